@@ -21,9 +21,14 @@ TUS = ["src/Cuda/Scan/JuicerCudaScanPipeline.cu", "src/Cuda/Film/JuicerCudaFilmP
        "src/Cuda/JuicerCudaAutoExposure.cu"]
 
 
+def sources_present() -> bool:
+    """An empty mount point counts as absent."""
+    return all(os.path.exists(os.path.join(REF, t)) for t in TUS)
+
+
 def main() -> int:
-    if not os.path.isdir(REF):
-        print("reference tree absent; keeping any prebuilt", LIB)
+    if not sources_present():
+        print("reference sources absent; keeping any prebuilt", LIB)
         return 0
     os.makedirs(OUT, exist_ok=True)
     srcs = [os.path.join(REF, t) for t in TUS] + [os.path.join(HERE, "ref_shim.cu")]
@@ -75,6 +80,6 @@ def build_fft() -> int:
 
 if __name__ == "__main__":
     rc = main()
-    if rc == 0 and os.path.isdir(REF):
+    if rc == 0 and sources_present():
         rc = build_fft()
     sys.exit(rc)
