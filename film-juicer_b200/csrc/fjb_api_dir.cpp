@@ -81,6 +81,8 @@ cudaError_t dir_blur_planes(const DirPlan& plan, const float* const in[3], float
     DirBlurParams bp{};
     bp.width = width;
     bp.height = height;
+    bp.region = scratch + 3 * plane;
+    bp.region_floats = fjb_spatial_dir_scratch_bytes(width, height) / sizeof(float) - 3 * plane;
     {
         const size_t planes_bytes = ((size_t)(3 + 3 * kDirMaxComponents) * plane * sizeof(float) + 255) / 256 * 256;
         char* rec = reinterpret_cast<char*>(scratch) + planes_bytes;

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/juicer_cuda_api.h"
+#include "fjb_line_pairs.cuh"
 
 namespace fjb {
 
@@ -47,15 +48,16 @@ struct DirComponentDev {
     int v_len, v_tsize;
     double v_term[9];
     double seg[9]; // recursion state map over kDirSeg zero-input steps (row-major 3x3)
-    double seg4[9]; // the same over 4 kDirSeg steps
     // Factored FP32 form of the recursion (factored != 0): a unit-DC first-order section
     // u += c0 (x - u) into the second-order section v = c2 v + c1 (u - y), y += v, with
     // state (u, y, v); to_fac / from_fac map direct states (y[n-1], y[n-2], y[n-3]) to it
-    // and back, seg_f / seg4_f are its zero-input maps over kDirSeg and 4 kDirSeg steps.
+    // and back, step_f is one zero-input step.
     int factored;
     float fac[3];
     double to_fac[9], from_fac[9];
-    double seg_f[9], seg4_f[9];
+    double step_f[9];
+    lp::LineMaps row_maps, col_maps; // its powers over a piece of a row and of a column
+    float host_taps[19];             // FIR up to radius 9: the taps again
 };
 
 constexpr int kDirSeg = 64; // segment length of the block-parallel recursions
@@ -72,6 +74,18 @@ struct DirBlurParams {
     double* carry;
     double* start;
     int lines_max, segs_max;
+    // everything after the scratch's first three planes; one warp per pair of lines: the
+    // recursions a column CTA holds at once, the rows and column CTAs between a CTA and the one
+    // after it, the planes the column launch adds its components to (null: nothing) with the
+    // identity component's weight in them, and the reflected starts of rows and columns (direct
+    // form, per channel, component and line)
+    float* region;
+    size_t region_floats;
+    int recursions, rows_ahead, cols_ahead;
+    float* base[3];
+    float raw_weight;
+    double* row_start;
+    double* col_start;
 };
 
 // Bytes of the recursion buffers for a width x height frame.
@@ -80,7 +94,13 @@ size_t dir_recursion_bytes(int width, int height);
 // Segments of the block-parallel recursions along a line of n samples.
 int dir_segments(int n);
 
-cudaError_t launch_dir_blur(const DirBlurParams& p, cudaStream_t stream);
+cudaError_t launch_dir_blur(DirBlurParams& p, cudaStream_t stream);
+
+// One warp per pair of lines (fjb_dir_lines.cu): false when the pass is out of its range
+// (line lengths, a component in the FP64 direct form, taps beyond radius 9); true lays the
+// pass out for launch_dir_lines.
+bool dir_lines_plan(DirBlurParams& p);
+cudaError_t launch_dir_lines(DirBlurParams& p, cudaStream_t stream);
 
 // Device-resident operator tables for one frame geometry.
 struct DirPlan {

@@ -275,18 +275,11 @@ size_t dir_scratch_floats(int width, int height) {
 
 namespace {
 
-void mat3_mul(const double* a, const double* b, double* o) {
-    double t[9];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) t[i * 3 + j] = a[i * 3] * b[j] + a[i * 3 + 1] * b[3 + j] + a[i * 3 + 2] * b[6 + j];
-    std::memcpy(o, t, sizeof(t));
-}
-
 // The recursion 1 / (1 - fb0 z^-1 - fb1 z^-2 - fb2 z^-3) as (1 - p z^-1)(1 - a1 z^-1 -
 // a2 z^-2): the real pole p by Newton's method from z = 1 (the Gaussian recursions
 // have one real pole in (0, 1) and a complex pair), then the FP32 coefficients
 // c0 = 1 - p, c2 = -a2, c1 = 1 - a1 - a2 and, from those rounded values, the basis
-// maps and zero-input state maps. In this form the state holds the first-order output,
+// maps and the zero-input step. In this form the state holds the first-order output,
 // the output and its last difference, so FP32 rounding is not amplified by the
 // recursion's DC gain as it is in the direct form (about 1 / ff). factored stays 0
 // (the FP64 direct form runs) when the coefficients do not have that structure.
@@ -312,12 +305,7 @@ void factor_recursion(DirComponentDev& c) {
     const double T[9] = {1.0 / C1, -A1 / C1, -A2 / C1, 1, 0, 0, 1, -1, 0};
     const double Ti[9] = {0, 1, 0, 0, 1, -1, -C1 / A2, (1.0 - A1) / A2, A1 / A2};
     const double F[9] = {P, 0, 0, C1 * P, 1.0 - C1, C2, C1 * P, -C1, C2};
-    double r[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    for (int step = 1; step <= 4 * kDirSeg; ++step) {
-        mat3_mul(F, r, r);
-        if (step == kDirSeg) std::memcpy(c.seg_f, r, sizeof(r));
-    }
-    std::memcpy(c.seg4_f, r, sizeof(r));
+    std::memcpy(c.step_f, F, sizeof(F));
     std::memcpy(c.to_fac, T, sizeof(T));
     std::memcpy(c.from_fac, Ti, sizeof(Ti));
     c.fac[0] = c0;
@@ -378,6 +366,7 @@ bool dir_plan_create(const FjSpatialDir& sd, int width, int height, cudaStream_t
                     return false;
                 if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return false;
                 c.taps = static_cast<const float*>(d);
+                for (int i = 0; i < 19 && i < (int)taps.size(); ++i) c.host_taps[i] = taps[i];
                 c.symmetric_taps = 1;
                 for (int i = 0; i <= 2 * g.radius; ++i)
                     if (std::memcmp(&taps[i], &taps[2 * g.radius - i], sizeof(float)) != 0) c.symmetric_taps = 0;
@@ -395,18 +384,11 @@ bool dir_plan_create(const FjSpatialDir& sd, int width, int height, cudaStream_t
                 c.ff = g.feedforward;
                 for (int k = 0; k < 3; ++k) c.fb[k] = g.feedback[k];
                 {
-                    // companion map (s0, s1, s2) -> (fb0 s0 + fb1 s1 + fb2 s2, s0, s1) over kDirSeg and 4 kDirSeg steps
+                    // companion map (s0, s1, s2) -> (fb0 s0 + fb1 s1 + fb2 s2, s0, s1) over kDirSeg steps
+                    static_assert((kDirSeg & (kDirSeg - 1)) == 0, "the segment map is built by squaring");
                     const double m[9] = {c.fb[0], c.fb[1], c.fb[2], 1, 0, 0, 0, 1, 0};
-                    double r[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-                    for (int step = 1; step <= 4 * kDirSeg; ++step) {
-                        double t[9];
-                        for (int i = 0; i < 3; ++i)
-                            for (int j = 0; j < 3; ++j)
-                                t[i * 3 + j] = m[i * 3] * r[j] + m[i * 3 + 1] * r[3 + j] + m[i * 3 + 2] * r[6 + j];
-                        std::memcpy(r, t, sizeof(r));
-                        if (step == kDirSeg) std::memcpy(c.seg, r, sizeof(r));
-                    }
-                    std::memcpy(c.seg4, r, sizeof(r));
+                    std::memcpy(c.seg, m, sizeof(m));
+                    for (int n = 1; n < kDirSeg; n *= 2) lp::mat3_mul(c.seg, c.seg, c.seg);
                 }
                 factor_recursion(c);
                 DirAxisBoundary hb, vb;

@@ -1,0 +1,338 @@
+// fjb_dir_lines.cu -- the spatial DIR filter, one warp per pair of lines (a7).
+//
+// The operators are those of fjb_dir_blur.cu (the reference's
+// src/Cuda/Film/JuicerCudaFilmPipeline.cu:388-780): FP64 taps with half-sample
+// reflection, and the third-order recursion with its reflected start and end block, here
+// in the factored FP32 form with FP64 states between pieces. Five launches: the short
+// components, both axes, summed into one plane per channel (fjb_fir2d.cuh); the rows'
+// reflected starts; the recursive components' rows, four rows per CTA (fjb_line_pairs.cuh);
+// the columns' reflected starts; the columns, one warp per pair of columns and recursive
+// component, then the weighted sum of all of them and the plane of the first launch.
+//
+// The starts are launches of their own because their weights (three doubles for each of the
+// first 21 sigma samples, 55 KB at 3840x2160) do not fit what the line kernels leave of L1:
+// inside those kernels every warp fetched them from L2, all SMs the same lines at the
+// same time, and they took 176 of the rows' 388 us and 121 of the columns' 419 us.
+#include <cuda_runtime.h>
+
+#include "fjb_dir.h"
+#include "fjb_fir2d.cuh"
+#include "fjb_launches.h"
+#include "fjb_line_pairs.cuh"
+
+namespace fjb {
+
+namespace {
+
+using lp::Pair;
+
+__device__ __forceinline__ void map_state(const double* T, const double d[3], double o[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[i] = T[3 * i] * d[0] + T[3 * i + 1] * d[1] + T[3 * i + 2] * d[2];
+}
+
+// Direct-form starts (y[n-1], y[n-2], y[n-3]) of the pair's lines as the step's state.
+__device__ __forceinline__ void state_from(const DirComponentDev& c, const double a[3], const double b[3],
+                                           Pair (&s)[3]) {
+    double oa[3], ob[3];
+    map_state(c.to_fac, a, oa);
+    map_state(c.to_fac, b, ob);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s[i] = lp::pack((float)oa[i], (float)ob[i]);
+}
+
+// End block of one line from its final state: the last `ts` outputs in `term`, and the
+// direct-form start of the way back.
+__device__ __forceinline__ void end_block(const DirComponentDev& c, const double* T, int ts, const double f[3],
+                                          double (&term)[3], double (&back)[3]) {
+    double d[3];
+    map_state(c.from_fac, f, d);
+    for (int r = 0; r < 3; ++r) {
+        double t = 0.0;
+        if (r < ts) {
+            t = d[0];
+            for (int q = 0; q < ts; ++q) t += T[r * ts + q] * (d[ts - 1 - q] - d[0]);
+        }
+        term[r] = t;
+        back[r] = r < ts ? t : d[r];
+    }
+}
+
+// Reflected starts of the recursive components' lines: anchor + sum_i w[i] (x_i - anchor) over
+// the first `len` samples, FP64. A warp takes four lines of a component (rows y .. y + 3, or
+// two pairs of columns), lanes stride the samples, so that a weight serves four lines.
+constexpr int kStartWarps = 8;
+
+template <bool kCols>
+__global__ void __launch_bounds__(32 * kStartWarps) dir_starts_kernel(const __grid_constant__ DirBlurParams P) {
+    const int ch = blockIdx.y, lane = threadIdx.x & 31;
+    const int W = P.width, H = P.height;
+    const int lines = kCols ? 2 * lp::plane_pairs(W) : H;
+    const int l0 = 4 * (blockIdx.x * kStartWarps + (threadIdx.x >> 5));
+    if (l0 >= lines) return;
+    const int words = lp::line_words(H);
+#pragma unroll 1
+    for (int k = 0; k < P.count; ++k) {
+        const DirComponentDev& c = P.comp[k];
+        if (c.op != kDirOpYvv) continue;
+        const int len = kCols ? c.v_len : c.h_len;
+        const double* w = kCols ? c.v_init : c.h_init;
+        const float2* pair = reinterpret_cast<const float2*>(P.temp[ch][k]) + (size_t)(l0 / 2) * words + H - 1;
+        auto samples = [&](int i, float (&v)[4]) {
+            if (kCols) {
+                const float2 a = pair[-i], b = pair[words - i];
+                v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+            } else {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) v[r] = P.raw[ch][(size_t)min(l0 + r, H - 1) * W + i];
+            }
+        };
+        float f[4];
+        samples(0, f);
+        const double anchor[4] = {f[0], f[1], f[2], f[3]};
+        double a[4][3] = {};
+#pragma unroll 4
+        for (int i = lane; i < len; i += 32) {
+            const double w0 = __ldg(w + i), w1 = __ldg(w + len + i), w2 = __ldg(w + 2 * len + i);
+            samples(i, f);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const double d = (double)f[r] - anchor[r];
+                a[r][0] += w0 * d;
+                a[r][1] += w1 * d;
+                a[r][2] += w2 * d;
+            }
+        }
+        double* out = (kCols ? P.col_start : P.row_start) + (((size_t)ch * kDirMaxComponents + k) * lines + l0) * 3;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int h = 0; h < 3; ++h) {
+                for (int o = 16; o > 0; o >>= 1) a[r][h] += __shfl_xor_sync(0xffffffffu, a[r][h], o);
+                if (lane == 0 && l0 + r < lines) out[3 * r + h] = anchor[r] + a[r][h];
+            }
+    }
+}
+
+// One recursive component over a pair of lines of n samples, in place: from the reflected
+// starts at `from` (of the pair's two lines) out, the end block at the last `ts` samples, the
+// way back from it. Rows count samples from position 0 up, columns (kDown) from position
+// n - 1 down.
+template <bool kDown>
+__device__ __forceinline__ void filter(const DirComponentDev& c, const double* from, Pair* line, int n, int lane) {
+    const lp::LineMaps& maps = kDown ? c.col_maps : c.row_maps;
+    const double* T = kDown ? c.v_term : c.h_term;
+    const int ts = kDown ? c.v_tsize : c.h_tsize;
+    const lp::FactoredStep op(c.fac[0], c.fac[1], c.fac[2]);
+    const lp::Piece piece(n, lane);
+    auto sample = [&](int i) { return line + (kDown ? n - 1 - i : i); };
+    Pair start[3], s[3];
+    {
+        const double a[3] = {from[0], from[1], from[2]}, b[3] = {from[3], from[4], from[5]};
+        state_from(c, a, b, start);
+    }
+    const bool low = lane == 0, high = piece.lo < piece.hi && piece.hi == n;
+    const int up = lane, down = lp::kPieces - 1 - lane;
+    lp::direction<!kDown>(op, maps, line, piece, kDown ? down : up, kDown ? high : low, start, s);
+    // the lane that holds the line's end makes the end block; everyone gets the way back's start
+    const int end_lane = kDown ? 0 : (n - 1) / piece.k;
+    {
+        const float2 f0 = lp::unpack(s[0]), f1 = lp::unpack(s[1]), f2 = lp::unpack(s[2]);
+        const double fa[3] = {f0.x, f1.x, f2.x}, fb[3] = {f0.y, f1.y, f2.y};
+        double ta[3], tb[3], ba[3], bb[3];
+        end_block(c, T, ts, fa, ta, ba);
+        end_block(c, T, ts, fb, tb, bb);
+        __syncwarp();
+        if (lane == end_lane)
+            for (int r = 0; r < ts; ++r)
+                if (n - ts + r >= 0) *sample(n - ts + r) = lp::pack((float)ta[r], (float)tb[r]);
+        state_from(c, ba, bb, s);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) start[i].v = __shfl_sync(0xffffffffu, s[i].v, end_lane);
+    }
+    // the way back leaves out the end block: the last ts positions, or the first (kDown)
+    lp::Piece back = piece;
+    if (kDown)
+        back.lo = min(max(piece.lo, ts), piece.hi);
+    else
+        back.hi = max(min(piece.hi, n - ts), piece.lo);
+    if (n > ts)
+        lp::direction<kDown>(op, maps, line, back, kDown ? up : down,
+                             back.lo < back.hi && (kDown ? back.lo == ts : back.hi == n - ts), start, s);
+    __syncwarp();
+}
+
+// Four rows of one channel per CTA through every recursive component.
+__global__ void __launch_bounds__(32 * lp::kRowWarps) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const int ch = blockIdx.y;
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int words = lp::line_words(W);
+    Pair* rows = reinterpret_cast<Pair*>(sm);
+    Pair* buf = rows + warp * words;
+    // rows past the frame's end repeat the last one; their results land in the planes' padding
+    const int y0 = 2 * lp::kRowWarps * blockIdx.x, y = y0 + 2 * warp;
+    const float* a = P.raw[ch] + (size_t)min(y, H - 1) * W;
+    const float* b = P.raw[ch] + (size_t)min(y + 1, H - 1) * W;
+    if (lane < 2 && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (size_t)(lane + P.rows_ahead) * W, W);
+#pragma unroll 1
+    for (int k = 0; k < P.count; ++k) {
+        const DirComponentDev& c = P.comp[k];
+        if (c.op != kDirOpYvv) continue;
+        // the last row's start again for a row past the frame's end
+        const double* starts = P.row_start + ((size_t)ch * kDirMaxComponents + k) * H * 3;
+        double from[6];
+#pragma unroll
+        for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + (size_t)min(y + h / 3, H - 1) * 3 + h % 3);
+        lp::load_rows(buf, a, b, W, lane);
+        filter<false>(c, from, buf, W, lane);
+        lp::store_pairs(rows, words, P.temp[ch][k], W, H, y0);
+    }
+}
+
+// Two pairs of columns per CTA, P.recursions recursive components at a time; the sum so far
+// waits in the first launch's plane between the rounds (more than one only for columns too
+// long for all of them to fit).
+__global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kColPairs * kDirMaxComponents)
+    dir_cols_kernel(const __grid_constant__ DirBlurParams P) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const auto cluster = cooperative_groups::this_cluster();
+    const int ch = blockIdx.y;
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Pair* lines = reinterpret_cast<Pair*>(sm);
+    Pair* line = lines + warp * lp::line_words(H);
+    if (lane == 0) {
+        const unsigned next = blockIdx.y * gridDim.x + blockIdx.x + P.cols_ahead;
+        if (next < gridDim.x * gridDim.y) {
+            const int first = next % gridDim.x * lp::kColPairs, nch = next / gridDim.x;
+            int slot = 0;
+            for (int i = 0; i < P.count; ++i)
+                if (P.comp[i].op == kDirOpYvv && slot++ == warp / lp::kColPairs)
+                    lp::prefetch_line(P.temp[nch][i], first + warp % lp::kColPairs, H);
+            if (P.base[nch] && warp < lp::kColPairs) lp::prefetch_line(P.base[nch], first + warp, H);
+        }
+    }
+    int k = 0;
+    do {
+        float weight[lp::kMaxRecursions];
+        int count = 0;
+#pragma unroll 1
+        for (; k < P.count && count < P.recursions; ++k) {
+            const DirComponentDev& c = P.comp[k];
+            if (c.op != kDirOpYvv) continue;
+            if (warp / lp::kColPairs == count) {
+                const int pair = blockIdx.x * lp::kColPairs + warp % lp::kColPairs;
+                const double* starts =
+                    P.col_start + (((size_t)ch * kDirMaxComponents + k) * 2 * lp::plane_pairs(W) + 2 * pair) * 3;
+                double from[6];
+#pragma unroll
+                for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + h);
+                lp::load_line(line, P.temp[ch][k], pair, H, lane);
+                filter<true>(c, from, line, H, lane);
+            }
+            weight[count++] = c.weight;
+        }
+        while (k < P.count && P.comp[k].op != kDirOpYvv) ++k;
+        cluster.sync();
+        lp::strip_sum(lp::StripSum{P.base[ch], P.filtered[ch], W, k >= P.count}, lines, weight, count, W, H);
+        cluster.sync(); // the other CTA has read these lines
+    } while (k < P.count);
+}
+
+} // namespace
+
+bool dir_lines_plan(DirBlurParams& P) {
+    int lines = 0;
+    bool base = false;
+    for (int k = 0; k < P.count; ++k) {
+        const DirComponentDev& c = P.comp[k];
+        if (c.op == kDirOpFir ? c.radius < 1 || c.radius > fir::kMaxRadius
+                              : c.op == kDirOpYvv ? !c.factored : c.op != kDirOpIdentity)
+            return false;
+        lines += c.op == kDirOpYvv;
+        base |= c.op != kDirOpYvv;
+    }
+    const int recursions = lp::recursions_per_cta(lines, P.height);
+    if (lp::kRowWarps * lp::line_bytes(P.width) > lp::kSmemLimit || recursions < 1) return false;
+    base |= lines > recursions; // the sum waits there between the rounds
+    const size_t plane = lp::plane_floats(P.width, P.height);
+    float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.region) + 31) / 32 * 32);
+    const size_t starts = 3 * (size_t)kDirMaxComponents * 3 * (P.height + 2 * (size_t)lp::plane_pairs(P.width)) * 2; // floats
+    if ((size_t)(next - P.region) + 3 * (size_t)(lines + base) * plane + starts > P.region_floats) return false;
+    P.recursions = recursions;
+    P.raw_weight = 0.0f;
+    for (int k = 0; k < P.count; ++k) {
+        DirComponentDev& c = P.comp[k];
+        if (c.op == kDirOpIdentity) P.raw_weight += c.weight;
+        if (c.op != kDirOpYvv) continue;
+        for (int ch = 0; ch < 3; ++ch, next += plane) P.temp[ch][k] = next;
+        c.row_maps = lp::line_maps(c.step_f, lp::piece_len(P.width));
+        c.col_maps = lp::line_maps(c.step_f, lp::piece_len(P.height));
+    }
+    for (int ch = 0; ch < 3; ++ch) {
+        P.base[ch] = base ? next : nullptr;
+        if (base) next += plane;
+    }
+    P.row_start = reinterpret_cast<double*>(next);
+    P.col_start = P.row_start + 3 * (size_t)kDirMaxComponents * 3 * P.height;
+    return true;
+}
+
+cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
+    bool lines = false;
+    fir::Jobs F{};
+    F.width = P.width;
+    F.height = P.height;
+    F.dst_pairs = lp::plane_pairs(P.width);
+    F.dst_words = lp::line_words(P.height);
+    for (int ch = 0; ch < 3; ++ch) {
+        fir::Job f{};
+        f.src = P.raw[ch];
+        f.stride = P.width;
+        f.dst = P.base[ch];
+        f.src_weight = P.raw_weight;
+        for (int k = 0; k < P.count; ++k) {
+            const DirComponentDev& c = P.comp[k];
+            lines |= c.op == kDirOpYvv;
+            if (c.op != kDirOpFir) continue;
+            fir::Taps& t = f.set[f.count++];
+            t.radius = c.radius;
+            t.weight = c.weight;
+            for (int i = 0; i < 2 * fir::kMaxRadius + 1; ++i) t.w[i] = c.host_taps[i];
+        }
+        if (f.dst) F.job[F.count++] = f;
+    }
+    cudaError_t e = cudaSuccess;
+    if (F.count) {
+        fjb::count_launch();
+        fir::kernel<double><<<fir::grid(F), fir::kThreads, 0, s>>>(F);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    constexpr int kLinesPerCta = 4 * kStartWarps;
+    if (lines) {
+        fjb::count_launch();
+        dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3), 32 * kStartWarps, 0, s>>>(P);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
+        e = cudaFuncSetAttribute(dir_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        P.rows_ahead = 2 * lp::kRowWarps * lp::resident_ctas(smem);
+        fjb::count_launch();
+        dir_rows_kernel<<<dim3((P.height + 3) / 4, 3), 32 * lp::kRowWarps, smem, s>>>(P);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        fjb::count_launch();
+        dir_starts_kernel<true>
+            <<<dim3((2 * lp::plane_pairs(P.width) + kLinesPerCta - 1) / kLinesPerCta, 3), 32 * kStartWarps, 0, s>>>(P);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    const int warps = P.recursions * lp::kColPairs;
+    const size_t smem = warps * lp::line_bytes(P.height);
+    e = cudaFuncSetAttribute(dir_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    P.cols_ahead = lp::resident_ctas(smem);
+    fjb::count_launch();
+    dir_cols_kernel<<<dim3(lp::plane_pairs(P.width) / lp::kColPairs, 3), 32 * warps, smem, s>>>(P);
+    return cudaGetLastError();
+}
+
+} // namespace fjb

@@ -10,18 +10,16 @@
 // (:29-46 reflect rule, :183-198 recursion steps, :201-282 row passes, :283-345
 // column passes).
 //
-// B200 schedule: the reference runs one read-modify-write accumulation pass per
-// Gaussian per channel (up to ~14 full-plane passes per channel). Here every
-// Gaussian that reads the same source plane is evaluated in the same sweep: the row
-// kernels write one row-filtered plane per Gaussian, and the last column kernel runs
-// all column filters of a channel together and applies the scatter/bounce
-// combination in its epilogue, so the tail accumulator never touches HBM. All three
-// channels run in each launch (grid.z = channel); the recursions are block-parallel
-// (below).
+// B200 schedule: fjb_halation_lines.cu. The kernels of this file are the form for what that
+// one does not cover: frames above 14528 samples in a line, and frames a few samples wide
+// whose padded planes exceed the stage's scratch. Here the recursions run block-parallel
+// over global memory; the row kernels write one row-filtered plane per Gaussian, and the
+// last column kernel runs all column filters of a channel together and applies the
+// scatter/bounce combination in its epilogue. All three channels run in each launch
+// (grid.z = channel).
 #include <cuda_runtime.h>
 
 #include "fjb_launches.h"
-#include "fjb_lines.cuh"
 #include "fjb_optics.h"
 
 namespace fjb {
@@ -467,316 +465,39 @@ __global__ void __launch_bounds__(kColThreads) cols_final_combine_kernel(const _
     }
 }
 
-// ---------------------------------------------------------------------------
-// Shared-memory form, used when whole lines fit on chip (the usual case): a CTA
-// holds kRowsPerCta full rows, or a kStripCols-wide strip of full columns, and runs
-// the block-parallel recursion of fjb_lines.cuh on them, so each Gaussian costs one
-// read and one write of the plane per direction pair.
-// ---------------------------------------------------------------------------
-constexpr int kRowsPerCta = 4;
-constexpr int kStripCols = 8;
-// CTA sizes (threads, resident CTAs per SM) that bound registers so shared memory,
-// not registers, sets the occupancy
-constexpr int kRowsThreads = 256, kRowsBlocks = 3;
-constexpr int kColsThreads = 288, kColsBlocks = 3;
-constexpr size_t kSmemLimit = 200 * 1024;
-static_assert(kOpticSeg == lines::kLineSeg, "segment maps are built for the line segment length");
-
-// One recursive Gaussian (kFactored: h, g, t form; else legacy B, B1, B2, B3) with its
-// coefficients held in registers (read once per CTA, not once per sample through the
-// parameter block).
-template <bool kFactored>
-struct HalStep {
-    using Real = float;
-    float c0, c1, c2, c3;
-    const double* seg;
-    const double* seg4;
-    __device__ explicit HalStep(const OpticGauss& g)
-        : c0(g.yvv[0]), c1(g.yvv[1]), c2(g.yvv[2]), c3(g.yvv[3]), seg(g.seg), seg4(g.seg4) {}
-    __device__ __forceinline__ float step(float x, float s[3]) const {
-        if (kFactored) {
-            s[0] += c0 * (x - s[0]);
-            s[2] = c2 * s[2] + c1 * (s[0] - s[1]);
-            s[1] += s[2];
-            return s[1];
-        }
-        const float v = __fmaf_rn(c1, s[0], __fmaf_rn(c2, s[1], __fmaf_rn(c3, s[2], c0 * x)));
-        s[2] = s[1];
-        s[1] = s[0];
-        s[0] = v;
-        return v;
-    }
-    __device__ __forceinline__ const double* map() const { return seg; }
-    __device__ __forceinline__ const double* map4() const { return seg4; }
-};
-
-// Replicate start of each line from its first sample in processing order (position
-// `first`), into entry (L x 3).
-template <int ES, typename Buf>
-__device__ __forceinline__ void replicate_starts(const OpticGauss& g, Buf buf, int L, int first, float* entry) {
-    for (int r = threadIdx.x; r < L; r += blockDim.x) {
-        YvvState st;
-        yvv_init(g, buf(r)[lines::at(first) * ES], st);
-        entry[r * 3] = st.s1;
-        entry[r * 3 + 1] = st.s2;
-        entry[r * 3 + 2] = st.s3;
-    }
-    __syncthreads();
-}
-
-// Both passes of one recursive Gaussian over L lines of n samples held in shared
-// memory: kFirstForward runs ascending positions first (rows: left to right, then
-// back), else descending first (columns: bottom-up, then top-down).
-template <int ES, bool kFirstForward, bool kFactored, typename Buf>
-__device__ __forceinline__ void yvv_lines(const OpticGauss& g, Buf buf, int L, int n, float* exits, double* carry,
-                                          float* entry) {
-    const HalStep<kFactored> op(g);
-    replicate_starts<ES>(g, buf, L, kFirstForward ? 0 : n - 1, entry);
-    lines::run_direction<ES, kFirstForward>(op, buf, L, 0, n, entry, exits, carry, (float*)nullptr, ES != 1);
-    replicate_starts<ES>(g, buf, L, kFirstForward ? n - 1 : 0, entry);
-    lines::run_direction<ES, !kFirstForward>(op, buf, L, 0, n, entry, exits, carry, (float*)nullptr, ES != 1);
-}
-
-// Dynamic shared memory: scan carries (doubles) first, then the lines, exit states and
-// entry states (floats).
-__host__ __device__ inline size_t carry_doubles(int L, int n) { return (size_t)L * lines::scan_chunks(lines::segs(n)) * 3; }
-
-size_t rows_smem_bytes(int W) {
-    return carry_doubles(kRowsPerCta, W) * sizeof(double) +
-           ((size_t)kRowsPerCta * lines::padded(W) + (size_t)kRowsPerCta * lines::segs(W) * 3 +
-            (size_t)kRowsPerCta * 3) *
-               sizeof(float);
-}
-
-size_t cols_smem_bytes(int H) {
-    return carry_doubles(kStripCols, H) * sizeof(double) +
-           ((size_t)kStripCols * lines::padded(H) + (size_t)kStripCols * lines::segs(H) * 3 +
-            (size_t)kStripCols * 3) *
-               sizeof(float);
-}
-
-// Rows: every Gaussian of the job into its row-filtered plane (recursive: left to
-// right then right to left; FIR: reflect taps).
-__global__ void __launch_bounds__(kRowsThreads, kRowsBlocks) rows_smem_kernel(const __grid_constant__ OpticPass P) {
-    extern __shared__ __align__(16) float sm[];
-    const int job = blockIdx.y;
-    const OpticJob& J = P.job[job];
-    const int W = P.width, H = P.height;
-    const int row0 = blockIdx.x * kRowsPerCta;
-    const int L = min(kRowsPerCta, H - row0);
-    const int pw = lines::padded(W);
-    double* carry = reinterpret_cast<double*>(sm);
-    float* buf = reinterpret_cast<float*>(carry + carry_doubles(kRowsPerCta, W));
-    float* exits = buf + (size_t)kRowsPerCta * pw;
-    float* entry = exits + (size_t)kRowsPerCta * lines::segs(W) * 3;
-    auto line = [&](int r) { return buf + (size_t)r * pw; };
-    for (int gi = 0; gi < J.count; ++gi) {
-        const OpticGauss& g = J.g[gi];
-        if (g.kind == kGaussFir) {
-            // reflect-boundary taps over the densely staged rows
-            lines::load_rows_dense(buf, J.src, J.stride, row0, L, W);
-            const int rad = g.radius;
-            for (int r = 0; r < L; ++r) {
-                const float* row = buf + (size_t)r * W;
-                float* out = J.temp[gi] + (long long)(row0 + r) * W;
-                for (int x = threadIdx.x; x < W; x += blockDim.x) {
-                    float sum = 0.0f;
-                    if (x - rad >= 0 && x + rad < W)
-                        for (int o = -rad; o <= rad; ++o) sum += row[x + o] * g.w[o + rad];
-                    else
-                        for (int o = -rad; o <= rad; ++o) sum += row[reflect_half(x + o, W)] * g.w[o + rad];
-                    out[x] = sum;
-                }
-            }
-            __syncthreads();
-            continue;
-        }
-        if (!is_yvv(g.kind)) continue;
-        lines::load_rows(buf, J.src, J.stride, row0, L, W);
-        if (g.kind == kGaussYvvFactored)
-            yvv_lines<1, true, true>(g, line, L, W, exits, carry, entry);
-        else
-            yvv_lines<1, true, false>(g, line, L, W, exits, carry, entry);
-        lines::store_rows(buf, J.temp[gi], row0, L, W);
-    }
-}
-
-// Columns of a kStripCols-wide strip: every Gaussian (recursive: bottom-up then
-// top-down; FIR: reflect taps; identity) in order, accumulated as the reference
-// combines them, then the scatter/bounce combination into the carrier plane. The
-// running sum of the Gaussians so far is parked in the strip of the row-filtered plane
-// this CTA has just consumed (it stays in L2), which keeps shared memory to one strip.
-__global__ void __launch_bounds__(kColsThreads, kColsBlocks) cols_smem_kernel(const __grid_constant__ OpticPass P) {
-    extern __shared__ __align__(16) float sm[];
-    const int job = blockIdx.y;
-    const OpticJob& J = P.job[job];
-    const int W = P.width, H = P.height;
-    const int x0 = blockIdx.x * kStripCols;
-    const int C = min(kStripCols, W - x0);
-    const int ph = lines::padded(H);
-    double* carry = reinterpret_cast<double*>(sm);
-    float* work = reinterpret_cast<float*>(carry + carry_doubles(kStripCols, H)); // [padded(H)][kStripCols]
-    float* exits = work + (size_t)ph * kStripCols;
-    float* entry = exits + (size_t)kStripCols * lines::segs(H) * 3;
-    auto column = [&](int c) { return work + c; };
-    const int count = J.count;
-    const bool scatter = J.mode == kOpticScatter;
-    for (int gi = 0; gi < count; ++gi) {
-        const OpticGauss& g = J.g[gi];
-        // roles of this Gaussian in the combination
-        const bool finishes = scatter ? gi >= J.tail_count : gi == count - 1; // writes the carrier plane
-        const bool reads_acc = gi > 0 && (!scatter || J.tail_count > 0);    // a running sum exists
-        const bool reads_src = g.kind == kGaussIdentity || finishes;
-        const float* acc_in = reads_acc ? J.temp[scatter && finishes ? J.tail_count - 1 : gi - 1] : nullptr;
-        float* acc_out = finishes ? nullptr : J.temp[gi];
-        // full strips on 16-byte aligned planes move four columns per access
-        const bool vec = C == kStripCols && W % 4 == 0 && J.stride % 4 == 0 && lines::aligned16(J.src) &&
-                         (g.kind == kGaussIdentity || lines::aligned16(J.temp[gi])) &&
-                         (!acc_in || lines::aligned16(acc_in)) && (!acc_out || lines::aligned16(acc_out));
-        const bool dense_fir = vec && g.kind == kGaussFir;
-        if (dense_fir)
-            lines::load_strip8_dense(work, J.temp[gi], W, H, x0);
-        else if (g.kind != kGaussIdentity)
-            lines::load_strip8(work, J.temp[gi], W, H, x0, C);
-        if (g.kind == kGaussYvvFactored)
-            yvv_lines<kStripCols, false, true>(g, column, kStripCols, H, exits, carry, entry);
-        else if (g.kind == kGaussYvv)
-            yvv_lines<kStripCols, false, false>(g, column, kStripCols, H, exits, carry, entry);
-        const float coef = J.coef[gi];
-        // running sum after this Gaussian, and the carrier value when it finishes the job
-        auto running = [&](float v, float a) { return gi == 0 ? coef * v : a + coef * v; };
-        auto finish = [&](float v, float a, float source) {
-            if (scatter) {
-                // the core is the job's last Gaussian
-                const float tail = J.tail_count > 0 ? a : 0.0f;
-                const float coreTerm = (1.0f - J.tail_weight) * v;
-                const float tailTerm = J.tail_weight * tail;
-                const float scattered = coreTerm + tailTerm;
-                const float sourceTerm = (1.0f - J.amount) * source;
-                const float scatteredTerm = J.amount * scattered;
-                return sourceTerm + scatteredTerm;
-            }
-            const float added = source + J.amount * running(v, a);
-            return J.renormalize ? added / (1.0f + J.amount) : added;
-        };
-        if (vec) {
-            // thread -> (row, half strip); global reads go kBatch rows at a time
-            constexpr int kBatch = 4;
-            const int h = threadIdx.x & 1, ys = blockDim.x >> 1;
-            for (int y0 = threadIdx.x >> 1; y0 < H; y0 += kBatch * ys) {
-                float4 srcv[kBatch], accv[kBatch];
-#pragma unroll
-                for (int b = 0; b < kBatch; ++b) {
-                    const int y = y0 + b * ys;
-                    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    srcv[b] = reads_src && y < H
-                                  ? *reinterpret_cast<const float4*>(J.src + (long long)y * J.stride + x0 + 4 * h)
-                                  : z;
-                    accv[b] = reads_acc && y < H
-                                  ? *reinterpret_cast<const float4*>(acc_in + (long long)y * W + x0 + 4 * h)
-                                  : z;
-                }
-#pragma unroll
-                for (int b = 0; b < kBatch; ++b) {
-                    const int y = y0 + b * ys;
-                    if (y >= H) continue;
-                    float4 v;
-                    if (g.kind == kGaussIdentity) {
-                        v = srcv[b];
-                    } else if (g.kind == kGaussFir) {
-                        float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        for (int o = -g.radius; o <= g.radius; ++o) {
-                            const float4 t = *reinterpret_cast<const float4*>(work + reflect_half(y - o, H) * 8 + 4 * h);
-                            const float wt = g.w[o + g.radius];
-                            sum.x += t.x * wt;
-                            sum.y += t.y * wt;
-                            sum.z += t.z * wt;
-                            sum.w += t.w * wt;
-                        }
-                        v = sum;
-                    } else {
-                        v = *reinterpret_cast<const float4*>(work + lines::at(y) * 8 + 4 * h);
-                    }
-                    const float4 a = accv[b];
-                    if (finishes) {
-                        const float4 o4 = make_float4(finish(v.x, a.x, srcv[b].x), finish(v.y, a.y, srcv[b].y),
-                                                      finish(v.z, a.z, srcv[b].z), finish(v.w, a.w, srcv[b].w));
-                        *reinterpret_cast<float4*>(J.src + (long long)y * J.stride + x0 + 4 * h) = o4;
-                    } else {
-                        const float4 o4 = make_float4(running(v.x, a.x), running(v.y, a.y), running(v.z, a.z),
-                                                      running(v.w, a.w));
-                        *reinterpret_cast<float4*>(acc_out + (long long)y * W + x0 + 4 * h) = o4;
-                    }
-                }
-            }
-        } else {
-            // one column per thread (the block size is a multiple of kStripCols)
-            constexpr int kBatch = 8;
-            const int c = threadIdx.x % kStripCols, ystep = blockDim.x / kStripCols;
-            for (int y0 = threadIdx.x / kStripCols; y0 < H; y0 += kBatch * ystep) {
-                float srcv[kBatch], accv[kBatch];
-#pragma unroll
-                for (int b = 0; b < kBatch; ++b) {
-                    const int y = y0 + b * ystep;
-                    const bool in = y < H && c < C;
-                    srcv[b] = reads_src && in ? J.src[(long long)y * J.stride + x0 + c] : 0.0f;
-                    accv[b] = reads_acc && in ? acc_in[(long long)y * W + x0 + c] : 0.0f;
-                }
-#pragma unroll
-                for (int b = 0; b < kBatch; ++b) {
-                    const int y = y0 + b * ystep;
-                    if (y >= H || c >= C) continue;
-                    float v;
-                    if (g.kind == kGaussIdentity) {
-                        v = srcv[b];
-                    } else if (g.kind == kGaussFir) {
-                        float sum = 0.0f;
-                        for (int o = -g.radius; o <= g.radius; ++o)
-                            sum += work[lines::at(reflect_half(y - o, H)) * kStripCols + c] * g.w[o + g.radius];
-                        v = sum;
-                    } else {
-                        v = work[lines::at(y) * kStripCols + c];
-                    }
-                    if (finishes)
-                        J.src[(long long)y * J.stride + x0 + c] = finish(v, accv[b], srcv[b]);
-                    else
-                        acc_out[(long long)y * W + x0 + c] = running(v, accv[b]);
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
 } // namespace
 
 int optic_segments(int n) { return seg_count(n); }
 
-cudaError_t launch_optic_pass(const OpticPass& P, cudaStream_t stream) {
+namespace {
+
+// The state map over kOpticSeg zero-input steps, in FP64: the operator that carries a
+// segment's entry state to its exit state.
+void segment_map(OpticGauss& g) {
+    static_assert((kOpticSeg & (kOpticSeg - 1)) == 0, "the segment map is built by squaring");
+    optic_step_map(g, g.seg);
+    for (int n = 1; n < kOpticSeg; n *= 2) lp::mat3_mul(g.seg, g.seg, g.seg);
+}
+
+} // namespace
+
+cudaError_t launch_optic_pass(OpticPass& P, cudaStream_t stream) {
     if (P.jobs <= 0 || P.width <= 0 || P.height <= 0) return cudaSuccess;
+    if (optic_lines_plan(P)) return launch_optic_lines(P, stream);
     bool anyYvv = false, anyFir = false;
     for (int j = 0; j < P.jobs; ++j)
         for (int g = 0; g < P.job[j].count; ++g) {
-            anyYvv |= is_yvv(P.job[j].g[g].kind);
-            anyFir |= P.job[j].g[g].kind == kGaussFir;
+            OpticGauss& q = P.job[j].g[g];
+            if (is_yvv(q.kind)) segment_map(q);
+            anyYvv |= is_yvv(q.kind);
+            anyFir |= q.kind == kGaussFir;
         }
     const int W = P.width, H = P.height;
     const int sw = seg_count(W), sh = seg_count(H);
     const dim3 rows_grid((H + 31) / 32, sw, P.jobs);
     const dim3 cols_grid((W + kColThreads - 1) / kColThreads, sh, P.jobs);
     cudaError_t e = cudaSuccess;
-    // whole rows / column strips in shared memory when they fit, else the global form
-    const size_t rs = rows_smem_bytes(W), cs = cols_smem_bytes(H);
-    const bool rows_on_chip = rs <= kSmemLimit, cols_on_chip = cs <= kSmemLimit;
-    if ((anyYvv || anyFir) && rows_on_chip) {
-        if ((e = cudaFuncSetAttribute(rows_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rs)) !=
-            cudaSuccess)
-            return e;
-        fjb::count_launch();
-        rows_smem_kernel<<<dim3((H + kRowsPerCta - 1) / kRowsPerCta, P.jobs), lines::line_threads(kRowsPerCta, W, kRowsThreads), rs,
-                           stream>>>(P);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    } else if (anyYvv) {
+    if (anyYvv) {
         const dim3 row_lines((H + 127) / 128, P.jobs);
         fjb::count_launch();
         rows_partial_fwd_kernel<<<rows_grid, 32, 0, stream>>>(P);
@@ -792,20 +513,11 @@ cudaError_t launch_optic_pass(const OpticPass& P, cudaStream_t stream) {
         rows_final_bwd_kernel<<<rows_grid, 32, 0, stream>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if (anyFir && !rows_on_chip) {
+    if (anyFir) {
         const dim3 block(32, 8);
         fjb::count_launch();
         rows_fir_kernel<<<dim3((W + 31) / 32, (H + 7) / 8, P.jobs), block, 0, stream>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if (cols_on_chip) {
-        if ((e = cudaFuncSetAttribute(cols_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cs)) !=
-            cudaSuccess)
-            return e;
-        fjb::count_launch();
-        cols_smem_kernel<<<dim3((W + kStripCols - 1) / kStripCols, P.jobs), lines::line_threads(kStripCols, H, kColsThreads), cs,
-                           stream>>>(P);
-        return cudaGetLastError();
     }
     if (anyYvv) {
         const dim3 col_lines((W + 127) / 128, P.jobs);

@@ -1,0 +1,235 @@
+// fjb_halation_lines.cu -- scatter/halation passes, one warp per pair of lines (a16).
+//
+// The operators are those of fjb_halation.cu (the reference's
+// src/Cuda/Film/JuicerCudaScatterHalation.cu:690-852). Both combinations are weighted sums
+// of the carrier and its Gaussians, so a pass is
+//   taps    : the carrier's own share and every short Gaussian, both axes, summed into one
+//             plane per channel (fjb_fir2d.cuh);
+//   rows    : every recursive Gaussian's row pass, two rows per warp (fjb_line_pairs.cuh);
+//   columns : a strip of columns per CTA, one warp per pair of columns and recursive
+//             Gaussian, then the weighted sum of all of them and the plane of the first
+//             launch into the carrier, so that no running sum leaves the CTA.
+#include <cuda_runtime.h>
+
+#include <cmath>
+
+#include "fjb_fir2d.cuh"
+#include "fjb_launches.h"
+#include "fjb_line_pairs.cuh"
+#include "fjb_optics.h"
+
+namespace fjb {
+
+namespace {
+
+using lp::Pair;
+
+__host__ __device__ __forceinline__ bool is_yvv(int kind) { return kind == kGaussYvv || kind == kGaussYvvFactored; }
+
+// Both directions of one recursive Gaussian over a pair of lines of n samples, from
+// replicate starts: ascending first (rows), or descending first (columns, kDown).
+template <bool kDown, bool kFactored, typename Op>
+__device__ __forceinline__ void filter(const Op& op, const lp::LineMaps& maps, Pair* line, int n, int lane) {
+    const lp::Piece piece(n, lane);
+    const bool low = lane == 0, high = piece.lo < piece.hi && piece.hi == n;
+    const int up = lane, down = lp::kPieces - 1 - lane;
+    const Pair zero{0ull};
+    const Pair v0 = line[kDown ? n - 1 : 0];
+    Pair start[3] = {v0, v0, kFactored ? zero : v0}, s[3];
+    lp::direction<!kDown>(op, maps, line, piece, kDown ? down : up, kDown ? high : low, start, s);
+    const Pair v1 = kFactored ? s[1] : s[0];
+    start[0] = start[1] = v1;
+    start[2] = kFactored ? zero : v1;
+    lp::direction<kDown>(op, maps, line, piece, kDown ? up : down, kDown ? low : high, start, s);
+    __syncwarp();
+}
+
+template <bool kDown>
+__device__ __forceinline__ void filter(const OpticGauss& g, Pair* line, int n, int lane) {
+    const lp::LineMaps& maps = kDown ? g.col_maps : g.row_maps;
+    if (g.kind == kGaussYvvFactored)
+        filter<kDown, true>(lp::FactoredStep(g.yvv[0], g.yvv[1], g.yvv[2]), maps, line, n, lane);
+    else
+        filter<kDown, false>(lp::DirectStep(g.yvv[0], g.yvv[1], g.yvv[2], g.yvv[3]), maps, line, n, lane);
+}
+
+// Four rows of one channel per CTA through every recursive Gaussian of the job.
+__global__ void __launch_bounds__(32 * lp::kRowWarps) optic_rows_kernel(const __grid_constant__ OpticPass P) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const OpticJob& J = P.job[blockIdx.y];
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int words = lp::line_words(W);
+    Pair* rows = reinterpret_cast<Pair*>(sm);
+    Pair* buf = rows + warp * words;
+    // rows past the frame's end repeat the last one; their results land in the planes' padding
+    const int y0 = 2 * lp::kRowWarps * blockIdx.x, y = y0 + 2 * warp;
+    const float* a = J.src + (long long)min(y, H - 1) * J.stride;
+    const float* b = J.src + (long long)min(y + 1, H - 1) * J.stride;
+    if (lane < 2 && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (long long)(lane + P.rows_ahead) * J.stride, W);
+#pragma unroll 1
+    for (int gi = 0; gi < J.count; ++gi) {
+        const OpticGauss& g = J.g[gi];
+        if (!is_yvv(g.kind)) continue;
+        lp::load_rows(buf, a, b, W, lane);
+        filter<false>(g, buf, W, lane);
+        lp::store_pairs(rows, words, J.temp[gi], W, H, y0);
+    }
+}
+
+// Two pairs of columns per CTA, P.recursions recursive Gaussians at a time; the sum so far
+// waits in the first launch's plane between the rounds (more than one only for columns too
+// long for all recursions of the channel to fit).
+__global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kMaxColWarps)
+    optic_cols_kernel(const __grid_constant__ OpticPass P) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const auto cluster = cooperative_groups::this_cluster();
+    const OpticJob& J = P.job[blockIdx.y];
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Pair* lines = reinterpret_cast<Pair*>(sm);
+    Pair* line = lines + warp * lp::line_words(H);
+    if (lane == 0) {
+        const unsigned next = blockIdx.y * gridDim.x + blockIdx.x + P.cols_ahead;
+        if (next < gridDim.x * gridDim.y) {
+            const OpticJob& N = P.job[next / gridDim.x];
+            int slot = 0;
+            for (int i = 0; i < N.count; ++i)
+                if (is_yvv(N.g[i].kind) && slot++ == warp / lp::kColPairs)
+                    lp::prefetch_line(N.temp[i], next % gridDim.x * lp::kColPairs + warp % lp::kColPairs, H);
+            if (warp < lp::kColPairs) lp::prefetch_line(N.base, next % gridDim.x * lp::kColPairs + warp, H);
+        }
+    }
+    int gi = 0;
+    do {
+        float weight[lp::kMaxRecursions];
+        int count = 0;
+#pragma unroll 1
+        for (; gi < J.count && count < P.recursions; ++gi) {
+            const OpticGauss& g = J.g[gi];
+            if (!is_yvv(g.kind)) continue;
+            if (warp / lp::kColPairs == count) {
+                lp::load_line(line, J.temp[gi], blockIdx.x * lp::kColPairs + warp % lp::kColPairs, H, lane);
+                filter<true>(g, line, H, lane);
+            }
+            weight[count++] = J.weight[gi];
+        }
+        while (gi < J.count && !is_yvv(J.g[gi].kind)) ++gi;
+        cluster.sync();
+        lp::strip_sum(lp::StripSum{J.base, J.src, J.stride, gi >= J.count}, lines, weight, count, W, H);
+        cluster.sync(); // the other CTA has read these lines
+    } while (gi < J.count);
+}
+
+} // namespace
+
+// Rounding the weights to FP32 one by one would change their sum (the gain of a flat field)
+// by up to 1e-7: the smallest Gaussian's weight, whose own rounding step is the finest, takes
+// up what the others' rounding left over.
+static void balance_weights(OpticJob& J, double carrier, const double* exact) {
+    double left = carrier - (double)J.carrier_weight;
+    int least = -1;
+    for (int g = 0; g < J.count; ++g) {
+        if (J.g[g].kind == kGaussIdentity || J.weight[g] == 0.0f) continue;
+        left += exact[g] - (double)J.weight[g];
+        if (least < 0 || std::fabs(J.weight[g]) < std::fabs(J.weight[least])) least = g;
+    }
+    if (least >= 0) J.weight[least] = (float)((double)J.weight[least] + left);
+}
+
+// Whether this form covers the pass: four rows and two pairs of columns fit in shared memory,
+// and the planes between the launches fit the pass's scratch.
+bool optic_lines_plan(OpticPass& P) {
+    int most = 1;
+    size_t planes = 0;
+    for (int j = 0; j < P.jobs; ++j) {
+        const OpticJob& J = P.job[j];
+        int n = 0;
+        for (int g = 0; g < J.count; ++g) n += is_yvv(J.g[g].kind);
+        planes += n + 1;
+        most = n > most ? n : most;
+    }
+    const int recursions = lp::recursions_per_cta(most, P.height);
+    if (lp::kRowWarps * lp::line_bytes(P.width) > lp::kSmemLimit || recursions < 1) return false;
+    const size_t plane = lp::plane_floats(P.width, P.height);
+    float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.scratch) + 31) / 32 * 32);
+    if ((size_t)(next - P.scratch) + planes * plane > P.scratch_floats) return false;
+    P.recursions = recursions;
+    for (int j = 0; j < P.jobs; ++j) {
+        OpticJob& J = P.job[j];
+        // the combination as weights: scatter (1 - a) x + a ((1 - w) core + w sum_i amp_i tail_i),
+        // bounce (x + s sum_b weight_b G_b) / (1 + s or 1)
+        const double a = J.amount, w = J.tail_weight;
+        const double scale = J.mode == kOpticScatter ? a : a / (J.renormalize ? 1.0 + a : 1.0);
+        double carrier = J.mode == kOpticScatter ? 1.0 - a : 1.0 / (J.renormalize ? 1.0 + a : 1.0);
+        double exact[kOpticMaxGauss];
+        for (int g = 0; g < J.count; ++g) {
+            OpticGauss& q = J.g[g];
+            const double part = J.mode == kOpticScatter ? (g < J.tail_count ? w * J.coef[g] : 1.0 - w) : J.coef[g];
+            J.weight[g] = (float)(scale * part);
+            exact[g] = scale * part;
+            if (q.kind == kGaussIdentity) carrier += scale * part;
+            if (!is_yvv(q.kind)) continue;
+            J.temp[g] = next;
+            next += plane;
+            double m[9];
+            optic_step_map(q, m);
+            q.row_maps = lp::line_maps(m, lp::piece_len(P.width));
+            q.col_maps = lp::line_maps(m, lp::piece_len(P.height));
+        }
+        J.carrier_weight = (float)carrier;
+        balance_weights(J, carrier, exact);
+        J.base = next;
+        next += plane;
+    }
+    return true;
+}
+
+cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
+    fir::Jobs F{};
+    F.width = P.width;
+    F.height = P.height;
+    F.dst_pairs = lp::plane_pairs(P.width);
+    F.dst_words = lp::line_words(P.height);
+    bool rows = false;
+    for (int j = 0; j < P.jobs; ++j) {
+        const OpticJob& J = P.job[j];
+        fir::Job f{};
+        f.src = J.src;
+        f.stride = J.stride;
+        f.dst = J.base;
+        f.src_weight = J.carrier_weight;
+        for (int g = 0; g < J.count; ++g) {
+            const OpticGauss& q = J.g[g];
+            rows |= is_yvv(q.kind);
+            if (q.kind != kGaussFir) continue;
+            fir::Taps& t = f.set[f.count++];
+            t.radius = q.radius;
+            t.flip_columns = 1; // the column pass runs bottom-up
+            t.weight = J.weight[g];
+            for (int i = 0; i < 2 * kOpticMaxFirRadius + 1; ++i) t.w[i] = q.w[i];
+        }
+        F.job[F.count++] = f;
+    }
+    cudaError_t e = cudaSuccess;
+    fjb::count_launch();
+    fir::kernel<float><<<fir::grid(F), fir::kThreads, 0, s>>>(F);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (rows) {
+        const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
+        e = cudaFuncSetAttribute(optic_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        P.rows_ahead = 2 * lp::kRowWarps * lp::resident_ctas(smem);
+        fjb::count_launch();
+        optic_rows_kernel<<<dim3((P.height + 3) / 4, P.jobs), 32 * lp::kRowWarps, smem, s>>>(P);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    const int warps = P.recursions * lp::kColPairs;
+    const size_t smem = warps * lp::line_bytes(P.height);
+    e = cudaFuncSetAttribute(optic_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    P.cols_ahead = lp::resident_ctas(smem);
+    fjb::count_launch();
+    optic_cols_kernel<<<dim3(lp::plane_pairs(P.width) / lp::kColPairs, P.jobs), 32 * warps, smem, s>>>(P);
+    return cudaGetLastError();
+}
+
+} // namespace fjb

@@ -1,0 +1,401 @@
+// fjb_line_pairs.cuh -- third-order linear recursions along lines, one warp per pair of lines.
+//
+// A warp holds two neighbouring lines (rows, or columns of a strip) of n samples in shared
+// memory, interleaved so that the two samples of a position are one 8-byte word. The
+// lines are cut into 32 pieces of K samples, one per lane, and a direction of a
+// recursion is
+//   partial : every piece runs from a zero state (the first from the line's start);
+//   scan    : exit states become entry states, entry_{t+1} = M^K entry_t + exit_t, by
+//             FP64 shuffles (Kogge-Stone over powers of M^K);
+//   final   : every piece runs again from its entry state, in place.
+// In exact arithmetic this is the sequential recursion; in floating point it differs
+// from it by rounding (the states between pieces are FP64). Successive pieces start an odd
+// number of words apart, so the lanes of a half warp fall in distinct banks. A step
+// handles both lines with packed FP32 instructions.
+//
+// Rows: a CTA holds four rows (two warps). Between the passes a plane lies by pairs of
+// columns, each pair's samples of all rows together, so that a row CTA writes a whole
+// 32-byte sector per pair of columns and a column warp reads its lines as one contiguous
+// block. Columns: a CTA holds two pairs of columns for each of a channel's recursions, one
+// warp per pair and recursion; two CTAs (a cluster) sum eight columns in their epilogue
+// through each other's shared memory and write whole sectors of the frame's rows.
+//
+// What bounds it: shared-memory bandwidth, seven 8-byte accesses per pair and position and
+// recursion (28 bytes per sample; 128 bytes per clock and SM), next to one read and one
+// write of the planes. Within a direction no warp waits for another, so what a warp waits
+// for (its loads, its scan) is covered by the others of its SM.
+#pragma once
+
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+namespace fjb {
+namespace lp {
+
+constexpr int kLevels = 5;
+constexpr int kPieces = 32;
+constexpr int kRowWarps = 2;      // warps (pairs of rows) of a row CTA
+constexpr int kMaxRecursions = 5; // of one channel
+constexpr int kColPairs = 2;      // pairs of columns of a column CTA
+constexpr int kColCluster = 2;    // column CTAs that write rows together
+constexpr int kMaxColWarps = kMaxRecursions * kColPairs;
+constexpr size_t kSmemLimit = 227 * 1024;
+
+// M^(K 2^i): the powers of the one-step zero-input map over one piece.
+struct LineMaps {
+    double m[kLevels][9];
+};
+
+// Samples per piece of a line of n samples (odd).
+__host__ __device__ inline int piece_len(int n) { return ((n + kPieces - 1) / kPieces) | 1; }
+// Words (pairs of samples) of a line as stored, a whole number of 32-byte sectors.
+__host__ __device__ inline int line_words(int n) { return (n + 3) / 4 * 4; }
+__host__ __device__ inline size_t line_bytes(int n) { return (size_t)line_words(n) * sizeof(float2); }
+// Pairs of columns of a plane between the passes (whole clusters), and its floats.
+__host__ __device__ inline int plane_pairs(int width) { return (width + 7) / 8 * 4; }
+__host__ __device__ inline size_t plane_floats(int width, int height) {
+    return (size_t)plane_pairs(width) * line_words(height) * 2;
+}
+
+inline void mat3_mul(const double* a, const double* b, double* o) {
+    double t[9];
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j) t[i * 3 + j] = a[i * 3] * b[j] + a[i * 3 + 1] * b[3 + j] + a[i * 3 + 2] * b[6 + j];
+    for (int i = 0; i < 9; ++i) o[i] = t[i];
+}
+
+inline LineMaps line_maps(const double* step, int k) {
+    LineMaps out;
+    auto power = [&](int n, double* o) {
+        double base[9], r[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
+        for (int i = 0; i < 9; ++i) base[i] = step[i];
+        for (; n > 0; n >>= 1) {
+            if (n & 1) mat3_mul(base, r, r);
+            mat3_mul(base, base, base);
+        }
+        for (int i = 0; i < 9; ++i) o[i] = r[i];
+    };
+    power(k, out.m[0]);
+    for (int l = 1; l < kLevels; ++l) mat3_mul(out.m[l - 1], out.m[l - 1], out.m[l]);
+    return out;
+}
+
+// ---------------------------------------------------------------------------
+// Two FP32 values in one 64-bit register; every operation rounds each half as the scalar
+// instruction does.
+// ---------------------------------------------------------------------------
+struct Pair {
+    unsigned long long v;
+};
+__device__ __forceinline__ Pair pack(float a, float b) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack(Pair p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// a - b (b's product with -1 is exact)
+__device__ __forceinline__ Pair sub2(Pair a, Pair b) { return fma2(b, pack(-1.0f, -1.0f), a); }
+
+// v = B x + B1 s0 + B2 s1 + B3 s2 with the last three outputs as state; the newest state
+// enters last, so the loop-carried dependency is one fused multiply-add.
+struct DirectStep {
+    Pair c0, c1, c2, c3;
+    __device__ DirectStep(float b, float b1, float b2, float b3)
+        : c0(pack(b, b)), c1(pack(b1, b1)), c2(pack(b2, b2)), c3(pack(b3, b3)) {}
+    __device__ __forceinline__ Pair step(Pair x, Pair (&s)[3]) const {
+        const Pair v = fma2(c1, s[0], fma2(c2, s[1], fma2(c3, s[2], mul2(c0, x))));
+        s[2] = s[1];
+        s[1] = s[0];
+        s[0] = v;
+        return v;
+    }
+};
+
+// The same recursion as a first-order section u += h (x - u) into a second-order one in
+// difference form, v = t v + g (u - y), y += v; state u, y, v.
+struct FactoredStep {
+    Pair h, g, t;
+    __device__ FactoredStep(float h_, float g_, float t_) : h(pack(h_, h_)), g(pack(g_, g_)), t(pack(t_, t_)) {}
+    __device__ __forceinline__ Pair step(Pair x, Pair (&s)[3]) const {
+        s[0] = fma2(h, sub2(x, s[0]), s[0]);
+        s[2] = fma2(t, s[2], mul2(g, sub2(s[0], s[1])));
+        s[1] = add2(s[1], s[2]);
+        return s[1];
+    }
+};
+
+// One piece of nv samples, the first processed one at `w` (kFwd: ascending positions).
+// Samples are read twelve at a time, so each group pays the shared-memory latency once, and
+// the direct form's state is back in its registers after a group (three shifts are none).
+template <bool kFwd, bool kWrite, typename Op>
+__device__ __forceinline__ void run(const Op& op, Pair* w, int nv, Pair (&s)[3]) {
+    constexpr int D = kFwd ? 1 : -1, U = 12;
+    int i = 0;
+#pragma unroll 1
+    for (; i + U <= nv; i += U, w += U * D) {
+        Pair x[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) x[k] = w[k * D];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const Pair v = op.step(x[k], s);
+            if (kWrite) w[k * D] = v;
+        }
+    }
+#pragma unroll 1
+    for (; i < nv; ++i, w += D) {
+        const Pair v = op.step(*w, s);
+        if (kWrite) *w = v;
+    }
+}
+
+// FP64 states of the pair's two lines.
+struct State2 {
+    double a[3], b[3];
+    __device__ __forceinline__ void set(const Pair (&s)[3]) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float2 f = unpack(s[i]);
+            a[i] = (double)f.x;
+            b[i] = (double)f.y;
+        }
+    }
+    __device__ __forceinline__ void get(Pair (&s)[3]) const {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s[i] = pack((float)a[i], (float)b[i]);
+    }
+    // += M t
+    __device__ __forceinline__ void add(const double* M, const State2& t) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = fma(M[3 * i], t.a[0], fma(M[3 * i + 1], t.a[1], fma(M[3 * i + 2], t.a[2], a[i])));
+            b[i] = fma(M[3 * i], t.b[0], fma(M[3 * i + 1], t.b[1], fma(M[3 * i + 2], t.b[2], b[i])));
+        }
+    }
+    // The state of the lane d places earlier in processing order.
+    template <bool kFwd>
+    __device__ __forceinline__ State2 from(int d) const {
+        State2 t;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            t.a[i] = kFwd ? __shfl_up_sync(0xffffffffu, a[i], d) : __shfl_down_sync(0xffffffffu, a[i], d);
+            t.b[i] = kFwd ? __shfl_up_sync(0xffffffffu, b[i], d) : __shfl_down_sync(0xffffffffu, b[i], d);
+        }
+        return t;
+    }
+};
+
+// This lane's piece of a pair of lines of n samples: positions [base, base + k) as far as
+// they lie in [lo, hi).
+struct Piece {
+    int base, k, lo, hi;
+    __device__ Piece(int n, int lane) : k(piece_len(n)) {
+        base = lane * k;
+        lo = min(base, n);
+        hi = min(base + k, n);
+    }
+};
+
+// One direction of a recursion over the pair of lines at `line`; `order` counts lanes in
+// processing order; `start` is the line's start state on the piece that is processed first
+// (`first`). Returns the piece's exit state in `s`.
+template <bool kFwd, typename Op>
+__device__ __forceinline__ void direction(const Op& op, const LineMaps& m, Pair* line, Piece pc, int order, bool first,
+                                          const Pair (&start)[3], Pair (&s)[3]) {
+    const Pair zero{0ull};
+    const int nv = pc.hi - pc.lo;
+    Pair* w = line + (kFwd ? pc.lo : pc.hi - 1);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s[i] = first ? start[i] : zero;
+    run<kFwd, false>(op, w, nv, s);
+    State2 S;
+    S.set(s);
+#pragma unroll 1
+    for (int l = 0; l < kLevels; ++l) {
+        const State2 t = S.from<kFwd>(1 << l);
+        if (order >= (1 << l)) S.add(m.m[l], t);
+    }
+    S.from<kFwd>(1).get(s);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s[i] = first ? start[i] : s[i];
+    run<kFwd, true>(op, w, nv, s);
+}
+
+// Brings a block of global memory into L2. The CTAs of a launch start together and would all
+// load, then all compute: each one asks for what the CTA that takes its place will load.
+__device__ __forceinline__ void prefetch_block(const float* p, size_t floats) {
+    const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+    const uintptr_t b = reinterpret_cast<uintptr_t>(p + floats) & ~(uintptr_t)15;
+    if (a < b)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(b - a)) : "memory");
+}
+// CTAs that the device holds at once, by shared memory alone.
+inline int resident_ctas(size_t smem) {
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return sms * (int)std::min<size_t>(32, kSmemLimit / std::max<size_t>(smem, 1));
+}
+
+// ---------------------------------------------------------------------------
+// Rows: from a plane, to a plane by pairs of columns
+// ---------------------------------------------------------------------------
+// Two rows of n floats, interleaved, by one warp (4-byte asynchronous copies: no alignment
+// asked for, everything in flight at once). The copies are in place when this returns.
+__device__ __forceinline__ void load_rows(Pair* buf, const float* a, const float* b, int n, int lane) {
+    unsigned d = (unsigned)__cvta_generic_to_shared(buf) + 8u * (unsigned)lane;
+#pragma unroll 4
+    for (int p = lane; p < n; p += 32, d += 256) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(a + p));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4), "l"(b + p));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+}
+
+// The CTA's four rows y .. y + 3 (two pairs, `words` apart) of `width` samples to the plane
+// by pairs of columns: one sector per pair of columns and thread. A barrier before (the
+// rows are complete) and after (the buffers are free).
+__device__ __forceinline__ void store_pairs(const Pair* buf, int words, float* plane, int width, int height, int y) {
+    __syncthreads();
+    const int pitch = 2 * line_words(height);
+    float* out = plane + 2 * y;
+#pragma unroll 2
+    for (int j = threadIdx.x; 2 * j < width; j += 32 * kRowWarps) {
+        const float4 a = *reinterpret_cast<const float4*>(buf + 2 * j);         // rows y, y + 1 of two columns
+        const float4 b = *reinterpret_cast<const float4*>(buf + words + 2 * j); // rows y + 2, y + 3
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + (size_t)j * pitch), "f"(a.x),
+                     "f"(a.z), "f"(a.y), "f"(a.w), "f"(b.x), "f"(b.z), "f"(b.y), "f"(b.w)
+                     : "memory");
+    }
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Columns
+// ---------------------------------------------------------------------------
+// One pair of columns of n rows by one warp, a contiguous block.
+__device__ __forceinline__ void load_line(Pair* buf, const float* plane, int pair, int n, int lane) {
+    const int words = line_words(n);
+    const float* src = plane + (size_t)pair * 2 * words;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(buf);
+#pragma unroll 4
+    for (int i = 2 * lane; i < words; i += 64)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + 8u * (unsigned)i), "l"(src + 2 * i));
+    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+}
+
+// The line of load_line into L2, by one lane.
+__device__ __forceinline__ void prefetch_line(const float* plane, int pair, int n) {
+    const size_t floats = 2 * (size_t)line_words(n);
+    prefetch_block(plane + pair * floats, floats);
+}
+
+// Where a cluster's results go: base + sum_i weight[i] * recursion i, to the frame's rows,
+// or back to the base while recursions are left over (columns too long for all at once).
+struct StripSum {
+    float* base; // by pairs of columns; null: no such term
+    float* dst;  // rows
+    long long dst_stride;
+    bool last;
+};
+
+// The epilogue of a column cluster: `count` recursions' lines in both CTAs' shared memory
+// (line i * kColPairs + pair), eight columns of an n x width plane, each CTA half of the
+// rows. The caller has synchronised the cluster and does so again before the lines go.
+__device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const float* weight, int count, int width, int n) {
+    constexpr int kBatch = 2, kAll = kColPairs * kColCluster;
+    const int words = line_words(n);
+    const unsigned rank = blockIdx.x % kColCluster;
+    const int pair0 = blockIdx.x / kColCluster * kAll, x0 = 2 * pair0;
+    const Pair* side[kColCluster];
+#pragma unroll
+    for (int r = 0; r < kColCluster; ++r) side[r] = cooperative_groups::this_cluster().map_shared_rank(lines, r);
+    const int half = (n + kColCluster - 1) / kColCluster;
+    const int ylo = rank * half, yhi = min(n, ylo + half);
+    float2* base = S.base ? reinterpret_cast<float2*>(S.base) + (size_t)pair0 * words : nullptr;
+    const unsigned align = S.dst_stride % 8 == 0 ? (unsigned)(reinterpret_cast<uintptr_t>(S.dst) & 31u) : 4u;
+    for (int y0 = ylo + threadIdx.x; y0 < yhi; y0 += kBatch * blockDim.x) {
+        float2 sum[kBatch][kAll];
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const int y = min(y0 + r * (int)blockDim.x, yhi - 1);
+#pragma unroll
+            for (int q = 0; q < kAll; ++q)
+                sum[r][q] = base ? base[(size_t)q * words + y] : make_float2(0.0f, 0.0f);
+        }
+#pragma unroll 1
+        for (int i = 0; i < count; ++i) {
+            const float w = weight[i];
+#pragma unroll
+            for (int r = 0; r < kBatch; ++r) {
+                const int y = min(y0 + r * (int)blockDim.x, yhi - 1);
+#pragma unroll
+                for (int q = 0; q < kAll; ++q) {
+                    const float2 v = unpack(side[q / kColPairs][(size_t)(i * kColPairs + q % kColPairs) * words + y]);
+                    sum[r][q].x = fmaf(w, v.x, sum[r][q].x);
+                    sum[r][q].y = fmaf(w, v.y, sum[r][q].y);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const int y = y0 + r * blockDim.x;
+            if (y >= yhi) break;
+            if (!S.last) {
+#pragma unroll
+                for (int q = 0; q < kAll; ++q) base[(size_t)q * words + y] = sum[r][q];
+                continue;
+            }
+            float* d = S.dst + (long long)y * S.dst_stride + x0;
+            if (x0 + 2 * kAll <= width && align == 0) {
+                asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(d), "f"(sum[r][0].x),
+                             "f"(sum[r][0].y), "f"(sum[r][1].x), "f"(sum[r][1].y), "f"(sum[r][2].x), "f"(sum[r][2].y),
+                             "f"(sum[r][3].x), "f"(sum[r][3].y)
+                             : "memory");
+            } else {
+#pragma unroll
+                for (int q = 0; q < kAll; ++q) {
+                    if (x0 + 2 * q < width) d[2 * q] = sum[r][q].x;
+                    if (x0 + 2 * q + 1 < width) d[2 * q + 1] = sum[r][q].y;
+                }
+            }
+        }
+    }
+}
+
+// Recursions a column CTA holds at once: two CTAs per SM (one loads while the other
+// computes) where that takes all of them, else as many as fit; 0: not one.
+inline int recursions_per_cta(int count, int n) {
+    const size_t bytes = kColPairs * line_bytes(n);
+    count = std::max(1, std::min(count, kMaxRecursions));
+    return std::min(count, (int)(kSmemLimit / bytes));
+}
+
+} // namespace lp
+} // namespace fjb

@@ -7,6 +7,7 @@
 #include <string>
 
 #include "../../include/juicer_cuda_api.h"
+#include "fjb_line_pairs.cuh"
 
 namespace fjb {
 
@@ -23,8 +24,10 @@ struct OpticGauss {
     int radius;   // FIR only
     float w[19];  // FIR weights, w[radius] is the centre tap
     float yvv[4]; // legacy: B, B1, B2, B3; factored: h, g, t, 0
-    double seg[9]; // recursive kinds: the state map over kOpticSeg zero-input steps (row-major 3x3)
-    double seg4[9]; // the same over 4 kOpticSeg steps
+    // recursive kinds, the zero-input state maps (row-major 3x3) that the pass's form needs:
+    // over a piece of a row and of a column and their powers, or over kOpticSeg steps
+    lp::LineMaps row_maps, col_maps;
+    double seg[9];
 };
 
 enum OpticMode : int { kOpticScatter = 0, kOpticBounce = 1 };
@@ -42,6 +45,11 @@ struct OpticJob {
     float tail_weight; // scatter only
     float amount;      // scatter amount, or bounce total strength
     int renormalize;   // bounce only
+    // one warp per pair of lines: the combination as weights of the carrier and of each
+    // Gaussian, and the plane the column launch adds its Gaussians to
+    float carrier_weight;
+    float weight[kOpticMaxGauss];
+    float* base;
 };
 
 struct OpticPass {
@@ -53,9 +61,22 @@ struct OpticPass {
     float* edge_a;
     float* edge_b;
     int lines_max, segs_max;
+    // the whole scratch of the stage; one warp per pair of lines: the recursions a column
+    // CTA holds at once, and the rows and column CTAs between a CTA and the one after it
+    float* scratch;
+    size_t scratch_floats;
+    int recursions, rows_ahead, cols_ahead;
 };
 
-cudaError_t launch_optic_pass(const OpticPass& P, cudaStream_t stream);
+cudaError_t launch_optic_pass(OpticPass& P, cudaStream_t stream);
+
+// One warp per pair of lines (fjb_halation_lines.cu): false when the pass's lines or planes are
+// out of its range; true lays the pass out for launch_optic_lines.
+bool optic_lines_plan(OpticPass& P);
+cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t stream);
+
+// One zero-input step of a recursive Gaussian's state (row-major 3x3).
+void optic_step_map(const OpticGauss& g, double m[9]);
 
 // Segments of the block-parallel recursions along a line of n samples.
 int optic_segments(int n);

@@ -16,8 +16,6 @@ namespace fjb {
 
 namespace {
 
-void segment_map(OpticGauss& g);
-
 const float kTailAmplitudes[3] = {0.1633f, 0.6496f, 0.1870f};
 
 bool decode_gauss(const FjHalationGaussian& s, OpticGauss& g) {
@@ -46,7 +44,6 @@ bool decode_gauss(const FjHalationGaussian& s, OpticGauss& g) {
     g.radius = s.radius;
     std::memcpy(g.w, s.fir_weights, sizeof(g.w));
     std::memcpy(g.yvv, s.yvv, sizeof(g.yvv));
-    segment_map(g);
     return true;
 }
 
@@ -56,34 +53,20 @@ namespace {
 
 int segments(int n) { return optic_segments(n); }
 
-// The recursion's state map over kOpticSeg steps with zero input, in FP64: the
-// operator that carries a segment's entry state to its exit state.
-void segment_map(OpticGauss& g) {
-    double m[9] = {0};
+} // namespace
+
+void optic_step_map(const OpticGauss& g, double m[9]) {
     if (g.kind == kGaussYvv) {
         // (s1, s2, s3) -> (B1 s1 + B2 s2 + B3 s3, s1, s2)
         const double m0[9] = {g.yvv[1], g.yvv[2], g.yvv[3], 1, 0, 0, 0, 1, 0};
-        std::memcpy(m, m0, sizeof(m));
-    } else if (g.kind == kGaussYvvFactored) {
+        std::memcpy(m, m0, sizeof(m0));
+    } else {
         // s1' = (1-h) s1; s3' = t s3 + g (s1' - s2); s2' = s2 + s3'
         const double h = g.yvv[0], gg = g.yvv[1], t = g.yvv[2];
         const double m0[9] = {1 - h, 0, 0, gg * (1 - h), 1 - gg, t, gg * (1 - h), -gg, t};
-        std::memcpy(m, m0, sizeof(m));
-    } else {
-        return;
+        std::memcpy(m, m0, sizeof(m0));
     }
-    double r[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    for (int step = 1; step <= 4 * kOpticSeg; ++step) {
-        double t[9];
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) t[i * 3 + j] = m[i * 3] * r[j] + m[i * 3 + 1] * r[3 + j] + m[i * 3 + 2] * r[6 + j];
-        std::memcpy(r, t, sizeof(r));
-        if (step == kOpticSeg) std::memcpy(g.seg, r, sizeof(r));
-    }
-    std::memcpy(g.seg4, r, sizeof(r));
 }
-
-} // namespace
 
 size_t halation_scratch_floats(int width, int height) {
     const size_t lines = (size_t)(width > height ? width : height);
@@ -110,6 +93,8 @@ bool scatter_halation(const FjScatterHalation& d, float* planes_rgb[3], long lon
         const int segs = segments(width) > segments(height) ? segments(width) : segments(height);
         float* tail = scratch + (size_t)3 * kOpticMaxGauss * plane;
         for (OpticPass* P : {&scatter, &bounce}) {
+            P->scratch = scratch;
+            P->scratch_floats = halation_scratch_floats(width, height);
             P->lines_max = lines;
             P->segs_max = segs;
             P->carry = tail;
