@@ -168,33 +168,38 @@ extern "C" FjStatus fjb_diffusion(const FjDiffusionComponents* components, int32
             if (!fjb::diffusion_psf_rows(components->lambda_px, weights[c], radius_px, rows[c], taps, why))
                 return fail_status(FJ_STATUS_PREPARATION_FAILURE, error, why);
         cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-        float* d_psf = nullptr;
+        // one allocation: the PSF rows, then for the FFT forms the PSF spectrum and the
+        // row-spectrum workspace (none for tiles)
         const size_t n = rows[0].size();
-        cudaError_t e = cudaMalloc(&d_psf, 3 * n * sizeof(float));
-        for (int c = 0; c < 3 && e == cudaSuccess; ++c)
-            e = cudaMemcpyAsync(d_psf + c * n, rows[c].data(), n * sizeof(float), cudaMemcpyHostToDevice, s);
-        float* d_fft = nullptr; // FFT form: PSF spectrum, then the row-spectrum workspace
+        fjb::DiffusionFftPlan plan;
+        const bool fft = fjb::diffusion_prefers_fft(width, height, radius_px) &&
+                         fjb::diffusion_fft_plan(width, height, radius_px, plan);
+        const size_t psf_floats = (3 * n + 63) / 64 * 64;
+        float* d_psf = nullptr;
+        cudaError_t e = cudaMalloc(
+            &d_psf, (psf_floats + (fft ? plan.spectrum_floats + plan.work_floats : 0)) * sizeof(float));
+        rows[0].insert(rows[0].end(), rows[1].begin(), rows[1].end());
+        rows[0].insert(rows[0].end(), rows[2].begin(), rows[2].end());
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(d_psf, rows[0].data(), 3 * n * sizeof(float), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) {
             const float* psf[3] = {d_psf, d_psf + n, d_psf + 2 * n};
             float* dst[3] = {dst_r, dst_g, dst_b};
             const float* src[3] = {src_r, src_g, src_b};
-            fjb::DiffusionFftPlan plan;
-            if (fjb::diffusion_prefers_fft(width, height, radius_px) &&
-                fjb::diffusion_fft_plan(width, height, radius_px, plan)) {
-                e = cudaMalloc(&d_fft, (plan.spectrum_floats + plan.work_floats) * sizeof(float));
-                float* work = d_fft + plan.spectrum_floats;
-                if (e == cudaSuccess) e = fjb::launch_diffusion_fft_spectrum(plan, psf, taps, d_fft, work, s);
+            if (fft) {
+                float* spectrum = d_psf + psf_floats;
+                float* work = spectrum + plan.spectrum_floats;
+                e = fjb::launch_diffusion_fft_spectrum(plan, psf, taps, spectrum, work, s);
                 if (e == cudaSuccess)
-                    e = fjb::launch_diffusion_fft(plan, d_fft, (float)scatter_fraction, dst, src, stride, work, s);
+                    e = fjb::launch_diffusion_fft(plan, spectrum, (float)scatter_fraction, dst, src, stride, work, s);
             } else {
                 e = fjb::launch_diffusion(psf, radius_px, taps, (float)scatter_fraction, dst, src, stride, width,
                                           height, s);
             }
         }
-        // the host rows and the device buffers must outlive the copies and the kernels
+        // the host rows and the device buffer must outlive the copies and the kernels
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (d_psf) cudaFree(d_psf);
-        if (d_fft) cudaFree(d_fft);
         if (e != cudaSuccess) return cuda_status(e, error, "diffusion");
         write_error(error, "");
         return ok_status();

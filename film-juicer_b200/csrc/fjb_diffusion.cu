@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include "fjb_diffusion.h"
@@ -119,22 +120,25 @@ bool diffusion_psf_rows(const double lambda_px[9], const double weights[9], int 
         return false;
     }
     const int d = 2 * radius + 1;
-    std::vector<float> grid((size_t)d * d);
+    // a value depends on dx^2 + dy^2 alone: one per 0 <= dx <= dy <= r (210 of 1521 at r = 19)
+    std::vector<float> octant((size_t)(radius + 1) * (radius + 1));
     double sum = 0.0;
     const double kTwoPi = 6.283185307179586476925286766559;
-    for (int iy = 0; iy < d; ++iy)
-        for (int ix = 0; ix < d; ++ix) {
-            const int dx = ix - radius, dy = iy - radius;
+    for (int dy = 0; dy <= radius; ++dy)
+        for (int dx = 0; dx <= dy; ++dx) {
             const double rho = std::sqrt((double)dx * (double)dx + (double)dy * (double)dy);
             double v = 0.0;
             for (int k = 0; k < 9; ++k) {
                 const double l = lambda_px[k];
                 v += weights[k] * std::exp(-rho / l) / (kTwoPi * l * l);
             }
-            const float stored = (float)v;
-            grid[(size_t)iy * d + ix] = stored;
-            sum += (double)stored;
+            octant[(size_t)dy * (radius + 1) + dx] = octant[(size_t)dx * (radius + 1) + dy] = (float)v;
         }
+    auto grid = [&](int iy, int ix) {
+        return octant[(size_t)std::abs(iy - radius) * (radius + 1) + std::abs(ix - radius)];
+    };
+    for (int iy = 0; iy < d; ++iy)
+        for (int ix = 0; ix < d; ++ix) sum += (double)grid(iy, ix);
     if (!(std::isfinite(sum) && sum > 0.0)) {
         why = "diffusion PSF does not normalise";
         return false;
@@ -143,7 +147,7 @@ bool diffusion_psf_rows(const double lambda_px[9], const double weights[9], int 
     rows.assign((size_t)(radius + 1) * taps, 0.0f);
     for (int dy = 0; dy <= radius; ++dy)
         for (int ix = 0; ix < d; ++ix)
-            rows[(size_t)dy * taps + ix] = (float)((double)grid[(size_t)(dy + radius) * d + ix] / sum);
+            rows[(size_t)dy * taps + ix] = (float)((double)grid(dy + radius, ix) / sum);
     return true;
 }
 

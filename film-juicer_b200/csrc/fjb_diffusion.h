@@ -21,12 +21,17 @@ size_t diffusion_smem_bytes(int radius);
 cudaError_t launch_diffusion(const float* const psf_rows[3], int radius, int taps, float fraction, float* dst[3],
                              const float* src[3], long long stride, int width, int height, cudaStream_t stream);
 
-// FFT form (fjb_diffusion_fft.cu), used from kDiffusionFftMinRadius up: the
-// reflect-extended frame convolved circularly on an nx x ny power-of-two grid.
+// FFT form, used from kDiffusionFftMinRadius up: tiles of kDiffusionTile x kDiffusionTile of
+// the reflect-extended frame convolved circularly in shared memory (fjb_diffusion_tile.cu),
+// or, above kDiffusionTileMaxRadius, the whole extended frame on an nx x ny grid
+// (fjb_diffusion_fft.cu).
 constexpr int kDiffusionFftMinRadius = 8;
+constexpr int kDiffusionTile = 128;
+constexpr int kDiffusionTileMaxRadius = 40;
 
 struct DiffusionFftPlan {
     int width, height, radius;
+    bool tile; // tiles: the sizes below are not used
     int m, log2m;     // nx / 2 complex points per row transform
     int ny, log2ny;   // column transform length 2^a 3^ny3 (log2ny: a when ny3 == 0, else -1)
     int ny3;          // factors of 3 in ny (0, 1 or 2)
@@ -51,5 +56,11 @@ cudaError_t launch_diffusion_fft_spectrum(const DiffusionFftPlan& plan, const fl
 // dst[c] = (1 - fraction) src[c] + fraction (PSF_c * src[c]) through the spectrum.
 cudaError_t launch_diffusion_fft(const DiffusionFftPlan& plan, const float* spectrum, float fraction, float* dst[3],
                                  const float* src[3], long long stride, float* work, cudaStream_t stream);
+
+// The tile form of the two (plan.tile).
+cudaError_t launch_diffusion_tile_spectrum(const DiffusionFftPlan& plan, const float* const psf_rows[3], int taps,
+                                           float* spectrum, cudaStream_t stream);
+cudaError_t launch_diffusion_tile(const DiffusionFftPlan& plan, const float* spectrum, float fraction, float* dst[3],
+                                  const float* src[3], long long stride, cudaStream_t stream);
 
 } // namespace fjb

@@ -1,4 +1,5 @@
-// fjb_diffusion_fft.cu -- diffusion (a17) as an FFT convolution, for large radii.
+// fjb_diffusion_fft.cu -- diffusion (a17) as an FFT convolution of the frame, for radii above
+// the tile form's (fjb_diffusion_tile.cu).
 //
 // Same result as the direct kernel of fjb_diffusion.cu up to FP32 round-off: the
 // reflect-extended frame (whole-sample reflection, r samples on every side) is
@@ -514,6 +515,14 @@ cudaError_t set_smem(const void* fn, size_t bytes) {
 bool diffusion_fft_plan(int width, int height, int radius, DiffusionFftPlan& p) {
     p = DiffusionFftPlan{};
     if (width <= 0 || height <= 0 || radius < 0) return false;
+    if (radius <= kDiffusionTileMaxRadius) {
+        p.width = width;
+        p.height = height;
+        p.radius = radius;
+        p.tile = true;
+        p.spectrum_floats = (size_t)3 * kDiffusionTile * kDiffusionTile;
+        return true;
+    }
     const long long wx = (long long)width + 2LL * radius, hy = (long long)height + 2LL * radius;
     if (wx > 2LL * kFftMaxLen || hy > kFftMaxLen) return false;
     const int nx = pow2_at_least((int)(wx < 16 ? 16 : wx));
@@ -563,6 +572,7 @@ bool diffusion_prefers_fft(int width, int height, int radius) {
 
 cudaError_t launch_diffusion_fft_spectrum(const DiffusionFftPlan& p, const float* const psf_rows[3], int taps,
                                           float* spectrum, float* work, cudaStream_t stream) {
+    if (p.tile) return launch_diffusion_tile_spectrum(p, psf_rows, taps, spectrum, stream);
     FftPass F{};
     F.p = p;
     float2* tw = reinterpret_cast<float2*>(spectrum);
@@ -595,6 +605,7 @@ cudaError_t launch_diffusion_fft_spectrum(const DiffusionFftPlan& p, const float
 
 cudaError_t launch_diffusion_fft(const DiffusionFftPlan& p, const float* spectrum, float fraction, float* dst[3],
                                  const float* src[3], long long stride, float* work, cudaStream_t stream) {
+    if (p.tile) return launch_diffusion_tile(p, spectrum, fraction, dst, src, stride, stream);
     FftPass F{};
     F.p = p;
     F.tw = reinterpret_cast<const float2*>(spectrum);

@@ -24,8 +24,6 @@ namespace fjb {
 
 namespace {
 
-using lp::Pair;
-
 __device__ __forceinline__ void map_state(const double* T, const double d[3], double o[3]) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) o[i] = T[3 * i] * d[0] + T[3 * i + 1] * d[1] + T[3 * i + 2] * d[2];
@@ -38,7 +36,7 @@ __device__ __forceinline__ void state_from(const DirComponentDev& c, const doubl
     map_state(c.to_fac, a, oa);
     map_state(c.to_fac, b, ob);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) s[i] = lp::pack((float)oa[i], (float)ob[i]);
+    for (int i = 0; i < 3; ++i) s[i] = pack((float)oa[i], (float)ob[i]);
 }
 
 // End block of one line from its final state: the last `ts` outputs in `term`, and the
@@ -137,7 +135,7 @@ __device__ __forceinline__ void filter(const DirComponentDev& c, const double* f
     // the lane that holds the line's end makes the end block; everyone gets the way back's start
     const int end_lane = kDown ? 0 : (n - 1) / piece.k;
     {
-        const float2 f0 = lp::unpack(s[0]), f1 = lp::unpack(s[1]), f2 = lp::unpack(s[2]);
+        const float2 f0 = unpack(s[0]), f1 = unpack(s[1]), f2 = unpack(s[2]);
         const double fa[3] = {f0.x, f1.x, f2.x}, fb[3] = {f0.y, f1.y, f2.y};
         double ta[3], tb[3], ba[3], bb[3];
         end_block(c, T, ts, fa, ta, ba);
@@ -145,7 +143,7 @@ __device__ __forceinline__ void filter(const DirComponentDev& c, const double* f
         __syncwarp();
         if (lane == end_lane)
             for (int r = 0; r < ts; ++r)
-                if (n - ts + r >= 0) *sample(n - ts + r) = lp::pack((float)ta[r], (float)tb[r]);
+                if (n - ts + r >= 0) *sample(n - ts + r) = pack((float)ta[r], (float)tb[r]);
         state_from(c, ba, bb, s);
 #pragma unroll
         for (int i = 0; i < 3; ++i) start[i].v = __shfl_sync(0xffffffffu, s[i].v, end_lane);

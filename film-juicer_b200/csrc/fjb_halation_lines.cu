@@ -22,8 +22,6 @@ namespace fjb {
 
 namespace {
 
-using lp::Pair;
-
 __host__ __device__ __forceinline__ bool is_yvv(int kind) { return kind == kGaussYvv || kind == kGaussYvvFactored; }
 
 // Both directions of one recursive Gaussian over a pair of lines of n samples, from

@@ -386,8 +386,9 @@ FjStatus apply_diffusion(FjCuda* cuda, const FjDiffusion& d, int stage, const fl
     if (fft || measure) {
         // the PSF spectrum depends on the descriptor and the transform sizes
         const uint64_t skey = (cache.key * 0x100000001b3ULL) ^ ((uint64_t)width << 32) ^ (uint64_t)height;
-        e = ensure_buffer(cuda, cuda->diffusion_fft_work, cuda->diffusion_fft_work_bytes,
-                          plan.work_floats * sizeof(float));
+        if (plan.work_floats)
+            e = ensure_buffer(cuda, cuda->diffusion_fft_work, cuda->diffusion_fft_work_bytes,
+                              plan.work_floats * sizeof(float));
         if (e != cudaSuccess) return fjb::cuda_status(e, error, "diffusion FFT workspace");
         if (skey != cache.spectrum_key || !cache.spectrum) {
             cache.spectrum_key = 0;
