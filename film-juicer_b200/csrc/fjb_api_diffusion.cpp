@@ -3,6 +3,7 @@
 
 #include <cmath>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -16,6 +17,58 @@ using fjb::ok_status;
 using fjb::write_error;
 
 namespace {
+
+// Device memory of one call, on the call's stream, from a pool of the library's own: a
+// cudaMalloc and cudaFree pair per call took from 50 to 600 us here, depending on the box. The
+// pool keeps at most kKeep bytes between calls (it grows by chunks of 32 MB: with a smaller
+// bound each synchronisation gave the chunk back, and the next call took 2.5 ms); what a call
+// needs beyond that goes back at the next synchronisation. Allocation is ordered by stream
+// and safe from several threads.
+class CallMemory {
+  public:
+    cudaError_t allocate(size_t bytes, cudaStream_t s) {
+        stream_ = s;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = device_pool(pool);
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&data_, bytes, pool, s);
+        return e;
+    }
+    float* data() const { return static_cast<float*>(data_); }
+    ~CallMemory() {
+        if (data_) cudaFreeAsync(data_, stream_);
+    }
+
+  private:
+    static constexpr uint64_t kKeep = 64ull << 20;
+    static constexpr int kMaxDevices = 64;
+    static cudaError_t device_pool(cudaMemPool_t& pool) {
+        static std::mutex gate;
+        static cudaMemPool_t pools[kMaxDevices] = {};
+        int device = 0;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return e;
+        if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+        std::lock_guard<std::mutex> lock(gate);
+        if (!pools[device]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            cudaMemPool_t fresh = nullptr;
+            if ((e = cudaMemPoolCreate(&fresh, &props)) != cudaSuccess) return e;
+            uint64_t keep = kKeep;
+            if ((e = cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+                cudaMemPoolDestroy(fresh);
+                return e;
+            }
+            pools[device] = fresh;
+        }
+        pool = pools[device];
+        return cudaSuccess;
+    }
+    void* data_ = nullptr;
+    cudaStream_t stream_ = nullptr;
+};
 
 double ordered_max(double v, double floor_value) { return v > floor_value ? v : floor_value; }
 
@@ -175,9 +228,9 @@ extern "C" FjStatus fjb_diffusion(const FjDiffusionComponents* components, int32
         const bool fft = fjb::diffusion_prefers_fft(width, height, radius_px) &&
                          fjb::diffusion_fft_plan(width, height, radius_px, plan);
         const size_t psf_floats = (3 * n + 63) / 64 * 64;
-        float* d_psf = nullptr;
-        cudaError_t e = cudaMalloc(
-            &d_psf, (psf_floats + (fft ? plan.spectrum_floats + plan.work_floats : 0)) * sizeof(float));
+        CallMemory memory;
+        cudaError_t e = memory.allocate((psf_floats + (fft ? plan.spectrum_floats + plan.work_floats : 0)) * sizeof(float), s);
+        float* d_psf = memory.data();
         rows[0].insert(rows[0].end(), rows[1].begin(), rows[1].end());
         rows[0].insert(rows[0].end(), rows[2].begin(), rows[2].end());
         if (e == cudaSuccess)
@@ -197,9 +250,8 @@ extern "C" FjStatus fjb_diffusion(const FjDiffusionComponents* components, int32
                                           height, s);
             }
         }
-        // the host rows and the device buffer must outlive the copies and the kernels
+        // the host rows must outlive the copy
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (d_psf) cudaFree(d_psf);
         if (e != cudaSuccess) return cuda_status(e, error, "diffusion");
         write_error(error, "");
         return ok_status();
