@@ -45,13 +45,16 @@ constexpr float kLn10 = 2.30258509299404568402f;
 
 struct FitTheta {
     float ev[3], gamma[3], pgamma[3], k[3], pev;
+    bool dir_guess = true; // the compensated axes as staged are strictly increasing
 };
 
 // Curve value and its slope dy / dxq at xq = logE * gamma (the interval the render
 // path's curve_sample selects; slope 0 at and beyond the sampled ends). `knot` and
 // `frac` receive the interval's left sample and the position in it (knot -1 outside).
-__device__ float curve_with_slope(const float* __restrict__ blob, const CurveRef& c, float logE, float gamma,
-                                  float& slope, int& knot, float& frac) {
+// `guess`: the recipe's first cell may start the lookup (the axis is the recipe's, or the
+// staging found the moved one strictly increasing too); it steps from there.
+__device__ __forceinline__ float curve_with_slope(const float* __restrict__ blob, const CurveRef& c, bool guess,
+                                                  float logE, float gamma, float& slope, int& knot, float& frac) {
     slope = 0.0f;
     knot = -1;
     frac = 0.0f;
@@ -63,6 +66,14 @@ __device__ float curve_with_slope(const float* __restrict__ blob, const CurveRef
     if (!(x[last] >= x[0])) return y[0];
     if (xq <= x[0]) return y[0];
     if (xq >= x[last]) return y[last];
+    if (guess && c.guess && xq == xq) {
+        float xa, xb;
+        knot = curve_interval(blob, c, xq, xa, xb);
+        const float y0 = y[knot], dy = y[knot + 1] - y0, den = xb - xa;
+        slope = fabsf(dy) <= 1e15f ? quotient(dy, den) : dy / den;
+        frac = quotient(xq - xa, den);
+        return y0 + frac * dy;
+    }
     const int i1 = curve_interval_search(x, last, xq);
     if (i1 > last) return y[last];
     const int i0 = i1 - 1;
@@ -170,26 +181,34 @@ __device__ bool scan_lut_sample_d(const PixelParams& p, const double n[3], float
 // q[3c + j] ln 2. One exp2 per wavelength serves the value and its derivative.
 __device__ __forceinline__ void print_spectral_moments(const PrintSpectral& s, const float d[3], float raw[3],
                                                        float q[9]) {
-    float a0[3] = {0.0f, 0.0f, 0.0f}, a1[3] = {0.0f, 0.0f, 0.0f};
+    const Pair zero = pack(0.0f, 0.0f);
+    const Pair d0 = pack(d[0], d[0]), d1 = pack(d[1], d[1]), d2 = pack(d[2], d[2]);
+    Pair a[3] = {zero, zero, zero}, m[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) q[k] = 0.0f;
+    for (int k = 0; k < 9; ++k) m[k] = zero;
 #pragma unroll
-    for (int i = 0; i < kSpectralSamples; ++i) {
-        const float dl = fmaf(d[0], s.nd[i][0], fmaf(d[1], s.nd[i][1], d[2] * s.nd[i][2]));
-        const float t = mufu_exp2(dl);
-        float* a = (i & 1) ? a1 : a0;
+    for (int i = 0; i < kSpectralPairs; ++i) {
+        const Pair* w = reinterpret_cast<const Pair*>(s.pairs[i]);
+        const float2 dl = unpack(fma2(d0, w[0], fma2(d1, w[1], mul2(d2, w[2]))));
+        const Pair t = pack(mufu_exp2(dl.x), mufu_exp2(dl.y));
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            a[c] = fmaf(t, s.sens[i][c], a[c]);
-            const float w = t * s.sens[i][c];
-            q[3 * c + 0] = fmaf(w, s.nd[i][0], q[3 * c + 0]);
-            q[3 * c + 1] = fmaf(w, s.nd[i][1], q[3 * c + 1]);
-            q[3 * c + 2] = fmaf(w, s.nd[i][2], q[3 * c + 2]);
+            a[c] = fma2(t, w[3 + c], a[c]);
+            const Pair v = mul2(t, w[3 + c]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) m[3 * c + j] = fma2(v, w[j], m[3 * c + j]);
         }
     }
-    raw[0] = a0[0] + a1[0];
-    raw[1] = a0[1] + a1[1];
-    raw[2] = a0[2] + a1[2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float2 v = unpack(a[c]);
+        raw[c] = v.x + v.y;
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const float2 v = unpack(m[k]);
+        q[k] = v.x + v.y;
+    }
 }
 
 // One pixel: the linear output RGB for theta; with kGrad, also adds the pixel's
@@ -216,7 +235,7 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
         if (!isfinite(logS[c])) return false;
         int kn;
         float fr;
-        layer[c] = curve_with_slope(blob, p.film_curve[c], logS[c], th.gamma[c], sl[c], kn, fr);
+        layer[c] = curve_with_slope(blob, p.film_curve[c], true, logS[c], th.gamma[c], sl[c], kn, fr);
     }
     float D[3], logC[3] = {0.0f, 0.0f, 0.0f}, sd[3] = {0.0f, 0.0f, 0.0f}, dv[3] = {0.0f, 0.0f, 0.0f},
                 dk[3] = {0.0f, 0.0f, 0.0f}, dfr[3] = {0.0f, 0.0f, 0.0f};
@@ -270,7 +289,7 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
         }
         for (int j = 0; j < 3; ++j) {
             logC[j] = logS[j] - corr[j];
-            D[2 - j] = curve_with_slope(blob, p.dir_curve[j], logC[j], th.gamma[j], sd[j], dkn[j], dfr[j]);
+            D[2 - j] = curve_with_slope(blob, p.dir_curve[j], th.dir_guess, logC[j], th.gamma[j], sd[j], dkn[j], dfr[j]);
         }
     } else {
         for (int c = 0; c < 3; ++c) D[2 - c] = layer[c];
@@ -296,10 +315,10 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
             v *= spev;
             v *= p.print_route_correction;
             rawp[c] = v;
-            lp[c] = log10f(v + 1e-10f);
+            lp[c] = log10_any(v + 1e-10f);
             int kn;
             float fr;
-            scanD[c] = curve_with_slope(blob, p.print_curve[c], lp[c], th.pgamma[c], sp[c], kn, fr);
+            scanD[c] = curve_with_slope(blob, p.print_curve[c], true, lp[c], th.pgamma[c], sp[c], kn, fr);
         }
     } else {
         for (int c = 0; c < 3; ++c) scanD[c] = D[c];
@@ -422,7 +441,7 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
 //   axis_j[i] += sum_d M[d][j] (L(y_d[i], k0_d) - L(y_d[i], k_d))
 // (the host builds axis_j[i] = logE[i] - sum_d M[d][j] L(y_d[i], k0_d):
 // rust/film-juicer-core/src/film/dir.rs:258-290). The recipe's knees leave them as given.
-__device__ __forceinline__ const float* stage_blob(const PixelParams& p, const FitTheta& th, float* smem) {
+__device__ __forceinline__ const float* stage_blob(const PixelParams& p, FitTheta& th, float* smem) {
     const float4* g = reinterpret_cast<const float4*>(p.curve_blob);
     float4* s4 = reinterpret_cast<float4*>(smem);
     for (int i = threadIdx.x; i < (p.curve_blob_floats >> 2); i += blockDim.x) s4[i] = __ldg(g + i);
@@ -442,6 +461,14 @@ __device__ __forceinline__ const float* stage_blob(const PixelParams& p, const F
             ax[i] = (float)((double)ax[i] + delta);
         }
         __syncthreads();
+        bool increasing = true;
+        for (int e = threadIdx.x; e < 3 * (n - 1); e += blockDim.x) {
+            const int j = e / (n - 1);
+            const float* ax = smem + p.dir_curve[j].x + (e - j * (n - 1));
+            const float step = ax[1] - ax[0];
+            increasing &= step > 1e-20f && step < 1e20f;
+        }
+        th.dir_guess = __syncthreads_and(increasing) != 0;
     }
     return smem;
 }
@@ -622,7 +649,7 @@ __device__ bool dir_source_pixel(const PixelParams& p, const float* __restrict__
         if (!isfinite(logS[c])) return false;
         int kn;
         float fr;
-        layer[c] = curve_with_slope(blob, p.film_curve[c], logS[c], th.gamma[c], sl[c], kn, fr);
+        layer[c] = curve_with_slope(blob, p.film_curve[c], true, logS[c], th.gamma[c], sl[c], kn, fr);
         const float v = layer[c];
         if (p.dir_mode == kDirPositiveReceiver) {
             donor[c] = p.dir_dmax[c] - v;

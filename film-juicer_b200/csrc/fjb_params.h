@@ -34,9 +34,12 @@ struct CurveRef {
     int x;   // offset of the ascending abscissa
     int y;   // offset of the ordinate
     int n;   // sample count (accepted domain is [0, n-1])
-    int guess;    // 1: the abscissa is strictly increasing and close to uniform
+    int guess;    // the abscissa is strictly increasing and 1: close to uniform; 2: see table
     float x0;     // first abscissa
-    float inv_dx; // (n - 1) / (x[n-1] - x[0])
+    float inv_dx; // cells / (x[n-1] - x[0])
+    float x1;     // last abscissa
+    int cells;    // n - 1, or the table's cells
+    int table;    // offset of the table: per cell (u16) the last sample at or below its start
 };
 
 // Print 81-lambda coefficients, pre-folded on the host:
@@ -48,10 +51,14 @@ struct CurveRef {
 // illuminant is NaN, are dropped and the remaining ones packed first; the unused tail
 // slots hold (0, 0, 0, -inf) and zero sensitivities, so they contribute exactly +0 for
 // finite densities. A NaN channel of a kept wavelength contributes zero.
+constexpr int kSpectralPairs = (kSpectralSamples + 1) / 2;
 struct PrintSpectral {
     float nd[kSpectralSamples][4];
     float sens[kSpectralSamples][3];
     int count;
+    // the same by pairs of wavelengths (2 i, 2 i + 1), for the packed form: the three exponents'
+    // factors, then the three weights; the last one's second half is padding (weight 0)
+    float2 pairs[kSpectralPairs][6];
 };
 
 struct PixelParams {

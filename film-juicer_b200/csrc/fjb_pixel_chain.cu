@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kPixelThreads) pixel_chain_kernel(const __grid
         }
         if constexpr (Out == kOutEnlargerDevelop) {
             // :1449-1488 with print_log_encode_diffused_device (:1025) and the print curves
-            for (int c = 0; c < 3; ++c) d[c] = curve_sample(blob, p.print_curve[c], log10f(fmaxf(d[c], 0.0f) + 1e-10f), 1.0f);
+            for (int c = 0; c < 3; ++c) d[c] = curve_sample(blob, p.print_curve[c], log_exposure(d[c]), 1.0f);
             p.density_c[idx] = d[0];
             p.density_m[idx] = d[1];
             p.density_y[idx] = d[2];

@@ -12,6 +12,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "fjb_math.cuh"
+#include "fjb_packed.cuh"
 #include "fjb_params.h"
 
 namespace fjb {
@@ -78,6 +80,27 @@ __device__ __forceinline__ float mitchell(float t) {
     return 0.0f;
 }
 
+// The four taps around a sample at fraction f in [0, 1], mitchell(f + 1), mitchell(f),
+// mitchell(f - 1), mitchell(f - 2), each on the branch it is known to be on (at the
+// branches' meeting points, f = 0 and 1, they agree but for rounding).
+__device__ __forceinline__ void mitchell_taps(float f, float w[4]) {
+    const float B = 1.0f / 3.0f;
+    const float C = 1.0f / 3.0f;
+    auto inner = [](float x) {
+        return (1.0f / 6.0f) * ((12.0f - 9.0f * B - 6.0f * C) * x * x * x +
+                                (-18.0f + 12.0f * B + 6.0f * C) * x * x + (6.0f - 2.0f * B));
+    };
+    auto outer = [](float x) {
+        const float v = (1.0f / 6.0f) * ((-B - 6.0f * C) * x * x * x + (6.0f * B + 30.0f * C) * x * x +
+                                         (-12.0f * B - 48.0f * C) * x + (8.0f * B + 24.0f * C));
+        return x < 2.0f ? v : 0.0f;
+    };
+    w[0] = outer(f + 1.0f);
+    w[1] = inner(f);
+    w[2] = inner(1.0f - f);
+    w[3] = outer(2.0f - f);
+}
+
 __device__ __forceinline__ void tc_coordinate(float normalized, int& base, float& frac) {
     const float top = (float)(kTcLutExtent - 1);
     const float coord = fminf(1.0f, fmaxf(0.0f, normalized)) * top;
@@ -128,8 +151,9 @@ __device__ __forceinline__ void tc_lut_sample(const float4* __restrict__ lut, fl
     float cf, mf;
     tc_coordinate(qx, cb, cf);
     tc_coordinate(qy, mb, mf);
-    const float wc[4] = {mitchell(cf + 1.0f), mitchell(cf), mitchell(cf - 1.0f), mitchell(cf - 2.0f)};
-    const float wm[4] = {mitchell(mf + 1.0f), mitchell(mf), mitchell(mf - 1.0f), mitchell(mf - 2.0f)};
+    float wc[4], wm[4];
+    mitchell_taps(cf, wc);
+    mitchell_taps(mf, wm);
     float acc[3] = {0.0f, 0.0f, 0.0f};
     float wsum = 0.0f;
     if (cb >= 1 && cb <= kTcLutExtent - 3 && mb >= 1 && mb <= kTcLutExtent - 3) {
@@ -151,7 +175,9 @@ __device__ __forceinline__ void tc_lut_sample(const float4* __restrict__ lut, fl
     } else {
         tc_lut_edge(lut, cb, mb, cf, mf, acc, wsum);
     }
-    for (int k = 0; k < 3; ++k) rgb[k] = wsum != 0.0f ? acc[k] / wsum : 0.0f;
+    // the taps add up to one but for rounding; the table's values may be anything
+    for (int k = 0; k < 3; ++k)
+        rgb[k] = fabsf(acc[k]) <= 1e30f && wsum > 0.5f ? quotient(acc[k], wsum) : (wsum != 0.0f ? acc[k] / wsum : 0.0f);
 }
 
 __device__ __forceinline__ void working_xyz(const PixelParams& p, const float in[3], float xyz[3]) {
@@ -174,13 +200,14 @@ __device__ __forceinline__ void tc_exposure(const PixelParams& p, const float in
     const float Z = keep_finite(in_xyz[2]);
     const float sum = X + Y + Z;
     const float den = fmaxf(sum, 1e-10f);
-    const float tx = X / den;
-    const float ty = Y / den;
+    const bool quick = fmaxf(fmaxf(fabsf(X), fabsf(Y)), den) <= 1e30f; // den >= 1e-10
+    const float tx = quick ? quotient(X, den) : X / den;
+    const float ty = quick ? quotient(Y, den) : Y / den;
     // triangle -> square mapping of chromaticity
     const float one_minus = 1.0f - tx;
     const float qden = fmaxf(one_minus, 1e-10f);
     const float qx = fminf(1.0f, fmaxf(0.0f, one_minus * one_minus));
-    const float qy = fminf(1.0f, fmaxf(0.0f, ty / qden));
+    const float qy = fminf(1.0f, fmaxf(0.0f, fabsf(ty) <= 1e30f && qden <= 1e30f ? quotient(ty, qden) : ty / qden));
     float rgb[3];
     tc_lut_sample(p.tc_lut, qx, qy, rgb);
     e_bgr[0] = keep_finite(sum * keep_finite(rgb[2]));
@@ -258,7 +285,7 @@ __device__ __forceinline__ void camera_linear_exposure(const PixelParams& p, con
 // strictly above the query" rule as the reference, so the chosen interval index is
 // identical for identical queries.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float log_exposure(float e) { return log10f(fmaxf(e, 0.0f) + 1e-10f); }
+__device__ __forceinline__ float log_exposure(float e) { return log10_any(fmaxf(e, 0.0f) + 1e-10f); }
 
 // First index i1 in [1, last] with xq < x[i1] (last + 1 when none): the reference's
 // binary search (src/Cuda/JuicerCudaDeviceHelpers.cuh:59-71).
@@ -276,38 +303,42 @@ static __device__ __noinline__ int curve_interval_search(const float* x, int las
     return i1;
 }
 
-__device__ __forceinline__ float curve_sample(const float* __restrict__ blob, const CurveRef& c, float logE,
-                                              float gamma) {
-    if (!isfinite(logE)) return nanf("");
+// Interval of xq on a strictly increasing axis (CurveRef::guess): the unique g with x[g] <= xq
+// < x[g + 1], for x[0] < xq < x[last], which is the interval the binary search selects. It
+// starts from the uniform grid's cell, or from the interval the cell begins in (a table
+// over twice as many cells as samples, for axes that are not near uniform), and steps: none
+// or one on the axes hosts prepare.
+__device__ __forceinline__ int curve_interval(const float* __restrict__ blob, const CurveRef& c, float xq, float& xa,
+                                              float& xb) {
     const float* x = blob + c.x;
-    const float* y = blob + c.y;
-    const int last = c.n - 1;
-    const float xq = logE * gamma;
+    int g = (int)((xq - c.x0) * c.inv_dx);
+    g = max(0, min(g, c.cells - 1));
+    if (c.guess == 2) g = reinterpret_cast<const unsigned short*>(blob + c.table)[g];
+    xa = x[g];
+    xb = x[g + 1];
+    while (xq < xa) {
+        --g;
+        xb = xa;
+        xa = x[g];
+    }
+    while (xq >= xb) {
+        ++g;
+        xa = xb;
+        xb = x[g + 1];
+    }
+    return g;
+}
+
+// Any other axis, as the reference samples it. Cold path, out of line.
+static __device__ __noinline__ float curve_sample_general(const float* __restrict__ x, const float* __restrict__ y, int n,
+                                                          float xq) {
+    const int last = n - 1;
     const float xmin = x[0];
     const float xmax = x[last];
     if (!(xmax >= xmin)) return y[0];
     if (xq <= xmin) return y[0];
     if (xq >= xmax) return y[last];
-    int i1 = last + 1;
-    bool found = false;
-    if (c.guess) {
-        // Strictly increasing, near-uniform abscissa: start from the uniform-grid cell
-        // and step to the unique i1 with x[i1-1] <= xq < x[i1] (the interval the
-        // reference's binary search selects). Two steps either way cover the spacing
-        // jitter the host admitted; otherwise fall through to the binary search.
-        int g = (int)((xq - c.x0) * c.inv_dx);
-        g = g < 0 ? 0 : (g > last - 1 ? last - 1 : g);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            if (g > 0 && xq < x[g]) --g;
-            if (g < last - 1 && xq >= x[g + 1]) ++g;
-        }
-        if (x[g] <= xq && xq < x[g + 1]) {
-            i1 = g + 1;
-            found = true;
-        }
-    }
-    if (!found) i1 = curve_interval_search(x, last, xq);
+    const int i1 = curve_interval_search(x, last, xq);
     if (i1 > last) return y[last];
     const int i0 = i1 - 1;
     const float x0 = x[i0], x1 = x[i1], y0 = y[i0], y1 = y[i1];
@@ -315,6 +346,20 @@ __device__ __forceinline__ float curve_sample(const float* __restrict__ blob, co
     if (!(den > 0.0f) || !isfinite(den)) return y0;
     const float t = (xq - x0) / den;
     return y0 + t * (y1 - y0);
+}
+
+__device__ __forceinline__ float curve_sample(const float* __restrict__ blob, const CurveRef& c, float logE,
+                                              float gamma) {
+    if (!isfinite(logE)) return nanf("");
+    const float xq = logE * gamma;
+    const float* y = blob + c.y;
+    if (!c.guess) return curve_sample_general(blob + c.x, y, c.n, xq);
+    if (xq <= c.x0) return y[0];
+    if (!(xq < c.x1)) return y[c.n - 1];
+    float xa, xb;
+    const int g = curve_interval(blob, c, xq, xa, xb);
+    const float y0 = y[g], y1 = y[g + 1];
+    return y0 + quotient(xq - xa, xb - xa) * (y1 - y0);
 }
 
 __device__ __forceinline__ float clamp_infinite_log(const float* __restrict__ blob, CurveRef c, float logE) {
@@ -351,10 +396,15 @@ static __device__ __noinline__ bool langmuir_guarded(float value, float knee, fl
 }
 
 __device__ __forceinline__ bool langmuir(float value, float knee, float ref, float& out) {
-    out = nanf("");
-    if (!isfinite(value) || !isfinite(knee) || !(knee > 0.0f) || !isfinite(ref)) return false;
     const float den = knee + value;
     const float kr = knee + ref;
+    // the ordinary range: everything finite, the quotient far from the pole
+    if (knee > 0.0f && fabsf(ref) <= 1e15f && fabsf(value) <= 1e15f && fabsf(den) >= 1e-15f && den <= 1e15f) {
+        out = quotient(value * kr, den);
+        return true;
+    }
+    out = nanf("");
+    if (!isfinite(value) || !isfinite(knee) || !(knee > 0.0f) || !isfinite(ref)) return false;
     const bool direct = isfinite(den) && den != 0.0f && isfinite(kr) &&
                         (value == 0.0f || fabsf(value) <= FLT_MAX / fabsf(kr));
     if (direct) {
@@ -490,14 +540,6 @@ __device__ __forceinline__ void develop_capture_spatial(const PixelParams& p, co
 // a8: enlarger print exposure + development (src/Cuda/JuicerCudaDeviceHelpers.cuh:860-1071)
 // The 81-wavelength coefficients are read straight from the constant bank.
 // ---------------------------------------------------------------------------
-// 2^x on the MUFU (ex2.approx.ftz.f32: relative error about 2^-22, flushes subnormal
-// results to zero; transmittances here are >= 2^-40, far above the subnormal range).
-__device__ __forceinline__ float mufu_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Non-finite density (a failed DIR pixel): the reference's per-sample NaN rule
 // (src/Cuda/JuicerCudaDeviceHelpers.cuh:856-864). Cold path, out of line.
 static __device__ __noinline__ void print_spectral_nonfinite(const PrintSpectral& s, const float d[3], float raw[3]) {
@@ -517,22 +559,22 @@ static __device__ __noinline__ void print_spectral_nonfinite(const PrintSpectral
 
 __device__ __forceinline__ void print_spectral(const PrintSpectral& s, const float d[3], float raw[3]) {
     if (isfinite(d[0]) && isfinite(d[1]) && isfinite(d[2])) {
-        // Fast path: all 81 slots unrolled, coefficients are constant-bank operands
-        // (one per instruction: the film base sits in the weights, fjb_params.h).
-        // Finite densities give finite exponents, so no NaN guard is needed; padded
-        // slots evaluate 2^0 * 0 = +0. Two partial sums per channel (even / odd
-        // wavelength) halve the dependent FMA chain.
-        float a0[3] = {0.0f, 0.0f, 0.0f}, a1[3] = {0.0f, 0.0f, 0.0f};
+        // Fast path: all slots unrolled, two wavelengths per packed instruction (even ones in
+        // the low half, so the halves are the two partial sums per channel that keep the
+        // dependent chains short). Finite densities give finite exponents, so no NaN guard is
+        // needed; padded slots add 2^0 * 0 = +0.
+        const Pair d0 = pack(d[0], d[0]), d1 = pack(d[1], d[1]), d2 = pack(d[2], d[2]);
+        Pair a[3] = {pack(0.0f, 0.0f), pack(0.0f, 0.0f), pack(0.0f, 0.0f)};
 #pragma unroll
-        for (int i = 0; i < kSpectralSamples; ++i) {
-            const float dl = fmaf(d[0], s.nd[i][0], fmaf(d[1], s.nd[i][1], d[2] * s.nd[i][2]));
-            const float t = mufu_exp2(dl);
-            float* a = (i & 1) ? a1 : a0;
-            a[0] = fmaf(t, s.sens[i][0], a[0]);
-            a[1] = fmaf(t, s.sens[i][1], a[1]);
-            a[2] = fmaf(t, s.sens[i][2], a[2]);
+        for (int i = 0; i < kSpectralPairs; ++i) {
+            const Pair* q = reinterpret_cast<const Pair*>(s.pairs[i]);
+            const float2 dl = unpack(fma2(d0, q[0], fma2(d1, q[1], mul2(d2, q[2]))));
+            const Pair t = pack(mufu_exp2(dl.x), mufu_exp2(dl.y));
+#pragma unroll
+            for (int c = 0; c < 3; ++c) a[c] = fma2(t, q[3 + c], a[c]);
         }
-        const float ac = a0[0] + a1[0], am = a0[1] + a1[1], ay = a0[2] + a1[2];
+        const float2 c2 = unpack(a[0]), m2 = unpack(a[1]), y2 = unpack(a[2]);
+        const float ac = c2.x + c2.y, am = m2.x + m2.y, ay = y2.x + y2.y;
         raw[0] = ac;
         raw[1] = am;
         raw[2] = ay;
@@ -558,7 +600,7 @@ __device__ __forceinline__ void print_finish(const PixelParams& p, const float* 
     for (int c = 0; c < 3; ++c) raw[c] *= p.print_exposure;
     for (int c = 0; c < 3; ++c) raw[c] *= p.print_route_correction;
     for (int c = 0; c < 3; ++c) {
-        const float lp = log10f(raw[c] + 1e-10f);
+        const float lp = log10_any(raw[c] + 1e-10f);
         d[c] = curve_sample(blob, p.print_curve[c], lp, 1.0f);
     }
 }
@@ -676,29 +718,32 @@ __device__ __constant__ const float kOkLabToLmsRoot[9] = {1.0f, 0.3963377774f,  
                                                           1.0f, -0.1055613458f, -0.0638541728f,
                                                           1.0f, -0.0894841775f, -1.2914855480f};
 
-__device__ __forceinline__ float signed_cbrt(float v) { return v < 0.0f ? -cbrtf(-v) : cbrtf(v); }
-
+// v above the knee's start: start + span n / (1 + n^p)^(1/p), n = (v - start) / span
 __device__ __forceinline__ float reinhard_knee(float v, const float knee[3]) {
     if (!(v > knee[0])) return v;
     const float span = knee[1] - knee[0];
-    const float nrm = (v - knee[0]) / span;
-    return knee[0] + span * nrm / powf(1.0f + powf(nrm, knee[2]), 1.0f / knee[2]);
+    const float nrm = divides(span) && v <= 1e30f ? quotient(v - knee[0], span) : (v - knee[0]) / span;
+    const float den = powf(1.0f + powf(nrm, knee[2]), 1.0f / knee[2]);
+    return knee[0] + (divides(den) && nrm <= 1e28f ? quotient(span * nrm, den) : span * nrm / den);
 }
 
 __device__ __forceinline__ float gamut_boundary(const float* __restrict__ cmax, float L, float h) {
     const float kPi = 3.14159265358979323846f;
     const float kTwoPi = 2.0f * kPi;
     const float Lc = fminf(fmaxf(L, 0.02f), 1.0f);
-    const float lp = (Lc - 0.02f) / (1.0f - 0.02f) * (float)(kGamutLightness - 1);
-    const int l0 = (int)floorf(lp);
+    const float lp = (Lc - 0.02f) * ((float)(kGamutLightness - 1) / (1.0f - 0.02f));
+    const int l0 = min((int)floorf(lp), kGamutLightness - 1);
     const int l1 = l0 + 1 < kGamutLightness ? l0 + 1 : l0;
     const float lf = lp - (float)l0;
-    float wh = fmodf(h + kPi, kTwoPi);
-    if (wh < 0.0f) wh += kTwoPi;
-    const float hp = wh / kTwoPi * (float)kGamutHue;
-    const int h0 = (int)floorf(hp) % kGamutHue;
-    const int h1 = (h0 + 1) % kGamutHue;
-    const float hf = hp - floorf(hp);
+    // h + pi lies in [0, 2 pi]
+    float wh = h + kPi;
+    if (wh >= kTwoPi) wh -= kTwoPi;
+    const float hp = fmaxf(wh, 0.0f) * ((float)kGamutHue / kTwoPi);
+    const float hb = floorf(hp);
+    int h0 = (int)hb;
+    if (h0 >= kGamutHue) h0 -= kGamutHue;
+    const int h1 = h0 + 1 < kGamutHue ? h0 + 1 : 0;
+    const float hf = hp - hb;
     const int r0 = l0 * kGamutHue, r1 = l1 * kGamutHue;
     const float c00 = __ldg(cmax + r0 + h0), c01 = __ldg(cmax + r0 + h1);
     const float c10 = __ldg(cmax + r1 + h0), c11 = __ldg(cmax + r1 + h1);
@@ -711,17 +756,21 @@ __device__ __forceinline__ void gamut_compress(const PixelParams& p, float rgb[3
     float xyz[3], lms[3], lab[3];
     mat3_apply(p.gamut_native_to_xyz, rgb, xyz);
     mat3_apply(kOkXyzToLms, xyz, lms);
-    for (int c = 0; c < 3; ++c) lms[c] = signed_cbrt(lms[c]);
+    for (int c = 0; c < 3; ++c) lms[c] = cube_root(lms[c]);
     mat3_apply(kOkLmsRootToLab, lms, lab);
     lab[0] = reinhard_knee(lab[0], p.gamut_lightness_knee);
-    const float chroma = hypotf(lab[1], lab[2]);
-    if (chroma > 0.0f) {
-        const float hue = atan2f(lab[2], lab[1]);
-        const float bound = fmaxf(gamut_boundary(p.gamut_cmax, lab[0], hue), 1.0e-9f);
-        const float comp = reinhard_knee(chroma / bound, p.gamut_chroma_knee) * bound;
-        const float sc = comp / chroma;
-        lab[1] *= sc;
-        lab[2] *= sc;
+    // a chroma below 1e-15 has no direction to speak of and lies inside any boundary; the
+    // roots above are below 1e13
+    const float square = fmaf(lab[1], lab[1], lab[2] * lab[2]);
+    if (square >= 1e-30f) {
+        const float chroma = root(square);
+        const float bound = fmaxf(gamut_boundary(p.gamut_cmax, lab[0], angle(lab[2], lab[1])), 1.0e-9f);
+        const float ratio = quotient(chroma, bound);
+        if (ratio > p.gamut_chroma_knee[0]) {
+            const float sc = quotient(reinhard_knee(ratio, p.gamut_chroma_knee) * bound, chroma);
+            lab[1] *= sc;
+            lab[2] *= sc;
+        }
     }
     mat3_apply(kOkLabToLmsRoot, lab, lms);
     for (int c = 0; c < 3; ++c) lms[c] = lms[c] * lms[c] * lms[c];
@@ -743,7 +792,8 @@ static __device__ __noinline__ float encode_channel_other(const PixelParams& p, 
 __device__ __forceinline__ float encode_channel(const PixelParams& p, float v) {
     if (p.cctf_kind == 2) {
         if (v <= 0.0031308f) return 12.92f * v;
-        return 1.055f * powf(v, 1.0f / 2.4f) - 0.055f;
+        // what lies above 2 encodes above 1, which the output clamps to 1 (a NaN stays one)
+        return 1.055f * pow_5_12(v >= 2.0f ? 2.0f : v) - 0.055f;
     }
     return encode_channel_other(p, v);
 }

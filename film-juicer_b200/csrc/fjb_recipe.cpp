@@ -44,23 +44,57 @@ cudaError_t upload(T** dst, const void* src, size_t bytes, cudaStream_t stream) 
     return cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, stream);
 }
 
-// Enables the uniform-grid interval guess for a curve whose abscissa is strictly
-// increasing with every step within 25 % of the mean step (then the guessed cell is
-// at most one off and two correction steps always land on the exact interval).
-void set_curve_guess(const std::vector<float>& blob, CurveRef& c) {
+// Floats of staged curves up to which lookup tables are added (48 KB: four blocks of the pixel
+// kernels share an SM; ordinary recipes hold 10 to 18 KB).
+constexpr int kMaxTabledBlob = 12288;
+
+// Where a lookup starts on the curve's axis, if that is strictly increasing: the uniform
+// grid's cell (every step within 25 % of the mean step), or else a table over twice as many
+// cells as samples, appended to the blob (the DIR couplers' compensated axes: spacings 0.17 to
+// 1.3 of the mean, for which the lookup was an eight-step search). Curves that share an axis
+// share the table.
+void set_curve_guess(std::vector<float>& blob, CurveRef& c, std::vector<CurveRef>& done) {
     c.guess = 0;
-    if (c.n < 2) return;
+    if (c.n < 2 || c.n > 65535) return;
+    for (const CurveRef& d : done)
+        if (d.x == c.x && d.n == c.n) {
+            const int y = c.y;
+            c = d;
+            c.y = y;
+            return;
+        }
     const float* x = blob.data() + c.x;
     const double span = (double)x[c.n - 1] - (double)x[0];
     if (!(span > 0.0) || !std::isfinite(span)) return;
     const double mean = span / (c.n - 1);
+    bool uniform = true;
     for (int i = 0; i + 1 < c.n; ++i) {
         const double d = (double)x[i + 1] - (double)x[i];
-        if (!(d > 0.0) || std::fabs(d - mean) > 0.25 * mean) return;
+        if (!(d > 1e-20) || !(d < 1e20)) return; // in the range of the device's quotient
+        uniform &= std::fabs(d - mean) <= 0.25 * mean;
     }
     c.x0 = x[0];
-    c.inv_dx = (float)((c.n - 1) / span);
-    c.guess = 1;
+    c.x1 = x[c.n - 1];
+    c.cells = uniform ? c.n - 1 : 2 * c.n;
+    c.inv_dx = (float)(c.cells / span);
+    c.guess = uniform ? 1 : 2;
+    if (!uniform) {
+        std::vector<float> table((c.cells + 1) / 2);
+        if (blob.size() + table.size() > (size_t)kMaxTabledBlob) {
+            c.guess = 0;
+            return;
+        }
+        unsigned short* t = reinterpret_cast<unsigned short*>(table.data());
+        int g = 0;
+        for (int i = 0; i < c.cells; ++i) {
+            const double start = (double)x[0] + span * i / c.cells;
+            while (g + 2 < c.n && (double)x[g + 1] <= start) ++g;
+            t[i] = (unsigned short)g;
+        }
+        c.table = (int)blob.size();
+        blob.insert(blob.end(), table.begin(), table.end());
+    }
+    done.push_back(c);
 }
 
 } // namespace
@@ -364,10 +398,20 @@ bool create_recipe(const FjPreparedHostData& h, cudaStream_t stream, Recipe& r, 
                 p.spectral.nd[l][3] = -INFINITY;
                 p.spectral.sens[l][0] = p.spectral.sens[l][1] = p.spectral.sens[l][2] = 0.0f;
             }
+            for (int i = 0; i < kSpectralPairs; ++i) {
+                const int l = 2 * i, m = l + 1;
+                for (int c = 0; c < 3; ++c) {
+                    p.spectral.pairs[i][c] =
+                        make_float2(p.spectral.nd[l][c], m < kSpectralSamples ? p.spectral.nd[m][c] : 0.0f);
+                    p.spectral.pairs[i][3 + c] =
+                        make_float2(p.spectral.sens[l][c], m < kSpectralSamples ? p.spectral.sens[m][c] : 0.0f);
+                }
+            }
         }
+        std::vector<CurveRef> done;
         for (CurveRef* c : {&p.film_curve[0], &p.film_curve[1], &p.film_curve[2], &p.dir_curve[0], &p.dir_curve[1],
                             &p.dir_curve[2], &p.print_curve[0], &p.print_curve[1], &p.print_curve[2]})
-            set_curve_guess(blob, *c);
+            set_curve_guess(blob, *c, done);
         while (blob.size() % 4) blob.push_back(0.0f);
         if ((e = upload(&r.curves, blob.data(), blob.size() * 4, stream)) != cudaSuccess) goto cuda_fail;
         p.curve_blob = r.curves;
