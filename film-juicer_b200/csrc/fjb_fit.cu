@@ -325,8 +325,7 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
     }
     double nd[3];
     for (int c = 0; c < 3; ++c)
-        nd[c] = p.scan_medium_negative ? ((double)scanD[c] + (double)p.scan_min_cmy[c]) * (double)p.scan_inv_span_cmy[c]
-                                       : ((double)scanD[c] - (double)p.scan_min_cmy[c]) * (double)p.scan_inv_span_cmy[c];
+        nd[c] = ((double)scanD[c] + p.scan_shift[c]) * p.scan_span[c];
     float l2[3], dl2[3][3];
     if constexpr (kGrad) {
         if (!scan_lut_sample_d(p, nd, l2, dl2)) return false;
@@ -336,17 +335,15 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
     double xyz[3] = {(double)exp2f(l2[0]), (double)exp2f(l2[1]), (double)exp2f(l2[2])};
     double xc[3] = {xyz[0], xyz[1], xyz[2]}, sc = 1.0, dsc = 0.0;
     if (p.correction_active) {
-        const double t = (double)p.correction_slope * xyz[1] + (double)p.correction_offset;
+        const double t = p.correction_slope * xyz[1] + p.correction_offset;
         const double cy = fmin(fmax(t, 0.0), 1.0);
         const double den = xyz[1] + 1e-10;
         sc = cy / den;
-        const double dcy = (t > 0.0 && t < 1.0) ? (double)p.correction_slope : 0.0;
+        const double dcy = (t > 0.0 && t < 1.0) ? p.correction_slope : 0.0;
         dsc = (dcy * den - cy) / (den * den);
         for (int c = 0; c < 3; ++c) xc[c] = xyz[c] * sc;
     }
-    double ad[3];
-    mat3_apply_d(p.cat02, xc, ad);
-    mat3_apply_d(p.xyz_to_rgb, ad, rgb);
+    mat3_apply_d(p.xyz_to_native, xc, rgb);
     if (!isfinite(rgb[0]) || !isfinite(rgb[1]) || !isfinite(rgb[2])) return false;
     if constexpr (!kGrad) return true;
 

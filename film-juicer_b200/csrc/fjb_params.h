@@ -42,23 +42,27 @@ struct CurveRef {
     int table;    // offset of the table: per cell (u16) the last sample at or below its start
 };
 
-// Print 81-lambda coefficients, pre-folded on the host:
-//   nd[l]   = (-(eps_c, eps_m, eps_y) * log2(10), 0)     (so T = 2^(D . nd))
-//   sens[l] = (sens_c, sens_m, sens_y) * filtered illuminant * 10^-base
+// Print 81-lambda coefficients, pre-folded on the host, by pairs of wavelengths (2 i, 2 i + 1)
+// for the packed form: pairs[i][0..2] = -(eps_c, eps_m, eps_y) * log2(10) (so T = 2^(D . nd)),
+// pairs[i][3..5] = (sens_c, sens_m, sens_y) * filtered illuminant * 10^-base
 // (the film base's transmittance is the same at every pixel, so it sits in the
-// weights and the per-pixel exponent has the three dye terms only; nd[l][3] stays 0).
+// weights and the per-pixel exponent has the three dye terms only).
 // Wavelengths whose three sensitivities are all NaN, or whose dye or base density or
 // illuminant is NaN, are dropped and the remaining ones packed first; the unused tail
-// slots hold (0, 0, 0, -inf) and zero sensitivities, so they contribute exactly +0 for
-// finite densities. A NaN channel of a kept wavelength contributes zero.
+// slots hold zeros, so they contribute exactly +0 for finite densities. A NaN channel of a
+// kept wavelength contributes zero.
 constexpr int kSpectralPairs = (kSpectralSamples + 1) / 2;
 struct PrintSpectral {
-    float nd[kSpectralSamples][4];
-    float sens[kSpectralSamples][3];
-    int count;
-    // the same by pairs of wavelengths (2 i, 2 i + 1), for the packed form: the three exponents'
-    // factors, then the three weights; the last one's second half is padding (weight 0)
     float2 pairs[kSpectralPairs][6];
+    int count;
+
+    // slot l's exponent factor (k = 0..2) or weight (k = 3..5)
+    __host__ __device__ __forceinline__ float at(int l, int k) const {
+        return (l & 1) ? pairs[l >> 1][k].y : pairs[l >> 1][k].x;
+    }
+    __host__ __forceinline__ void set(int l, int k, float v) {
+        ((l & 1) ? pairs[l >> 1][k].y : pairs[l >> 1][k].x) = v;
+    }
 };
 
 struct PixelParams {
@@ -149,14 +153,18 @@ struct PixelParams {
 
     // ---- scanner ----
     int scan_medium_negative;
-    float scan_min_cmy[3];
     float scan_inv_span_cmy[3];
+    // normalized density = (d + shift) * span in FP64. The scanner's and the output's FP64
+    // factors are stored as such: converting them at each pixel took a fifth of the print/scan
+    // kernel's conversion and transcendental unit.
+    double scan_shift[3];
+    double scan_span[3];
     int scan_res;
     const float4* scan_nodes; // [(c*r+m)*r+y][3 outputs] of (value, slope_c, slope_m, slope_y)
     const float4* scan_cells; // [(c*s+m)*s+y][2] of (min xyz, max x), (max y, max z, 0, 0)
     int correction_active;
-    float correction_slope;
-    float correction_offset;
+    double correction_slope;
+    double correction_offset;
     // scanner post effects: glare percent plane added in XYZ (may be null), the scan
     // illuminant it is scaled by, and linear output-RGB planes written instead of the
     // encoded pixels when the stage stops before encoding
@@ -183,15 +191,16 @@ struct PixelParams {
     // ---- output colour ----
     float cat02[9];
     float xyz_to_rgb[9];
+    double xyz_to_native[9]; // xyz_to_rgb cat02
     int gamut_active;
     const float* gamut_cmax; // [64][720]
-    float gamut_native_to_xyz[9];
-    float gamut_xyz_to_native[9];
+    float gamut_native_to_lms[9]; // native RGB to OkLab's cone responses
+    float gamut_lms_to_native[9];
     float gamut_lightness_knee[3];
     float gamut_chroma_knee[3];
     int encode_input_is_output;
     int encode_apply_cctf;
-    float encode_dwg_to_output[9];
+    double encode_dwg_to_output[9];
     int cctf_kind;
     float cctf_gamma, cctf_a, cctf_b, cctf_c, cctf_d, cctf_linear_cutoff;
 

@@ -28,10 +28,10 @@ __device__ __forceinline__ void mat3_apply(const float m[9], const float v[3], f
     o[2] = m[6] * v[0] + m[7] * v[1] + m[8] * v[2];
 }
 
-__device__ __forceinline__ void mat3_apply_d(const float m[9], const double v[3], double o[3]) {
-    o[0] = (double)m[0] * v[0] + (double)m[1] * v[1] + (double)m[2] * v[2];
-    o[1] = (double)m[3] * v[0] + (double)m[4] * v[1] + (double)m[5] * v[2];
-    o[2] = (double)m[6] * v[0] + (double)m[7] * v[1] + (double)m[8] * v[2];
+__device__ __forceinline__ void mat3_apply_d(const double m[9], const double v[3], double o[3]) {
+    o[0] = m[0] * v[0] + m[1] * v[1] + m[2] * v[2];
+    o[1] = m[3] * v[0] + m[4] * v[1] + m[5] * v[2];
+    o[2] = m[6] * v[0] + m[7] * v[1] + m[8] * v[2];
 }
 
 // ---------------------------------------------------------------------------
@@ -545,12 +545,12 @@ __device__ __forceinline__ void develop_capture_spatial(const PixelParams& p, co
 static __device__ __noinline__ void print_spectral_nonfinite(const PrintSpectral& s, const float d[3], float raw[3]) {
     float ac = 0.0f, am = 0.0f, ay = 0.0f;
     for (int i = 0; i < s.count; ++i) {
-        const float dl = d[0] * s.nd[i][0] + d[1] * s.nd[i][1] + d[2] * s.nd[i][2] + s.nd[i][3];
+        const float dl = d[0] * s.at(i, 0) + d[1] * s.at(i, 1) + d[2] * s.at(i, 2);
         float t = exp2f(dl);
         t = isnan(t) ? 0.0f : t;
-        ac += t * s.sens[i][0];
-        am += t * s.sens[i][1];
-        ay += t * s.sens[i][2];
+        ac += t * s.at(i, 3);
+        am += t * s.at(i, 4);
+        ay += t * s.at(i, 5);
     }
     raw[0] = ac;
     raw[1] = am;
@@ -705,12 +705,6 @@ __device__ __forceinline__ bool scan_lut_sample(const PixelParams& p, const doub
 // ---------------------------------------------------------------------------
 // a11: OkLch output gamut compression (src/GamutCompression.h:110-216)
 // ---------------------------------------------------------------------------
-__device__ __constant__ const float kOkXyzToLms[9] = {0.8189330101f, 0.3618667424f, -0.1288597137f,
-                                                      0.0329845436f, 0.9293118715f, 0.0361456387f,
-                                                      0.0482003018f, 0.2643662691f, 0.6338517070f};
-__device__ __constant__ const float kOkLmsToXyz[9] = {1.2270138511f,  -0.5577999807f, 0.2812561490f,
-                                                      -0.0405801784f, 1.1122568696f,  -0.0716766787f,
-                                                      -0.0763812845f, -0.4214819784f, 1.5861632204f};
 __device__ __constant__ const float kOkLmsRootToLab[9] = {0.2104542553f, 0.7936177850f,  -0.0040720468f,
                                                           1.9779984951f, -2.4285922050f, 0.4505937099f,
                                                           0.0259040371f, 0.7827717662f,  -0.8086757660f};
@@ -753,9 +747,8 @@ __device__ __forceinline__ float gamut_boundary(const float* __restrict__ cmax, 
 }
 
 __device__ __forceinline__ void gamut_compress(const PixelParams& p, float rgb[3]) {
-    float xyz[3], lms[3], lab[3];
-    mat3_apply(p.gamut_native_to_xyz, rgb, xyz);
-    mat3_apply(kOkXyzToLms, xyz, lms);
+    float lms[3], lab[3];
+    mat3_apply(p.gamut_native_to_lms, rgb, lms);
     for (int c = 0; c < 3; ++c) lms[c] = cube_root(lms[c]);
     mat3_apply(kOkLmsRootToLab, lms, lab);
     lab[0] = reinhard_knee(lab[0], p.gamut_lightness_knee);
@@ -774,8 +767,7 @@ __device__ __forceinline__ void gamut_compress(const PixelParams& p, float rgb[3
     }
     mat3_apply(kOkLabToLmsRoot, lab, lms);
     for (int c = 0; c < 3; ++c) lms[c] = lms[c] * lms[c] * lms[c];
-    mat3_apply(kOkLmsToXyz, lms, xyz);
-    mat3_apply(p.gamut_xyz_to_native, xyz, rgb);
+    mat3_apply(p.gamut_lms_to_native, lms, rgb);
 }
 
 // ---------------------------------------------------------------------------
@@ -824,21 +816,18 @@ static __device__ __noinline__ float encode_channel_other(const PixelParams& p, 
     }
 }
 
-__device__ __forceinline__ void encode_output(const PixelParams& p, double rgb[3]) {
-    double lin[3];
-    if (p.encode_input_is_output) {
-        lin[0] = rgb[0];
-        lin[1] = rgb[1];
-        lin[2] = rgb[2];
-    } else {
-        mat3_apply_d(p.encode_dwg_to_output, rgb, lin);
-    }
+__device__ __forceinline__ void encode_output(const PixelParams& p, const double rgb[3], float out[3]) {
+    double lin[3] = {rgb[0], rgb[1], rgb[2]};
+    if (!p.encode_input_is_output) mat3_apply_d(p.encode_dwg_to_output, rgb, lin);
     if (p.encode_apply_cctf) {
-        for (int c = 0; c < 3; ++c) rgb[c] = encode_channel(p, (float)lin[c]);
+        // the encoded value is FP32: clamping it there is the same
+        for (int c = 0; c < 3; ++c) {
+            const float v = encode_channel(p, (float)lin[c]);
+            out[c] = v <= 0.0f ? 0.0f : (v >= 1.0f ? 1.0f : v);
+        }
     } else {
-        for (int c = 0; c < 3; ++c) rgb[c] = lin[c];
+        for (int c = 0; c < 3; ++c) out[c] = (float)clamp01(lin[c]);
     }
-    for (int c = 0; c < 3; ++c) rgb[c] = clamp01(rgb[c]);
 }
 
 // ---------------------------------------------------------------------------
@@ -852,13 +841,7 @@ __device__ __forceinline__ void encode_output(const PixelParams& p, double rgb[3
 __device__ __forceinline__ bool scan_to_linear(const PixelParams& p, const float d[3], double rgb[3],
                                                float glare_percent = -1.0f, const float* dust = nullptr) {
     double nd[3];
-    for (int c = 0; c < 3; ++c) {
-        if (p.scan_medium_negative) {
-            nd[c] = ((double)d[c] + (double)p.scan_min_cmy[c]) * (double)p.scan_inv_span_cmy[c];
-        } else {
-            nd[c] = ((double)d[c] - (double)p.scan_min_cmy[c]) * (double)p.scan_inv_span_cmy[c];
-        }
-    }
+    for (int c = 0; c < 3; ++c) nd[c] = ((double)d[c] + p.scan_shift[c]) * p.scan_span[c];
     float l2[3];
     if (!scan_lut_sample(p, nd, l2)) return false;
     double xyz[3] = {(double)exp2f(l2[0]), (double)exp2f(l2[1]), (double)exp2f(l2[2])};
@@ -869,7 +852,7 @@ __device__ __forceinline__ bool scan_to_linear(const PixelParams& p, const float
         xyz[2] *= t;
     }
     if (p.correction_active) {
-        const double cy = fmin(fmax((double)p.correction_slope * xyz[1] + (double)p.correction_offset, 0.0), 1.0);
+        const double cy = fmin(fmax(p.correction_slope * xyz[1] + p.correction_offset, 0.0), 1.0);
         const double sc = cy / (xyz[1] + 1e-10);
         xyz[0] *= sc;
         xyz[1] *= sc;
@@ -882,9 +865,7 @@ __device__ __forceinline__ bool scan_to_linear(const PixelParams& p, const float
         xyz[1] += glare * (double)p.scan_illuminant_xyz[1];
         xyz[2] += glare * (double)p.scan_illuminant_xyz[2];
     }
-    double ad[3];
-    mat3_apply_d(p.cat02, xyz, ad);
-    mat3_apply_d(p.xyz_to_rgb, ad, rgb);
+    mat3_apply_d(p.xyz_to_native, xyz, rgb);
     if (!isfinite(rgb[0]) || !isfinite(rgb[1]) || !isfinite(rgb[2])) return false;
     if (p.gamut_active) {
         float f[3] = {(float)rgb[0], (float)rgb[1], (float)rgb[2]};

@@ -3,16 +3,16 @@
 //
 // Reference: print_spectral_integrate_device (src/Cuda/JuicerCudaDeviceHelpers.cuh:866-935)
 //   D(l) = sum_c d_c eps_c(l) + base(l),  T(l) = 10^-D(l) I_filt(l),  raw_c = sum_l T(l) S_c(l).
-// The recipe folds it into nd(l) = -(eps_c, eps_m, eps_y)(l) log2(10), nd3(l) = 0 and
-// sens(l) = S(l) I_filt(l) 10^-base(l) (fjb_params.h), so T(l) = 2^(d . nd(l) + nd3(l))
-// and raw_c = sum_l T(l) sens_c(l); nd3 is -inf on the padded wavelengths.
+// The recipe folds it into nd(l) = -(eps_c, eps_m, eps_y)(l) log2(10) and
+// sens(l) = S(l) I_filt(l) 10^-base(l) (fjb_params.h), so T(l) = 2^(d . nd(l))
+// and raw_c = sum_l T(l) sens_c(l).
 //
 // One persistent CTA of 128 threads takes tiles of 128 consecutive pixels (one per
 // thread, one TMEM lane per pixel):
 //   GEMM1  D1[128 x 96] = A1[128 x 16] B1[96 x 16]^T  (M = pixels, N = wavelengths
 //          padded 81 -> 96, K = 16). A1 row = (d_hi[3], d_lo[3], d_hi[3], 1, 1, 0...),
-//          B1 row = (nd_hi[3], nd_hi[3], nd_lo[3], nd3_hi, nd3_lo, 0...): BF16 hi + lo
-//          pairs of both sides, so d . nd + nd3 is carried to about 2^-17 relative
+//          B1 row = (nd_hi[3], nd_hi[3], nd_lo[3], 0...): BF16 hi + lo
+//          pairs of both sides, so d . nd is carried to about 2^-17 relative
 //          (only d_lo nd_lo is dropped), accumulated in FP32 in TMEM.
 //   exp2   per pixel and wavelength in FP32 on the MUFU, read from TMEM with
 //          tcgen05.ld; T rounded to BF16 (kPrintTensor) or to a BF16 pair hi + lo
@@ -167,7 +167,6 @@ __device__ __forceinline__ void write_a1(unsigned char* a1, int tid, const float
             a[3 + c] = lo;
             a[6 + c] = hi;
         }
-        a[9] = a[10] = __float2bfloat16_rn(1.0f);
     }
     *reinterpret_cast<uint4*>(a1 + kmajor(tid, 0, kTcK1)) = *reinterpret_cast<const uint4*>(a);
     *reinterpret_cast<uint4*>(a1 + kmajor(tid, 8, kTcK1)) = *reinterpret_cast<const uint4*>(a + 8);
@@ -202,7 +201,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) print_raw_tc_kernel(const __gri
     const uint32_t bar1[2] = {smem_addr(bars), smem_addr(bars + 1)};
     const uint32_t bar2[2] = {smem_addr(bars + 2), smem_addr(bars + 3)};
 
-    // B1: per wavelength (nd_hi[3], nd_hi[3], nd_lo[3], nd3_hi, nd3_lo, 0 x 5)
+    // B1: per wavelength (nd_hi[3], nd_hi[3], nd_lo[3], 0 x 7)
     const int count = p.spectral.count;
     for (int l = tid; l < kTcLambda; l += kTcThreads) {
         __nv_bfloat16 row[kTcK1];
@@ -210,12 +209,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) print_raw_tc_kernel(const __gri
         if (l < count) {
             for (int c = 0; c < 3; ++c) {
                 __nv_bfloat16 hi, lo;
-                split_bf16(p.spectral.nd[l][c], hi, lo);
+                split_bf16(p.spectral.at(l, c), hi, lo);
                 row[c] = hi;
                 row[3 + c] = hi;
                 row[6 + c] = lo;
             }
-            split_bf16(p.spectral.nd[l][3], row[9], row[10]);
         }
         for (int k = 0; k < kTcK1; ++k)
             *reinterpret_cast<__nv_bfloat16*>(tc_smem + kOffB1 + kmajor(l, k, kTcK1)) = row[k];
@@ -226,7 +224,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) print_raw_tc_kernel(const __gri
         __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
         if (n < 6 && l < count) {
             __nv_bfloat16 hi, lo;
-            split_bf16(p.spectral.sens[l][n % 3], hi, lo);
+            split_bf16(p.spectral.at(l, 3 + n % 3), hi, lo);
             v = n < 3 ? hi : lo;
         }
         *reinterpret_cast<__nv_bfloat16*>(tc_smem + kOffB2 + kmajor(n, l, kTcLambda)) = v;

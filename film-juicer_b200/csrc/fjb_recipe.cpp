@@ -44,6 +44,23 @@ cudaError_t upload(T** dst, const void* src, size_t bytes, cudaStream_t stream) 
     return cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, stream);
 }
 
+// OkLab: D65 XYZ to cone responses and back (src/GamutCompression.h:110-216)
+constexpr float kOkXyzToLms[9] = {0.8189330101f, 0.3618667424f, -0.1288597137f, 0.0329845436f, 0.9293118715f,
+                                  0.0361456387f, 0.0482003018f, 0.2643662691f,  0.6338517070f};
+constexpr float kOkLmsToXyz[9] = {1.2270138511f,  -0.5577999807f, 0.2812561490f,  -0.0405801784f, 1.1122568696f,
+                                  -0.0716766787f, -0.0763812845f, -0.4214819784f, 1.5861632204f};
+
+// a b in FP64, row major
+template <typename T>
+void matrix_product(const float* a, const float* b, T* out) {
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j) {
+            double s = 0.0;
+            for (int k = 0; k < 3; ++k) s += (double)a[3 * i + k] * (double)b[3 * k + j];
+            out[3 * i + j] = (T)s;
+        }
+}
+
 // Floats of staged curves up to which lookup tables are added (48 KB: four blocks of the pixel
 // kernels share an SM; ordinary recipes hold 10 to 18 KB).
 constexpr int kMaxTabledBlob = 12288;
@@ -381,32 +398,19 @@ bool create_recipe(const FjPreparedHostData& h, cudaStream_t stream, Recipe& r, 
                 if (std::isnan(eps[0]) || std::isnan(eps[1]) || std::isnan(eps[2]) ||
                     std::isnan(pr.film_base_density.data[l]) || std::isnan(il))
                     continue;
-                for (int c = 0; c < 3; ++c) p.spectral.nd[count][c] = -(pr.film_density_cmy.data[l * 3 + c] * kLog2Of10);
+                for (int c = 0; c < 3; ++c) p.spectral.set(count, c, -(pr.film_density_cmy.data[l * 3 + c] * kLog2Of10));
                 // the film base transmits the same 2^nd3 at every pixel: it is folded into
                 // the wavelength's weights, so the per-pixel exponent is d . nd alone
                 const float nd3 = -(pr.film_base_density.data[l] * kLog2Of10);
                 const double base_t = std::exp2((double)nd3);
-                p.spectral.nd[count][3] = 0.0f;
                 for (int c = 0; c < 3; ++c)
-                    p.spectral.sens[count][c] =
-                        (std::isnan(s[c]) || std::isnan(il)) ? 0.0f : (float)((double)s[c] * (double)il * base_t);
+                    p.spectral.set(count, 3 + c,
+                                   (std::isnan(s[c]) || std::isnan(il)) ? 0.0f : (float)((double)s[c] * (double)il * base_t));
                 ++count;
             }
             p.spectral.count = count;
-            for (int l = count; l < kSpectralSamples; ++l) {
-                p.spectral.nd[l][0] = p.spectral.nd[l][1] = p.spectral.nd[l][2] = 0.0f;
-                p.spectral.nd[l][3] = -INFINITY;
-                p.spectral.sens[l][0] = p.spectral.sens[l][1] = p.spectral.sens[l][2] = 0.0f;
-            }
-            for (int i = 0; i < kSpectralPairs; ++i) {
-                const int l = 2 * i, m = l + 1;
-                for (int c = 0; c < 3; ++c) {
-                    p.spectral.pairs[i][c] =
-                        make_float2(p.spectral.nd[l][c], m < kSpectralSamples ? p.spectral.nd[m][c] : 0.0f);
-                    p.spectral.pairs[i][3 + c] =
-                        make_float2(p.spectral.sens[l][c], m < kSpectralSamples ? p.spectral.sens[m][c] : 0.0f);
-                }
-            }
+            for (int l = count; l < 2 * kSpectralPairs; ++l)
+                for (int k = 0; k < 6; ++k) p.spectral.set(l, k, 0.0f);
         }
         std::vector<CurveRef> done;
         for (CurveRef* c : {&p.film_curve[0], &p.film_curve[1], &p.film_curve[2], &p.dir_curve[0], &p.dir_curve[1],
@@ -423,8 +427,9 @@ bool create_recipe(const FjPreparedHostData& h, cudaStream_t stream, Recipe& r, 
         const FjDensityBounds& b = h.scanner_bounds;
         p.scan_medium_negative = print ? 0 : 1;
         for (int c = 0; c < 3; ++c) {
-            p.scan_min_cmy[c] = print ? b.min_cmy[c] : -b.min_cmy[c];
             p.scan_inv_span_cmy[c] = b.inv_span_cmy[c];
+            p.scan_shift[c] = -(double)b.min_cmy[c];
+            p.scan_span[c] = b.inv_span_cmy[c];
         }
         const FjScannerSpectra& sp = h.scanner_spectra;
         const int res = (int)h.scanner_lut.resolution;
@@ -446,7 +451,7 @@ bool create_recipe(const FjPreparedHostData& h, cudaStream_t stream, Recipe& r, 
         ls.k = kSpectralSamples;
         ls.inv_yn = sp.inverse_y_normalization;
         for (int c = 0; c < 3; ++c) {
-            ls.range_min_cmy[c] = p.scan_min_cmy[c];
+            ls.range_min_cmy[c] = print ? b.min_cmy[c] : -b.min_cmy[c];
             ls.inverse_span_cmy[c] = p.scan_inv_span_cmy[c];
         }
         ls.medium = print ? 1 : 0;
@@ -480,6 +485,7 @@ bool create_recipe(const FjPreparedHostData& h, cudaStream_t stream, Recipe& r, 
         std::memcpy(p.cat02, oc.cat02, sizeof(p.cat02));
         std::memcpy(p.scan_illuminant_xyz, oc.illuminant_xyz, sizeof(p.scan_illuminant_xyz));
         std::memcpy(p.xyz_to_rgb, oc.xyz_to_rgb, sizeof(p.xyz_to_rgb));
+        matrix_product(oc.xyz_to_rgb, oc.cat02, p.xyz_to_native);
         p.gamut_active = (oc.flags & FJ_COLOR_GAMUT_COMPRESSION) ? 1 : 0;
         if (p.gamut_active) {
             if (!span_ok(oc.gamut_cmax, (size_t)kGamutLightness * kGamutHue)) {
@@ -490,13 +496,13 @@ bool create_recipe(const FjPreparedHostData& h, cudaStream_t stream, Recipe& r, 
                 goto cuda_fail;
         }
         p.gamut_cmax = r.gamut_cmax;
-        std::memcpy(p.gamut_native_to_xyz, oc.native_rgb_to_d65_xyz, sizeof(p.gamut_native_to_xyz));
-        std::memcpy(p.gamut_xyz_to_native, oc.d65_xyz_to_native_rgb, sizeof(p.gamut_xyz_to_native));
+        matrix_product(kOkXyzToLms, oc.native_rgb_to_d65_xyz, p.gamut_native_to_lms);
+        matrix_product(oc.d65_xyz_to_native_rgb, kOkLmsToXyz, p.gamut_lms_to_native);
         std::memcpy(p.gamut_lightness_knee, oc.lightness_knee, sizeof(p.gamut_lightness_knee));
         std::memcpy(p.gamut_chroma_knee, oc.chroma_knee, sizeof(p.gamut_chroma_knee));
         p.encode_input_is_output = (oc.flags & FJ_COLOR_INPUT_IS_OUTPUT_SPACE) ? 1 : 0;
         p.encode_apply_cctf = (oc.flags & FJ_COLOR_ENCODE_CCTF) ? 1 : 0;
-        std::memcpy(p.encode_dwg_to_output, oc.encoding.dwg_to_output, sizeof(p.encode_dwg_to_output));
+        for (int c = 0; c < 9; ++c) p.encode_dwg_to_output[c] = oc.encoding.dwg_to_output[c];
         p.cctf_kind = (int)oc.encoding.cctf_kind;
         p.cctf_gamma = oc.encoding.gamma;
         p.cctf_a = oc.encoding.a;
