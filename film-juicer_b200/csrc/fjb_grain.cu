@@ -27,6 +27,7 @@
 // reconstruction in one pass) and taps passed as kernel parameters.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "fjb_grain.h"
@@ -85,136 +86,207 @@ __device__ __forceinline__ uint32_t hash_u32(int x, int y, uint64_t seed, uint64
     return (uint32_t)(h & 0xFFFFFFFFu);
 }
 
-__device__ __forceinline__ float value_noise(float cx, float cy, uint64_t seed) {
-    const int ix = (int)floorf(cx), iy = (int)floorf(cy);
-    const float fx = cx - (float)ix, fy = cy - (float)iy;
-    const float sx = smoothstep(fx), sy = smoothstep(fy);
-    const float v00 = spatial_hash01(ix, iy, seed);
-    const float v10 = spatial_hash01(ix + 1, iy, seed);
-    const float v01 = spatial_hash01(ix, iy + 1, seed);
-    const float v11 = spatial_hash01(ix + 1, iy + 1, seed);
-    const float v0 = __fmaf_rn(v10 - v00, sx, v00);
-    const float v1 = __fmaf_rn(v11 - v01, sx, v01);
-    return __fmaf_rn(v1 - v0, sy, v0);
+// A coordinate of a value-noise lattice: the cell and the smoothed position in it.
+struct NoiseAxis {
+    int i;
+    float s;
+};
+__device__ __forceinline__ NoiseAxis noise_axis(float c) {
+    const int i = (int)floorf(c);
+    return {i, smoothstep(c - (float)i)};
+}
+
+// Value noise between the corners of a cell.
+template <typename Corner>
+__device__ __forceinline__ float value_noise(const NoiseAxis& x, const NoiseAxis& y, Corner corner) {
+    const float v00 = corner(x.i, y.i);
+    const float v10 = corner(x.i + 1, y.i);
+    const float v01 = corner(x.i, y.i + 1);
+    const float v11 = corner(x.i + 1, y.i + 1);
+    const float v0 = __fmaf_rn(v10 - v00, x.s, v00);
+    const float v1 = __fmaf_rn(v11 - v01, x.s, v01);
+    return __fmaf_rn(v1 - v0, y.s, v0);
 }
 
 constexpr uint32_t kPhiloxGlobalSeed = 0xAAAAAAAAu;
 
-struct GrainRng {
-    Philox philox;
-    const GrainFrame* f;
-    uint64_t abs_x, abs_y, seed;
-    uint32_t draw;
-    int use_stbn, off_x, off_y;
-    int64_t pitch_offset;
-    size_t frame_row_base;
-    const uint8_t* frame_base; // the blue-noise frame's first row
-    int mask_w, mask_h;
+// What a block of the sample kernel prepares for its pixels.
+//
+// The kernel is bound by integer instruction issue, and most of it was the same for many
+// pixels: the blue-noise offsets of draw d hash the pass's seed and d alone; a blue-noise
+// uniform has 256 values, so the normal's radius and cosine do too; Wang cells and noise
+// lattice cells cover many pixels; coordinates (divisions and 64-bit conversions) depend on
+// the column or the row. The block evaluates each once, with the functions the pixels would
+// call, so the results keep their bits. 3840x2160, one pass of three sublayers: 2880 -> 1190
+// instructions per warp of pixels, 857 -> 459 us. What is left waits on the scattered
+// blue-noise bytes (the Wang shift differs from pixel to pixel) as much as on issue.
+constexpr int kSampleColumns = 32, kSampleRows = 8;
+constexpr int kSampleThreads = kSampleColumns * kSampleRows;
+static_assert(kSampleThreads == 256, "one thread per value of a noise byte and sample of the axis");
+constexpr int kBlockRows = 8 * kSampleRows; // rows of pixels of a tile, at most
+constexpr int kTableDraws = 32; // a Poisson count of a mean below 10 draws rarely more
+constexpr int kWangCells = kSampleThreads;
+constexpr int kSampleBlocks = 3; // per SM (2: 586 us; 4, in 64 registers: 495; 3: 459)
 
-    __device__ GrainRng(const GrainFrame* frame, uint64_t s, uint64_t ax, uint64_t ay, int stbn, int frame_offset,
-                        int wang_x, int wang_y)
-        : philox(s, (uint32_t)ax, kPhiloxGlobalSeed, (uint32_t)ay), f(frame), abs_x(ax), abs_y(ay), seed(s),
-          draw(0), use_stbn(stbn), off_x(wang_x), off_y(wang_y), pitch_offset(0), frame_row_base(0),
-          frame_base(nullptr), mask_w(-1), mask_h(-1) {
-        if (!use_stbn) return;
-        if ((f->stbn_w & (f->stbn_w - 1)) == 0 && (f->stbn_h & (f->stbn_h - 1)) == 0) {
-            mask_w = f->stbn_w - 1;
-            mask_h = f->stbn_h - 1;
-        }
-        if (f->pitch_px > 0) pitch_offset = (int64_t)f->pitch_px * (f->frame_index + (int64_t)frame_offset);
-        const int wf = wrap_coordinate((int64_t)f->stbn_frame + (int64_t)frame_offset, f->stbn_frames);
-        frame_row_base = (size_t)wf * (size_t)f->stbn_h;
-        frame_base = f->stbn + frame_row_base * (size_t)f->stbn_w;
-    }
+// Value-noise fields and the coordinates they are read at: breathing at its small and its
+// large cells with two seeds each, and the two uniforms of the clump normal.
+constexpr int kNoiseCoords = 4; // breathing small, breathing large, clump, clump (shifted)
+constexpr int kNoiseFields = 6; // small a, b, large a, b, clump, clump (shifted)
+__host__ __device__ constexpr int noise_coord(int field) { return field < 4 ? field >> 1 : field - 2; }
+constexpr int kLattice = 192; // corners held of a field: cells are at least 4 pixels wide
 
-    // The blue-noise uniform of draw d (its table address depends on d alone).
-    __device__ __forceinline__ float stbn_at(uint32_t d) const {
-        const uint64_t h = splitmix64(seed + (uint64_t)d * 0x9E3779B97F4A7C15ULL);
-        const int ox = (int)(h & 0xFFFFu) + off_x;
-        const int oy = (int)((h >> 16) & 0xFFFFu) + off_y;
-        if (mask_w >= 0) {
-            // power-of-two table: the masked coordinate keeps only low bits of the
-            // 64-bit sum, which the 32-bit sum of the addends' low words already has
-            const uint32_t xm = ((uint32_t)abs_x + (uint32_t)ox + (uint32_t)f->stbn_offset_x) & (uint32_t)mask_w;
-            const uint32_t ym =
-                ((uint32_t)abs_y + (uint32_t)oy + (uint32_t)f->stbn_offset_y + (uint32_t)pitch_offset) & (uint32_t)mask_h;
-            const uint8_t v = __ldg(frame_base + ((size_t)ym * (size_t)(uint32_t)f->stbn_w + xm));
-            return ((float)v + 0.5f) * (1.0f / 256.0f);
-        }
-        const int64_t xc = (int64_t)abs_x + (int64_t)ox + (int64_t)f->stbn_offset_x;
-        const int64_t yc = (int64_t)abs_y + (int64_t)oy + (int64_t)f->stbn_offset_y + pitch_offset;
-        const int x = wrap_coordinate(xc, f->stbn_w);
-        const int y = wrap_coordinate(yc, f->stbn_h);
-        const uint8_t v = __ldg(f->stbn + ((frame_row_base + (size_t)y) * (size_t)f->stbn_w + (size_t)x));
-        return ((float)v + 0.5f) * (1.0f / 256.0f);
-    }
+struct NoiseField {
+    uint64_t seed;
+    int x0, y0, nx, ny; // lattice corners held (nx 0: none)
+};
 
-    __device__ __forceinline__ float uniform() {
-        if (use_stbn) return stbn_at(draw++);
-        // u01: x * 2^-32 + 2^-33 (the product is exact, so the fma is too)
-        return __fmaf_rn((float)philox.next(), 1.0f / 4294967296.0f, 0.5f / 4294967296.0f);
-    }
+struct WangRow {
+    int cell, near, far; // row of cells held, rows of the tile
+};
 
-    __device__ __forceinline__ float normal() {
-        float u1 = uniform();
-        u1 = clamp01(u1, 1e-7f, 1.0f);
-        const float u2 = uniform();
-        const float r = sqrtf(-2.0f * logf(u1));
-        return r * cosf(kTwoPi * u2);
+struct GrainTables {
+    GrainFrameUniforms u;
+    uint32_t draws[2][3][kTableDraws]; // [frame, next frame][sublayer][draw]: low word of the hash
+    float radius[256], cosine[256];    // sqrt(-2 ln u), cos(2 pi u) of the noise byte's uniform u
+    float axis[256];                   // layer lookup axis, in lookup sign
+    const uint8_t* frame_base[2];      // the blue-noise frame's first row
+    size_t frame_row[2];
+    int64_t pitch_offset[2];
+    NoiseField field[kNoiseFields];
+    float lattice[kNoiseFields][kLattice];
+    NoiseAxis row[kNoiseCoords][kBlockRows];
+    int wang_tile[kWangCells];
+    WangRow wang_row[kBlockRows];
+    int64_t wang_x; // first column of cells
+    int wang_nx;    // columns held (0: none)
+};
+
+__device__ __forceinline__ uint32_t draw_hash(uint64_t seed, uint32_t d) {
+    return (uint32_t)splitmix64(seed + (uint64_t)d * 0x9E3779B97F4A7C15ULL);
+}
+
+// (v + 1/2) / 256, all steps exact
+__device__ __forceinline__ float noise_uniform(uint32_t v) {
+    return __uint_as_float(0x3f800000u + (v << 15)) - (1.0f - 0.5f / 256.0f);
+}
+
+// sqrt(-2 ln u1) and cos(2 pi u2) of the Box-Muller normal
+__device__ __forceinline__ float normal_radius(float u1) {
+    u1 = clamp01(u1, 1e-7f, 1.0f);
+    return sqrtf(-2.0f * logf(u1));
+}
+__device__ __forceinline__ float normal_cosine(float u2) { return cosf(kTwoPi * u2); }
+
+struct PixelContext {
+    uint64_t ax, ay;
+    int use_stbn, wang_x, wang_y;
+    float breathing, clump;
+    bool retime;
+    float time_alpha;
+};
+
+// Where a pass's blue-noise draws fall for a pixel: the table is a power of two on both sides,
+// so the masked coordinate keeps only low bits of the 64-bit sum, which the 32-bit sum of the
+// addends' low words already has.
+struct NoisePlace {
+    const uint8_t* frame; // its first row
+    uint32_t width, mask_x, mask_y, x, y;
+    __device__ __forceinline__ uint32_t byte(uint32_t h) const {
+        const uint32_t u = (x + (h & 0xFFFFu)) & mask_x, v = (y + (h >> 16)) & mask_y;
+        return __ldg(frame + ((size_t)v * (size_t)width + u));
     }
 };
 
+// The low word of the hash of draw d of the pass's `seed`. `draws`: its table, or null.
+__device__ __forceinline__ uint32_t draw_word(const uint32_t* draws, uint64_t seed, uint32_t d) {
+    return draws && d < (uint32_t)kTableDraws ? draws[d] : draw_hash(seed, d);
+}
+
 constexpr int kStbnBatch = 4;
 
-__device__ __forceinline__ int poisson(float lambda, GrainRng& rng) {
-    if (!finite(lambda) || !(lambda > 0.0f)) return 0;
-    if (lambda < 10.0f) {
-        const float L = expf(-lambda);
-        float p = 1.0f;
-        int k = 0;
-        if (rng.use_stbn) {
-            // The same draws in the same order, fetched kStbnBatch at a time: the
-            // blue-noise addresses do not depend on earlier draws, so the table loads
-            // overlap instead of paying one cache latency per draw. Draws fetched past
-            // the stop are not consumed (the draw index advances by the draws used).
-            while (p > L && k < 1024) {
-                float u[kStbnBatch];
+// Poisson count of a mean below 10: a product of uniforms. The draws are fetched kStbnBatch
+// at a time: the blue-noise addresses do not depend on earlier draws, so the table loads
+// overlap instead of paying one cache latency per draw.
+__device__ __forceinline__ int poisson_product(float lambda, const uint32_t* draws, uint64_t seed, const uint8_t* frame,
+                                            uint32_t width, uint32_t mask_x, uint32_t mask_y, uint32_t x, uint32_t y) {
+    const NoisePlace at{frame, width, mask_x, mask_y, x, y};
+    const float L = expf(-lambda);
+    float p = 1.0f;
+    int k = 0;
+    while (p > L && k < 1024) {
+        uint32_t v[kStbnBatch];
 #pragma unroll
-                for (int j = 0; j < kStbnBatch; ++j) u[j] = rng.stbn_at(rng.draw + (uint32_t)j);
-                uint32_t used = 0;
+        for (int j = 0; j < kStbnBatch; ++j) v[j] = at.byte(draw_word(draws, seed, (uint32_t)(k + j)));
+        int used = 0;
 #pragma unroll
-                for (int j = 0; j < kStbnBatch; ++j) {
-                    if (p > L && k < 1024) {
-                        ++k;
-                        ++used;
-                        p *= clamp01(u[j], 1e-7f, 1.0f);
-                    }
-                }
-                rng.draw += used;
+        for (int j = 0; j < kStbnBatch; ++j) {
+            if (p > L && k + used < 1024) {
+                ++used;
+                p *= noise_uniform(v[j]); // within the draws' clamp to [1e-7, 1]
             }
-            return k - 1;
         }
-        while (p > L && k < 1024) {
-            ++k;
-            p *= clamp01(rng.uniform(), 1e-7f, 1.0f);
-        }
-        return k - 1;
+        k += used;
     }
-    const float z = rng.normal();
+    return k - 1;
+}
+
+// Poisson count of a normal deviate z (means of 10 and more).
+__device__ __forceinline__ int poisson_normal(float lambda, float z) {
     float s = __fmaf_rn(sqrtf(lambda), z, lambda);
     if (!finite(s)) s = 0.0f;
     int k = (int)floorf(s + 0.5f);
     return k < 0 ? 0 : k;
 }
 
+// Poisson count with uniforms from `uniform`, lambda > 0.
+template <typename Uniform>
+__device__ __forceinline__ int poisson_stream(float lambda, Uniform uniform) {
+    if (lambda < 10.0f) {
+        const float L = expf(-lambda);
+        float p = 1.0f;
+        int k = 0;
+        while (p > L && k < 1024) {
+            ++k;
+            p *= clamp01(uniform(), 1e-7f, 1.0f);
+        }
+        return k - 1;
+    }
+    const float r = normal_radius(uniform());
+    return poisson_normal(lambda, r * normal_cosine(uniform()));
+}
+
+// The counter stream (no blue noise).
+__device__ __noinline__ int poisson_philox(float lambda, uint64_t seed, uint32_t ax, uint32_t ay) {
+    Philox philox(seed, ax, kPhiloxGlobalSeed, ay);
+    // u01: x * 2^-32 + 2^-33 (the product is exact, so the fma is too)
+    return poisson_stream(lambda, [&]() {
+        return __fmaf_rn((float)philox.next(), 1.0f / 4294967296.0f, 0.5f / 4294967296.0f);
+    });
+}
+
+// Blue-noise tables of other sizes.
+__device__ __noinline__ int poisson_wrapped(float lambda, uint64_t seed, const GrainFrame* f, const GrainTables* t,
+                                            int frame, uint64_t ax, uint64_t ay, int wang_x, int wang_y) {
+    uint32_t d = 0;
+    return poisson_stream(lambda, [&]() {
+        const uint32_t h = draw_hash(seed, d++);
+        const int ox = (int)(h & 0xFFFFu) + wang_x;
+        const int oy = (int)(h >> 16) + wang_y;
+        const int64_t xc = (int64_t)ax + (int64_t)ox + (int64_t)f->stbn_offset_x;
+        const int64_t yc = (int64_t)ay + (int64_t)oy + (int64_t)f->stbn_offset_y + t->pitch_offset[frame];
+        const int x = wrap_coordinate(xc, f->stbn_w);
+        const int y = wrap_coordinate(yc, f->stbn_h);
+        return noise_uniform(__ldg(f->stbn + ((t->frame_row[frame] + (size_t)y) * (size_t)f->stbn_w + (size_t)x)));
+    });
+}
+
 struct ParticleSample {
     float density, density_max, n_particles, od_particle, uniformity;
-    uint64_t seed;
-    int frame_offset;
 };
 
-__device__ __forceinline__ float particle_model(const GrainFrame* f, const ParticleSample& s, uint64_t ax,
-                                                uint64_t ay, int use_stbn, int wang_x, int wang_y) {
+// `slot`: the sublayer's place in the draw tables (beyond them the draws are hashed here).
+__device__ __forceinline__ float particle_model(const GrainFrame* f, const GrainTables* t, const ParticleSample& s,
+                                                const PixelContext& px, int slot, int frame, uint64_t seed) {
     float density = s.density;
     if (!finite(density) || density < 0.0f) density = 0.0f;
     float p = density / s.density_max;
@@ -222,24 +294,76 @@ __device__ __forceinline__ float particle_model(const GrainFrame* f, const Parti
     const float u = finite(s.uniformity) ? clamp01(s.uniformity, 0.0f, 1.0f) : 0.0f;
     float sat = __fmaf_rn(-(p * u), 1.0f - 1e-6f, 1.0f);
     if (!finite(sat) || sat <= 0.0f) sat = 1e-6f;
-    GrainRng rng(f, s.seed, ax, ay, use_stbn, s.frame_offset, wang_x, wang_y);
-    const float lambda = s.n_particles / sat;
-    const int count = poisson(lambda * p, rng);
+    const float lambda = s.n_particles / sat * p;
+    int count = 0;
+    if (finite(lambda) && lambda > 0.0f) {
+        const bool pow2 = (f->stbn_w & (f->stbn_w - 1)) == 0 && (f->stbn_h & (f->stbn_h - 1)) == 0;
+        if (!px.use_stbn) {
+            count = poisson_philox(lambda, seed, (uint32_t)px.ax, (uint32_t)px.ay);
+        } else if (!pow2) {
+            count = poisson_wrapped(lambda, seed, f, t, frame, px.ax, px.ay, px.wang_x, px.wang_y);
+        } else {
+            const uint32_t* draws = slot < 3 ? t->draws[frame][slot] : nullptr;
+            const NoisePlace at{t->frame_base[frame],
+                                (uint32_t)f->stbn_w,
+                                (uint32_t)f->stbn_w - 1,
+                                (uint32_t)f->stbn_h - 1,
+                                (uint32_t)px.ax + (uint32_t)px.wang_x + (uint32_t)f->stbn_offset_x,
+                                (uint32_t)px.ay + (uint32_t)px.wang_y + (uint32_t)f->stbn_offset_y +
+                                    (uint32_t)t->pitch_offset[frame]};
+            if (lambda < 10.0f) {
+                count = poisson_product(lambda, draws, seed, at.frame, at.width, at.mask_x, at.mask_y, at.x, at.y);
+            } else {
+                const uint32_t v1 = at.byte(draw_word(draws, seed, 0)), v2 = at.byte(draw_word(draws, seed, 1));
+                count = poisson_normal(lambda, t->radius[v1] * t->cosine[v2]);
+            }
+        }
+    }
     return sanitize((float)count * s.od_particle * sat);
 }
 
-__device__ __forceinline__ void wang_offsets(const GrainFrame* f, uint64_t ax, uint64_t ay, int& ox, int& oy) {
-    ox = 0;
-    oy = 0;
-    if (!f->wang_tiles || !f->wang_lut || f->wang_w <= 0 || f->wang_h <= 0 || f->wang_count <= 0) return;
-    if (!(f->pixel_size_um > 0.0f) || !(f->wang_cell_mm > 0.0f)) return;
-    const float xmm = (float)ax * (f->pixel_size_um * 0.001f);
-    const float ymm = (float)ay * (f->pixel_size_um * 0.001f);
+// Particle samples of one sublayer in this frame and the next, modulated and retimed.
+__device__ __forceinline__ float blend_frames(const PixelContext& px, float density, float g, float gn) {
+    g = __fmaf_rn((g - density) * px.breathing, px.clump, density);
+    if (px.retime) {
+        gn = __fmaf_rn((gn - density) * px.breathing, px.clump, density);
+        const float d0 = g - density, d1 = gn - density;
+        const float blend = __fmaf_rn(d1 - d0, px.time_alpha, d0);
+        const float w0 = 1.0f - px.time_alpha;
+        const float den = __fmaf_rn(w0, w0, px.time_alpha * px.time_alpha) + 1e-6f;
+        g = __fmaf_rn(blend, rsqrtf(den), density);
+    }
+    return g;
+}
+
+__device__ __forceinline__ bool wang_active(const GrainFrame* f) {
+    return f->wang_tiles && f->wang_lut && f->wang_w > 0 && f->wang_h > 0 && f->wang_count > 0 &&
+           f->pixel_size_um > 0.0f && f->wang_cell_mm > 0.0f && f->wang_colors > 0;
+}
+
+// A pixel coordinate in FP32 (rounded once either way).
+__device__ __forceinline__ float coordinate(uint64_t a) {
+    return (a >> 31) == 0 ? (float)(int)a : (float)a;
+}
+
+// Position of a pixel coordinate in Wang cells.
+__device__ __forceinline__ float wang_position(const GrainFrame* f, uint64_t a) {
+    const float mm = coordinate(a) * (f->pixel_size_um * 0.001f);
     const float inv = 1.0f / f->wang_cell_mm;
-    const float cx = xmm * inv, cy = ymm * inv;
-    const float fx = cx - floorf(cx), fy = cy - floorf(cy);
-    const int64_t mx = (int64_t)floorf(cx), my = (int64_t)floorf(cy);
-    if (f->wang_colors <= 0) return;
+    return mm * inv;
+}
+
+// Rows (or columns) of a tile of size n that position c reads: where it lies in its cell, and
+// half a tile on, wrapped.
+__device__ __forceinline__ void wang_samples(float c, int n, int& near, int& far) {
+    near = (int)floorf((c - floorf(c)) * (float)n);
+    if (near >= n) near = n - 1;
+    far = near + (n >> 1);
+    if (far >= n) far -= n;
+}
+
+// The tile of cell (mx, my): its edges' colours are hashes of the cells they separate.
+__device__ __forceinline__ int wang_tile(const GrainFrame* f, int64_t mx, int64_t my) {
     const int colors = f->wang_colors;
     const uint64_t s0 = f->clip_token != 0 ? f->clip_token : f->session_seed;
     const uint64_t base = s0 != 0 ? s0 : 1ULL;
@@ -248,20 +372,19 @@ __device__ __forceinline__ void wang_offsets(const GrainFrame* f, uint64_t ax, u
     const uint32_t t = hash_u32((int)mx, (int)my, base, 0xC3C3C3C3u) % colors;
     const uint32_t b = hash_u32((int)mx, (int)(my + 1), base, 0x3C3C3C3Cu) % colors;
     const size_t c = (size_t)colors;
-    const int tile = (int)f->wang_lut[(((size_t)l * c + r) * c + t) * c + b];
+    return (int)f->wang_lut[(((size_t)l * c + r) * c + t) * c + b];
+}
+
+// Shift of the blue-noise lookup by two samples of the pixel's tile (0 where there is none).
+__device__ __forceinline__ void wang_shift(const GrainFrame* f, int tile, int tx, int hx, int ty, int hy, int& ox,
+                                           int& oy) {
     const int w = f->wang_w, h = f->wang_h;
-    int tx = (int)floorf(fx * (float)w), ty = (int)floorf(fy * (float)h);
-    if (tx >= w) tx = w - 1;
-    if (ty >= h) ty = h - 1;
-    auto sample = [&](int x, int y) -> float {
-        if (tile < 0 || tile >= f->wang_count) return 0.0f;
-        x = x < 0 ? 0 : (x >= w ? w - 1 : x);
-        y = y < 0 ? 0 : (y >= h ? h - 1 : y);
-        const uint8_t v = f->wang_tiles[((size_t)tile * (size_t)h + (size_t)y) * (size_t)w + (size_t)x];
-        return ((float)v + 0.5f) * (1.0f / 256.0f);
-    };
-    const float v0 = sample(tx, ty);
-    const float v1 = sample((tx + (w >> 1)) % w, (ty + (h >> 1)) % h);
+    float v0 = 0.0f, v1 = 0.0f;
+    if (tile >= 0 && tile < f->wang_count) {
+        const uint8_t* t = f->wang_tiles + (size_t)tile * (size_t)h * (size_t)w;
+        v0 = noise_uniform(__ldg(t + ((size_t)ty * (size_t)w + tx)));
+        v1 = noise_uniform(__ldg(t + ((size_t)hy * (size_t)w + hx)));
+    }
     const int warp_x = f->stbn_w > 0 ? ((f->stbn_w / 8) > 4 ? f->stbn_w / 8 : 4) : 0;
     const int warp_y = f->stbn_h > 0 ? ((f->stbn_h / 8) > 4 ? f->stbn_h / 8 : 4) : 0;
     if (warp_x == 0 || warp_y == 0) return;
@@ -269,17 +392,50 @@ __device__ __forceinline__ void wang_offsets(const GrainFrame* f, uint64_t ax, u
     oy = (int)floorf((v1 - 0.5f) * 2.0f * (float)warp_y);
 }
 
-__device__ __forceinline__ float breathing_factor(const GrainFrame* f, const GrainFrameUniforms& u, uint64_t ax,
-                                                  uint64_t ay) {
+// The shift where the block holds no cells (negative or far coordinates).
+__device__ __noinline__ void wang_offsets(const GrainFrame* f, uint64_t ax, uint64_t ay, int& ox, int& oy) {
+    const float cx = wang_position(f, ax), cy = wang_position(f, ay);
+    int tx, hx, ty, hy;
+    wang_samples(cx, f->wang_w, tx, hx);
+    wang_samples(cy, f->wang_h, ty, hy);
+    wang_shift(f, wang_tile(f, (int64_t)floorf(cx), (int64_t)floorf(cy)), tx, hx, ty, hy, ox, oy);
+}
+
+// Coordinate `k` of the noise fields (kNoiseCoords) at column ax or row ay.
+__device__ __forceinline__ float noise_x(const GrainFrameUniforms& u, int k, uint64_t ax) {
+    if (k < 2) return (coordinate(ax) + u.breathing_drift_x) / (k == 0 ? u.breathing_cell_small_px : u.breathing_cell_large_px);
+    const float xs = coordinate(ax) / u.clump_cell_px;
+    return k == 2 ? xs : xs + 19.19f;
+}
+__device__ __forceinline__ float noise_y(const GrainFrameUniforms& u, int k, uint64_t ay) {
+    if (k < 2)
+        return (coordinate(ay) + u.breathing_drift_y + u.breathing_roll_y) /
+               (k == 0 ? u.breathing_cell_small_px : u.breathing_cell_large_px);
+    const float ys = (coordinate(ay) + u.clump_roll_y) / u.clump_cell_px;
+    return k == 2 ? ys : ys + 7.23f;
+}
+__device__ __forceinline__ uint64_t noise_seed(const GrainFrameUniforms& u, int field) {
+    const uint64_t seed = field >= 4 ? u.clump_static_seed : (field & 1) ? u.breathing_seed_b : u.breathing_seed_a;
+    return seed ^ (field == 2 || field == 3 || field == 5 ? 0xBF58476D1CE4E5B9ULL : 0x9E3779B97F4A7C15ULL);
+}
+
+__device__ __forceinline__ float field_noise(const GrainTables& t, int field, const NoiseAxis& x, const NoiseAxis& y) {
+    const NoiseField& q = t.field[field];
+    if (q.nx > 0) {
+        const float* v = t.lattice[field] + ((y.i - q.y0) * q.nx + (x.i - q.x0));
+        return value_noise(x, y, [&](int i, int j) { return v[(j - y.i) * q.nx + (i - x.i)]; });
+    }
+    return value_noise(x, y, [&](int i, int j) { return spatial_hash01(i, j, q.seed); });
+}
+
+__device__ __forceinline__ float breathing_factor(const GrainFrame* f, const GrainFrameUniforms& u,
+                                                  const GrainTables& t, const NoiseAxis x[kNoiseCoords],
+                                                  const NoiseAxis y[kNoiseCoords]) {
     if (!u.breathing_active) return 1.0f;
-    const float bx = (float)ax + u.breathing_drift_x;
-    const float by = (float)ay + u.breathing_drift_y + u.breathing_roll_y;
-    const float xs = bx / u.breathing_cell_small_px, ys = by / u.breathing_cell_small_px;
-    const float xl = bx / u.breathing_cell_large_px, yl = by / u.breathing_cell_large_px;
-    const float sa = value_noise(xs, ys, u.breathing_seed_a ^ 0x9E3779B97F4A7C15ULL);
-    const float sb = value_noise(xs, ys, u.breathing_seed_b ^ 0x9E3779B97F4A7C15ULL);
-    const float la = value_noise(xl, yl, u.breathing_seed_a ^ 0xBF58476D1CE4E5B9ULL);
-    const float lb = value_noise(xl, yl, u.breathing_seed_b ^ 0xBF58476D1CE4E5B9ULL);
+    const float sa = field_noise(t, 0, x[0], y[0]);
+    const float sb = field_noise(t, 1, x[0], y[0]);
+    const float la = field_noise(t, 2, x[1], y[1]);
+    const float lb = field_noise(t, 3, x[1], y[1]);
     const float ns = __fmaf_rn(sb - sa, u.breathing_t, sa);
     const float nl = __fmaf_rn(lb - la, u.breathing_t, la);
     const float noise = __fmaf_rn(u.breathing_mix, ns, (1.0f - u.breathing_mix) * nl);
@@ -288,13 +444,11 @@ __device__ __forceinline__ float breathing_factor(const GrainFrame* f, const Gra
     return factor > 0.0f ? factor : 0.0f;
 }
 
-__device__ __forceinline__ float clump_factor(const GrainFrameUniforms& u, uint64_t ax, uint64_t ay) {
+__device__ __forceinline__ float clump_factor(const GrainFrameUniforms& u, const GrainTables& t,
+                                              const NoiseAxis x[kNoiseCoords], const NoiseAxis y[kNoiseCoords]) {
     if (!u.clump_active) return 1.0f;
-    const float bx = (float)ax;
-    const float by = (float)ay + u.clump_roll_y;
-    const float xs = bx / u.clump_cell_px, ys = by / u.clump_cell_px;
-    const float a = value_noise(xs, ys, u.clump_static_seed ^ 0x9E3779B97F4A7C15ULL);
-    const float b = value_noise(xs + 19.19f, ys + 7.23f, u.clump_static_seed ^ 0xBF58476D1CE4E5B9ULL);
+    const float a = field_noise(t, 4, x[2], y[2]);
+    const float b = field_noise(t, 5, x[3], y[3]);
     const float u1 = clamp01(a, 1e-6f, 1.0f - 1e-6f);
     const float u2 = clamp01(b, 0.0f, 1.0f);
     const float r = sqrtf(-2.0f * logf(u1));
@@ -306,15 +460,31 @@ __device__ __forceinline__ float clump_factor(const GrainFrameUniforms& u, uint6
 
 // Density of one sublayer at the given total density: linear interpolation of the
 // layer curve over the capture density curve (negated for positive film), with the
-// 16-block prefix-maximum search for finite 256-sample axes.
-__device__ float layer_density(const GrainFrame* f, int ch, int layer, float density) {
+// 16-block prefix-maximum search for finite 256-sample axes (on a rising axis a binary search
+// finds the same sample). The place on the axis is the same for all layers.
+struct LayerPlace {
+    int i0;  // sample, or -1: the density itself
+    float t; // position to the next sample; below 0: the sample's value
+};
+
+__device__ __forceinline__ LayerPlace layer_place(const GrainFrame* f, const float* rising, int ch, float density) {
     const float* x = f->base_curve[ch];
-    const float* y = f->layer_curve[layer][ch];
     const int n = f->base_curve_n[ch];
-    if (!x || !y || n <= 0) return density;
-    if (!finite(density)) return __ldg(y);
+    if (!x || n <= 0) return {-1, 0.0f};
+    if (!finite(density)) return {0, -1.0f};
     const bool pos = f->positive_film != 0;
     const float q = pos ? -density : density;
+    if (rising) { // 256 finite samples
+        if (q <= rising[0]) return {0, -1.0f};
+        if (q >= rising[255]) return {255, -1.0f};
+        int lo = 0; // rising[lo] < q
+#pragma unroll
+        for (int step = 128; step > 0; step >>= 1)
+            if (lo + step < 256 && rising[lo + step] < q) lo += step;
+        const float den = rising[lo + 1] - rising[lo];
+        if (!(den > 0.0f) || !finite(den)) return {lo, -1.0f};
+        return {lo, (q - rising[lo]) / den};
+    }
     auto axis = [&](int i) {
         const float v = __ldg(x + i);
         return pos ? -v : v;
@@ -323,13 +493,13 @@ __device__ float layer_density(const GrainFrame* f, int ch, int layer, float den
     int b0 = 0, b1 = n - 1;
     if (!bounded) {
         while (b0 < n && !finite(axis(b0))) ++b0;
-        if (b0 >= n) return density;
+        if (b0 >= n) return {-1, 0.0f};
         while (b1 > b0 && !finite(axis(b1))) --b1;
     }
     const float xmin = axis(b0), xmax = axis(b1);
-    if (!finite(xmin) || !finite(xmax) || !(xmax >= xmin)) return __ldg(y + b0);
-    if (q <= xmin) return __ldg(y + b0);
-    if (q >= xmax) return __ldg(y + b1);
+    if (!finite(xmin) || !finite(xmax) || !(xmax >= xmin)) return {b0, -1.0f};
+    if (q <= xmin) return {b0, -1.0f};
+    if (q >= xmax) return {b1, -1.0f};
     int i1 = b0 + 1;
     if (bounded) {
         const float* prefix = f->axis_block_prefix_max[ch];
@@ -348,131 +518,228 @@ __device__ float layer_density(const GrainFrame* f, int ch, int layer, float den
     } else {
         while (i1 <= b1 && axis(i1) < q) ++i1;
     }
-    if (i1 > b1) return __ldg(y + b1);
+    if (i1 > b1) return {b1, -1.0f};
     const int i0 = i1 - 1;
     const float x0 = axis(i0), x1v = axis(i1);
-    const float y0 = __ldg(y + i0), y1 = __ldg(y + i1);
     const float den = x1v - x0;
-    if (!(den > 0.0f) || !finite(den)) return y0;
-    const float t = (q - x0) / den;
-    return __fmaf_rn(t, y1 - y0, y0);
+    if (!(den > 0.0f) || !finite(den)) return {i0, -1.0f};
+    return {i0, (q - x0) / den};
 }
 
-struct PixelContext {
-    uint64_t ax, ay;
-    int use_stbn, wang_x, wang_y;
-    float breathing, clump;
-    bool retime;
-    float time_alpha;
-};
-
-// One layer's particle sample with the breathing/clump modulation and retiming.
-__device__ __forceinline__ float modulated_sample(const GrainFrame* f, const PixelContext& px, ParticleSample s,
-                                                  uint64_t seed_next) {
-    const float density = s.density;
-    float g = particle_model(f, s, px.ax, px.ay, px.use_stbn, px.wang_x, px.wang_y);
-    float gn = 0.0f;
-    if (px.retime) {
-        s.seed = seed_next;
-        s.frame_offset = 1;
-        gn = particle_model(f, s, px.ax, px.ay, px.use_stbn, px.wang_x, px.wang_y);
-    }
-    g = __fmaf_rn((g - density) * px.breathing, px.clump, density);
-    if (px.retime) {
-        gn = __fmaf_rn((gn - density) * px.breathing, px.clump, density);
-        const float d0 = g - density, d1 = gn - density;
-        const float blend = __fmaf_rn(d1 - d0, px.time_alpha, d0);
-        const float w0 = 1.0f - px.time_alpha;
-        const float den = __fmaf_rn(w0, w0, px.time_alpha * px.time_alpha) + 1e-6f;
-        g = __fmaf_rn(blend, rsqrtf(den), density);
-    }
-    return g;
+__device__ __forceinline__ float layer_density(const GrainFrame* f, int ch, int layer, const LayerPlace& at,
+                                               float density) {
+    const float* y = f->layer_curve[layer][ch];
+    if (!y || at.i0 < 0) return density;
+    const float y0 = __ldg(y + at.i0);
+    if (!(at.t >= 0.0f)) return y0;
+    return __fmaf_rn(at.t, __ldg(y + at.i0 + 1) - y0, y0);
 }
 
+// The tables that hold for the whole pass; returns whether tables.axis holds a rising axis.
 template <int Mode>
-__global__ void __launch_bounds__(256) grain_sample_kernel(const __grid_constant__ GrainFrame f, int ch, int layer,
-                                                           const float* __restrict__ density_in, long long din_stride,
-                                                           GrainPlane out, GrainSampleEpilogue ep, int width,
-                                                           int height) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= width || y >= height) return;
-    const GrainFrameUniforms u = *f.uniforms;
-    const float in_density = density_in[(long long)y * din_stride + x];
+__device__ __forceinline__ bool prepare_pass(const GrainFrame& f, GrainTables& tables, int ch, bool use_stbn,
+                                             bool retime) {
+    const int tid = threadIdx.x;
+    if (tid == 0) tables.u = *f.uniforms;
+    if (use_stbn) {
+        if (tid < (retime ? 6 : 3) * kTableDraws) {
+            const int frame = tid / (3 * kTableDraws), slot = tid / kTableDraws % 3, d = tid % kTableDraws;
+            const uint64_t salt = (uint64_t)ch + (uint64_t)slot * 10ULL;
+            tables.draws[frame][slot][d] = draw_hash((frame ? f.seed_base_next : f.seed_base) ^ salt, (uint32_t)d);
+        }
+        tables.radius[tid] = normal_radius(noise_uniform((uint32_t)tid));
+        tables.cosine[tid] = normal_cosine(noise_uniform((uint32_t)tid));
+        if (tid < 2) {
+            tables.pitch_offset[tid] = f.pitch_px > 0 ? (int64_t)f.pitch_px * (f.frame_index + (int64_t)tid) : 0;
+            const int wf = wrap_coordinate((int64_t)f.stbn_frame + (int64_t)tid, f.stbn_frames);
+            tables.frame_row[tid] = (size_t)wf * (size_t)f.stbn_h;
+            tables.frame_base[tid] = f.stbn + tables.frame_row[tid] * (size_t)f.stbn_w;
+        }
+    }
+    bool rising = false;
+    if constexpr (Mode != kGrainSimple) {
+        rising = f.base_curve[ch] && f.base_curve_n[ch] == 256 && f.axis_finite[ch] != 0;
+        if (rising) {
+            const float v = __ldg(f.base_curve[ch] + tid);
+            tables.axis[tid] = f.positive_film != 0 ? -v : v;
+        }
+    }
+    __syncthreads();
+    if constexpr (Mode != kGrainSimple) {
+        if (rising) {
+            bool ok = finite(tables.axis[tid]) && (tid == 0 || tables.axis[tid - 1] <= tables.axis[tid]);
+            if (tid < 16) ok = ok && f.axis_block_prefix_max[ch][tid] == tables.axis[16 * tid + 15];
+            rising = __syncthreads_and(ok) != 0;
+        }
+    }
+    return rising;
+}
+
+// The tables of a tile: rows y0 .. y1 - 1, columns x0 .. x1 - 1. One warp per noise field, one
+// for the Wang cells; the rows' coordinates by the first four.
+__device__ __forceinline__ void prepare_tile(const GrainFrame& f, GrainTables& tables, bool use_stbn, int x0, int x1,
+                                             int y0, int y1) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const GrainFrameUniforms& u = tables.u;
+    const int64_t ax = (int64_t)f.origin_x + x0, ay = (int64_t)f.origin_y + y0;
+    const int64_t bx = (int64_t)f.origin_x + x1 - 1, by = (int64_t)f.origin_y + y1 - 1;
+    // coordinates are unsigned 64-bit: a tile that holds negative ones is not in order
+    const bool ordered = ax >= 0 && ay >= 0;
+    static_assert(kSampleThreads >= 32 * (kNoiseFields + 1) && kNoiseCoords * kBlockRows <= kSampleThreads,
+                  "a warp per noise field, one for the Wang cells");
+    if (warp < kNoiseFields) {
+        const int field = warp;
+        if (field < 4 ? u.breathing_active : u.clump_active) {
+            const int k = noise_coord(field);
+            const uint64_t seed = noise_seed(u, field);
+            NoiseField q{seed, 0, 0, 0, 0};
+            if (ordered) {
+                const float px = noise_x(u, k, (uint64_t)ax), py = noise_y(u, k, (uint64_t)ay);
+                const float qx = noise_x(u, k, (uint64_t)bx), qy = noise_y(u, k, (uint64_t)by);
+                if (fabsf(px) < 1e9f && fabsf(py) < 1e9f && qx - px < (float)kLattice && qy - py < (float)kLattice) {
+                    q.x0 = (int)floorf(px);
+                    q.y0 = (int)floorf(py);
+                    q.nx = (int)floorf(qx) - q.x0 + 2;
+                    q.ny = (int)floorf(qy) - q.y0 + 2;
+                    if (q.nx < 2 || q.ny < 2 || q.nx * q.ny > kLattice) q.nx = 0;
+                }
+            }
+            for (int i = lane; i < q.nx * q.ny; i += 32)
+                tables.lattice[field][i] = spatial_hash01(q.x0 + i % q.nx, q.y0 + i / q.nx, seed);
+            if (lane == 0) tables.field[field] = q;
+        }
+    } else if (warp == kNoiseFields && use_stbn && wang_active(&f)) {
+        int64_t mx = 0, my = 0;
+        int nx = 0, ny = 0;
+        if (ordered) {
+            const float px = wang_position(&f, (uint64_t)ax), py = wang_position(&f, (uint64_t)ay);
+            const float qx = wang_position(&f, (uint64_t)bx), qy = wang_position(&f, (uint64_t)by);
+            if (qx < 1e9f && qy < 1e9f && qx - px < (float)kWangCells && qy - py < (float)kWangCells) {
+                mx = (int64_t)floorf(px);
+                my = (int64_t)floorf(py);
+                nx = (int)((int64_t)floorf(qx) - mx) + 1;
+                ny = (int)((int64_t)floorf(qy) - my) + 1;
+                if (nx < 1 || ny < 1 || nx * ny > kWangCells) nx = ny = 0;
+            }
+        }
+        for (int i = lane; i < nx * ny; i += 32) tables.wang_tile[i] = wang_tile(&f, mx + i % nx, my + i / nx);
+        for (int i = lane; nx > 0 && i < y1 - y0; i += 32) {
+            const float cy = wang_position(&f, (uint64_t)(ay + i));
+            WangRow r;
+            r.cell = ((int)floorf(cy) - (int)my) * nx;
+            wang_samples(cy, f.wang_h, r.near, r.far);
+            tables.wang_row[i] = r;
+        }
+        if (lane == 0) {
+            tables.wang_x = mx;
+            tables.wang_nx = nx;
+        }
+    }
+    if (tid < kNoiseCoords * kBlockRows) {
+        const int k = tid / kBlockRows, r = tid % kBlockRows;
+        if (r < y1 - y0 && (k < 2 ? u.breathing_active : u.clump_active))
+            tables.row[k][r] = noise_axis(noise_y(u, k, (uint64_t)(ay + r)));
+    }
+}
+
+// The grid's blocks walk tiles of kSampleColumns x `rows` pixels, `columns` tiles to a row.
+template <int Mode>
+__global__ void __launch_bounds__(kSampleThreads, kSampleBlocks)
+    grain_sample_kernel(const __grid_constant__ GrainFrame f, int ch, int layer, const float* __restrict__ density_in,
+                        long long din_stride, GrainPlane out, GrainSampleEpilogue ep, int width, int height, int rows,
+                        int columns, int tiles) {
+    __shared__ GrainTables tables;
+    const int lane = threadIdx.x % kSampleColumns, line = threadIdx.x / kSampleColumns;
     PixelContext px;
-    px.ax = (uint64_t)((int64_t)f.origin_x + x);
-    px.ay = (uint64_t)((int64_t)f.origin_y + y);
     px.time_alpha = f.time_alpha;
     px.retime = f.time_alpha > 1e-6f && f.time_alpha < 0.999999f;
     px.use_stbn = (f.stbn && f.stbn_w > 0 && f.stbn_h > 0 && f.stbn_frames > 0) ? 1 : 0;
-    px.wang_x = px.wang_y = 0;
-    px.clump = clump_factor(u, px.ax, px.ay);
-    if (px.use_stbn) wang_offsets(&f, px.ax, px.ay, px.wang_x, px.wang_y);
-    px.breathing = breathing_factor(&f, u, px.ax, px.ay);
-
-    float value;
-    if (Mode == kGrainSimple) {
-        const float density = in_density + f.density_min[ch];
-        const int nsub = f.n_sublayers > 0 ? f.n_sublayers : 1;
-        float acc = 0.0f, accn = 0.0f;
-        for (int sl = 0; sl < nsub; ++sl) {
-            const uint64_t salt = (uint64_t)ch + (uint64_t)sl * 10ULL;
-            ParticleSample s{density, f.density_max[ch], f.n_particles[ch], f.od_particle[ch], f.uniformity[ch],
-                             f.seed_base ^ salt, 0};
-            acc += particle_model(&f, s, px.ax, px.ay, px.use_stbn, px.wang_x, px.wang_y);
-            if (px.retime) {
-                s.seed = f.seed_base_next ^ salt;
-                s.frame_offset = 1;
-                accn += particle_model(&f, s, px.ax, px.ay, px.use_stbn, px.wang_x, px.wang_y);
+    const bool rising = prepare_pass<Mode>(f, tables, ch, px.use_stbn != 0, px.retime);
+    const GrainFrameUniforms& u = tables.u;
+    const bool wang = px.use_stbn && wang_active(&f);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int x0 = tile % columns * kSampleColumns, y0 = tile / columns * rows, y1 = min(y0 + rows, height);
+        __syncthreads();
+        prepare_tile(f, tables, px.use_stbn != 0, x0, min(x0 + kSampleColumns, width), y0, y1);
+        __syncthreads();
+        const int x = x0 + lane;
+        if (x >= width) continue;
+        px.ax = (uint64_t)((int64_t)f.origin_x + x);
+        NoiseAxis noise_col[kNoiseCoords];
+#pragma unroll
+        for (int k = 0; k < kNoiseCoords; ++k)
+            noise_col[k] =
+                (k < 2 ? u.breathing_active : u.clump_active) ? noise_axis(noise_x(u, k, px.ax)) : NoiseAxis{0, 0.0f};
+        const bool wang_held = wang && tables.wang_nx > 0;
+        int wang_cell = 0, wang_near = 0, wang_far = 0;
+        if (wang_held) {
+            const float cx = wang_position(&f, px.ax);
+            wang_cell = (int)floorf(cx) - (int)tables.wang_x;
+            wang_samples(cx, f.wang_w, wang_near, wang_far);
+        }
+#pragma unroll 1
+        for (int y = y0 + line; y < y1; y += kSampleRows) {
+            const float in_density = density_in[(long long)y * din_stride + x];
+            px.ay = (uint64_t)((int64_t)f.origin_y + y);
+            px.wang_x = px.wang_y = 0;
+            if (wang_held) {
+                const WangRow r = tables.wang_row[y - y0];
+                wang_shift(&f, tables.wang_tile[r.cell + wang_cell], wang_near, wang_far, r.near, r.far, px.wang_x,
+                           px.wang_y);
+            } else if (wang) {
+                wang_offsets(&f, px.ax, px.ay, px.wang_x, px.wang_y);
             }
-        }
-        acc /= (float)nsub;
-        if (px.retime) accn /= (float)nsub;
-        acc = __fmaf_rn((acc - density) * px.breathing, px.clump, density);
-        if (px.retime) {
-            accn = __fmaf_rn((accn - density) * px.breathing, px.clump, density);
-            const float d0 = acc - density, d1 = accn - density;
-            const float blend = __fmaf_rn(d1 - d0, px.time_alpha, d0);
-            const float w0 = 1.0f - px.time_alpha;
-            const float den = __fmaf_rn(w0, w0, px.time_alpha * px.time_alpha) + 1e-6f;
-            acc = __fmaf_rn(blend, rsqrtf(den), density);
-        }
-        value = sanitize(acc);
-    } else if (Mode == kGrainLayer) {
-        const float density = layer_density(&f, ch, layer, in_density) + f.density_min_layers[layer][ch];
-        const uint64_t salt = (uint64_t)ch + (uint64_t)layer * 10ULL;
-        const ParticleSample s{density,
-                               f.density_max_layers[layer][ch],
-                               f.n_particles_layers[layer][ch],
-                               f.od_particle_layers[layer][ch],
-                               f.uniformity[ch],
-                               f.seed_base ^ salt,
-                               0};
-        value = sanitize(modulated_sample(&f, px, s, f.seed_base_next ^ salt));
-    } else {
-        float sum = 0.0f;
-        for (int l = 0; l < 3; ++l) {
-            const float density = layer_density(&f, ch, l, in_density) + f.density_min_layers[l][ch];
-            const uint64_t salt = (uint64_t)ch + (uint64_t)l * 10ULL;
-            const ParticleSample s{density,
-                                   f.density_max_layers[l][ch],
-                                   f.n_particles_layers[l][ch],
-                                   f.od_particle_layers[l][ch],
-                                   f.uniformity[ch],
-                                   f.seed_base ^ salt,
-                                   0};
-            sum += sanitize(modulated_sample(&f, px, s, f.seed_base_next ^ salt));
-        }
-        value = sanitize(sum);
-    }
+            NoiseAxis noise_row[kNoiseCoords];
+#pragma unroll
+            for (int k = 0; k < kNoiseCoords; ++k) noise_row[k] = tables.row[k][y - y0];
 
-    float* o = out.p + (long long)y * out.stride + x;
-    if (ep.accumulate) value = sanitize((ep.init ? 0.0f : *o) + value);
-    if (ep.form_delta) {
-        if (ep.density_bias != 0.0f) value = sanitize(value + ep.density_bias);
-        value = sanitize(value - in_density);
+            px.clump = clump_factor(u, tables, noise_col, noise_row);
+            px.breathing = breathing_factor(&f, u, tables, noise_col, noise_row);
+
+            float value;
+            if (Mode == kGrainSimple) {
+                const float density = in_density + f.density_min[ch];
+                const int nsub = f.n_sublayers > 0 ? f.n_sublayers : 1;
+                const ParticleSample s{density, f.density_max[ch], f.n_particles[ch], f.od_particle[ch],
+                                       f.uniformity[ch]};
+                float acc[2] = {0.0f, 0.0f};
+#pragma unroll 1
+                for (int sl = 0; sl < nsub; ++sl) {
+                    const uint64_t salt = (uint64_t)ch + (uint64_t)sl * 10ULL;
+                    acc[0] += particle_model(&f, &tables, s, px, sl, 0, f.seed_base ^ salt);
+                    if (px.retime) acc[1] += particle_model(&f, &tables, s, px, sl, 1, f.seed_base_next ^ salt);
+                }
+                acc[0] /= (float)nsub;
+                if (px.retime) acc[1] /= (float)nsub;
+                value = sanitize(blend_frames(px, density, acc[0], acc[1]));
+            } else {
+                const LayerPlace at = layer_place(&f, rising ? tables.axis : nullptr, ch, in_density);
+                const int first = Mode == kGrainLayer ? layer : 0, last = Mode == kGrainLayer ? layer : 2;
+                float sum = 0.0f;
+#pragma unroll 3
+                for (int l = first; l <= last; ++l) {
+                    const uint64_t salt = (uint64_t)ch + (uint64_t)l * 10ULL;
+                    const float density = layer_density(&f, ch, l, at, in_density) + f.density_min_layers[l][ch];
+                    const ParticleSample s{density, f.density_max_layers[l][ch], f.n_particles_layers[l][ch],
+                                           f.od_particle_layers[l][ch], f.uniformity[ch]};
+                    const float g = particle_model(&f, &tables, s, px, l, 0, f.seed_base ^ salt);
+                    float gn = 0.0f;
+                    if (px.retime) gn = particle_model(&f, &tables, s, px, l, 1, f.seed_base_next ^ salt);
+                    const float v = sanitize(blend_frames(px, density, g, gn));
+                    sum = Mode == kGrainLayer ? v : sum + v;
+                }
+                value = sanitize(sum);
+            }
+
+            float* o = out.p + (long long)y * out.stride + x;
+            if (ep.accumulate) value = sanitize((ep.init ? 0.0f : *o) + value);
+            if (ep.form_delta) {
+                if (ep.density_bias != 0.0f) value = sanitize(value + ep.density_bias);
+                value = sanitize(value - in_density);
+            }
+            *o = value;
+        }
     }
-    *o = value;
 }
 
 __device__ __forceinline__ int reflect_half(int i, int n) {
@@ -719,24 +986,21 @@ cudaError_t launch_grain_sample(const GrainFrame& f, int mode, int channel, int 
                                 long long density_stride, GrainPlane out, const GrainSampleEpilogue& ep, int width,
                                 int height, cudaStream_t s) {
     if (width <= 0 || height <= 0) return cudaSuccess;
-    const dim3 block(32, 8), grid = plane_grid(width, height);
-    switch (mode) {
-    case kGrainSimple:
-        fjb::count_launch();
-        grain_sample_kernel<kGrainSimple><<<grid, block, 0, s>>>(f, channel, layer, density, density_stride, out, ep,
-                                                                 width, height);
-        break;
-    case kGrainLayer:
-        fjb::count_launch();
-        grain_sample_kernel<kGrainLayer><<<grid, block, 0, s>>>(f, channel, layer, density, density_stride, out, ep,
-                                                                width, height);
-        break;
-    default:
-        fjb::count_launch();
-        grain_sample_kernel<kGrainTriplet><<<grid, block, 0, s>>>(f, channel, layer, density, density_stride, out,
-                                                                  ep, width, height);
-        break;
-    }
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int resident = (sms > 0 ? sms : 148) * kSampleBlocks;
+    // tiles of several rows per thread share the tables, unless that leaves blocks without one
+    int rows = kBlockRows;
+    const int columns = (width + kSampleColumns - 1) / kSampleColumns;
+    while (rows > kSampleRows && (long long)columns * ((height + rows - 1) / rows) < resident) rows /= 2;
+    const long long tiles = (long long)columns * ((height + rows - 1) / rows);
+    auto* k = mode == kGrainSimple  ? grain_sample_kernel<kGrainSimple>
+              : mode == kGrainLayer ? grain_sample_kernel<kGrainLayer>
+                                    : grain_sample_kernel<kGrainTriplet>;
+    fjb::count_launch();
+    k<<<(unsigned)std::min<long long>(tiles, resident), kSampleThreads, 0, s>>>(
+        f, channel, layer, density, density_stride, out, ep, width, height, rows, columns, (int)tiles);
     return cudaGetLastError();
 }
 
