@@ -469,7 +469,7 @@ extern "C" FjStatus fjb_visual_grain(FjbRecipe* recipe, const FjVisualGrain* gra
                     e = fjb::launch_grain_clear(sc.accum, width, height, sc.s);
                 }
                 if (e == cudaSuccess)
-                    e = fjb::launch_grain_finish(density[c], ds, sc.accum.p, sc.accum.stride, nullptr, 0.0f, 0.0f,
+                    e = fjb::launch_grain_finish({{density[c]}}, 1, ds, sc.accum.p, sc.accum.stride, nullptr, 0.0f, 0.0f,
                                                  0.0f, grain->amplitude, 0, width, height, sc.s);
             }
         } else {
@@ -481,11 +481,13 @@ extern "C" FjStatus fjb_visual_grain(FjbRecipe* recipe, const FjVisualGrain* gra
                 sf.seed_base_next ^= kSaltShared;
                 e = sc.mix(sf, density_m, ds, 1, sc.shared);
             }
-            for (int c = 0; c < 3 && e == cudaSuccess; ++c) {
-                const bool independent = grain->chroma_independent_weight > 0.0f || !shared_chroma;
+            const bool independent = grain->chroma_independent_weight > 0.0f || !shared_chroma;
+            for (int c = 0; c < (independent ? 3 : 1) && e == cudaSuccess; ++c) {
                 if (independent) e = sc.mix(f, density[c], ds, c, sc.accum);
+                const fjb::GrainDensity planes = independent ? fjb::GrainDensity{{density[c]}}
+                                                             : fjb::GrainDensity{{density_c, density_m, density_y}};
                 if (e == cudaSuccess)
-                    e = fjb::launch_grain_finish(density[c], ds, sc.accum.p, sc.accum.stride,
+                    e = fjb::launch_grain_finish(planes, independent ? 1 : 3, ds, sc.accum.p, sc.accum.stride,
                                                  shared_chroma ? sc.shared.p : nullptr, grain->chroma_shared_weight,
                                                  grain->chroma_independent_weight, grain->amplitude,
                                                  shared_chroma ? 1.0f : grain->amplitude,

@@ -112,11 +112,17 @@ cudaError_t launch_grain_accumulate_weighted(GrainPlane dst, const float* src, l
                                              int init, int apply_gain, float gain, int width, int height,
                                              cudaStream_t s);
 cudaError_t launch_grain_clear(GrainPlane dst, int width, int height, cudaStream_t s);
+// Density planes that take the same delta.
+struct GrainDensity {
+    float* p[3];
+};
+
 // density = sanitize(fma(scale, delta', add_mean ? density : 0)) with delta' the delta
 // (independent) or the shared/independent mix when `shared` is non-null.
-cudaError_t launch_grain_finish(float* density, long long density_stride, const float* delta, long long delta_stride,
-                                const float* shared, float shared_weight, float independent_weight, float amplitude,
-                                float scale, int add_mean, int width, int height, cudaStream_t s);
+cudaError_t launch_grain_finish(const GrainDensity& density, int planes, long long density_stride, const float* delta,
+                                long long delta_stride, const float* shared, float shared_weight,
+                                float independent_weight, float amplitude, float scale, int add_mean, int width,
+                                int height, cudaStream_t s);
 // debug: all three planes = offset + mean(c, m, y) * scale
 cudaError_t launch_grain_debug_average(float* c, float* m, float* y, long long stride, float offset, float scale,
                                        int width, int height, cudaStream_t s);
