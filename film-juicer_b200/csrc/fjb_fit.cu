@@ -37,6 +37,10 @@ namespace fjb {
 namespace {
 
 constexpr int kFitThreads = 256;
+// Blocks per SM, the grids' too (one wave). 16 frames of 512x512: forward 454 us at two, 391 at
+// four; adjoint 870 at two, 826 at three, 970 at four (its state spills in 64 registers).
+constexpr int kForwardBlocks = 4;
+constexpr int kVjpBlocks = 3;
 static_assert((kFitThreads & (kFitThreads - 1)) == 0, "the block sum is a power-of-two tree");
 // Per-thread gradient sums (a thread adds a few tens of pixels); blocks sum in FP64.
 using FitAcc = float;
@@ -505,8 +509,7 @@ struct FitCarrier {
 // exposure, or from the carrier planes as the capture stage reads them
 // (max(0, carrier x route correction)).
 template <bool kCarrier>
-__device__ __forceinline__ void load_exposure(const PixelParams& p, const FitCarrier& cr, long long idx, float e0[3]) {
-    const int y = (int)(idx / p.width), x = (int)(idx - (long long)y * p.width);
+__device__ __forceinline__ void load_exposure(const PixelParams& p, const FitCarrier& cr, int x, int y, float e0[3]) {
     if constexpr (kCarrier) {
         const long long ci = (long long)y * cr.stride + x;
         e0[0] = fmaxf(0.0f, cr.b[ci] * p.route_correction_scale);
@@ -521,8 +524,7 @@ __device__ __forceinline__ void load_exposure(const PixelParams& p, const FitCar
 }
 
 // The filtered DIR corrections of pixel idx (spatial DIR, carrier layout).
-__device__ __forceinline__ void load_filtered(const PixelParams& p, const FitCarrier& cr, long long idx, float cf[3]) {
-    const int y = (int)(idx / p.width), x = (int)(idx - (long long)y * p.width);
+__device__ __forceinline__ void load_filtered(const PixelParams& p, const FitCarrier& cr, int x, int y, float cf[3]) {
     const long long ci = (long long)y * cr.stride + x;
     cf[0] = cr.fy[ci];
     cf[1] = cr.fm[ci];
@@ -531,17 +533,19 @@ __device__ __forceinline__ void load_filtered(const PixelParams& p, const FitCar
 
 // Linear output RGB planes for theta (NaN where the chain rejects a pixel).
 template <bool kPrint, bool kCarrier, bool kSpatial = false>
-__global__ void __launch_bounds__(kFitThreads, 2) fit_forward_kernel(const __grid_constant__ PixelParams p, FitTheta th,
+__global__ void __launch_bounds__(kFitThreads, kForwardBlocks) fit_forward_kernel(const __grid_constant__ PixelParams p, FitTheta th,
                                                                   FitCarrier cr, float* out_r, float* out_g,
                                                                   float* out_b) {
     extern __shared__ float4 fit_smem4[];
     const float* blob = stage_blob(p, th, reinterpret_cast<float*>(fit_smem4));
     const long long total = (long long)p.width * p.height;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
+    const int stride = (int)(gridDim.x * blockDim.x);
+    for (PixelWalk at(p.width, stride); at.idx < total; at.next(p.width, stride)) {
+        const long long idx = at.idx;
+        const int x = at.x, y = at.y;
         float e0[3], cf[3] = {0.0f, 0.0f, 0.0f};
-        load_exposure<kCarrier>(p, cr, idx, e0);
-        if constexpr (kSpatial) load_filtered(p, cr, idx, cf);
+        load_exposure<kCarrier>(p, cr, x, y, e0);
+        if constexpr (kSpatial) load_filtered(p, cr, x, y, cf);
         double rgb[3];
         const bool ok =
             fit_pixel<kPrint, false, kSpatial>(p, blob, th, e0, rgb, nullptr, nullptr, nullptr, nullptr, cf, nullptr);
@@ -557,7 +561,7 @@ constexpr int kFitParams = 13;
 // carrier input and gradient planes, also d <g, rgb> / d carrier per pixel (zero where
 // the chain rejects the pixel or the cotangent is zero).
 template <bool kPrint, bool kCarrier, bool kSpatial = false>
-__global__ void __launch_bounds__(kFitThreads, 2) fit_vjp_kernel(const __grid_constant__ PixelParams p, FitTheta th,
+__global__ void __launch_bounds__(kFitThreads, kVjpBlocks) fit_vjp_kernel(const __grid_constant__ PixelParams p, FitTheta th,
                                                               FitCarrier cr, const float* __restrict__ g_r,
                                                               const float* __restrict__ g_g,
                                                               const float* __restrict__ g_b, double* partials) {
@@ -577,15 +581,17 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_vjp_kernel(const __grid_co
     for (int k = 0; k < kFitParams; ++k) acc[k] = 0.0f;
     const bool carrier_grad = kCarrier && cr.gb != nullptr;
     const long long total = (long long)p.width * p.height;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
+    const int stride = (int)(gridDim.x * blockDim.x);
+    for (PixelWalk at(p.width, stride); at.idx < total; at.next(p.width, stride)) {
+        const long long idx = at.idx;
+        const int x = at.x, y = at.y;
         const float g[3] = {g_r[idx], g_g[idx], g_b[idx]};
         float ge[3] = {0.0f, 0.0f, 0.0f}, gcf[3] = {0.0f, 0.0f, 0.0f};
         float e0[3] = {0.0f, 0.0f, 0.0f};
         if (g[0] != 0.0f || g[1] != 0.0f || g[2] != 0.0f) {
-            load_exposure<kCarrier>(p, cr, idx, e0);
+            load_exposure<kCarrier>(p, cr, x, y, e0);
             float cf[3] = {0.0f, 0.0f, 0.0f};
-            if constexpr (kSpatial) load_filtered(p, cr, idx, cf);
+            if constexpr (kSpatial) load_filtered(p, cr, x, y, cf);
             double rgb[3];
             if (!fit_pixel<kPrint, true, kSpatial>(p, blob, th, e0, rgb, g, acc, dldk, carrier_grad ? ge : nullptr, cf,
                                                    gcf)) {
@@ -594,7 +600,6 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_vjp_kernel(const __grid_co
             }
         }
         if constexpr (kSpatial) {
-            const int y = (int)(idx / p.width), x = (int)(idx - (long long)y * p.width);
             const long long ci = (long long)y * cr.stride + x;
             cr.gfy[ci] = gcf[0];
             cr.gfm[ci] = gcf[1];
@@ -602,7 +607,6 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_vjp_kernel(const __grid_co
         }
         if (carrier_grad) {
             // e0 = max(0, carrier x route): the route factor inside, zero where clamped
-            const int y = (int)(idx / p.width), x = (int)(idx - (long long)y * p.width);
             const long long ci = (long long)y * cr.stride + x;
             const float rc = p.route_correction_scale;
             cr.gb[ci] = e0[0] > 0.0f ? ge[0] * rc : 0.0f;
@@ -622,12 +626,20 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_vjp_kernel(const __grid_co
     }
 }
 
-__global__ void fit_reduce_kernel(const double* __restrict__ partials, int blocks, double* out) {
-    const int k = threadIdx.x;
-    if (k >= kFitParams) return;
-    double s = 0.0;
-    for (int b = 0; b < blocks; ++b) s += partials[(size_t)b * kFitParams + k];
-    out[k] = s;
+// One block per parameter: the blocks' partials in a fixed order. 592 partials: 23 -> 3 us
+// against one thread per parameter, which paid a memory latency per partial.
+__global__ void __launch_bounds__(kFitThreads) fit_reduce_kernel(const double* __restrict__ partials, int blocks,
+                                                                double* out) {
+    __shared__ double red[kFitThreads];
+    double v = 0.0;
+    for (int b = threadIdx.x; b < blocks; b += kFitThreads) v += partials[(size_t)b * kFitParams + blockIdx.x];
+    red[threadIdx.x] = v;
+    __syncthreads();
+    for (int s = kFitThreads / 2; s > 0; s >>= 1) {
+        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
 }
 
 // Spatial-DIR source of one pixel for theta (src/Cuda/Film/JuicerCudaFilmPipeline.cu:124-214):
@@ -690,12 +702,13 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_dir_source_kernel(const __
     extern __shared__ float4 fit_smem4[];
     const float* blob = stage_blob(p, th, reinterpret_cast<float*>(fit_smem4));
     const long long total = (long long)p.width * p.height;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
+    const int stride = (int)(gridDim.x * blockDim.x);
+    for (PixelWalk at(p.width, stride); at.idx < total; at.next(p.width, stride)) {
+        const long long idx = at.idx;
+        const int x = at.x, y = at.y;
         float e0[3], corr[3];
-        load_exposure<kCarrier>(p, cr, idx, e0);
+        load_exposure<kCarrier>(p, cr, x, y, e0);
         const bool ok = dir_source_pixel<false>(p, blob, th, e0, corr, nullptr, nullptr, nullptr);
-        const int y = (int)(idx / p.width), x = (int)(idx - (long long)y * p.width);
         const long long ci = (long long)y * cr.stride + x;
         out_y[ci] = ok ? corr[0] : nanf("");
         out_m[ci] = ok ? corr[1] : nanf("");
@@ -720,14 +733,15 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_dir_source_vjp_kernel(cons
     for (int k = 0; k < kFitParams; ++k) acc[k] = 0.0f;
     const bool carrier_grad = kCarrier && cr.gb != nullptr;
     const long long total = (long long)p.width * p.height;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(idx / p.width), x = (int)(idx - (long long)y * p.width);
+    const int stride = (int)(gridDim.x * blockDim.x);
+    for (PixelWalk at(p.width, stride); at.idx < total; at.next(p.width, stride)) {
+        const long long idx = at.idx;
+        const int x = at.x, y = at.y;
         const long long ci = (long long)y * cr.stride + x;
         const float g[3] = {g_y[ci], g_m[ci], g_c[ci]};
         if (g[0] == 0.0f && g[1] == 0.0f && g[2] == 0.0f) continue;
         float e0[3], corr[3], ge[3] = {0.0f, 0.0f, 0.0f};
-        load_exposure<kCarrier>(p, cr, idx, e0);
+        load_exposure<kCarrier>(p, cr, x, y, e0);
         if (!dir_source_pixel<true>(p, blob, th, e0, corr, g, acc, carrier_grad ? ge : nullptr)) continue;
         if (carrier_grad) {
             const float rc = p.route_correction_scale;
@@ -748,12 +762,16 @@ __global__ void __launch_bounds__(kFitThreads, 2) fit_dir_source_vjp_kernel(cons
     }
 }
 
-int fit_blocks() {
+int fit_blocks(int per_sm) {
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    return (sms > 0 ? sms : 148) * 4;
+    return (sms > 0 ? sms : 148) * per_sm;
 }
+
+// Blocks that the scratch holds partial sums of (the adjoints launch no more).
+constexpr int kPartialBlocks = 4;
+static_assert(kVjpBlocks <= kPartialBlocks && kForwardBlocks <= kPartialBlocks, "partials fit the scratch");
 
 bool theta_from(const FjbFitParams& f, FitTheta& th) {
     for (int c = 0; c < 3; ++c) {
@@ -784,11 +802,11 @@ cudaError_t launch_fit_forward(const PixelParams& p, const FitTheta& th, const F
     if (p.route == kRoutePrint) {
         auto* k = fit_forward_kernel<true, kCarrier, kSpatial>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<fit_blocks(), kFitThreads, smem, s>>>(p, th, cr, out_r, out_g, out_b);
+        k<<<fit_blocks(kForwardBlocks), kFitThreads, smem, s>>>(p, th, cr, out_r, out_g, out_b);
     } else {
         auto* k = fit_forward_kernel<false, kCarrier, kSpatial>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<fit_blocks(), kFitThreads, smem, s>>>(p, th, cr, out_r, out_g, out_b);
+        k<<<fit_blocks(kForwardBlocks), kFitThreads, smem, s>>>(p, th, cr, out_r, out_g, out_b);
     }
     return cudaGetLastError();
 }
@@ -797,7 +815,7 @@ template <bool kCarrier, bool kSpatial = false>
 cudaError_t launch_fit_vjp(const PixelParams& p, const FitTheta& th, const FitCarrier& cr, const float* grad_r,
                            const float* grad_g, const float* grad_b, double* partials, double* grad_params,
                            cudaStream_t s) {
-    const int blocks = fit_blocks();
+    const int blocks = fit_blocks(kVjpBlocks);
     const size_t smem = fit_vjp_smem(p);
     count_launch();
     if (p.route == kRoutePrint) {
@@ -812,7 +830,7 @@ cudaError_t launch_fit_vjp(const PixelParams& p, const FitTheta& th, const FitCa
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
         count_launch();
-        fit_reduce_kernel<<<1, 32, 0, s>>>(partials, blocks, grad_params);
+        fit_reduce_kernel<<<kFitParams, kFitThreads, 0, s>>>(partials, blocks, grad_params);
         e = cudaGetLastError();
     }
     return e;
@@ -824,14 +842,14 @@ cudaError_t launch_fit_dir_source(const PixelParams& p, const FitTheta& th, cons
     count_launch();
     auto* k = fit_dir_source_kernel<true>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<fit_blocks(), kFitThreads, smem, s>>>(p, th, cr, out_y, out_m, out_c);
+    k<<<fit_blocks(kPartialBlocks), kFitThreads, smem, s>>>(p, th, cr, out_y, out_m, out_c);
     return cudaGetLastError();
 }
 
 cudaError_t launch_fit_dir_source_vjp(const PixelParams& p, const FitTheta& th, const FitCarrier& cr, const float* g_y,
                                       const float* g_m, const float* g_c, double* partials, double* grad_params,
                                       cudaStream_t s) {
-    const int blocks = fit_blocks();
+    const int blocks = fit_blocks(kPartialBlocks);
     const size_t smem = (size_t)p.curve_blob_floats * sizeof(float);
     count_launch();
     auto* k = fit_dir_source_vjp_kernel<true>;
@@ -840,7 +858,7 @@ cudaError_t launch_fit_dir_source_vjp(const PixelParams& p, const FitTheta& th, 
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
         count_launch();
-        fit_reduce_kernel<<<1, 32, 0, s>>>(partials, blocks, grad_params);
+        fit_reduce_kernel<<<kFitParams, kFitThreads, 0, s>>>(partials, blocks, grad_params);
         e = cudaGetLastError();
     }
     return e;
@@ -856,7 +874,7 @@ using fjb::write_error;
 
 extern "C" {
 
-size_t fjb_fit_scratch_bytes(void) { return (size_t)fjb::fit_blocks() * fjb::kFitParams * sizeof(double); }
+size_t fjb_fit_scratch_bytes(void) { return (size_t)fjb::fit_blocks(fjb::kPartialBlocks) * fjb::kFitParams * sizeof(double); }
 
 FjStatus fjb_fit_defaults(FjbRecipe* recipe, FjbFitParams* out, FjErrorBuffer* error) {
     if (!recipe || !out) return fail_status(FJ_STATUS_INTERNAL_FAILURE, error, "null argument");
@@ -915,7 +933,7 @@ FjStatus fjb_fit_vjp(FjbRecipe* recipe, const FjbFitParams* params, const float*
     if (st.category != FJ_STATUS_SUCCESS) return st;
     if (!grad_r || !grad_g || !grad_b || !grad_params || !scratch)
         return fail_status(FJ_STATUS_INTERNAL_FAILURE, error, "null argument");
-    if (scratch_bytes < (size_t)fjb::fit_blocks() * fjb::kFitParams * sizeof(double))
+    if (scratch_bytes < (size_t)fjb::fit_blocks(fjb::kPartialBlocks) * fjb::kFitParams * sizeof(double))
         return fail_status(FJ_STATUS_UNSUPPORTED_INPUT, error, "fit scratch smaller than fjb_fit_scratch_bytes()");
     fjb::PixelParams p = recipe->r.params;
     p.src = reinterpret_cast<const char*>(src);
@@ -967,7 +985,7 @@ FjStatus fjb_fit_vjp_carrier(FjbRecipe* recipe, const FjbFitParams* params, cons
     const bool planes = grad_carrier_b || grad_carrier_g || grad_carrier_r;
     if (planes && !(grad_carrier_b && grad_carrier_g && grad_carrier_r))
         return fail_status(FJ_STATUS_INTERNAL_FAILURE, error, "carrier gradient planes: all three or none");
-    if (scratch_bytes < (size_t)fjb::fit_blocks() * fjb::kFitParams * sizeof(double))
+    if (scratch_bytes < (size_t)fjb::fit_blocks(fjb::kPartialBlocks) * fjb::kFitParams * sizeof(double))
         return fail_status(FJ_STATUS_UNSUPPORTED_INPUT, error, "fit scratch smaller than fjb_fit_scratch_bytes()");
     fjb::PixelParams p = recipe->r.params;
     p.width = width;
@@ -1063,7 +1081,7 @@ FjStatus fjb_fit_vjp_spatial_carrier(FjbRecipe* recipe, const FjbFitParams* para
     const bool planes = grad_carrier_b || grad_carrier_g || grad_carrier_r;
     if (planes && !(grad_carrier_b && grad_carrier_g && grad_carrier_r))
         return fail_status(FJ_STATUS_INTERNAL_FAILURE, error, "carrier gradient planes: all three or none");
-    if (scratch_bytes < (size_t)fjb::fit_blocks() * fjb::kFitParams * sizeof(double))
+    if (scratch_bytes < (size_t)fjb::fit_blocks(fjb::kPartialBlocks) * fjb::kFitParams * sizeof(double))
         return fail_status(FJ_STATUS_UNSUPPORTED_INPUT, error, "fit scratch smaller than fjb_fit_scratch_bytes()");
     fjb::PixelParams p = recipe->r.params;
     p.width = width;
@@ -1099,7 +1117,7 @@ FjStatus fjb_fit_dir_source_vjp_carrier(FjbRecipe* recipe, const FjbFitParams* p
     const bool planes = grad_carrier_b || grad_carrier_g || grad_carrier_r;
     if (planes && !(grad_carrier_b && grad_carrier_g && grad_carrier_r))
         return fail_status(FJ_STATUS_INTERNAL_FAILURE, error, "carrier gradient planes: all three or none");
-    if (scratch_bytes < (size_t)fjb::fit_blocks() * fjb::kFitParams * sizeof(double))
+    if (scratch_bytes < (size_t)fjb::fit_blocks(fjb::kPartialBlocks) * fjb::kFitParams * sizeof(double))
         return fail_status(FJ_STATUS_UNSUPPORTED_INPUT, error, "fit scratch smaller than fjb_fit_scratch_bytes()");
     fjb::PixelParams p = recipe->r.params;
     p.width = width;

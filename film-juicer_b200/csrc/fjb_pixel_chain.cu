@@ -31,30 +31,6 @@ enum OutputKind : int {
     kOutEnlargerDevelop = 6, // print density from the diffused print-linear exposure
 };
 
-// A thread's pixels, one grid stride apart, with their coordinates: one division per thread
-// instead of a 64-bit one per pixel.
-struct PixelWalk {
-    long long idx;
-    int x, y, step_x, step_y;
-    __device__ __forceinline__ PixelWalk(int width, int stride) {
-        const unsigned first = blockIdx.x * blockDim.x + threadIdx.x;
-        idx = first;
-        y = (int)(first / (unsigned)width);
-        x = (int)(first - (unsigned)y * (unsigned)width);
-        step_y = stride / width;
-        step_x = stride - step_y * width;
-    }
-    __device__ __forceinline__ void next(int width, int stride) {
-        idx += stride;
-        x += step_x;
-        y += step_y;
-        if (x >= width) {
-            x -= width;
-            ++y;
-        }
-    }
-};
-
 // Spatial-DIR source (src/Cuda/Film/JuicerCudaFilmPipeline.cu:124-214): raw log
 // exposure, pre-DIR layer densities and the donor corrections they release.
 __device__ __forceinline__ void dir_source(const PixelParams& p, const float* __restrict__ blob, const float e[3],

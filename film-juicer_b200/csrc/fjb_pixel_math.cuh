@@ -22,6 +22,30 @@ __device__ __forceinline__ bool finite_f(float v) { return isfinite(v); }
 __device__ __forceinline__ float keep_finite(float v) { return isfinite(v) ? v : 0.0f; }
 __device__ __forceinline__ float keep_finite_nonneg(float v) { return isfinite(v) ? fmaxf(0.0f, v) : 0.0f; }
 
+// A thread's pixels, one grid stride apart, with their coordinates: one division per thread
+// instead of a 64-bit one per pixel.
+struct PixelWalk {
+    long long idx;
+    int x, y, step_x, step_y;
+    __device__ __forceinline__ PixelWalk(int width, int stride) {
+        const unsigned first = blockIdx.x * blockDim.x + threadIdx.x;
+        idx = first;
+        y = (int)(first / (unsigned)width);
+        x = (int)(first - (unsigned)y * (unsigned)width);
+        step_y = stride / width;
+        step_x = stride - step_y * width;
+    }
+    __device__ __forceinline__ void next(int width, int stride) {
+        idx += stride;
+        x += step_x;
+        y += step_y;
+        if (x >= width) {
+            x -= width;
+            ++y;
+        }
+    }
+};
+
 __device__ __forceinline__ void mat3_apply(const float m[9], const float v[3], float o[3]) {
     o[0] = m[0] * v[0] + m[1] * v[1] + m[2] * v[2];
     o[1] = m[3] * v[0] + m[4] * v[1] + m[5] * v[2];
