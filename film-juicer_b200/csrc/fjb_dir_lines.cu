@@ -59,6 +59,9 @@ __device__ __forceinline__ void end_block(const DirComponentDev& c, const double
 // Reflected starts of the recursive components' lines: anchor + sum_i w[i] (x_i - anchor) over
 // the first `len` samples, FP64. A warp takes four lines of a component (rows y .. y + 3, or
 // two pairs of columns), lanes stride the samples, so that a weight serves four lines.
+// Bound by the latency of its loads: a launch has few warps, so the components run side by side
+// and eight samples of a lane are in flight (3840x2160: rows 23 us, columns 39 us; one
+// component after the other, four samples: 57 and 56).
 constexpr int kStartWarps = 8;
 
 template <bool kCols>
@@ -69,47 +72,45 @@ __global__ void __launch_bounds__(32 * kStartWarps) dir_starts_kernel(const __gr
     const int l0 = 4 * (blockIdx.x * kStartWarps + (threadIdx.x >> 5));
     if (l0 >= lines) return;
     const int words = lp::line_words(H);
-#pragma unroll 1
-    for (int k = 0; k < P.count; ++k) {
-        const DirComponentDev& c = P.comp[k];
-        if (c.op != kDirOpYvv) continue;
-        const int len = kCols ? c.v_len : c.h_len;
-        const double* w = kCols ? c.v_init : c.h_init;
-        const float2* pair = reinterpret_cast<const float2*>(P.temp[ch][k]) + (size_t)(l0 / 2) * words + H - 1;
-        auto samples = [&](int i, float (&v)[4]) {
-            if (kCols) {
-                const float2 a = pair[-i], b = pair[words - i];
-                v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
-            } else {
+    const int k = blockIdx.z;
+    const DirComponentDev& c = P.comp[k];
+    if (c.op != kDirOpYvv) return;
+    const int len = kCols ? c.v_len : c.h_len;
+    const double* w = kCols ? c.v_init : c.h_init;
+    const float2* pair = reinterpret_cast<const float2*>(P.temp[ch][k]) + (size_t)(l0 / 2) * words + H - 1;
+    auto samples = [&](int i, float (&v)[4]) {
+        if (kCols) {
+            const float2 a = pair[-i], b = pair[words - i];
+            v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+        } else {
 #pragma unroll
-                for (int r = 0; r < 4; ++r) v[r] = P.raw[ch][(size_t)min(l0 + r, H - 1) * W + i];
-            }
-        };
-        float f[4];
-        samples(0, f);
-        const double anchor[4] = {f[0], f[1], f[2], f[3]};
-        double a[4][3] = {};
-#pragma unroll 4
-        for (int i = lane; i < len; i += 32) {
-            const double w0 = __ldg(w + i), w1 = __ldg(w + len + i), w2 = __ldg(w + 2 * len + i);
-            samples(i, f);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const double d = (double)f[r] - anchor[r];
-                a[r][0] += w0 * d;
-                a[r][1] += w1 * d;
-                a[r][2] += w2 * d;
-            }
+            for (int r = 0; r < 4; ++r) v[r] = P.raw[ch][(size_t)min(l0 + r, H - 1) * W + i];
         }
-        double* out = (kCols ? P.col_start : P.row_start) + (((size_t)ch * kDirMaxComponents + k) * lines + l0) * 3;
+    };
+    float f[4];
+    samples(0, f);
+    const double anchor[4] = {f[0], f[1], f[2], f[3]};
+    double a[4][3] = {};
+#pragma unroll 8
+    for (int i = lane; i < len; i += 32) {
+        const double w0 = __ldg(w + i), w1 = __ldg(w + len + i), w2 = __ldg(w + 2 * len + i);
+        samples(i, f);
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int h = 0; h < 3; ++h) {
-                for (int o = 16; o > 0; o >>= 1) a[r][h] += __shfl_xor_sync(0xffffffffu, a[r][h], o);
-                if (lane == 0 && l0 + r < lines) out[3 * r + h] = anchor[r] + a[r][h];
-            }
+        for (int r = 0; r < 4; ++r) {
+            const double d = (double)f[r] - anchor[r];
+            a[r][0] += w0 * d;
+            a[r][1] += w1 * d;
+            a[r][2] += w2 * d;
+        }
     }
+    double* out = (kCols ? P.col_start : P.row_start) + (((size_t)ch * kDirMaxComponents + k) * lines + l0) * 3;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+            for (int o = 16; o > 0; o >>= 1) a[r][h] += __shfl_xor_sync(0xffffffffu, a[r][h], o);
+            if (lane == 0 && l0 + r < lines) out[3 * r + h] = anchor[r] + a[r][h];
+        }
 }
 
 // One recursive component over a pair of lines of n samples, in place: from the reflected
@@ -309,7 +310,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
     constexpr int kLinesPerCta = 4 * kStartWarps;
     if (lines) {
         fjb::count_launch();
-        dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3), 32 * kStartWarps, 0, s>>>(P);
+        dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
         e = cudaFuncSetAttribute(dir_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -320,7 +321,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         fjb::count_launch();
         dir_starts_kernel<true>
-            <<<dim3((2 * lp::plane_pairs(P.width) + kLinesPerCta - 1) / kLinesPerCta, 3), 32 * kStartWarps, 0, s>>>(P);
+            <<<dim3((2 * lp::plane_pairs(P.width) + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     const int warps = P.recursions * lp::kColPairs;
