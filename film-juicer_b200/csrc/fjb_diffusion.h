@@ -24,7 +24,10 @@ cudaError_t launch_diffusion(const float* const psf_rows[3], int radius, int tap
 // FFT form, used from kDiffusionFftMinRadius up: tiles of kDiffusionTile x kDiffusionTile of
 // the reflect-extended frame convolved circularly in shared memory (fjb_diffusion_tile.cu),
 // or, above kDiffusionTileMaxRadius, the whole extended frame on an nx x ny grid
-// (fjb_diffusion_fft.cu).
+// (fjb_diffusion_fft.cu). Measured at radius 19, tiles against the whole frame: 1920x1080 64
+// and 217 us, 3840x2160 233 and 780, 7680x4320 885 and 4300. A tile's inner share is
+// (128 - 2 r)^2 / 128^2, so at radius 40 there are 3.5 times as many tiles: 225, 820 and
+// 3100 us, where the two forms meet; the whole-frame form hardly depends on the radius.
 constexpr int kDiffusionFftMinRadius = 8;
 constexpr int kDiffusionTile = 128;
 constexpr int kDiffusionTileMaxRadius = 40;

@@ -3,11 +3,15 @@
 // function it stands for), without the library's handling of the rest: callers send
 // arguments outside the stated range to the library.
 //
-// Why: the print/scan chain is bound by instruction issue (about 2300 per pixel), and the
-// general functions -- division with its range fix-up, log10f, powf, cbrtf, atan2f, hypotf,
-// fmodf -- were more than half of that. Seeds come from the MUFU, accuracy from one
-// Newton-Raphson step on the defining equation; logarithm, arctangent and exponential are
-// series or fits derived here.
+// Why: the print/scan chain is bound by instruction issue (2300 per pixel with the general
+// functions, division with its range fix-up, log10f, cbrtf, atan2f, hypotf, fmodf and the
+// lookups' searches making up more than half). Seeds come from the MUFU, accuracy from one
+// Newton-Raphson step on the defining equation; the logarithm is a series, the arctangent a fit,
+// both derived here. With the packed spectrum and the table-started lookups: 1720 per pixel,
+// 3840x2160 print scan 743 -> 609 us.
+// Largest and rms error in ulp against FP64, here and the library: quotient and root 0.50 /
+// 0.29, the same (correctly rounded); log10 1.4 / 0.4 and 2.1 / 0.54; cube root 0.73 / 0.31
+// and 1.15 / 0.33; x^(5/12) 1.2 / 0.34 and 1.55 / 0.52; angle 1.7 / 0.36 and 1.95 / 0.46.
 #pragma once
 
 #include <cuda_runtime.h>
