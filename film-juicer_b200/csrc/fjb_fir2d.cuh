@@ -26,7 +26,12 @@ namespace fir {
 constexpr int kMaxRadius = 9;
 constexpr int kTileW = 64, kTileH = 32, kThreads = 256;
 constexpr int kHalo = 12; // columns on each side: the widest halo in whole float4
-constexpr int kInPitch = kTileW + 2 * kHalo;
+constexpr int kInCols = kTileW + 2 * kHalo;
+// Rows 4 banks apart (modulo 32): a quarter warp's 16-byte accesses to eight rows are
+// conflict-free.
+constexpr int kInPitch = kInCols + 4;
+constexpr int kMidPitch = kTileW + 4;
+static_assert(kInPitch % 32 == 28 && kMidPitch % 32 == 4, "eight rows in distinct banks");
 
 constexpr int kMaxSets = 5;
 struct Taps {
@@ -71,17 +76,17 @@ __device__ __forceinline__ void stage(const Jobs& P, const Job& J, int rad, floa
     const int x0 = blockIdx.x * kTileW - kHalo, y0 = blockIdx.y * kTileH - rad;
     const int rows = kTileH + 2 * rad;
     const unsigned base = (unsigned)__cvta_generic_to_shared(in);
-    if (x0 >= 0 && x0 + kInPitch <= W && J.stride % 4 == 0 && (reinterpret_cast<uintptr_t>(J.src) & 15u) == 0) {
-        for (int i = threadIdx.x; i < rows * (kInPitch / 4); i += kThreads) {
-            const int r = i / (kInPitch / 4), c = i % (kInPitch / 4) * 4;
+    if (x0 >= 0 && x0 + kInCols <= W && J.stride % 4 == 0 && (reinterpret_cast<uintptr_t>(J.src) & 15u) == 0) {
+        for (int i = threadIdx.x; i < rows * (kInCols / 4); i += kThreads) {
+            const int r = i / (kInCols / 4), c = i % (kInCols / 4) * 4;
             const float* src = J.src + (long long)reflect(y0 + r, H) * J.stride + x0 + c;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(base + 16u * (unsigned)i), "l"(src));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(base + 4u * (unsigned)(r * kInPitch + c)), "l"(src));
         }
     } else {
-        for (int i = threadIdx.x; i < rows * kInPitch; i += kThreads) {
-            const int r = i / kInPitch, c = i % kInPitch;
+        for (int i = threadIdx.x; i < rows * kInCols; i += kThreads) {
+            const int r = i / kInCols, c = i % kInCols;
             const float* src = J.src + (long long)reflect(y0 + r, H) * J.stride + reflect(x0 + c, W);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(base + 4u * (unsigned)i), "l"(src));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(base + 4u * (unsigned)(r * kInPitch + c)), "l"(src));
         }
     }
     asm volatile("cp.async.commit_group;\n" ::);
@@ -99,7 +104,7 @@ __device__ __forceinline__ void taps(const Taps& T, int rad, const float* in, fl
     for (int o = 0; o <= 2 * RAD; ++o) t[o] = (Acc)T.w[o];
     __syncthreads();
     for (int task = threadIdx.x; task < kRows * (kTileW / 8); task += kThreads) {
-        const int r = task / (kTileW / 8), c = task % (kTileW / 8) * 8;
+        const int r = task % kRows, c = task / kRows * 8; // neighbouring lanes, neighbouring rows
         const float4* q = reinterpret_cast<const float4*>(in + (r + rad - RAD) * kInPitch + kHalo - kPad + c);
         Acc win[8 + 2 * kPad];
 #pragma unroll
@@ -118,7 +123,7 @@ __device__ __forceinline__ void taps(const Taps& T, int rad, const float* in, fl
             for (int o = 0; o <= 2 * RAD; ++o) s += win[kPad - RAD + j + o] * t[o];
             o8[j] = rounded(s);
         }
-        float4* m = reinterpret_cast<float4*>(mid + r * kTileW + c);
+        float4* m = reinterpret_cast<float4*>(mid + r * kMidPitch + c);
         m[0] = make_float4(o8[0], o8[1], o8[2], o8[3]);
         m[1] = make_float4(o8[4], o8[5], o8[6], o8[7]);
     }
@@ -131,10 +136,10 @@ __device__ __forceinline__ void taps(const Taps& T, int rad, const float* in, fl
             t[2 * RAD - o] = a;
         }
     }
-    const float* col = mid + threadIdx.x / kTileW * 8 * kTileW + threadIdx.x % kTileW;
+    const float* col = mid + threadIdx.x / kTileW * 8 * kMidPitch + threadIdx.x % kTileW;
     Acc win[8 + 2 * RAD];
 #pragma unroll
-    for (int i = 0; i < 8 + 2 * RAD; ++i) win[i] = (Acc)col[i * kTileW];
+    for (int i = 0; i < 8 + 2 * RAD; ++i) win[i] = (Acc)col[i * kMidPitch];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         Acc s = 0;
@@ -147,7 +152,7 @@ __device__ __forceinline__ void taps(const Taps& T, int rad, const float* in, fl
 template <typename Acc>
 __global__ void __launch_bounds__(kThreads, 3) kernel(const __grid_constant__ Jobs P) {
     __shared__ __align__(16) float in[(kTileH + 2 * kMaxRadius) * kInPitch];
-    __shared__ __align__(16) float mid[(kTileH + 2 * kMaxRadius) * kTileW];
+    __shared__ __align__(16) float mid[(kTileH + 2 * kMaxRadius) * kMidPitch];
     const Job& J = P.job[blockIdx.z];
     int rad = 0;
     for (int i = 0; i < J.count; ++i) rad = max(rad, J.set[i].radius);
