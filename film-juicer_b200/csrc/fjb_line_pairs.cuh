@@ -26,7 +26,7 @@
 // for (its loads, its scan) is covered by the others of its SM.
 // Lines cut into blocks of 64 samples, a CTA's threads walking blocks between barriers, took
 // at 3840x2160 290 + 159 us for halation's rows and 499 + 283 for its columns; here 143 + 131
-// and 188 + 151, with the short taps apart (104 + 30). Loading rows through registers (half the
+// and 188 + 151, with the short taps apart (95 + 29). Loading rows through registers (half the
 // shared-memory passes of the 4-byte copies) took a fifth longer, and column CTAs of one pair
 // in clusters of four gained 4 % on DIR's columns and lost 19 % at 1283x719.
 #pragma once
