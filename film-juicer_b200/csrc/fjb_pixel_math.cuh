@@ -224,14 +224,15 @@ __device__ __forceinline__ void tc_exposure(const PixelParams& p, const float in
     const float Z = keep_finite(in_xyz[2]);
     const float sum = X + Y + Z;
     const float den = fmaxf(sum, 1e-10f);
-    const bool quick = fmaxf(fmaxf(fabsf(X), fabsf(Y)), den) <= 1e30f; // den >= 1e-10
+    // below 1e27 every quotient by 1e-10 or more is in range
+    const bool quick = fmaxf(fmaxf(fabsf(X), fabsf(Y)), den) <= 1e27f;
     const float tx = quick ? quotient(X, den) : X / den;
     const float ty = quick ? quotient(Y, den) : Y / den;
     // triangle -> square mapping of chromaticity
     const float one_minus = 1.0f - tx;
     const float qden = fmaxf(one_minus, 1e-10f);
     const float qx = fminf(1.0f, fmaxf(0.0f, one_minus * one_minus));
-    const float qy = fminf(1.0f, fmaxf(0.0f, fabsf(ty) <= 1e30f && qden <= 1e30f ? quotient(ty, qden) : ty / qden));
+    const float qy = fminf(1.0f, fmaxf(0.0f, fabsf(ty) <= 1e27f && qden <= 1e27f ? quotient(ty, qden) : ty / qden));
     float rgb[3];
     tc_lut_sample(p.tc_lut, qx, qy, rgb);
     e_bgr[0] = keep_finite(sum * keep_finite(rgb[2]));
