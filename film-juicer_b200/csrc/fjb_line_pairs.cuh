@@ -11,7 +11,8 @@
 // In exact arithmetic this is the sequential recursion; in floating point it differs
 // from it by rounding (the states between pieces are FP64). Successive pieces start an odd
 // number of words apart, so the lanes of a half warp fall in distinct banks. A step
-// handles both lines with packed FP32 instructions.
+// handles both lines with packed FP32 instructions. Long lines in the direct form take
+// their 32 pieces chunk by chunk (direct_chunks).
 //
 // Rows: a CTA holds four rows (two warps). Between the passes a plane lies by pairs of
 // columns, each pair's samples of all rows together, so that a row CTA writes a whole
@@ -58,6 +59,20 @@ struct LineMaps {
 
 // Samples per piece of a line of n samples (odd).
 __host__ __device__ inline int piece_len(int n) { return ((n + kPieces - 1) / kPieces) | 1; }
+// Chunks that a line in the direct form (DirectStep) is processed in, one after the other
+// with FP64 states between them, 32 pieces each. Its rounding errors are amplified by the
+// recursion's DC gain, and the longer a piece runs in FP32, the more of the gain they see.
+// Largest back-reflection of a 35 mm gate, both directions, rms error against 64 bits over
+// lines of 12 stops: 3840 samples 1.5e-5 for pieces of 121 as for 63; 5000: 3.0e-5 (157),
+// 2.6e-5 (63); 7680: 8.9e-5 (241), 5.5e-5 (63); 12288: 2.9e-4 (385), 9.7e-5 (63). So
+// pieces above 127 samples are cut to 63 at most; 7680x4320, both axes, 4560 -> 5670 us for
+// it (lines in blocks of 64 samples, whole CTAs: 6670). The factored form shows no such growth.
+__host__ __device__ inline int direct_chunks(int n) {
+    constexpr int kLongest = 127, kCut = 63;
+    return piece_len(n) <= kLongest ? 1 : (n + kPieces * kCut - 1) / (kPieces * kCut);
+}
+// Samples per piece of a line in so many chunks.
+__host__ __device__ inline int chunk_piece_len(int n, int chunks) { return piece_len((n + chunks - 1) / chunks); }
 // Words (pairs of samples) of a line as stored, a whole number of 32-byte sectors.
 __host__ __device__ inline int line_words(int n) { return (n + 3) / 4 * 4; }
 __host__ __device__ inline size_t line_bytes(int n) { return (size_t)line_words(n) * sizeof(float2); }
@@ -180,14 +195,26 @@ struct State2 {
         }
         return t;
     }
+    // The state of a lane.
+    __device__ __forceinline__ State2 of(int lane) const {
+        State2 t;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            t.a[i] = __shfl_sync(0xffffffffu, a[i], lane);
+            t.b[i] = __shfl_sync(0xffffffffu, b[i], lane);
+        }
+        return t;
+    }
 };
 
 // This lane's piece of a pair of lines of n samples: positions [base, base + k) as far as
 // they lie in [lo, hi).
 struct Piece {
     int base, k, lo, hi;
-    __device__ Piece(int n, int lane) : k(piece_len(n)) {
-        base = lane * k;
+    __device__ Piece(int n, int lane) : Piece(n, lane, 0, piece_len(n)) {}
+    // of the 32 pieces of `k_` samples from position `from` on
+    __device__ Piece(int n, int lane, int from, int k_) : k(k_) {
+        base = from + lane * k;
         lo = min(base, n);
         hi = min(base + k, n);
     }
@@ -216,6 +243,48 @@ __device__ __forceinline__ void direction(const Op& op, const LineMaps& m, Pair*
 #pragma unroll
     for (int i = 0; i < 3; ++i) s[i] = first ? start[i] : s[i];
     run<kFwd, true>(op, w, nv, s);
+}
+
+// The same over the line's chunks of 32 pieces of `k` samples, the chunk's entry state carried
+// in FP64 from the one processed before. `s` receives the exit state of the lane's piece in
+// the last chunk processed.
+template <bool kFwd>
+__device__ __forceinline__ void direction_chunks(const DirectStep& op, const LineMaps& m, Pair* line, int n, int k,
+                                                 int chunks, int lane, const Pair (&start)[3], Pair (&s)[3]) {
+    const Pair zero{0ull};
+    const int order = kFwd ? lane : kPieces - 1 - lane;
+    State2 carry;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+        const int from = (kFwd ? c : chunks - 1 - c) * kPieces * k;
+        const Piece pc(n, lane, from, k);
+        const bool first = kFwd ? lane == 0 : pc.lo < pc.hi && pc.hi == min(n, from + kPieces * k);
+        const int nv = pc.hi - pc.lo;
+        Pair* w = line + (kFwd ? pc.lo : pc.hi - 1);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s[i] = first && c == 0 ? start[i] : zero;
+        run<kFwd, false>(op, w, nv, s);
+        State2 S;
+        S.set(s);
+        if (first && c > 0) S.add(m.m[0], carry);
+#pragma unroll 1
+        for (int l = 0; l < kLevels; ++l) {
+            const State2 t = S.from<kFwd>(1 << l);
+            if (order >= (1 << l)) S.add(m.m[l], t);
+        }
+        S.from<kFwd>(1).get(s);
+        if (first) {
+            if (c == 0) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) s[i] = start[i];
+            } else {
+                carry.get(s);
+            }
+        }
+        // the chunks followed by another are whole: the lane processed last has their exit state
+        carry = S.of(kFwd ? kPieces - 1 : 0);
+        run<kFwd, true>(op, w, nv, s);
+    }
 }
 
 // Brings a block of global memory into L2. The CTAs of a launch start together and would all
