@@ -37,13 +37,18 @@ namespace fjb {
 namespace {
 
 constexpr int kFitThreads = 256;
+constexpr int kFitWarps = kFitThreads / 32;
 // Blocks per SM, the grids' too (one wave). 16 frames of 512x512: forward 454 us at two, 391 at
 // four; adjoint 870 at two, 826 at three, 970 at four (its state spills in 64 registers).
 constexpr int kForwardBlocks = 4;
 constexpr int kVjpBlocks = 3;
 static_assert((kFitThreads & (kFitThreads - 1)) == 0, "the block sum is a power-of-two tree");
-// Per-thread gradient sums (a thread adds a few tens of pixels); blocks sum in FP64.
+// Gradient sums: a thread adds kFitRun pixels in FP32, and its runs in FP64, in its column of
+// a table in shared memory (FP64 sums in registers or local memory cost 5 % of the adjoint,
+// FP64 for every pixel 2 %; this 0.5 %).
 using FitAcc = float;
+constexpr int kFitRun = 16;
+constexpr int kFitParams = 13;
 constexpr float kLn2 = 0.69314718055994530942f;
 constexpr float kLn10 = 2.30258509299404568402f;
 
@@ -383,13 +388,13 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
     } else {
         for (int c = 0; c < 3; ++c) g_D[c] = g_scan[c];
     }
-    float g_logS[3], g_layer[3];
+    float g_logS[3], g_layer[3], g_gamma[3] = {0.0f, 0.0f, 0.0f};
     if (dir) {
-        float g_corr[3];
+        float g_corr[3], g_knee[3] = {0.0f, 0.0f, 0.0f};
         for (int j = 0; j < 3; ++j) {
             const float g = g_D[2 - j];
             const float g_logC = g * sd[j] * th.gamma[j];
-            g_th[3 + j] += (g * sd[j] * logC[j]);
+            g_gamma[j] = g * sd[j] * logC[j];
             g_logS[j] = g_logC;
             g_corr[j] = -g_logC * dfin[j];
         }
@@ -403,7 +408,7 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
             for (int i = 0; i < 3; ++i) {
                 const float g_donor = M[3 * i] * g_corr[0] + M[3 * i + 1] * g_corr[1] + M[3 * i + 2] * g_corr[2];
                 g_layer[i] = g_donor * dv[i];
-                g_th[9 + i] += (g_donor * dk[i]);
+                g_knee[i] = g_donor * dk[i];
             }
         }
         // The compensated axes depend on the knees (axis_j[i] = logE[i] - sum_d M[d][j]
@@ -417,9 +422,10 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
             const float t = dfr[j];
             for (int d = 0; d < 3; ++d) {
                 const float s0 = dldk[d * n + i0], s1 = dldk[d * n + i0 + 1];
-                g_th[9 + d] += (w * M[3 * d + j] * ((1.0f - t) * s0 + t * s1));
+                g_knee[d] += w * M[3 * d + j] * ((1.0f - t) * s0 + t * s1);
             }
         }
+        for (int d = 0; d < 3; ++d) g_th[9 + d] += g_knee[d];
     } else {
         for (int c = 0; c < 3; ++c) {
             g_layer[c] = g_D[2 - c];
@@ -428,7 +434,7 @@ __device__ bool fit_pixel(const PixelParams& p, const float* __restrict__ blob, 
     }
     for (int c = 0; c < 3; ++c) {
         g_logS[c] += g_layer[c] * sl[c] * th.gamma[c];
-        g_th[3 + c] += (g_layer[c] * sl[c] * logS[c]);
+        g_th[3 + c] += g_gamma[c] + g_layer[c] * sl[c] * logS[c];
         const float g_e = e[c] > 0.0f ? g_logS[c] / ((e[c] + 1e-10f) * kLn10) : 0.0f;
         g_th[c] += (g_e * e[c] * kLn2);
         if (g_e0) g_e0[c] = g_e * exp2f(th.ev[c]);
@@ -555,7 +561,18 @@ __global__ void __launch_bounds__(kFitThreads, kForwardBlocks) fit_forward_kerne
     }
 }
 
-constexpr int kFitParams = 13;
+// Block sums of the table (a warp per parameter, fixed order).
+__device__ __forceinline__ void reduce_sums(const double* sums, double* out) {
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < kFitParams; k += kFitWarps) {
+        double v = 0.0;
+#pragma unroll
+        for (int i = 0; i < kFitWarps; ++i) v += sums[k * kFitThreads + i * 32 + lane];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) out[k] = v;
+    }
+}
 
 // Per-block sums (FP64, fixed order) of the pixels' vector-Jacobian products; with
 // carrier input and gradient planes, also d <g, rgb> / d carrier per pixel (zero where
@@ -576,54 +593,57 @@ __global__ void __launch_bounds__(kFitThreads, kVjpBlocks) fit_vjp_kernel(const 
         }
         __syncthreads();
     }
-    __shared__ double red[kFitThreads];
+    __shared__ double sums[kFitParams * kFitThreads];
     FitAcc acc[kFitParams];
-    for (int k = 0; k < kFitParams; ++k) acc[k] = 0.0f;
+    for (int k = 0; k < kFitParams; ++k) {
+        sums[k * kFitThreads + threadIdx.x] = 0.0;
+        acc[k] = 0.0f;
+    }
     const bool carrier_grad = kCarrier && cr.gb != nullptr;
     const long long total = (long long)p.width * p.height;
     const int stride = (int)(gridDim.x * blockDim.x);
-    for (PixelWalk at(p.width, stride); at.idx < total; at.next(p.width, stride)) {
-        const long long idx = at.idx;
-        const int x = at.x, y = at.y;
-        const float g[3] = {g_r[idx], g_g[idx], g_b[idx]};
-        float ge[3] = {0.0f, 0.0f, 0.0f}, gcf[3] = {0.0f, 0.0f, 0.0f};
-        float e0[3] = {0.0f, 0.0f, 0.0f};
-        if (g[0] != 0.0f || g[1] != 0.0f || g[2] != 0.0f) {
-            load_exposure<kCarrier>(p, cr, x, y, e0);
-            float cf[3] = {0.0f, 0.0f, 0.0f};
-            if constexpr (kSpatial) load_filtered(p, cr, x, y, cf);
-            double rgb[3];
-            if (!fit_pixel<kPrint, true, kSpatial>(p, blob, th, e0, rgb, g, acc, dldk, carrier_grad ? ge : nullptr, cf,
-                                                   gcf)) {
-                ge[0] = ge[1] = ge[2] = 0.0f;
-                gcf[0] = gcf[1] = gcf[2] = 0.0f;
+    PixelWalk at(p.width, stride);
+    while (at.idx < total) {
+#pragma unroll 1
+        for (int run = 0; run < kFitRun && at.idx < total; ++run, at.next(p.width, stride)) {
+            const long long idx = at.idx;
+            const int x = at.x, y = at.y;
+            const float g[3] = {g_r[idx], g_g[idx], g_b[idx]};
+            float ge[3] = {0.0f, 0.0f, 0.0f}, gcf[3] = {0.0f, 0.0f, 0.0f};
+            float e0[3] = {0.0f, 0.0f, 0.0f};
+            if (g[0] != 0.0f || g[1] != 0.0f || g[2] != 0.0f) {
+                load_exposure<kCarrier>(p, cr, x, y, e0);
+                float cf[3] = {0.0f, 0.0f, 0.0f};
+                if constexpr (kSpatial) load_filtered(p, cr, x, y, cf);
+                double rgb[3];
+                if (!fit_pixel<kPrint, true, kSpatial>(p, blob, th, e0, rgb, g, acc, dldk, carrier_grad ? ge : nullptr,
+                                                       cf, gcf)) {
+                    ge[0] = ge[1] = ge[2] = 0.0f;
+                    gcf[0] = gcf[1] = gcf[2] = 0.0f;
+                }
+            }
+            if constexpr (kSpatial) {
+                const long long ci = (long long)y * cr.stride + x;
+                cr.gfy[ci] = gcf[0];
+                cr.gfm[ci] = gcf[1];
+                cr.gfc[ci] = gcf[2];
+            }
+            if (carrier_grad) {
+                // e0 = max(0, carrier x route): the route factor inside, zero where clamped
+                const long long ci = (long long)y * cr.stride + x;
+                const float rc = p.route_correction_scale;
+                cr.gb[ci] = e0[0] > 0.0f ? ge[0] * rc : 0.0f;
+                cr.gg[ci] = e0[1] > 0.0f ? ge[1] * rc : 0.0f;
+                cr.gr[ci] = e0[2] > 0.0f ? ge[2] * rc : 0.0f;
             }
         }
-        if constexpr (kSpatial) {
-            const long long ci = (long long)y * cr.stride + x;
-            cr.gfy[ci] = gcf[0];
-            cr.gfm[ci] = gcf[1];
-            cr.gfc[ci] = gcf[2];
-        }
-        if (carrier_grad) {
-            // e0 = max(0, carrier x route): the route factor inside, zero where clamped
-            const long long ci = (long long)y * cr.stride + x;
-            const float rc = p.route_correction_scale;
-            cr.gb[ci] = e0[0] > 0.0f ? ge[0] * rc : 0.0f;
-            cr.gg[ci] = e0[1] > 0.0f ? ge[1] * rc : 0.0f;
-            cr.gr[ci] = e0[2] > 0.0f ? ge[2] * rc : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kFitParams; ++k) {
+            sums[k * kFitThreads + threadIdx.x] += (double)acc[k];
+            acc[k] = 0.0f;
         }
     }
-    for (int k = 0; k < kFitParams; ++k) {
-        red[threadIdx.x] = (double)acc[k];
-        __syncthreads();
-        for (int s = kFitThreads / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) partials[(size_t)blockIdx.x * kFitParams + k] = red[0];
-        __syncthreads();
-    }
+    reduce_sums(sums, partials + (size_t)blockIdx.x * kFitParams);
 }
 
 // One block per parameter: the blocks' partials in a fixed order. 592 partials: 23 -> 3 us
