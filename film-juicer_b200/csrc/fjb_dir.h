@@ -76,9 +76,9 @@ struct DirBlurParams {
     int lines_max, segs_max;
     // everything after the scratch's first three planes; one warp per pair of lines: the
     // recursions a column CTA holds at once, the rows and column CTAs between a CTA and the one
-    // after it, the planes the column launch adds its components to (null: nothing) with the
-    // identity component's weight in them, and the reflected starts of rows and columns (direct
-    // form, per channel, component and line)
+    // after it, the planes of the short components' sums that the column launch adds its own to
+    // (null: there are none), the identity component's weight, and the reflected starts of rows
+    // and columns (direct form, per channel, component and line)
     float* region;
     size_t region_floats;
     int recursions, rows_ahead, cols_ahead;

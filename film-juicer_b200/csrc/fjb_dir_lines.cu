@@ -4,10 +4,12 @@
 // src/Cuda/Film/JuicerCudaFilmPipeline.cu:388-780): FP64 taps with half-sample
 // reflection, and the third-order recursion with its reflected start and end block, here
 // in the factored FP32 form with FP64 states between pieces. Five launches: the short
-// components, both axes, summed into one plane per channel (fjb_fir2d.cuh); the rows'
+// components, if any, both axes, summed into one plane per channel (fjb_fir2d.cuh); the rows'
 // reflected starts; the recursive components' rows, four rows per CTA (fjb_line_pairs.cuh);
 // the columns' reflected starts; the columns, one warp per pair of columns and recursive
 // component, then the weighted sum of all of them and the plane of the first launch.
+// Only short components take a plane of their own, so the planes are never more than the
+// components, which is what the scratch holds.
 //
 // The starts are launches of their own because their weights (three doubles for each of the
 // first 21 sigma samples, 55 KB at 3840x2160) do not fit what the line kernels leave of L1:
@@ -190,9 +192,10 @@ __global__ void __launch_bounds__(32 * lp::kRowWarps) dir_rows_kernel(const __gr
 }
 
 // Two pairs of columns per CTA, P.recursions recursive components at a time; the sum so far
-// waits in the first launch's plane between the rounds (more than one only for columns too
-// long for all of them to fit).
-__global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kColPairs * kDirMaxComponents)
+// waits in the first launch's plane or, where there is none (kRow), in the filtered plane
+// between the rounds (more than one only for columns too long for all of them to fit).
+template <bool kRow>
+__global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kColPairs * kDirMaxComponents, 4)
     dir_cols_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();
@@ -211,6 +214,7 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
             if (P.base[nch] && warp < lp::kColPairs) lp::prefetch_line(P.base[nch], first + warp, H);
         }
     }
+    lp::StripSum out{P.base[ch], P.filtered[ch], W, false, P.raw_weight != 0.0f ? P.raw[ch] : nullptr, W, P.raw_weight};
     int k = 0;
     do {
         float weight[lp::kMaxRecursions];
@@ -233,7 +237,12 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         }
         while (k < P.count && P.comp[k].op != kDirOpYvv) ++k;
         cluster.sync();
-        lp::strip_sum(lp::StripSum{P.base[ch], P.filtered[ch], W, k >= P.count}, lines, weight, count, W, H);
+        out.last = k >= P.count;
+        lp::strip_sum<kRow>(out, lines, weight, count, W, H);
+        if constexpr (kRow) {
+            out.row = P.filtered[ch];
+            out.row_weight = 1.0f;
+        }
         cluster.sync(); // the other CTA has read these lines
     } while (k < P.count);
 }
@@ -249,11 +258,10 @@ bool dir_lines_plan(DirBlurParams& P) {
                               : c.op == kDirOpYvv ? !c.factored : c.op != kDirOpIdentity)
             return false;
         lines += c.op == kDirOpYvv;
-        base |= c.op != kDirOpYvv;
+        base |= c.op == kDirOpFir;
     }
     const int recursions = lp::recursions_per_cta(lines, P.height);
     if (lp::kRowWarps * lp::line_bytes(P.width) > lp::kSmemLimit || recursions < 1) return false;
-    base |= lines > recursions; // the sum waits there between the rounds
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.region) + 31) / 32 * 32);
     const size_t starts = 3 * (size_t)kDirMaxComponents * 3 * (P.height + 2 * (size_t)lp::plane_pairs(P.width)) * 2; // floats
@@ -326,11 +334,12 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
     }
     const int warps = P.recursions * lp::kColPairs;
     const size_t smem = warps * lp::line_bytes(P.height);
-    e = cudaFuncSetAttribute(dir_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto* k = P.base[0] ? dir_cols_kernel<false> : dir_cols_kernel<true>;
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);
     fjb::count_launch();
-    dir_cols_kernel<<<dim3(lp::plane_pairs(P.width) / lp::kColPairs, 3), 32 * warps, smem, s>>>(P);
+    k<<<dim3(lp::plane_pairs(P.width) / lp::kColPairs, 3), 32 * warps, smem, s>>>(P);
     return cudaGetLastError();
 }
 

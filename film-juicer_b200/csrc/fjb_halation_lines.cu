@@ -134,7 +134,7 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         }
         while (gi < J.count && !is_yvv(J.g[gi].kind)) ++gi;
         cluster.sync();
-        lp::strip_sum(lp::StripSum{J.base, J.src, J.stride, gi >= J.count}, lines, weight, count, W, H);
+        lp::strip_sum<false>(lp::StripSum{J.base, J.src, J.stride, gi >= J.count}, lines, weight, count, W, H);
         cluster.sync(); // the other CTA has read these lines
     } while (gi < J.count);
 }
