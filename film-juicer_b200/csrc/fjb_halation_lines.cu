@@ -4,7 +4,8 @@
 // src/Cuda/Film/JuicerCudaScatterHalation.cu:690-852). Both combinations are weighted sums
 // of the carrier and its Gaussians, so a pass is
 //   taps    : the carrier's own share and every short Gaussian, both axes, summed into one
-//             plane per channel (fjb_fir2d.cuh);
+//             plane per channel (fjb_fir2d.cuh); channels without a short Gaussian do
+//             without it where the scratch has no room for that plane;
 //   rows    : every recursive Gaussian's row pass, two rows per warp (fjb_line_pairs.cuh);
 //   columns : a strip of columns per CTA, one warp per pair of columns and recursive
 //             Gaussian, then the weighted sum of all of them and the plane of the first
@@ -96,9 +97,9 @@ __global__ void __launch_bounds__(32 * lp::kRowWarps) optic_rows_kernel(const __
 }
 
 // Two pairs of columns per CTA, P.recursions recursive Gaussians at a time; the sum so far
-// waits in the first launch's plane between the rounds (more than one only for columns too
-// long for all recursions of the channel to fit).
-template <bool kLong>
+// waits in the first launch's plane or, where channels have none (kRow), in the carrier between
+// the rounds (more than one only for columns too long for all recursions of the channel to fit).
+template <bool kLong, bool kRow>
 __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kMaxColWarps)
     optic_cols_kernel(const __grid_constant__ OpticPass P) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -115,9 +116,10 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
             for (int i = 0; i < N.count; ++i)
                 if (is_yvv(N.g[i].kind) && slot++ == warp / lp::kColPairs)
                     lp::prefetch_line(N.temp[i], next % gridDim.x * lp::kColPairs + warp % lp::kColPairs, H);
-            if (warp < lp::kColPairs) lp::prefetch_line(N.base, next % gridDim.x * lp::kColPairs + warp, H);
+            if (N.base && warp < lp::kColPairs) lp::prefetch_line(N.base, next % gridDim.x * lp::kColPairs + warp, H);
         }
     }
+    lp::StripSum out{J.base, J.src, J.stride, false, J.src, J.stride, J.carrier_weight};
     int gi = 0;
     do {
         float weight[lp::kMaxRecursions];
@@ -134,7 +136,12 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         }
         while (gi < J.count && !is_yvv(J.g[gi].kind)) ++gi;
         cluster.sync();
-        lp::strip_sum<false>(lp::StripSum{J.base, J.src, J.stride, gi >= J.count}, lines, weight, count, W, H);
+        out.last = gi >= J.count;
+        lp::strip_sum<kRow>(out, lines, weight, count, W, H);
+        if constexpr (kRow) {
+            out.base = nullptr;
+            out.row_weight = 1.0f;
+        }
         cluster.sync(); // the other CTA has read these lines
     } while (gi < J.count);
 }
@@ -155,23 +162,33 @@ static void balance_weights(OpticJob& J, double carrier, const double* exact) {
     if (least >= 0) J.weight[least] = (float)((double)J.weight[least] + left);
 }
 
-// Whether this form covers the pass: four rows and two pairs of columns fit in shared memory,
-// and the planes between the launches fit the pass's scratch.
+// Whether this form covers the pass: four rows and two pairs of columns fit in shared memory
+// (lines up to 14528 samples), and the planes between the launches, whole sectors of rows and
+// columns each, fit the pass's scratch (frames a few samples wide may exceed it).
 bool optic_lines_plan(OpticPass& P) {
     int most = 1;
-    size_t planes = 0;
+    size_t planes = 0, taps = 0;
+    bool fir[3] = {};
     for (int j = 0; j < P.jobs; ++j) {
         const OpticJob& J = P.job[j];
         int n = 0;
-        for (int g = 0; g < J.count; ++g) n += is_yvv(J.g[g].kind);
-        planes += n + 1;
+        for (int g = 0; g < J.count; ++g) {
+            n += is_yvv(J.g[g].kind);
+            fir[j] |= J.g[g].kind == kGaussFir;
+        }
+        planes += n;
+        taps += fir[j];
         most = n > most ? n : most;
     }
     const int recursions = lp::recursions_per_cta(most, P.height);
     if (lp::kRowWarps * lp::line_bytes(P.width) > lp::kSmemLimit || recursions < 1) return false;
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.scratch) + 31) / 32 * 32);
-    if ((size_t)(next - P.scratch) + planes * plane > P.scratch_floats) return false;
+    const size_t room = P.scratch_floats - (size_t)(next - P.scratch);
+    // one plane per channel for the taps' sums; with five recursive bounces on three channels
+    // only where there are taps
+    P.taps_for_all = (planes + P.jobs) * plane <= room;
+    if ((planes + taps) * plane > room) return false;
     P.recursions = recursions;
     for (int j = 0; j < P.jobs; ++j) {
         OpticJob& J = P.job[j];
@@ -198,8 +215,8 @@ bool optic_lines_plan(OpticPass& P) {
         }
         J.carrier_weight = (float)carrier;
         balance_weights(J, carrier, exact);
-        J.base = next;
-        next += plane;
+        J.base = P.taps_for_all || fir[j] ? next : nullptr;
+        if (J.base) next += plane;
     }
     return true;
 }
@@ -229,12 +246,14 @@ cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
             t.weight = J.weight[g];
             for (int i = 0; i < 2 * kOpticMaxFirRadius + 1; ++i) t.w[i] = q.w[i];
         }
-        F.job[F.count++] = f;
+        if (f.dst) F.job[F.count++] = f;
     }
     cudaError_t e = cudaSuccess;
-    fjb::count_launch();
-    fir::kernel<float><<<fir::grid(F), fir::kThreads, 0, s>>>(F);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (F.count) {
+        fjb::count_launch();
+        fir::kernel<float><<<fir::grid(F), fir::kThreads, 0, s>>>(F);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     if (rows) {
         const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
         auto* k = direct && lp::direct_chunks(P.width) > 1 ? optic_rows_kernel<true> : optic_rows_kernel<false>;
@@ -247,7 +266,9 @@ cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
     }
     const int warps = P.recursions * lp::kColPairs;
     const size_t smem = warps * lp::line_bytes(P.height);
-    auto* k = direct && lp::direct_chunks(P.height) > 1 ? optic_cols_kernel<true> : optic_cols_kernel<false>;
+    auto* k = direct && lp::direct_chunks(P.height) > 1
+                  ? (P.taps_for_all ? optic_cols_kernel<true, false> : optic_cols_kernel<true, true>)
+                  : (P.taps_for_all ? optic_cols_kernel<false, false> : optic_cols_kernel<false, true>);
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);

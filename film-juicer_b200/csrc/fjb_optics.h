@@ -46,7 +46,8 @@ struct OpticJob {
     float amount;      // scatter amount, or bounce total strength
     int renormalize;   // bounce only
     // one warp per pair of lines: the combination as weights of the carrier and of each
-    // Gaussian, and the plane the column launch adds its Gaussians to
+    // Gaussian, and the plane the column launch adds its Gaussians to (null: the carrier
+    // times its weight)
     float carrier_weight;
     float weight[kOpticMaxGauss];
     float* base;
@@ -62,10 +63,12 @@ struct OpticPass {
     float* edge_b;
     int lines_max, segs_max;
     // the whole scratch of the stage; one warp per pair of lines: the recursions a column
-    // CTA holds at once, and the rows and column CTAs between a CTA and the one after it
+    // CTA holds at once, the rows and column CTAs between a CTA and the one after it, and
+    // whether every job has a plane `base`
     float* scratch;
     size_t scratch_floats;
     int recursions, rows_ahead, cols_ahead;
+    bool taps_for_all;
 };
 
 cudaError_t launch_optic_pass(OpticPass& P, cudaStream_t stream);

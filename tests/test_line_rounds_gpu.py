@@ -64,3 +64,24 @@ def test_four_recursive_components(torch_cuda, w, h):
     # sigma 4 and up: starts, rows, starts, columns
     sd = descriptors.spatial_dir_record(5.0, w, h, diffusion_size_um=20.0, tail_um=60.0, tail_weight=0.3)
     check_dir(torch_cuda, sd, planes(w, h, 5), 4)
+
+
+@pytest.mark.parametrize("legacy", [True, False])
+@pytest.mark.parametrize("w,h,bounces", [(640, 360, 5), (643, 361, 5), (640, 360, 4), (800, 3300, 5)])
+def test_recursive_bounces_on_three_channels(torch_cuda, prepare, w, h, bounces, legacy):
+    """Five bounces take all planes of the scratch; 3300 rows take two rounds of columns."""
+    from film_juicer_b200 import runtime
+    from oracle import optics
+
+    torch = torch_cuda
+    weights = (0.4, 0.25, 0.15, 0.1, 0.1)[:bounces]
+    d = prepare.scatter_halation_record(9.11, scatter_amount=0.0, strength=(0.1, 0.05, 0.02), bounce_weights=weights,
+                                        legacy=legacy)
+    src = planes(w, h, 6)
+    dev = [torch.from_numpy(p).cuda() for p in src]
+    # rows and columns; at 640x360 four bounces leave room for the taps' plane, which carries
+    # the carrier's own share
+    assert launches(torch, lambda: runtime.scatter_halation(d, dev)) == (3 if bounces < 5 else 2)
+    for t, r in zip(dev, optics.scatter_halation(d, src)):
+        g = t.cpu().numpy()
+        assert np.all(np.abs(g - r) <= 2e-5 + 2e-5 * np.abs(r)), float(np.abs(g - r).max())
