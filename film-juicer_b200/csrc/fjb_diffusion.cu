@@ -174,7 +174,7 @@ cudaError_t launch_diffusion(const float* const psf_rows[3], int radius, int tap
     }
     const size_t smem = diffusion_smem_bytes(radius);
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(diffusion_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = fjb::allow_dynamic_smem(diffusion_kernel, smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((width + kTileW - 1) / kTileW, (height + kTileH - 1) / kTileH, 3);
     fjb::count_launch();

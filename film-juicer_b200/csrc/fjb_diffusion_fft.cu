@@ -506,10 +506,6 @@ size_t rows_smem(const DiffusionFftPlan& p) {
 }
 size_t cols_smem(const DiffusionFftPlan& p) { return ((size_t)p.cols_per_cta + 1) * p.ny * sizeof(float2); }
 
-cudaError_t set_smem(const void* fn, size_t bytes) {
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 } // namespace
 
 bool diffusion_fft_plan(int width, int height, int radius, DiffusionFftPlan& p) {
@@ -592,8 +588,8 @@ cudaError_t launch_diffusion_fft_spectrum(const DiffusionFftPlan& p, const float
     twiddle_kernel<<<(p.ny + 255) / 256, 256, 0, stream>>>(tw + p.ntw, p.ny);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t rs = rows_smem(p), cs = cols_smem(p);
-    if ((e = set_smem((const void*)rows_r2c_kernel<true>, rs)) != cudaSuccess) return e;
-    if ((e = set_smem((const void*)columns_kernel<true>, cs)) != cudaSuccess) return e;
+    if ((e = fjb::allow_dynamic_smem(rows_r2c_kernel<true>, rs)) != cudaSuccess) return e;
+    if ((e = fjb::allow_dynamic_smem(columns_kernel<true>, cs)) != cudaSuccess) return e;
     const int psf_rows_n = 2 * p.radius + 1;
     fjb::count_launch();
     rows_r2c_kernel<true><<<dim3((psf_rows_n + p.rows_per_cta - 1) / p.rows_per_cta, 3), kFftThreads, rs, stream>>>(F);
@@ -620,9 +616,9 @@ cudaError_t launch_diffusion_fft(const DiffusionFftPlan& p, const float* spectru
     F.fraction = fraction;
     cudaError_t e;
     const size_t rs = rows_smem(p), cs = cols_smem(p);
-    if ((e = set_smem((const void*)rows_r2c_kernel<false>, rs)) != cudaSuccess) return e;
-    if ((e = set_smem((const void*)columns_kernel<false>, cs)) != cudaSuccess) return e;
-    if ((e = set_smem((const void*)rows_c2r_kernel, rs)) != cudaSuccess) return e;
+    if ((e = fjb::allow_dynamic_smem(rows_r2c_kernel<false>, rs)) != cudaSuccess) return e;
+    if ((e = fjb::allow_dynamic_smem(columns_kernel<false>, cs)) != cudaSuccess) return e;
+    if ((e = fjb::allow_dynamic_smem(rows_c2r_kernel, rs)) != cudaSuccess) return e;
     fjb::count_launch();
     rows_r2c_kernel<false><<<dim3((p.ey + p.rows_per_cta - 1) / p.rows_per_cta, 3), kFftThreads, rs, stream>>>(F);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -321,7 +321,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
-        e = cudaFuncSetAttribute(dir_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = fjb::allow_dynamic_smem(dir_rows_kernel, smem);
         if (e != cudaSuccess) return e;
         P.rows_ahead = 2 * lp::kRowWarps * lp::resident_ctas(smem);
         fjb::count_launch();
@@ -335,7 +335,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
     const int warps = P.recursions * lp::kColPairs;
     const size_t smem = warps * lp::line_bytes(P.height);
     auto* k = P.base[0] ? dir_cols_kernel<false> : dir_cols_kernel<true>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = fjb::allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);
     fjb::count_launch();

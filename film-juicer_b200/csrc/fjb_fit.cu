@@ -49,6 +49,7 @@ static_assert((kFitThreads & (kFitThreads - 1)) == 0, "the block sum is a power-
 using FitAcc = float;
 constexpr int kFitRun = 16;
 constexpr int kFitParams = 13;
+constexpr size_t kFitSumsBytes = (size_t)kFitParams * kFitThreads * sizeof(double);
 constexpr float kLn2 = 0.69314718055994530942f;
 constexpr float kLn10 = 2.30258509299404568402f;
 
@@ -821,11 +822,13 @@ cudaError_t launch_fit_forward(const PixelParams& p, const FitTheta& th, const F
     count_launch();
     if (p.route == kRoutePrint) {
         auto* k = fit_forward_kernel<true, kCarrier, kSpatial>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_dynamic_smem(k, smem);
+        if (e != cudaSuccess) return e;
         k<<<fit_blocks(kForwardBlocks), kFitThreads, smem, s>>>(p, th, cr, out_r, out_g, out_b);
     } else {
         auto* k = fit_forward_kernel<false, kCarrier, kSpatial>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_dynamic_smem(k, smem);
+        if (e != cudaSuccess) return e;
         k<<<fit_blocks(kForwardBlocks), kFitThreads, smem, s>>>(p, th, cr, out_r, out_g, out_b);
     }
     return cudaGetLastError();
@@ -840,11 +843,13 @@ cudaError_t launch_fit_vjp(const PixelParams& p, const FitTheta& th, const FitCa
     count_launch();
     if (p.route == kRoutePrint) {
         auto* k = fit_vjp_kernel<true, kCarrier, kSpatial>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_dynamic_smem(k, smem, kFitSumsBytes);
+        if (e != cudaSuccess) return e;
         k<<<blocks, kFitThreads, smem, s>>>(p, th, cr, grad_r, grad_g, grad_b, partials);
     } else {
         auto* k = fit_vjp_kernel<false, kCarrier, kSpatial>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_dynamic_smem(k, smem, kFitSumsBytes);
+        if (e != cudaSuccess) return e;
         k<<<blocks, kFitThreads, smem, s>>>(p, th, cr, grad_r, grad_g, grad_b, partials);
     }
     cudaError_t e = cudaGetLastError();
@@ -861,7 +866,8 @@ cudaError_t launch_fit_dir_source(const PixelParams& p, const FitTheta& th, cons
     const size_t smem = (size_t)p.curve_blob_floats * sizeof(float);
     count_launch();
     auto* k = fit_dir_source_kernel<true>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_dynamic_smem(k, smem);
+    if (e != cudaSuccess) return e;
     k<<<fit_blocks(kPartialBlocks), kFitThreads, smem, s>>>(p, th, cr, out_y, out_m, out_c);
     return cudaGetLastError();
 }
@@ -873,9 +879,10 @@ cudaError_t launch_fit_dir_source_vjp(const PixelParams& p, const FitTheta& th, 
     const size_t smem = (size_t)p.curve_blob_floats * sizeof(float);
     count_launch();
     auto* k = fit_dir_source_vjp_kernel<true>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k, smem, kFitThreads * sizeof(double));
+    if (e != cudaSuccess) return e;
     k<<<blocks, kFitThreads, smem, s>>>(p, th, cr, g_y, g_m, g_c, partials);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e == cudaSuccess) {
         count_launch();
         fit_reduce_kernel<<<kFitParams, kFitThreads, 0, s>>>(partials, blocks, grad_params);

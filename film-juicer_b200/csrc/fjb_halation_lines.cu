@@ -257,7 +257,7 @@ cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
     if (rows) {
         const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
         auto* k = direct && lp::direct_chunks(P.width) > 1 ? optic_rows_kernel<true> : optic_rows_kernel<false>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = fjb::allow_dynamic_smem(k, smem);
         if (e != cudaSuccess) return e;
         P.rows_ahead = 2 * lp::kRowWarps * lp::resident_ctas(smem);
         fjb::count_launch();
@@ -269,7 +269,7 @@ cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
     auto* k = direct && lp::direct_chunks(P.height) > 1
                   ? (P.taps_for_all ? optic_cols_kernel<true, false> : optic_cols_kernel<true, true>)
                   : (P.taps_for_all ? optic_cols_kernel<false, false> : optic_cols_kernel<false, true>);
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = fjb::allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);
     fjb::count_launch();

@@ -346,10 +346,8 @@ static int persistent_grid(long long total, const void* kernel, size_t smem) {
 template <int In, int Out, bool Print, bool SpatialDir>
 static cudaError_t launch_variant(const PixelParams& p, long long total, size_t smem, cudaStream_t stream) {
     auto* k = pixel_chain_kernel<In, Out, Print, SpatialDir>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = fjb::allow_dynamic_smem(k, smem);
+    if (e != cudaSuccess) return e;
     const int grid = persistent_grid(total, reinterpret_cast<const void*>(k), smem);
     fjb::count_launch();
     k<<<grid, kPixelThreads, smem, stream>>>(p);

@@ -224,7 +224,7 @@ cudaError_t blur_rows(float* const* planes, float* const* tmps, int count, int w
         out.p[c] = tmps[c];
     }
     const size_t smem = rows_smem_bytes(radius);
-    cudaError_t e = cudaFuncSetAttribute(blur_rows_run_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = fjb::allow_dynamic_smem(blur_rows_run_kernel, smem);
     if (e != cudaSuccess) return e;
     fjb::count_launch();
     blur_rows_run_kernel<<<dim3((width + kSegment - 1) / kSegment, (height + kRowWarps - 1) / kRowWarps, count),
@@ -241,7 +241,7 @@ cudaError_t blur_cols(float* const* planes, float* const* tmps, int count, int w
         io.p[c] = planes[c];
     }
     const size_t smem = taps_bytes(radius);
-    cudaError_t e = cudaFuncSetAttribute(blur_cols_run_kernel<kUnsharp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = fjb::allow_dynamic_smem(blur_cols_run_kernel<kUnsharp>, smem);
     if (e != cudaSuccess) return e;
     const int runs = (height + kRun - 1) / kRun;
     fjb::count_launch();
