@@ -23,7 +23,8 @@ namespace {
 // pool keeps at most kKeep bytes between calls (it grows by chunks of 32 MB: with a smaller
 // bound each synchronisation gave the chunk back, and the next call took 2.5 ms); what a call
 // needs beyond that goes back at the next synchronisation. Allocation is ordered by stream
-// and safe from several threads.
+// and safe from several threads. There is a pool per device and context, so that a call
+// after cudaDeviceReset makes its own.
 class CallMemory {
   public:
     cudaError_t allocate(size_t bytes, cudaStream_t s) {
@@ -40,30 +41,50 @@ class CallMemory {
 
   private:
     static constexpr uint64_t kKeep = 64ull << 20;
-    static constexpr int kMaxDevices = 64;
+    // Number of the current context, never given twice: cudaDeviceReset destroys the pools of a
+    // device, and the context made after it has another number. 0 where the driver cannot tell.
+    static unsigned long long context_number() {
+        using GetId = int (*)(void*, unsigned long long*);
+        static const GetId get = [] {
+            void* f = nullptr;
+            cudaDriverEntryPointQueryResult found{};
+            const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found) == cudaSuccess &&
+                            found == cudaDriverEntryPointSuccess;
+            return ok ? reinterpret_cast<GetId>(f) : nullptr;
+        }();
+        unsigned long long id = 0;
+        return get && get(nullptr, &id) == 0 ? id : 0;
+    }
+    struct DevicePool {
+        int device;
+        unsigned long long context;
+        cudaMemPool_t pool;
+    };
     static cudaError_t device_pool(cudaMemPool_t& pool) {
         static std::mutex gate;
-        static cudaMemPool_t pools[kMaxDevices] = {};
+        static std::vector<DevicePool> pools;
         int device = 0;
         cudaError_t e = cudaGetDevice(&device);
+        if (e == cudaSuccess) e = cudaFree(nullptr); // makes the device's context current
         if (e != cudaSuccess) return e;
-        if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+        const unsigned long long context = context_number();
         std::lock_guard<std::mutex> lock(gate);
-        if (!pools[device]) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = device;
-            cudaMemPool_t fresh = nullptr;
-            if ((e = cudaMemPoolCreate(&fresh, &props)) != cudaSuccess) return e;
-            uint64_t keep = kKeep;
-            if ((e = cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-                cudaMemPoolDestroy(fresh);
-                return e;
+        for (const DevicePool& p : pools)
+            if (p.device == device && p.context == context) {
+                pool = p.pool;
+                return cudaSuccess;
             }
-            pools[device] = fresh;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+        uint64_t keep = kKeep;
+        if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
         }
-        pool = pools[device];
+        pools.push_back({device, context, pool});
         return cudaSuccess;
     }
     void* data_ = nullptr;

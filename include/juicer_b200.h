@@ -408,7 +408,9 @@ FjStatus fjb_diffusion_components_host(const FjDiffusion* diffusion, FjDiffusion
  * JuicerCuda::Diffusion::launch_stage): dst_c = (1 - f) src_c + f (PSF_c * src_c) with
  * PSF_c = sum_k w_ck exp(-rho / lambda_k) / (2 pi lambda_k^2) on the (2r+1)^2 grid,
  * normalised, and whole-sample reflection at the frame border. Planes R, G, B with
- * `stride` floats per row; dst must not alias src. radius_px <= 80. */
+ * `stride` floats per row; dst must not alias src. radius_px <= 80. Synchronises
+ * `stream`. Device memory for the PSF and the transforms comes from a pool of the
+ * library's, which keeps at most 64 MB per device between calls. */
 FjStatus fjb_diffusion(const FjDiffusionComponents* components, int32_t radius_px, double scatter_fraction,
                        const float* src_r, const float* src_g, const float* src_b, float* dst_r, float* dst_g,
                        float* dst_b, ptrdiff_t stride, int32_t width, int32_t height, void* stream,
