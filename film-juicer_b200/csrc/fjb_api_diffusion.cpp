@@ -24,11 +24,16 @@ namespace {
 // bound each synchronisation gave the chunk back, and the next call took 2.5 ms); what a call
 // needs beyond that goes back at the next synchronisation. Allocation is ordered by stream
 // and safe from several threads. There is a pool per device and context, so that a call
-// after cudaDeviceReset makes its own.
+// after cudaDeviceReset makes its own. Above kLargest a call is better off with a cudaMalloc and
+// cudaFree of its own than with the pool growing and giving back that much (7680x4320, radius
+// 41 and 60: 8.8 and 9.1 ms with the pool, 6.4 and 6.7 without; 3840x2160, 210 MB: the same;
+// 1920x1080: 0.55 and 1.23).
 class CallMemory {
   public:
     cudaError_t allocate(size_t bytes, cudaStream_t s) {
         stream_ = s;
+        pooled_ = bytes <= kLargest;
+        if (!pooled_) return cudaMalloc(&data_, bytes);
         cudaMemPool_t pool = nullptr;
         cudaError_t e = device_pool(pool);
         if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&data_, bytes, pool, s);
@@ -36,11 +41,16 @@ class CallMemory {
     }
     float* data() const { return static_cast<float*>(data_); }
     ~CallMemory() {
-        if (data_) cudaFreeAsync(data_, stream_);
+        if (!data_) return;
+        if (pooled_)
+            cudaFreeAsync(data_, stream_);
+        else
+            cudaFree(data_);
     }
 
   private:
     static constexpr uint64_t kKeep = 64ull << 20;
+    static constexpr size_t kLargest = (size_t)256 << 20;
     // Number of the current context, never given twice: cudaDeviceReset destroys the pools of a
     // device, and the context made after it has another number. 0 where the driver cannot tell.
     static unsigned long long context_number() {
@@ -88,6 +98,7 @@ class CallMemory {
         return cudaSuccess;
     }
     void* data_ = nullptr;
+    bool pooled_ = true;
     cudaStream_t stream_ = nullptr;
 };
 
