@@ -7,6 +7,8 @@
 // (src/Cuda/JuicerCudaDeviceHelpers.cuh:1267-1328).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include <string>
 
 #include "../../include/juicer_b200.h"
@@ -110,7 +112,9 @@ extern "C" {
 size_t fjb_spatial_dir_scratch_bytes(int32_t width, int32_t height) {
     if (width <= 0 || height <= 0) return 0;
     const size_t planes = (size_t)(3 + 3 * fjb::kDirMaxComponents) * (size_t)width * (size_t)height * sizeof(float);
-    return (planes + 255) / 256 * 256 + fjb::dir_recursion_bytes(width, height);
+    // frames a few samples wide: the line form's padded planes take more than the recursion buffers
+    const size_t lines = (3 * (size_t)width * (size_t)height + fjb::dir_lines_floats(width, height)) * sizeof(float);
+    return std::max((planes + 255) / 256 * 256 + fjb::dir_recursion_bytes(width, height), lines);
 }
 
 FjStatus fjb_spatial_dir_build(FjbRecipe* recipe, const FjSpatialDir* spatial_dir, const float* src,

@@ -75,13 +75,14 @@ struct DirBlurParams {
     double* start;
     int lines_max, segs_max;
     // everything after the scratch's first three planes; one warp per pair of lines: the
-    // recursions a column CTA holds at once, the rows and column CTAs between a CTA and the one
-    // after it, the planes of the short components' sums that the column launch adds its own to
-    // (null: there are none), the identity component's weight, and the reflected starts of rows
-    // and columns (direct form, per channel, component and line)
+    // pairs a row and a column CTA hold, the recursions a column CTA holds at once, the rows and
+    // column CTAs between a CTA and the one after it, the planes of the short components' sums
+    // that the column launch adds its own to (null: there are none), the identity component's
+    // weight, and the reflected starts of rows and columns (direct form, per channel, component
+    // and line)
     float* region;
     size_t region_floats;
-    int recursions, rows_ahead, cols_ahead;
+    int row_warps, col_pairs, recursions, rows_ahead, cols_ahead;
     float* base[3];
     float raw_weight;
     double* row_start;
@@ -95,6 +96,9 @@ size_t dir_recursion_bytes(int width, int height);
 int dir_segments(int n);
 
 cudaError_t launch_dir_blur(DirBlurParams& p, cudaStream_t stream);
+
+// Floats that the form with one warp per pair of lines needs after the scratch's first three planes.
+size_t dir_lines_floats(int width, int height);
 
 // One warp per pair of lines (fjb_dir_lines.cu): false when the pass is out of its range
 // (line lengths, a component in the FP64 direct form, taps beyond radius 9); true lays the

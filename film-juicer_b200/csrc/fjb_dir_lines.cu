@@ -163,8 +163,9 @@ __device__ __forceinline__ void filter(const DirComponentDev& c, const double* f
     __syncwarp();
 }
 
-// Four rows of one channel per CTA through every recursive component.
-__global__ void __launch_bounds__(32 * lp::kRowWarps) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
+// Four rows of one channel per CTA (kWarps pairs) through every recursive component.
+template <int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int ch = blockIdx.y;
     const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(32 * lp::kRowWarps) dir_rows_kernel(const __gr
     Pair* rows = reinterpret_cast<Pair*>(sm);
     Pair* buf = rows + warp * words;
     // rows past the frame's end repeat the last one; their results land in the planes' padding
-    const int y0 = 2 * lp::kRowWarps * blockIdx.x, y = y0 + 2 * warp;
+    const int y0 = 2 * kWarps * blockIdx.x, y = y0 + 2 * warp;
     const float* a = P.raw[ch] + (size_t)min(y, H - 1) * W;
     const float* b = P.raw[ch] + (size_t)min(y + 1, H - 1) * W;
     if (lane < 2 && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (size_t)(lane + P.rows_ahead) * W, W);
@@ -187,15 +188,16 @@ __global__ void __launch_bounds__(32 * lp::kRowWarps) dir_rows_kernel(const __gr
         for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + (size_t)min(y + h / 3, H - 1) * 3 + h % 3);
         lp::load_rows(buf, a, b, W, lane);
         filter<false>(c, from, buf, W, lane);
-        lp::store_pairs(rows, words, P.temp[ch][k], W, H, y0);
+        lp::store_pairs<kWarps>(rows, words, P.temp[ch][k], W, H, y0);
     }
 }
 
-// Two pairs of columns per CTA, P.recursions recursive components at a time; the sum so far
+// kPairs pairs of columns per CTA, P.recursions recursive components at a time; the sum so far
 // waits in the first launch's plane or, where there is none (kRow), in the filtered plane
 // between the rounds (more than one only for columns too long for all of them to fit).
-template <bool kRow>
-__global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kColPairs * kDirMaxComponents, 4)
+template <bool kRow, int kPairs>
+__global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
+    __launch_bounds__(32 * kPairs * kDirMaxComponents, kPairs == lp::kColPairs ? 4 : 1)
     dir_cols_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();
@@ -206,12 +208,12 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
     if (lane == 0) {
         const unsigned next = blockIdx.y * gridDim.x + blockIdx.x + P.cols_ahead;
         if (next < gridDim.x * gridDim.y) {
-            const int first = next % gridDim.x * lp::kColPairs, nch = next / gridDim.x;
+            const int first = next % gridDim.x * kPairs, nch = next / gridDim.x;
             int slot = 0;
             for (int i = 0; i < P.count; ++i)
-                if (P.comp[i].op == kDirOpYvv && slot++ == warp / lp::kColPairs)
-                    lp::prefetch_line(P.temp[nch][i], first + warp % lp::kColPairs, H);
-            if (P.base[nch] && warp < lp::kColPairs) lp::prefetch_line(P.base[nch], first + warp, H);
+                if (P.comp[i].op == kDirOpYvv && slot++ == warp / kPairs)
+                    lp::prefetch_line(P.temp[nch][i], first + warp % kPairs, H);
+            if (P.base[nch] && warp < kPairs) lp::prefetch_line(P.base[nch], first + warp, H);
         }
     }
     lp::StripSum out{P.base[ch], P.filtered[ch], W, false, P.raw_weight != 0.0f ? P.raw[ch] : nullptr, W, P.raw_weight};
@@ -223,8 +225,8 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         for (; k < P.count && count < P.recursions; ++k) {
             const DirComponentDev& c = P.comp[k];
             if (c.op != kDirOpYvv) continue;
-            if (warp / lp::kColPairs == count) {
-                const int pair = blockIdx.x * lp::kColPairs + warp % lp::kColPairs;
+            if (warp / kPairs == count) {
+                const int pair = blockIdx.x * kPairs + warp % kPairs;
                 const double* starts =
                     P.col_start + (((size_t)ch * kDirMaxComponents + k) * 2 * lp::plane_pairs(W) + 2 * pair) * 3;
                 double from[6];
@@ -238,16 +240,30 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         while (k < P.count && P.comp[k].op != kDirOpYvv) ++k;
         cluster.sync();
         out.last = k >= P.count;
-        lp::strip_sum<kRow>(out, lines, weight, count, W, H);
+        lp::strip_sum<kRow, kPairs>(out, lines, weight, count, W, H);
         if constexpr (kRow) {
             out.row = P.filtered[ch];
             out.row_weight = 1.0f;
         }
-        cluster.sync(); // the other CTA has read these lines
+        cluster.sync(); // the other CTAs have read these lines
     } while (k < P.count);
 }
 
 } // namespace
+
+namespace {
+
+constexpr size_t kAlignFloats = 8; // planes start on 32 bytes
+size_t starts_floats(int width, int height) {
+    return 3 * (size_t)kDirMaxComponents * 3 * ((size_t)height + 2 * (size_t)lp::plane_pairs(width)) * 2;
+}
+
+} // namespace
+
+// A plane for every component of the three channels (short ones share theirs), and the starts.
+size_t dir_lines_floats(int width, int height) {
+    return kAlignFloats + 3 * (size_t)kDirMaxComponents * lp::plane_floats(width, height) + starts_floats(width, height);
+}
 
 bool dir_lines_plan(DirBlurParams& P) {
     int lines = 0;
@@ -260,13 +276,14 @@ bool dir_lines_plan(DirBlurParams& P) {
         lines += c.op == kDirOpYvv;
         base |= c.op == kDirOpFir;
     }
-    const int recursions = lp::recursions_per_cta(lines, P.height);
-    if (lp::kRowWarps * lp::line_bytes(P.width) > lp::kSmemLimit || recursions < 1) return false;
+    P.row_warps = lp::rows_per_cta(P.width);
+    P.col_pairs = lp::pairs_per_cta(P.height);
+    if (P.row_warps < 1 || P.col_pairs < 1) return false;
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.region) + 31) / 32 * 32);
-    const size_t starts = 3 * (size_t)kDirMaxComponents * 3 * (P.height + 2 * (size_t)lp::plane_pairs(P.width)) * 2; // floats
-    if ((size_t)(next - P.region) + 3 * (size_t)(lines + base) * plane + starts > P.region_floats) return false;
-    P.recursions = recursions;
+    if ((size_t)(next - P.region) + 3 * (size_t)(lines + base) * plane + starts_floats(P.width, P.height) > P.region_floats)
+        return false;
+    P.recursions = lp::recursions_per_cta(lines, P.col_pairs, P.height);
     P.raw_weight = 0.0f;
     for (int k = 0; k < P.count; ++k) {
         DirComponentDev& c = P.comp[k];
@@ -320,26 +337,30 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         fjb::count_launch();
         dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
-        e = fjb::allow_dynamic_smem(dir_rows_kernel, smem);
+        const size_t smem = P.row_warps * lp::line_bytes(P.width);
+        auto* k = P.row_warps == lp::kRowWarps ? dir_rows_kernel<lp::kRowWarps> : dir_rows_kernel<1>;
+        e = fjb::allow_dynamic_smem(k, smem);
         if (e != cudaSuccess) return e;
-        P.rows_ahead = 2 * lp::kRowWarps * lp::resident_ctas(smem);
+        const int rows = 2 * P.row_warps;
+        P.rows_ahead = rows * lp::resident_ctas(smem);
         fjb::count_launch();
-        dir_rows_kernel<<<dim3((P.height + 3) / 4, 3), 32 * lp::kRowWarps, smem, s>>>(P);
+        k<<<dim3((P.height + rows - 1) / rows, 3), 32 * P.row_warps, smem, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         fjb::count_launch();
         dir_starts_kernel<true>
             <<<dim3((2 * lp::plane_pairs(P.width) + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    const int warps = P.recursions * lp::kColPairs;
+    const int warps = P.recursions * P.col_pairs;
     const size_t smem = warps * lp::line_bytes(P.height);
-    auto* k = P.base[0] ? dir_cols_kernel<false> : dir_cols_kernel<true>;
+    auto* k = P.col_pairs == lp::kColPairs
+                  ? (P.base[0] ? dir_cols_kernel<false, lp::kColPairs> : dir_cols_kernel<true, lp::kColPairs>)
+                  : (P.base[0] ? dir_cols_kernel<false, 1> : dir_cols_kernel<true, 1>);
     e = fjb::allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);
     fjb::count_launch();
-    k<<<dim3(lp::plane_pairs(P.width) / lp::kColPairs, 3), 32 * warps, smem, s>>>(P);
+    k<<<dim3(lp::plane_pairs(P.width) / P.col_pairs, 3), 32 * warps, smem, s>>>(P);
     return cudaGetLastError();
 }
 

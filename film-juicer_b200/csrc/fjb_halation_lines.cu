@@ -72,9 +72,9 @@ __device__ __forceinline__ void filter(const OpticGauss& g, Pair* line, int n, i
     }
 }
 
-// Four rows of one channel per CTA through every recursive Gaussian of the job.
-template <bool kLong>
-__global__ void __launch_bounds__(32 * lp::kRowWarps) optic_rows_kernel(const __grid_constant__ OpticPass P) {
+// Four rows of one channel per CTA (kWarps pairs) through every recursive Gaussian of the job.
+template <bool kLong, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) optic_rows_kernel(const __grid_constant__ OpticPass P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const OpticJob& J = P.job[blockIdx.y];
     const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(32 * lp::kRowWarps) optic_rows_kernel(const __
     Pair* rows = reinterpret_cast<Pair*>(sm);
     Pair* buf = rows + warp * words;
     // rows past the frame's end repeat the last one; their results land in the planes' padding
-    const int y0 = 2 * lp::kRowWarps * blockIdx.x, y = y0 + 2 * warp;
+    const int y0 = 2 * kWarps * blockIdx.x, y = y0 + 2 * warp;
     const float* a = J.src + (long long)min(y, H - 1) * J.stride;
     const float* b = J.src + (long long)min(y + 1, H - 1) * J.stride;
     if (lane < 2 && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (long long)(lane + P.rows_ahead) * J.stride, W);
@@ -92,15 +92,15 @@ __global__ void __launch_bounds__(32 * lp::kRowWarps) optic_rows_kernel(const __
         if (!is_yvv(g.kind)) continue;
         lp::load_rows(buf, a, b, W, lane);
         filter<false, kLong>(g, buf, W, lane);
-        lp::store_pairs(rows, words, J.temp[gi], W, H, y0);
+        lp::store_pairs<kWarps>(rows, words, J.temp[gi], W, H, y0);
     }
 }
 
-// Two pairs of columns per CTA, P.recursions recursive Gaussians at a time; the sum so far
+// kPairs pairs of columns per CTA, P.recursions recursive Gaussians at a time; the sum so far
 // waits in the first launch's plane or, where channels have none (kRow), in the carrier between
 // the rounds (more than one only for columns too long for all recursions of the channel to fit).
-template <bool kLong, bool kRow>
-__global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * lp::kMaxColWarps)
+template <bool kLong, bool kRow, int kPairs>
+__global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1) __launch_bounds__(32 * lp::kMaxRecursions * kPairs)
     optic_cols_kernel(const __grid_constant__ OpticPass P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();
@@ -114,9 +114,9 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
             const OpticJob& N = P.job[next / gridDim.x];
             int slot = 0;
             for (int i = 0; i < N.count; ++i)
-                if (is_yvv(N.g[i].kind) && slot++ == warp / lp::kColPairs)
-                    lp::prefetch_line(N.temp[i], next % gridDim.x * lp::kColPairs + warp % lp::kColPairs, H);
-            if (N.base && warp < lp::kColPairs) lp::prefetch_line(N.base, next % gridDim.x * lp::kColPairs + warp, H);
+                if (is_yvv(N.g[i].kind) && slot++ == warp / kPairs)
+                    lp::prefetch_line(N.temp[i], next % gridDim.x * kPairs + warp % kPairs, H);
+            if (N.base && warp < kPairs) lp::prefetch_line(N.base, next % gridDim.x * kPairs + warp, H);
         }
     }
     lp::StripSum out{J.base, J.src, J.stride, false, J.src, J.stride, J.carrier_weight};
@@ -128,8 +128,8 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         for (; gi < J.count && count < P.recursions; ++gi) {
             const OpticGauss& g = J.g[gi];
             if (!is_yvv(g.kind)) continue;
-            if (warp / lp::kColPairs == count) {
-                lp::load_line(line, J.temp[gi], blockIdx.x * lp::kColPairs + warp % lp::kColPairs, H, lane);
+            if (warp / kPairs == count) {
+                lp::load_line(line, J.temp[gi], blockIdx.x * kPairs + warp % kPairs, H, lane);
                 filter<true, kLong>(g, line, H, lane);
             }
             weight[count++] = J.weight[gi];
@@ -137,13 +137,20 @@ __global__ void __cluster_dims__(lp::kColCluster, 1, 1) __launch_bounds__(32 * l
         while (gi < J.count && !is_yvv(J.g[gi].kind)) ++gi;
         cluster.sync();
         out.last = gi >= J.count;
-        lp::strip_sum<kRow>(out, lines, weight, count, W, H);
+        lp::strip_sum<kRow, kPairs>(out, lines, weight, count, W, H);
         if constexpr (kRow) {
             out.base = nullptr;
             out.row_weight = 1.0f;
         }
-        cluster.sync(); // the other CTA has read these lines
+        cluster.sync(); // the other CTAs have read these lines
     } while (gi < J.count);
+}
+
+using ColsKernel = void (*)(OpticPass);
+template <int kPairs>
+ColsKernel cols_variant(bool chunks, bool row) {
+    return chunks ? (row ? optic_cols_kernel<true, true, kPairs> : optic_cols_kernel<true, false, kPairs>)
+                  : (row ? optic_cols_kernel<false, true, kPairs> : optic_cols_kernel<false, false, kPairs>);
 }
 
 } // namespace
@@ -162,9 +169,9 @@ static void balance_weights(OpticJob& J, double carrier, const double* exact) {
     if (least >= 0) J.weight[least] = (float)((double)J.weight[least] + left);
 }
 
-// Whether this form covers the pass: four rows and two pairs of columns fit in shared memory
-// (lines up to 14528 samples), and the planes between the launches, whole sectors of rows and
-// columns each, fit the pass's scratch (frames a few samples wide may exceed it).
+// Whether this form covers the pass: a pair of rows and a pair of columns fit in shared memory
+// (lines up to 29056 samples). The planes between the launches, whole sectors of rows and
+// columns each, fit the pass's scratch.
 bool optic_lines_plan(OpticPass& P) {
     int most = 1;
     size_t planes = 0, taps = 0;
@@ -180,8 +187,9 @@ bool optic_lines_plan(OpticPass& P) {
         taps += fir[j];
         most = n > most ? n : most;
     }
-    const int recursions = lp::recursions_per_cta(most, P.height);
-    if (lp::kRowWarps * lp::line_bytes(P.width) > lp::kSmemLimit || recursions < 1) return false;
+    P.row_warps = lp::rows_per_cta(P.width);
+    P.col_pairs = lp::pairs_per_cta(P.height);
+    if (P.row_warps < 1 || P.col_pairs < 1) return false;
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.scratch) + 31) / 32 * 32);
     const size_t room = P.scratch_floats - (size_t)(next - P.scratch);
@@ -189,7 +197,7 @@ bool optic_lines_plan(OpticPass& P) {
     // only where there are taps
     P.taps_for_all = (planes + P.jobs) * plane <= room;
     if ((planes + taps) * plane > room) return false;
-    P.recursions = recursions;
+    P.recursions = lp::recursions_per_cta(most, P.col_pairs, P.height);
     for (int j = 0; j < P.jobs; ++j) {
         OpticJob& J = P.job[j];
         // the combination as weights: scatter (1 - a) x + a ((1 - w) core + w sum_i amp_i tail_i),
@@ -255,25 +263,29 @@ cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (rows) {
-        const size_t smem = lp::kRowWarps * lp::line_bytes(P.width);
-        auto* k = direct && lp::direct_chunks(P.width) > 1 ? optic_rows_kernel<true> : optic_rows_kernel<false>;
+        const size_t smem = P.row_warps * lp::line_bytes(P.width);
+        const bool chunks = direct && lp::direct_chunks(P.width) > 1;
+        auto* k = P.row_warps == lp::kRowWarps
+                      ? (chunks ? optic_rows_kernel<true, lp::kRowWarps> : optic_rows_kernel<false, lp::kRowWarps>)
+                      : (chunks ? optic_rows_kernel<true, 1> : optic_rows_kernel<false, 1>);
         e = fjb::allow_dynamic_smem(k, smem);
         if (e != cudaSuccess) return e;
-        P.rows_ahead = 2 * lp::kRowWarps * lp::resident_ctas(smem);
+        const int lines = 2 * P.row_warps;
+        P.rows_ahead = lines * lp::resident_ctas(smem);
         fjb::count_launch();
-        k<<<dim3((P.height + 3) / 4, P.jobs), 32 * lp::kRowWarps, smem, s>>>(P);
+        k<<<dim3((P.height + lines - 1) / lines, P.jobs), 32 * P.row_warps, smem, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    const int warps = P.recursions * lp::kColPairs;
+    const int warps = P.recursions * P.col_pairs;
     const size_t smem = warps * lp::line_bytes(P.height);
-    auto* k = direct && lp::direct_chunks(P.height) > 1
-                  ? (P.taps_for_all ? optic_cols_kernel<true, false> : optic_cols_kernel<true, true>)
-                  : (P.taps_for_all ? optic_cols_kernel<false, false> : optic_cols_kernel<false, true>);
+    auto* k = P.col_pairs == lp::kColPairs
+                  ? cols_variant<lp::kColPairs>(direct && lp::direct_chunks(P.height) > 1, !P.taps_for_all)
+                  : cols_variant<1>(direct && lp::direct_chunks(P.height) > 1, !P.taps_for_all);
     e = fjb::allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);
     fjb::count_launch();
-    k<<<dim3(lp::plane_pairs(P.width) / lp::kColPairs, P.jobs), 32 * warps, smem, s>>>(P);
+    k<<<dim3(lp::plane_pairs(P.width) / P.col_pairs, P.jobs), 32 * warps, smem, s>>>(P);
     return cudaGetLastError();
 }
 

@@ -20,6 +20,9 @@
 // block. Columns: a CTA holds two pairs of columns for each of a channel's recursions, one
 // warp per pair and recursion; two CTAs (a cluster) sum eight columns in their epilogue
 // through each other's shared memory and write whole sectors of the frame's rows.
+// Lines above 14528 samples: a CTA holds one pair of rows, or of columns (clusters of four);
+// above 29056 not even one pair fits. 16000x2000: DIR 5.3 ms, scatter/halation 7.0; 2000x16000:
+// 5.8 and 7.7; as launches over segments in global memory 10.0, 13.9, 8.6 and 11.9 ms.
 //
 // What bounds it: shared-memory bandwidth, seven 8-byte accesses per pair and position and
 // recursion (28 bytes per sample; 128 bytes per clock and SM), next to one read and one
@@ -48,8 +51,7 @@ constexpr int kPieces = 32;
 constexpr int kRowWarps = 2;      // warps (pairs of rows) of a row CTA
 constexpr int kMaxRecursions = 5; // of one channel
 constexpr int kColPairs = 2;      // pairs of columns of a column CTA
-constexpr int kColCluster = 2;    // column CTAs that write rows together
-constexpr int kMaxColWarps = kMaxRecursions * kColPairs;
+constexpr int kStripPairs = 4;    // pairs of columns whose CTAs (a cluster) write rows together
 constexpr size_t kSmemLimit = 227 * 1024;
 
 // M^(K 2^i): the powers of the one-step zero-input map over one piece.
@@ -320,16 +322,22 @@ __device__ __forceinline__ void load_rows(Pair* buf, const float* a, const float
     __syncwarp();
 }
 
-// The CTA's four rows y .. y + 3 (two pairs, `words` apart) of `width` samples to the plane
-// by pairs of columns: one sector per pair of columns and thread. A barrier before (the
-// rows are complete) and after (the buffers are free).
+// The CTA's rows y .. y + 3 (two pairs, `words` apart) of `width` samples to the plane by
+// pairs of columns: one sector per pair of columns and thread; or its one pair of rows, half a
+// sector. A barrier before (the rows are complete) and after (the buffers are free).
+template <int kWarps>
 __device__ __forceinline__ void store_pairs(const Pair* buf, int words, float* plane, int width, int height, int y) {
+    static_assert(kWarps == 1 || kWarps == 2, "rows of a CTA");
     __syncthreads();
     const int pitch = 2 * line_words(height);
     float* out = plane + 2 * y;
 #pragma unroll 2
-    for (int j = threadIdx.x; 2 * j < width; j += 32 * kRowWarps) {
-        const float4 a = *reinterpret_cast<const float4*>(buf + 2 * j);         // rows y, y + 1 of two columns
+    for (int j = threadIdx.x; 2 * j < width; j += 32 * kWarps) {
+        const float4 a = *reinterpret_cast<const float4*>(buf + 2 * j); // rows y, y + 1 of two columns
+        if constexpr (kWarps == 1) {
+            *reinterpret_cast<float4*>(out + (size_t)j * pitch) = make_float4(a.x, a.z, a.y, a.w);
+            continue;
+        }
         const float4 b = *reinterpret_cast<const float4*>(buf + words + 2 * j); // rows y + 2, y + 3
         asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + (size_t)j * pitch), "f"(a.x),
                      "f"(a.z), "f"(a.y), "f"(a.w), "f"(b.x), "f"(b.z), "f"(b.y), "f"(b.w)
@@ -376,7 +384,7 @@ struct StripSum {
 };
 
 // Eight neighbouring samples of a row, `left` of them inside it; `wide`: in two 16-byte loads.
-__device__ __forceinline__ void row_samples(const float* p, bool wide, int left, float2 (&v)[kColPairs * kColCluster]) {
+__device__ __forceinline__ void row_samples(const float* p, bool wide, int left, float2 (&v)[kStripPairs]) {
     if (wide && left >= 8) {
         const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
         v[0] = make_float2(a.x, a.y);
@@ -390,23 +398,23 @@ __device__ __forceinline__ void row_samples(const float* p, bool wide, int left,
     }
 }
 
-// The epilogue of a column cluster: `count` recursions' lines in both CTAs' shared memory
-// (line i * kColPairs + pair), eight columns of an n x width plane, each CTA half of the
+// The epilogue of a column cluster: `count` recursions' lines in its CTAs' shared memory
+// (line i * kPairs + pair), eight columns of an n x width plane, each CTA its share of the
 // rows. The caller has synchronised the cluster and does so again before the lines go.
 // Without kRow there is a plane by pairs of columns (a variant of its own: with the rest,
 // scatter/halation took 784 us at 3840x2160 instead of 771).
-template <bool kRow>
+template <bool kRow, int kPairs>
 __device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const float* weight, int count, int width, int n) {
-    constexpr int kBatch = 2, kAll = kColPairs * kColCluster;
+    constexpr int kBatch = 2, kAll = kStripPairs, kCluster = kAll / kPairs;
     static_assert(kAll == 4, "row_samples takes eight columns");
     const int words = line_words(n);
-    const unsigned rank = blockIdx.x % kColCluster;
-    const int pair0 = blockIdx.x / kColCluster * kAll, x0 = 2 * pair0;
-    const Pair* side[kColCluster];
+    const unsigned rank = blockIdx.x % kCluster;
+    const int pair0 = blockIdx.x / kCluster * kAll, x0 = 2 * pair0;
+    const Pair* side[kCluster];
 #pragma unroll
-    for (int r = 0; r < kColCluster; ++r) side[r] = cooperative_groups::this_cluster().map_shared_rank(lines, r);
-    const int half = (n + kColCluster - 1) / kColCluster;
-    const int ylo = rank * half, yhi = min(n, ylo + half);
+    for (int r = 0; r < kCluster; ++r) side[r] = cooperative_groups::this_cluster().map_shared_rank(lines, r);
+    const int share = (n + kCluster - 1) / kCluster;
+    const int ylo = rank * share, yhi = min(n, ylo + share);
     float2* base = !kRow || S.base ? reinterpret_cast<float2*>(S.base) + (size_t)pair0 * words : nullptr;
     const bool wide = kRow && S.row && S.row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(S.row) & 15u) == 0;
     const unsigned align = S.dst_stride % 8 == 0 ? (unsigned)(reinterpret_cast<uintptr_t>(S.dst) & 31u) : 4u;
@@ -436,7 +444,7 @@ __device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const 
                 const int y = min(y0 + r * (int)blockDim.x, yhi - 1);
 #pragma unroll
                 for (int q = 0; q < kAll; ++q) {
-                    const float2 v = unpack(side[q / kColPairs][(size_t)(i * kColPairs + q % kColPairs) * words + y]);
+                    const float2 v = unpack(side[q / kPairs][(size_t)(i * kPairs + q % kPairs) * words + y]);
                     sum[r][q].x = fmaf(w, v.x, sum[r][q].x);
                     sum[r][q].y = fmaf(w, v.y, sum[r][q].y);
                 }
@@ -468,11 +476,14 @@ __device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const 
     }
 }
 
-// Recursions a column CTA holds at once, as many as fit; 0: not one.
-inline int recursions_per_cta(int count, int n) {
-    const size_t bytes = kColPairs * line_bytes(n);
+// Pairs of rows of a row CTA; 0: not one fits.
+inline int rows_per_cta(int n) { return std::min(kRowWarps, (int)(kSmemLimit / line_bytes(n))); }
+// Pairs of columns of a column CTA; 0: not one fits.
+inline int pairs_per_cta(int n) { return std::min(kColPairs, (int)(kSmemLimit / line_bytes(n))); }
+// Recursions a column CTA of `pairs` pairs holds at once, as many as fit.
+inline int recursions_per_cta(int count, int pairs, int n) {
     count = std::max(1, std::min(count, kMaxRecursions));
-    return std::min(count, (int)(kSmemLimit / bytes));
+    return std::min(count, (int)(kSmemLimit / (pairs * line_bytes(n))));
 }
 
 } // namespace lp

@@ -62,12 +62,12 @@ struct OpticPass {
     float* edge_a;
     float* edge_b;
     int lines_max, segs_max;
-    // the whole scratch of the stage; one warp per pair of lines: the recursions a column
-    // CTA holds at once, the rows and column CTAs between a CTA and the one after it, and
-    // whether every job has a plane `base`
+    // the whole scratch of the stage; one warp per pair of lines: the pairs a row and a column
+    // CTA hold, the recursions a column CTA holds at once, the rows and column CTAs between a
+    // CTA and the one after it, and whether every job has a plane `base`
     float* scratch;
     size_t scratch_floats;
-    int recursions, rows_ahead, cols_ahead;
+    int row_warps, col_pairs, recursions, rows_ahead, cols_ahead;
     bool taps_for_all;
 };
 

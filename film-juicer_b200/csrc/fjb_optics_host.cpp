@@ -71,9 +71,12 @@ void optic_step_map(const OpticGauss& g, double m[9]) {
 size_t halation_scratch_floats(int width, int height) {
     const size_t lines = (size_t)(width > height ? width : height);
     const size_t segs = (size_t)(segments(width) > segments(height) ? segments(width) : segments(height));
-    return (size_t)3 * kOpticMaxGauss * (size_t)width * (size_t)height // row-filtered planes
-           + (size_t)3 * kOpticMaxGauss * lines * segs * 3               // segment states
-           + (size_t)2 * 3 * kOpticMaxGauss * lines;                     // edge values
+    const size_t global = (size_t)3 * kOpticMaxGauss * (size_t)width * (size_t)height // row-filtered planes
+                          + (size_t)3 * kOpticMaxGauss * lines * segs * 3               // segment states
+                          + (size_t)2 * 3 * kOpticMaxGauss * lines;                     // edge values
+    // small frames: the line form's padded planes take more, from an address on 32 bytes on
+    const size_t pairs = 8 + (size_t)3 * kOpticMaxGauss * lp::plane_floats(width, height);
+    return global > pairs ? global : pairs;
 }
 
 bool scatter_halation(const FjScatterHalation& d, float* planes_rgb[3], long long stride, int width, int height,
