@@ -85,6 +85,7 @@ struct DirBlurParams {
     int row_warps, col_pairs, recursions, rows_ahead, cols_ahead;
     float* base[3];
     float raw_weight;
+    bool direct; // some component has no factored form
     double* row_start;
     double* col_start;
 };
@@ -101,8 +102,8 @@ cudaError_t launch_dir_blur(DirBlurParams& p, cudaStream_t stream);
 size_t dir_lines_floats(int width, int height);
 
 // One warp per pair of lines (fjb_dir_lines.cu): false when the pass is out of its range
-// (line lengths, a component in the FP64 direct form, taps beyond radius 9); true lays the
-// pass out for launch_dir_lines.
+// (line lengths, taps beyond radius 9); true lays the pass out for
+// launch_dir_lines.
 bool dir_lines_plan(DirBlurParams& p);
 cudaError_t launch_dir_lines(DirBlurParams& p, cudaStream_t stream);
 

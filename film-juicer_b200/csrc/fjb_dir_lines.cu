@@ -3,7 +3,8 @@
 // The operators are those of fjb_dir_blur.cu (the reference's
 // src/Cuda/Film/JuicerCudaFilmPipeline.cu:388-780): FP64 taps with half-sample
 // reflection, and the third-order recursion with its reflected start and end block, here
-// in the factored FP32 form with FP64 states between pieces. Five launches: the short
+// in the factored FP32 form with FP64 states between pieces, or, for coefficients without that
+// form, in the direct one in FP64. Five launches: the short
 // components, if any, both axes, summed into one plane per channel (fjb_fir2d.cuh); the rows'
 // reflected starts; the recursive components' rows, four rows per CTA (fjb_line_pairs.cuh);
 // the columns' reflected starts; the columns, one warp per pair of columns and recursive
@@ -41,12 +42,10 @@ __device__ __forceinline__ void state_from(const DirComponentDev& c, const doubl
     for (int i = 0; i < 3; ++i) s[i] = pack((float)oa[i], (float)ob[i]);
 }
 
-// End block of one line from its final state: the last `ts` outputs in `term`, and the
-// direct-form start of the way back.
-__device__ __forceinline__ void end_block(const DirComponentDev& c, const double* T, int ts, const double f[3],
-                                          double (&term)[3], double (&back)[3]) {
-    double d[3];
-    map_state(c.from_fac, f, d);
+// End block of one line from its final state `d` (direct form): the last `ts` outputs in `term`,
+// and the direct-form start of the way back.
+__device__ __forceinline__ void end_block(const double* T, int ts, const double (&d)[3], double (&term)[3],
+                                          double (&back)[3]) {
     for (int r = 0; r < 3; ++r) {
         double t = 0.0;
         if (r < ts) {
@@ -57,6 +56,39 @@ __device__ __forceinline__ void end_block(const DirComponentDev& c, const double
         back[r] = r < ts ? t : d[r];
     }
 }
+
+// A recursive component's step and state in each of its forms.
+struct Factored {
+    using State = Pair[3];
+    const DirComponentDev& c;
+    __device__ __forceinline__ lp::FactoredStep op() const { return lp::FactoredStep(c.fac[0], c.fac[1], c.fac[2]); }
+    // from direct-form states of the pair's lines, and back
+    __device__ __forceinline__ void from(const double a[3], const double b[3], State& s) const { state_from(c, a, b, s); }
+    __device__ __forceinline__ void to(const State& s, double (&a)[3], double (&b)[3]) const {
+        const float2 f0 = unpack(s[0]), f1 = unpack(s[1]), f2 = unpack(s[2]);
+        const double fa[3] = {f0.x, f1.x, f2.x}, fb[3] = {f0.y, f1.y, f2.y};
+        map_state(c.from_fac, fa, a);
+        map_state(c.from_fac, fb, b);
+    }
+    static __device__ __forceinline__ void of_lane(State& s, const State& t, int lane) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s[i].v = __shfl_sync(0xffffffffu, t[i].v, lane);
+    }
+};
+struct Direct {
+    using State = lp::State2;
+    const DirComponentDev& c;
+    __device__ __forceinline__ lp::DirectStep64 op() const { return {c.ff, c.fb[0], c.fb[1], c.fb[2]}; }
+    __device__ __forceinline__ void from(const double a[3], const double b[3], State& s) const {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s.a[i] = a[i], s.b[i] = b[i];
+    }
+    __device__ __forceinline__ void to(const State& s, double (&a)[3], double (&b)[3]) const {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) a[i] = s.a[i], b[i] = s.b[i];
+    }
+    static __device__ __forceinline__ void of_lane(State& s, const State& t, int lane) { s = t.of(lane); }
+};
 
 // Reflected starts of the recursive components' lines: anchor + sum_i w[i] (x_i - anchor) over
 // the first `len` samples, FP64. A warp takes four lines of a component (rows y .. y + 3, or
@@ -119,18 +151,19 @@ __global__ void __launch_bounds__(32 * kStartWarps) dir_starts_kernel(const __gr
 // starts at `from` (of the pair's two lines) out, the end block at the last `ts` samples, the
 // way back from it. Rows count samples from position 0 up, columns (kDown) from position
 // n - 1 down.
-template <bool kDown>
-__device__ __forceinline__ void filter(const DirComponentDev& c, const double* from, Pair* line, int n, int lane) {
+template <bool kDown, typename Form>
+__device__ __forceinline__ void filter(const Form& form, const double* from, Pair* line, int n, int lane) {
+    const DirComponentDev& c = form.c;
     const lp::LineMaps& maps = kDown ? c.col_maps : c.row_maps;
     const double* T = kDown ? c.v_term : c.h_term;
     const int ts = kDown ? c.v_tsize : c.h_tsize;
-    const lp::FactoredStep op(c.fac[0], c.fac[1], c.fac[2]);
+    const auto op = form.op();
     const lp::Piece piece(n, lane);
     auto sample = [&](int i) { return line + (kDown ? n - 1 - i : i); };
-    Pair start[3], s[3];
+    typename Form::State start, s;
     {
         const double a[3] = {from[0], from[1], from[2]}, b[3] = {from[3], from[4], from[5]};
-        state_from(c, a, b, start);
+        form.from(a, b, start);
     }
     const bool low = lane == 0, high = piece.lo < piece.hi && piece.hi == n;
     const int up = lane, down = lp::kPieces - 1 - lane;
@@ -138,18 +171,16 @@ __device__ __forceinline__ void filter(const DirComponentDev& c, const double* f
     // the lane that holds the line's end makes the end block; everyone gets the way back's start
     const int end_lane = kDown ? 0 : (n - 1) / piece.k;
     {
-        const float2 f0 = unpack(s[0]), f1 = unpack(s[1]), f2 = unpack(s[2]);
-        const double fa[3] = {f0.x, f1.x, f2.x}, fb[3] = {f0.y, f1.y, f2.y};
-        double ta[3], tb[3], ba[3], bb[3];
-        end_block(c, T, ts, fa, ta, ba);
-        end_block(c, T, ts, fb, tb, bb);
+        double da[3], db[3], ta[3], tb[3], ba[3], bb[3];
+        form.to(s, da, db);
+        end_block(T, ts, da, ta, ba);
+        end_block(T, ts, db, tb, bb);
         __syncwarp();
         if (lane == end_lane)
             for (int r = 0; r < ts; ++r)
                 if (n - ts + r >= 0) *sample(n - ts + r) = pack((float)ta[r], (float)tb[r]);
-        state_from(c, ba, bb, s);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) start[i].v = __shfl_sync(0xffffffffu, s[i].v, end_lane);
+        form.from(ba, bb, s);
+        form.of_lane(start, s, end_lane);
     }
     // the way back leaves out the end block: the last ts positions, or the first (kDown)
     lp::Piece back = piece;
@@ -163,8 +194,18 @@ __device__ __forceinline__ void filter(const DirComponentDev& c, const double* f
     __syncwarp();
 }
 
+// kDirect: some component has no factored form. A variant of its own: the FP64 states take
+// registers.
+template <bool kDown, bool kDirect>
+__device__ __forceinline__ void filter(const DirComponentDev& c, const double* from, Pair* line, int n, int lane) {
+    if (kDirect && !c.factored)
+        filter<kDown>(Direct{c}, from, line, n, lane);
+    else
+        filter<kDown>(Factored{c}, from, line, n, lane);
+}
+
 // Four rows of one channel per CTA (kWarps pairs) through every recursive component.
-template <int kWarps>
+template <int kWarps, bool kDirect>
 __global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int ch = blockIdx.y;
@@ -187,7 +228,7 @@ __global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_cons
 #pragma unroll
         for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + (size_t)min(y + h / 3, H - 1) * 3 + h % 3);
         lp::load_rows(buf, a, b, W, lane);
-        filter<false>(c, from, buf, W, lane);
+        filter<false, kDirect>(c, from, buf, W, lane);
         lp::store_pairs<kWarps>(rows, words, P.temp[ch][k], W, H, y0);
     }
 }
@@ -195,9 +236,9 @@ __global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_cons
 // kPairs pairs of columns per CTA, P.recursions recursive components at a time; the sum so far
 // waits in the first launch's plane or, where there is none (kRow), in the filtered plane
 // between the rounds (more than one only for columns too long for all of them to fit).
-template <bool kRow, int kPairs>
+template <bool kRow, int kPairs, bool kDirect>
 __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
-    __launch_bounds__(32 * kPairs * kDirMaxComponents, kPairs == lp::kColPairs ? 4 : 1)
+    __launch_bounds__(32 * kPairs * kDirMaxComponents, kPairs == lp::kColPairs && !kDirect ? 4 : 1)
     dir_cols_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();
@@ -233,7 +274,7 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
 #pragma unroll
                 for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + h);
                 lp::load_line(line, P.temp[ch][k], pair, H, lane);
-                filter<true>(c, from, line, H, lane);
+                filter<true, kDirect>(c, from, line, H, lane);
             }
             weight[count++] = c.weight;
         }
@@ -249,9 +290,17 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
     } while (k < P.count);
 }
 
-} // namespace
-
-namespace {
+using Kernel = void (*)(DirBlurParams);
+template <bool kDirect>
+Kernel rows_variant(const DirBlurParams& P) {
+    return P.row_warps == lp::kRowWarps ? dir_rows_kernel<lp::kRowWarps, kDirect> : dir_rows_kernel<1, kDirect>;
+}
+template <bool kDirect>
+Kernel cols_variant(const DirBlurParams& P) {
+    if (P.col_pairs == lp::kColPairs)
+        return P.base[0] ? dir_cols_kernel<false, lp::kColPairs, kDirect> : dir_cols_kernel<true, lp::kColPairs, kDirect>;
+    return P.base[0] ? dir_cols_kernel<false, 1, kDirect> : dir_cols_kernel<true, 1, kDirect>;
+}
 
 constexpr size_t kAlignFloats = 8; // planes start on 32 bytes
 size_t starts_floats(int width, int height) {
@@ -271,7 +320,7 @@ bool dir_lines_plan(DirBlurParams& P) {
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];
         if (c.op == kDirOpFir ? c.radius < 1 || c.radius > fir::kMaxRadius
-                              : c.op == kDirOpYvv ? !c.factored : c.op != kDirOpIdentity)
+                              : c.op != kDirOpYvv && c.op != kDirOpIdentity)
             return false;
         lines += c.op == kDirOpYvv;
         base |= c.op == kDirOpFir;
@@ -285,13 +334,17 @@ bool dir_lines_plan(DirBlurParams& P) {
         return false;
     P.recursions = lp::recursions_per_cta(lines, P.col_pairs, P.height);
     P.raw_weight = 0.0f;
+    P.direct = false;
     for (int k = 0; k < P.count; ++k) {
         DirComponentDev& c = P.comp[k];
         if (c.op == kDirOpIdentity) P.raw_weight += c.weight;
         if (c.op != kDirOpYvv) continue;
         for (int ch = 0; ch < 3; ++ch, next += plane) P.temp[ch][k] = next;
-        c.row_maps = lp::line_maps(c.step_f, lp::piece_len(P.width));
-        c.col_maps = lp::line_maps(c.step_f, lp::piece_len(P.height));
+        // one zero-input step: (s0, s1, s2) -> (fb0 s0 + fb1 s1 + fb2 s2, s0, s1) in the direct form
+        const double direct[9] = {c.fb[0], c.fb[1], c.fb[2], 1, 0, 0, 0, 1, 0};
+        c.row_maps = lp::line_maps(c.factored ? c.step_f : direct, lp::piece_len(P.width));
+        c.col_maps = lp::line_maps(c.factored ? c.step_f : direct, lp::piece_len(P.height));
+        P.direct |= !c.factored;
     }
     for (int ch = 0; ch < 3; ++ch) {
         P.base[ch] = base ? next : nullptr;
@@ -338,7 +391,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         const size_t smem = P.row_warps * lp::line_bytes(P.width);
-        auto* k = P.row_warps == lp::kRowWarps ? dir_rows_kernel<lp::kRowWarps> : dir_rows_kernel<1>;
+        auto* k = P.direct ? rows_variant<true>(P) : rows_variant<false>(P);
         e = fjb::allow_dynamic_smem(k, smem);
         if (e != cudaSuccess) return e;
         const int rows = 2 * P.row_warps;
@@ -353,9 +406,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
     }
     const int warps = P.recursions * P.col_pairs;
     const size_t smem = warps * lp::line_bytes(P.height);
-    auto* k = P.col_pairs == lp::kColPairs
-                  ? (P.base[0] ? dir_cols_kernel<false, lp::kColPairs> : dir_cols_kernel<true, lp::kColPairs>)
-                  : (P.base[0] ? dir_cols_kernel<false, 1> : dir_cols_kernel<true, 1>);
+    auto* k = P.direct ? cols_variant<true>(P) : cols_variant<false>(P);
     e = fjb::allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);

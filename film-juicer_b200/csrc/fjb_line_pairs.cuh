@@ -141,8 +141,8 @@ struct FactoredStep {
 // One piece of nv samples, the first processed one at `w` (kFwd: ascending positions).
 // Samples are read twelve at a time, so each group pays the shared-memory latency once, and
 // the direct form's state is back in its registers after a group (three shifts are none).
-template <bool kFwd, bool kWrite, typename Op>
-__device__ __forceinline__ void run(const Op& op, Pair* w, int nv, Pair (&s)[3]) {
+template <bool kFwd, bool kWrite, typename Op, typename State>
+__device__ __forceinline__ void run(const Op& op, Pair* w, int nv, State& s) {
     constexpr int D = kFwd ? 1 : -1, U = 12;
     int i = 0;
 #pragma unroll 1
@@ -209,6 +209,22 @@ struct State2 {
     }
 };
 
+// The direct form in FP64, its state too; the samples between the directions are FP32.
+struct DirectStep64 {
+    double b, b1, b2, b3;
+    __device__ __forceinline__ float step(float x, double (&s)[3]) const {
+        const double v = fma(b1, s[0], fma(b2, s[1], fma(b3, s[2], b * (double)x)));
+        s[2] = s[1];
+        s[1] = s[0];
+        s[0] = v;
+        return (float)v;
+    }
+    __device__ __forceinline__ Pair step(Pair x, State2& s) const {
+        const float2 f = unpack(x);
+        return pack(step(f.x, s.a), step(f.y, s.b));
+    }
+};
+
 // This lane's piece of a pair of lines of n samples: positions [base, base + k) as far as
 // they lie in [lo, hi).
 struct Piece {
@@ -247,7 +263,25 @@ __device__ __forceinline__ void direction(const Op& op, const LineMaps& m, Pair*
     run<kFwd, true>(op, w, nv, s);
 }
 
-// The same over the line's chunks of 32 pieces of `k` samples, the chunk's entry state carried
+// The same with FP64 states.
+template <bool kFwd>
+__device__ __forceinline__ void direction(const DirectStep64& op, const LineMaps& m, Pair* line, Piece pc, int order,
+                                          bool first, const State2& start, State2& s) {
+    const int nv = pc.hi - pc.lo;
+    Pair* w = line + (kFwd ? pc.lo : pc.hi - 1);
+    s = first ? start : State2{};
+    run<kFwd, false>(op, w, nv, s);
+#pragma unroll 1
+    for (int l = 0; l < kLevels; ++l) {
+        const State2 t = s.from<kFwd>(1 << l);
+        if (order >= (1 << l)) s.add(m.m[l], t);
+    }
+    s = s.from<kFwd>(1);
+    if (first) s = start;
+    run<kFwd, true>(op, w, nv, s);
+}
+
+// A direction in the direct form over the line's chunks of 32 pieces of `k` samples, the chunk's entry state carried
 // in FP64 from the one processed before. `s` receives the exit state of the lane's piece in
 // the last chunk processed.
 template <bool kFwd>

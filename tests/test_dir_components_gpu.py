@@ -1,0 +1,37 @@
+"""Spatial DIR records beyond those a host derives from the film: a recursion without a factored
+form (one real pole, or three), which runs in FP64 in the line form beside factored ones. Oracle
+and bounds are those of test_line_pairs_gpu.py; the launch count shows that the line form ran."""
+import pytest
+
+from test_line_rounds_gpu import check_dir, planes
+
+pytestmark = pytest.mark.gpu
+
+
+def recursion(component, feedback):
+    from film_juicer_b200 import abi
+
+    g = component
+    g.reference_operator = abi.FJ_DIR_OPERATOR_YVV_REFLECT
+    g.sigma_px = max(3.0, g.sigma_px)
+    g.radius = int(3.0 * g.sigma_px + 0.5)
+    for i in range(3):
+        g.feedback[i] = g.feedback_numerators[i] = feedback[i]
+    g.feedforward = g.feedforward_numerator = 1.0 - (feedback[0] + feedback[1] + feedback[2])
+    g.normalization_denominator = 1.0
+
+
+# real poles 0.9; 0.8, 0.5, 0.25; and a pair of 0.7 beside a negative one
+POLES = {"one": (0.9, 0.0, 0.0), "three": (1.55, -0.725, 0.1), "negative": (1.2, -0.21, -0.098)}
+
+
+@pytest.mark.parametrize("poles", sorted(POLES))
+@pytest.mark.parametrize("w,h,which", [(643, 361, (3,)), (640, 361, (0, 1, 2, 3)), (1600, 3700, (2, 3)), (9, 40, (3,)),
+                                       (14600, 9, (3,)), (9, 14600, (1, 3))])
+def test_recursions_without_a_factored_form(torch_cuda, w, h, which, poles):
+    from film_juicer_b200 import descriptors
+
+    sd = descriptors.spatial_dir_record(5.0, w, h, diffusion_size_um=20.0, tail_um=60.0, tail_weight=0.3)
+    for k in which:
+        recursion(sd.components[k], POLES[poles])
+    check_dir(torch_cuda, sd, planes(w, h, 11), 4)
