@@ -62,13 +62,14 @@ struct Factored {
     using State = Pair[3];
     const DirComponentDev& c;
     __device__ __forceinline__ lp::FactoredStep op() const { return lp::FactoredStep(c.fac[0], c.fac[1], c.fac[2]); }
-    // from direct-form states of the pair's lines, and back
+    // from direct-form states of the pair's lines, and back (one line's)
     __device__ __forceinline__ void from(const double a[3], const double b[3], State& s) const { state_from(c, a, b, s); }
-    __device__ __forceinline__ void to(const State& s, double (&a)[3], double (&b)[3]) const {
-        const float2 f0 = unpack(s[0]), f1 = unpack(s[1]), f2 = unpack(s[2]);
-        const double fa[3] = {f0.x, f1.x, f2.x}, fb[3] = {f0.y, f1.y, f2.y};
-        map_state(c.from_fac, fa, a);
-        map_state(c.from_fac, fb, b);
+    template <int kLine>
+    __device__ __forceinline__ void to(const State& s, double (&d)[3]) const {
+        double f[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) f[i] = kLine ? unpack(s[i]).y : unpack(s[i]).x;
+        map_state(c.from_fac, f, d);
     }
     static __device__ __forceinline__ void of_lane(State& s, const State& t, int lane) {
 #pragma unroll
@@ -83,9 +84,10 @@ struct Direct {
 #pragma unroll
         for (int i = 0; i < 3; ++i) s.a[i] = a[i], s.b[i] = b[i];
     }
-    __device__ __forceinline__ void to(const State& s, double (&a)[3], double (&b)[3]) const {
+    template <int kLine>
+    __device__ __forceinline__ void to(const State& s, double (&d)[3]) const {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) a[i] = s.a[i], b[i] = s.b[i];
+        for (int i = 0; i < 3; ++i) d[i] = kLine ? s.b[i] : s.a[i];
     }
     static __device__ __forceinline__ void of_lane(State& s, const State& t, int lane) { s = t.of(lane); }
 };
@@ -171,10 +173,11 @@ __device__ __forceinline__ void filter(const Form& form, const double* from, Pai
     // the lane that holds the line's end makes the end block; everyone gets the way back's start
     const int end_lane = kDown ? 0 : (n - 1) / piece.k;
     {
-        double da[3], db[3], ta[3], tb[3], ba[3], bb[3];
-        form.to(s, da, db);
-        end_block(T, ts, da, ta, ba);
-        end_block(T, ts, db, tb, bb);
+        double d[3], ta[3], tb[3], ba[3], bb[3];
+        form.template to<0>(s, d);
+        end_block(T, ts, d, ta, ba);
+        form.template to<1>(s, d);
+        end_block(T, ts, d, tb, bb);
         __syncwarp();
         if (lane == end_lane)
             for (int r = 0; r < ts; ++r)
