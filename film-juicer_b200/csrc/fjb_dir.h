@@ -102,8 +102,7 @@ cudaError_t launch_dir_blur(DirBlurParams& p, cudaStream_t stream);
 size_t dir_lines_floats(int width, int height);
 
 // One warp per pair of lines (fjb_dir_lines.cu): false when the pass is out of its range
-// (line lengths, taps beyond radius 9); true lays the pass out for
-// launch_dir_lines.
+// (line lengths); true lays the pass out for launch_dir_lines.
 bool dir_lines_plan(DirBlurParams& p);
 cudaError_t launch_dir_lines(DirBlurParams& p, cudaStream_t stream);
 

@@ -5,7 +5,8 @@
 // reflection, and the third-order recursion with its reflected start and end block, here
 // in the factored FP32 form with FP64 states between pieces, or, for coefficients without that
 // form, in the direct one in FP64. Five launches: the short
-// components, if any, both axes, summed into one plane per channel (fjb_fir2d.cuh); the rows'
+// components, if any, both axes, summed into one plane per channel (fjb_fir2d.cuh; taps beyond
+// radius 9 by two launches each, the post blurs' kernels); the rows'
 // reflected starts; the recursive components' rows, four rows per CTA (fjb_line_pairs.cuh);
 // the columns' reflected starts; the columns, one warp per pair of columns and recursive
 // component, then the weighted sum of all of them and the plane of the first launch.
@@ -22,6 +23,7 @@
 #include "fjb_fir2d.cuh"
 #include "fjb_launches.h"
 #include "fjb_line_pairs.cuh"
+#include "fjb_scanner_post.h"
 
 namespace fjb {
 
@@ -322,9 +324,6 @@ bool dir_lines_plan(DirBlurParams& P) {
     bool base = false;
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];
-        if (c.op == kDirOpFir ? c.radius < 1 || c.radius > fir::kMaxRadius
-                              : c.op != kDirOpYvv && c.op != kDirOpIdentity)
-            return false;
         lines += c.op == kDirOpYvv;
         base |= c.op == kDirOpFir;
     }
@@ -374,7 +373,7 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         for (int k = 0; k < P.count; ++k) {
             const DirComponentDev& c = P.comp[k];
             lines |= c.op == kDirOpYvv;
-            if (c.op != kDirOpFir) continue;
+            if (c.op != kDirOpFir || c.radius > fir::kMaxRadius) continue;
             fir::Taps& t = f.set[f.count++];
             t.radius = c.radius;
             t.weight = c.weight;
@@ -387,6 +386,13 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         fjb::count_launch();
         fir::kernel<double><<<fir::grid(F), fir::kThreads, 0, s>>>(F);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    // wider taps, a component after the other; the filtered planes hold its rows
+    for (int k = 0; k < P.count; ++k) {
+        const DirComponentDev& c = P.comp[k];
+        if (c.op != kDirOpFir || c.radius <= fir::kMaxRadius) continue;
+        e = launch_blur_into_pairs(P.raw, P.filtered, P.base, 3, P.width, P.height, c.taps, c.radius, c.weight, s);
+        if (e != cudaSuccess) return e;
     }
     constexpr int kLinesPerCta = 4 * kStartWarps;
     if (lines) {

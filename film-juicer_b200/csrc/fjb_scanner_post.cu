@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "fjb_launches.h"
+#include "fjb_line_pairs.cuh"
 #include "fjb_philox.cuh"
 #include "fjb_scanner_post.h"
 
@@ -169,9 +170,11 @@ __global__ void __launch_bounds__(32 * kRowWarps) blur_rows_run_kernel(const __g
 }
 
 // Vertical pass (plane blockIdx.z): a thread takes kRun rows of one column; the warp's
-// loads are rows of 32 consecutive columns. With kUnsharp, `io` holds the plane and
-// receives v + amount (v - blurred) in FP64; otherwise the blurred value goes to `io`.
-template <bool kUnsharp>
+// loads are rows of 32 consecutive columns. The blurred value goes to `io`; with kUnsharp, `io`
+// holds the plane and receives v + amount (v - blurred) in FP64; with kPairs it is a sum by pairs
+// of columns and receives v + amount blurred.
+enum ColumnsOut : int { kBlurred, kUnsharp, kPairs };
+template <ColumnsOut kOut>
 __global__ void __launch_bounds__(32 * kColWarps, 5) blur_cols_run_kernel(const __grid_constant__ Planes in,
                                                                        const __grid_constant__ Planes io, int width,
                                                                        int height, const float* __restrict__ w,
@@ -184,7 +187,10 @@ __global__ void __launch_bounds__(32 * kColWarps, 5) blur_cols_run_kernel(const 
     const int p0 = (blockIdx.y * kColWarps + (threadIdx.x >> 5)) * kRun;
     if (x >= width || p0 >= height) return;
     const float* src = in.p[blockIdx.z] + x;
-    float* dst = io.p[blockIdx.z] + ((size_t)p0 * width + x);
+    constexpr bool pairs = kOut == kPairs;
+    float* dst = io.p[blockIdx.z] + (pairs ? ((size_t)(x >> 1) * lp::line_words(height) + p0) * 2 + (x & 1)
+                                           : (size_t)p0 * width + x);
+    const size_t step = pairs ? 2 : width;
     const int rows = min(kRun, height - p0);
     double sum[kRun];
     if (p0 >= radius && p0 - radius + n + kRun <= height) {
@@ -201,14 +207,16 @@ __global__ void __launch_bounds__(32 * kColWarps, 5) blur_cols_run_kernel(const 
     for (int j = 0; j < kRun; ++j) {
         if (j >= rows) break;
         const float blurred = finite_d(sum[j]) ? (float)sum[j] : 0.0f;
-        if constexpr (kUnsharp) {
-            const double v = (double)dst[(size_t)j * width];
+        if constexpr (kOut == kUnsharp) {
+            const double v = (double)dst[j * step];
             const double vb = (double)blurred;
             const double a = (double)amount;
             const double o = v + a * (v - vb);
-            dst[(size_t)j * width] = finite_d(o) ? (float)o : 0.0f;
+            dst[j * step] = finite_d(o) ? (float)o : 0.0f;
+        } else if constexpr (pairs) {
+            dst[j * step] = fmaf(amount, blurred, dst[j * step]);
         } else {
-            dst[(size_t)j * width] = blurred;
+            dst[j * step] = blurred;
         }
     }
 }
@@ -232,7 +240,7 @@ cudaError_t blur_rows(float* const* planes, float* const* tmps, int count, int w
     return cudaGetLastError();
 }
 
-template <bool kUnsharp>
+template <ColumnsOut kOut>
 cudaError_t blur_cols(float* const* planes, float* const* tmps, int count, int width, int height, const float* w,
                       int radius, float amount, cudaStream_t stream) {
     Planes in{}, io{};
@@ -241,11 +249,11 @@ cudaError_t blur_cols(float* const* planes, float* const* tmps, int count, int w
         io.p[c] = planes[c];
     }
     const size_t smem = taps_bytes(radius);
-    cudaError_t e = fjb::allow_dynamic_smem(blur_cols_run_kernel<kUnsharp>, smem);
+    cudaError_t e = fjb::allow_dynamic_smem(blur_cols_run_kernel<kOut>, smem);
     if (e != cudaSuccess) return e;
     const int runs = (height + kRun - 1) / kRun;
     fjb::count_launch();
-    blur_cols_run_kernel<kUnsharp><<<dim3((width + 31) / 32, (runs + kColWarps - 1) / kColWarps, count), 32 * kColWarps,
+    blur_cols_run_kernel<kOut><<<dim3((width + 31) / 32, (runs + kColWarps - 1) / kColWarps, count), 32 * kColWarps,
                                      smem, stream>>>(in, io, width, height, w, radius, amount);
     return cudaGetLastError();
 }
@@ -267,7 +275,7 @@ cudaError_t launch_blur_planes(float* const* planes, float* const* tmps, int cou
     if (count > 3) return cudaErrorInvalidValue;
     cudaError_t e = blur_rows(planes, tmps, count, width, height, w, radius, stream);
     if (e != cudaSuccess) return e;
-    return blur_cols<false>(planes, tmps, count, width, height, w, radius, 0.0f, stream);
+    return blur_cols<kBlurred>(planes, tmps, count, width, height, w, radius, 0.0f, stream);
 }
 
 cudaError_t launch_unsharp_planes(float* const* planes, float* const* tmps, int count, int width, int height,
@@ -276,7 +284,19 @@ cudaError_t launch_unsharp_planes(float* const* planes, float* const* tmps, int 
     if (count > 3) return cudaErrorInvalidValue;
     cudaError_t e = blur_rows(planes, tmps, count, width, height, w, radius, stream);
     if (e != cudaSuccess) return e;
-    return blur_cols<true>(planes, tmps, count, width, height, w, radius, amount, stream);
+    return blur_cols<kUnsharp>(planes, tmps, count, width, height, w, radius, amount, stream);
+}
+
+cudaError_t launch_blur_into_pairs(const float* const* planes, float* const* tmps, float* const* sums, int count,
+                                   int width, int height, const float* w, int radius, float weight,
+                                   cudaStream_t stream) {
+    if (width <= 0 || height <= 0 || radius <= 0 || !w || count <= 0) return cudaSuccess;
+    if (count > 3) return cudaErrorInvalidValue;
+    float* in[3] = {};
+    for (int c = 0; c < count; ++c) in[c] = const_cast<float*>(planes[c]); // read only
+    cudaError_t e = blur_rows(in, tmps, count, width, height, w, radius, stream);
+    if (e != cudaSuccess) return e;
+    return blur_cols<kPairs>(sums, tmps, count, width, height, w, radius, weight, stream);
 }
 
 } // namespace fjb

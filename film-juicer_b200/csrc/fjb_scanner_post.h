@@ -28,6 +28,12 @@ cudaError_t launch_blur_planes(float* const* planes, float* const* tmps, int cou
 cudaError_t launch_unsharp_planes(float* const* planes, float* const* tmps, int count, int width, int height,
                                   const float* w, int radius, float amount, cudaStream_t stream);
 
+// sum += weight blur(plane) for `count` (1..3) planes, through `tmps`; the sums lie by pairs of
+// columns (fjb_line_pairs.cuh).
+cudaError_t launch_blur_into_pairs(const float* const* planes, float* const* tmps, float* const* sums, int count,
+                                   int width, int height, const float* w, int radius, float weight,
+                                   cudaStream_t stream);
+
 // Which effects a post-effects record turns on, with their Gaussian taps (host).
 struct PostPlan {
     bool active = false;

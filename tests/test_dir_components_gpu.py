@@ -1,6 +1,7 @@
 """Spatial DIR records beyond those a host derives from the film: a recursion without a factored
-form (one real pole, or three), which runs in FP64 in the line form beside factored ones. Oracle
-and bounds are those of test_line_pairs_gpu.py; the launch count shows that the line form ran."""
+form (one real pole, or three), which runs in FP64 in the line form beside factored ones, and taps of
+radius 10 to 64, two launches of their own each. Oracle and bounds are those of
+test_line_pairs_gpu.py; the launch count shows that the line form ran."""
 import pytest
 
 from test_line_rounds_gpu import check_dir, planes
@@ -35,3 +36,23 @@ def test_recursions_without_a_factored_form(torch_cuda, w, h, which, poles):
     for k in which:
         recursion(sd.components[k], POLES[poles])
     check_dir(torch_cuda, sd, planes(w, h, 11), 4)
+
+
+def taps(component, sigma, radius):
+    from film_juicer_b200 import abi
+
+    component.reference_operator = abi.FJ_DIR_OPERATOR_FIR_REFLECT
+    component.sigma_px, component.radius = sigma, radius
+
+
+@pytest.mark.parametrize("w,h", [(643, 361), (40, 3700), (7, 5), (1, 9), (9, 1), (289, 73), (14600, 9)])
+@pytest.mark.parametrize("radii", [(10,), (64,), (9, 10), (11, 40, 2, 64)])
+def test_wide_taps(torch_cuda, w, h, radii):
+    from film_juicer_b200 import descriptors
+
+    sd = descriptors.spatial_dir_record(5.0, w, h, diffusion_size_um=20.0, tail_um=60.0, tail_weight=0.3)
+    for k, r in enumerate(radii):
+        taps(sd.components[k], 2.9 if r > 2 else 0.7, r)
+    wide = sum(r > 9 for r in radii)
+    recursive = 3 if len(radii) < 4 else 0  # starts, rows, starts
+    check_dir(torch_cuda, sd, planes(w, h, 12), 1 + 2 * wide + recursive + 1)
