@@ -14,6 +14,7 @@
 // reference so results match it to the last bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "fjb_launches.h"
@@ -69,7 +70,8 @@ __global__ void glare_kernel(float* out, int width, int height, uint64_t seed, u
 // Bound by instruction issue at the ordinary radii, most of it around the sums: a warp
 // takes a segment of one row (no divisions to place a run or an output), loads are
 // asynchronous or unconditional where nothing is reflected. 1999x1333, glare, lens
-// blur and unsharp (seven planes): rows 122 -> 46 us, columns 84 -> 73 us.
+// blur and unsharp (seven planes): rows 122 -> 46 us, columns 84 -> 73 us. Radius 80, three
+// planes: 119 and 269 us (a 64-bit row index where rows are reflected: 306).
 // ---------------------------------------------------------------------------
 constexpr int kRun = 9; // odd: threads nine samples apart read distinct shared-memory banks
 constexpr int kSegment = 32 * kRun;
@@ -112,9 +114,49 @@ __device__ __forceinline__ void run_taps(const double* taps, int n, Get get, dou
 __host__ __device__ inline int segment_floats(int radius) { return kSegment + 2 * radius + kRun + 1; }
 
 size_t taps_bytes(int radius) { return (2 * (size_t)radius + 1) * sizeof(double); }
-// 183 KB at the largest radius the host prepares (2048)
+// 58 KB at radius 400, above which the segments of a row share their inputs
 size_t rows_smem_bytes(int radius) {
     return taps_bytes(radius) + (size_t)kRowWarps * (segment_floats(radius) + kSegment) * sizeof(float);
+}
+
+// `count` inputs from sample q0 on of a row of `width`, reflected at its ends, asynchronously, by
+// threads first, first + step, ...
+__device__ __forceinline__ void stage_inputs(float* line, const float* row, int q0, int count, int width, int outputs,
+                                             int radius, int first, int step) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(line);
+    if (q0 >= 0 && q0 + count <= width) {
+#pragma unroll 4
+        for (int i = first; i < count; i += step)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4u * (unsigned)i), "l"(row + q0 + i));
+    } else {
+        // what lies beyond the last output's inputs is not part of a sum that is kept
+        const int last = outputs + 2 * radius;
+        for (int i = first; i < count; i += step) {
+            const int q = q0 + i;
+            if (i < last)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4u * (unsigned)i),
+                             "l"(row + ((unsigned)q < (unsigned)width ? q : reflect_wide(q, width))));
+            else
+                line[i] = 0.0f;
+        }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+}
+
+// A warp's kSegment outputs of a row from its inputs at `in`, through its staging area `st`, to
+// dst, of which `left` are inside the row.
+__device__ __forceinline__ void segment_outputs(const double* taps, int n, const float* in, float* st, float* dst,
+                                                int left, int lane) {
+    if (lane * kRun < left) {
+        double sum[kRun];
+        run_taps(taps, n, [&](int i) { return in[lane * kRun + i]; }, sum);
+#pragma unroll
+        for (int j = 0; j < kRun; ++j) st[lane * kRun + j] = finite_d(sum[j]) ? (float)sum[j] : 0.0f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kRun; ++i)
+        if (i * 32 + lane < left) dst[i * 32 + lane] = st[i * 32 + lane];
 }
 
 // Horizontal pass (plane blockIdx.z): a warp stages the segment of a row, reflected at the
@@ -130,43 +172,42 @@ __global__ void __launch_bounds__(32 * kRowWarps) blur_rows_run_kernel(const __g
     float* line = reinterpret_cast<float*>(taps + n) + warp * (count + kSegment);
     float* st = line + count;
     const int x0 = blockIdx.x * kSegment, y = blockIdx.y * kRowWarps + warp;
-    if (y < height) {
-        const float* row = in.p[blockIdx.z] + (size_t)y * width;
-        const int q0 = x0 - radius;
-        const unsigned d = (unsigned)__cvta_generic_to_shared(line);
-        if (q0 >= 0 && q0 + count <= width) {
-#pragma unroll 4
-            for (int i = lane; i < count; i += 32)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4u * (unsigned)i), "l"(row + q0 + i));
-        } else {
-            // what lies beyond the last output's inputs is not part of a sum that is kept
-            const int last = min(kSegment, width - x0) + 2 * radius;
-            for (int i = lane; i < count; i += 32) {
-                const int q = q0 + i;
-                if (i < last)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4u * (unsigned)i),
-                                 "l"(row + ((unsigned)q < (unsigned)width ? q : reflect_wide(q, width))));
-                else
-                    line[i] = 0.0f;
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    }
+    if (y < height)
+        stage_inputs(line, in.p[blockIdx.z] + (size_t)y * width, x0 - radius, count, width, min(kSegment, width - x0),
+                     radius, lane, 32);
     stage_taps(taps, w, n); // its barrier is the last one: warps go on by themselves
     if (y >= height) return;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncwarp();
-    if (x0 + lane * kRun < width) {
-        double sum[kRun];
-        run_taps(taps, n, [&](int i) { return line[lane * kRun + i]; }, sum);
-#pragma unroll
-        for (int j = 0; j < kRun; ++j) st[lane * kRun + j] = finite_d(sum[j]) ? (float)sum[j] : 0.0f;
-    }
-    __syncwarp();
-    float* dst = out.p[blockIdx.z] + (size_t)y * width + x0;
-#pragma unroll
-    for (int i = 0; i < kRun; ++i)
-        if (x0 + i * 32 + lane < width) dst[i * 32 + lane] = st[i * 32 + lane];
+    segment_outputs(taps, n, line, st, out.p[blockIdx.z] + (size_t)y * width + x0, width - x0, lane);
+}
+
+// The same for large radii: the warps of a CTA take neighbouring segments of one row (blockIdx.x)
+// and share its inputs, of which a segment by itself has more around it than in it. 1999x1333,
+// three planes, a warp's own inputs and shared ones: radius 400 531 us both, 600 799 and 781,
+// 1200 1684 and 1530, 2000, where the first leave room for eight warps per SM, 4230 and 2590.
+constexpr int kSharedRadius = 400;
+size_t shared_rows_smem_bytes(int radius, int warps) {
+    return taps_bytes(radius) + ((size_t)segment_floats(radius) + (2 * (size_t)warps - 1) * kSegment) * sizeof(float);
+}
+__global__ void __launch_bounds__(32 * kRowWarps) blur_rows_shared_kernel(const __grid_constant__ Planes in,
+                                                                          const __grid_constant__ Planes out, int width,
+                                                                          int height, const float* __restrict__ w,
+                                                                          int radius) {
+    extern __shared__ __align__(16) unsigned char post_smem[];
+    double* taps = reinterpret_cast<double*>(post_smem);
+    const int n = 2 * radius + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int count = segment_floats(radius) + (warps - 1) * kSegment;
+    float* line = reinterpret_cast<float*>(taps + n);
+    const int first = blockIdx.y * warps * kSegment, x0 = first + warp * kSegment;
+    const size_t row = (size_t)blockIdx.x * width;
+    stage_inputs(line, in.p[blockIdx.z] + row, first - radius, count, width, min(warps * kSegment, width - first), radius,
+                 threadIdx.x, blockDim.x);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    stage_taps(taps, w, n);
+    if (x0 < width)
+        segment_outputs(taps, n, line + warp * kSegment, line + count + warp * kSegment, out.p[blockIdx.z] + row + x0,
+                        width - x0, lane);
 }
 
 // Vertical pass (plane blockIdx.z): a thread takes kRun rows of one column; the warp's
@@ -198,8 +239,8 @@ __global__ void __launch_bounds__(32 * kColWarps, 5) blur_cols_run_kernel(const 
         run_taps(taps, n, [&](int i) { return __ldg(top + (size_t)i * width); }, sum);
     } else {
         run_taps(taps, n, [&](int i) {
-            const long long q = (long long)p0 - radius + i;
-            const int y = (unsigned long long)q < (unsigned long long)height ? (int)q : reflect_wide(q, height);
+            const int q = p0 - radius + i;
+            const int y = (unsigned)q < (unsigned)height ? q : reflect_wide(q, height);
             return __ldg(src + (size_t)y * width);
         }, sum);
     }
@@ -231,6 +272,16 @@ cudaError_t blur_rows(float* const* planes, float* const* tmps, int count, int w
         in.p[c] = planes[c];
         out.p[c] = tmps[c];
     }
+    if (radius > kSharedRadius) {
+        const int segments = (width + kSegment - 1) / kSegment, warps = std::min(segments, kRowWarps);
+        const size_t smem = shared_rows_smem_bytes(radius, warps);
+        const cudaError_t e = fjb::allow_dynamic_smem(blur_rows_shared_kernel, smem);
+        if (e != cudaSuccess) return e;
+        fjb::count_launch();
+        blur_rows_shared_kernel<<<dim3(height, (segments + warps - 1) / warps, count), 32 * warps, smem, stream>>>(
+            in, out, width, height, w, radius);
+        return cudaGetLastError();
+    }
     const size_t smem = rows_smem_bytes(radius);
     cudaError_t e = fjb::allow_dynamic_smem(blur_rows_run_kernel, smem);
     if (e != cudaSuccess) return e;
@@ -248,13 +299,11 @@ cudaError_t blur_cols(float* const* planes, float* const* tmps, int count, int w
         in.p[c] = tmps[c];
         io.p[c] = planes[c];
     }
-    const size_t smem = taps_bytes(radius);
-    cudaError_t e = fjb::allow_dynamic_smem(blur_cols_run_kernel<kOut>, smem);
-    if (e != cudaSuccess) return e;
+    const size_t smem = taps_bytes(radius); // 33 KB at the largest radius: no setting needed
     const int runs = (height + kRun - 1) / kRun;
     fjb::count_launch();
     blur_cols_run_kernel<kOut><<<dim3((width + 31) / 32, (runs + kColWarps - 1) / kColWarps, count), 32 * kColWarps,
-                                     smem, stream>>>(in, io, width, height, w, radius, amount);
+                                 smem, stream>>>(in, io, width, height, w, radius, amount);
     return cudaGetLastError();
 }
 
