@@ -82,7 +82,7 @@ struct DirBlurParams {
     // and line)
     float* region;
     size_t region_floats;
-    int row_warps, col_pairs, recursions, rows_ahead, cols_ahead;
+    int row_pairs, col_pairs, recursions, rows_ahead, cols_ahead;
     float* base[3];
     float raw_weight;
     bool direct; // some component has no factored form

@@ -7,7 +7,7 @@
 // the visual top (last memory row) down, then back up.
 //
 // B200 schedule: fjb_dir_lines.cu. The kernels of this file are the form for what that one
-// does not cover: lines above 29056 samples.
+// does not cover: lines above 29020 samples.
 // The recursions are block-parallel: a line is cut into segments of
 // kDirSeg samples (the segment processed last in a direction is shorter, or absorbs
 // a remainder of fewer than 8 samples). A start kernel forms each line's reflected

@@ -199,6 +199,39 @@ __device__ __forceinline__ void filter(const Form& form, const double* from, Pai
     __syncwarp();
 }
 
+// The same by the CTA's team, factored form.
+template <bool kDown>
+__device__ __forceinline__ void filter_team(const DirComponentDev& c, const double* from, Pair* line, int n,
+                                            lp::TeamExchange& ex) {
+    const Factored form{c};
+    const lp::LineMaps& maps = kDown ? c.col_maps : c.row_maps;
+    const double* T = kDown ? c.v_term : c.h_term;
+    const int ts = kDown ? c.v_tsize : c.h_tsize, k = lp::team_piece_len(n, 1);
+    const auto op = form.op();
+    Pair start[3], s[3];
+    {
+        const double a[3] = {from[0], from[1], from[2]}, b[3] = {from[3], from[4], from[5]};
+        form.from(a, b, start);
+    }
+    lp::direction_team<!kDown>(op, maps, line, 0, n, k, 1, start, s, ex);
+    // the thread that holds the line's end makes the end block and the way back's start
+    if ((int)threadIdx.x == (kDown ? 0 : (n - 1) / k)) {
+        double d[3], ta[3], tb[3], ba[3], bb[3];
+        form.template to<0>(s, d);
+        end_block(T, ts, d, ta, ba);
+        form.template to<1>(s, d);
+        end_block(T, ts, d, tb, bb);
+        for (int r = 0; r < ts; ++r) line[kDown ? ts - 1 - r : n - ts + r] = pack((float)ta[r], (float)tb[r]);
+        form.from(ba, bb, s);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) ex.start[i] = s[i].v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 3; ++i) start[i].v = ex.start[i];
+    lp::direction_team<kDown>(op, maps, line, kDown ? ts : 0, kDown ? n : n - ts, k, 1, start, s, ex);
+}
+
 // kDirect: some component has no factored form. A variant of its own: the FP64 states take
 // registers.
 template <bool kDown, bool kDirect>
@@ -209,20 +242,26 @@ __device__ __forceinline__ void filter(const DirComponentDev& c, const double* f
         filter<kDown>(Factored{c}, from, line, n, lane);
 }
 
-// Four rows of one channel per CTA (kWarps pairs) through every recursive component.
-template <int kWarps, bool kDirect>
-__global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
+// Warps of a CTA of one pair of lines: a team, unless a component runs in FP64.
+template <bool kDirect>
+constexpr int team_warps() {
+    return kDirect ? 1 : lp::kTeam;
+}
+
+// Four rows of one channel per CTA (kPairs pairs) through every recursive component.
+template <int kPairs, bool kDirect>
+__global__ void __launch_bounds__(32 * (kPairs == 1 ? team_warps<kDirect>() : kPairs)) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int ch = blockIdx.y;
-    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = kPairs == 1 ? 0 : threadIdx.x >> 5;
     const int words = lp::line_words(W);
     Pair* rows = reinterpret_cast<Pair*>(sm);
     Pair* buf = rows + warp * words;
     // rows past the frame's end repeat the last one; their results land in the planes' padding
-    const int y0 = 2 * kWarps * blockIdx.x, y = y0 + 2 * warp;
+    const int y0 = 2 * kPairs * blockIdx.x, y = y0 + 2 * warp;
     const float* a = P.raw[ch] + (size_t)min(y, H - 1) * W;
     const float* b = P.raw[ch] + (size_t)min(y + 1, H - 1) * W;
-    if (lane < 2 && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (size_t)(lane + P.rows_ahead) * W, W);
+    if (lane < 2 && (kPairs > 1 || threadIdx.x < 2) && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (size_t)(lane + P.rows_ahead) * W, W);
 #pragma unroll 1
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];
@@ -232,9 +271,14 @@ __global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_cons
         double from[6];
 #pragma unroll
         for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + (size_t)min(y + h / 3, H - 1) * 3 + h % 3);
-        lp::load_rows(buf, a, b, W, lane);
-        filter<false, kDirect>(c, from, buf, W, lane);
-        lp::store_pairs<kWarps>(rows, words, P.temp[ch][k], W, H, y0);
+        if constexpr (kPairs == 1 && !kDirect) {
+            lp::load_rows<lp::kTeam>(buf, a, b, W, threadIdx.x);
+            filter_team<false>(c, from, buf, W, lp::exchange(buf, words));
+        } else {
+            lp::load_rows(buf, a, b, W, lane);
+            filter<false, kDirect>(c, from, buf, W, lane);
+        }
+        lp::store_pairs<kPairs>(rows, words, P.temp[ch][k], W, H, y0);
     }
 }
 
@@ -243,15 +287,15 @@ __global__ void __launch_bounds__(32 * kWarps) dir_rows_kernel(const __grid_cons
 // between the rounds (more than one only for columns too long for all of them to fit).
 template <bool kRow, int kPairs, bool kDirect>
 __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
-    __launch_bounds__(32 * kPairs * kDirMaxComponents, kPairs == lp::kColPairs && !kDirect ? 4 : 1)
+    __launch_bounds__(32 * (kPairs == 1 ? team_warps<kDirect>() : kPairs * kDirMaxComponents), kPairs == lp::kColPairs && !kDirect ? 4 : 1)
     dir_cols_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();
     const int ch = blockIdx.y;
-    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = kPairs == 1 ? 0 : threadIdx.x >> 5;
     Pair* lines = reinterpret_cast<Pair*>(sm);
     Pair* line = lines + warp * lp::line_words(H);
-    if (lane == 0) {
+    if (lane == 0 && (kPairs > 1 || threadIdx.x == 0)) {
         const unsigned next = blockIdx.y * gridDim.x + blockIdx.x + P.cols_ahead;
         if (next < gridDim.x * gridDim.y) {
             const int first = next % gridDim.x * kPairs, nch = next / gridDim.x;
@@ -278,8 +322,13 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
                 double from[6];
 #pragma unroll
                 for (int h = 0; h < 6; ++h) from[h] = __ldg(starts + h);
-                lp::load_line(line, P.temp[ch][k], pair, H, lane);
-                filter<true, kDirect>(c, from, line, H, lane);
+                if constexpr (kPairs == 1 && !kDirect) {
+                    lp::load_line<lp::kTeam>(line, P.temp[ch][k], pair, H, threadIdx.x);
+                    filter_team<true>(c, from, line, H, lp::exchange(line, lp::line_words(H)));
+                } else {
+                    lp::load_line(line, P.temp[ch][k], pair, H, lane);
+                    filter<true, kDirect>(c, from, line, H, lane);
+                }
             }
             weight[count++] = c.weight;
         }
@@ -298,13 +347,22 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
 using Kernel = void (*)(DirBlurParams);
 template <bool kDirect>
 Kernel rows_variant(const DirBlurParams& P) {
-    return P.row_warps == lp::kRowWarps ? dir_rows_kernel<lp::kRowWarps, kDirect> : dir_rows_kernel<1, kDirect>;
+    return P.row_pairs == lp::kRowWarps ? dir_rows_kernel<lp::kRowWarps, kDirect> : dir_rows_kernel<1, kDirect>;
 }
 template <bool kDirect>
 Kernel cols_variant(const DirBlurParams& P) {
     if (P.col_pairs == lp::kColPairs)
         return P.base[0] ? dir_cols_kernel<false, lp::kColPairs, kDirect> : dir_cols_kernel<true, lp::kColPairs, kDirect>;
     return P.base[0] ? dir_cols_kernel<false, 1, kDirect> : dir_cols_kernel<true, 1, kDirect>;
+}
+
+// Warps of a CTA of `lines` lines (pairs), and samples per piece of a line of n samples in a CTA of
+// `pairs` pairs.
+int warps_of(const DirBlurParams& P, int pairs, int lines) {
+    return pairs > 1 ? lines : P.direct ? team_warps<true>() : team_warps<false>();
+}
+int piece_of(const DirBlurParams& P, int n, int pairs) {
+    return pairs > 1 || P.direct ? lp::piece_len(n) : lp::team_piece_len(n, 1);
 }
 
 constexpr size_t kAlignFloats = 8; // planes start on 32 bytes
@@ -322,21 +380,22 @@ size_t dir_lines_floats(int width, int height) {
 bool dir_lines_plan(DirBlurParams& P) {
     int lines = 0;
     bool base = false;
+    P.direct = false;
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];
         lines += c.op == kDirOpYvv;
+        P.direct |= c.op == kDirOpYvv && !c.factored;
         base |= c.op == kDirOpFir;
     }
-    P.row_warps = lp::rows_per_cta(P.width);
+    P.row_pairs = lp::pairs_per_cta(P.width);
     P.col_pairs = lp::pairs_per_cta(P.height);
-    if (P.row_warps < 1 || P.col_pairs < 1) return false;
+    if (P.row_pairs < 1 || P.col_pairs < 1) return false;
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.region) + 31) / 32 * 32);
     if ((size_t)(next - P.region) + 3 * (size_t)(lines + base) * plane + starts_floats(P.width, P.height) > P.region_floats)
         return false;
     P.recursions = lp::recursions_per_cta(lines, P.col_pairs, P.height);
     P.raw_weight = 0.0f;
-    P.direct = false;
     for (int k = 0; k < P.count; ++k) {
         DirComponentDev& c = P.comp[k];
         if (c.op == kDirOpIdentity) P.raw_weight += c.weight;
@@ -344,9 +403,8 @@ bool dir_lines_plan(DirBlurParams& P) {
         for (int ch = 0; ch < 3; ++ch, next += plane) P.temp[ch][k] = next;
         // one zero-input step: (s0, s1, s2) -> (fb0 s0 + fb1 s1 + fb2 s2, s0, s1) in the direct form
         const double direct[9] = {c.fb[0], c.fb[1], c.fb[2], 1, 0, 0, 0, 1, 0};
-        c.row_maps = lp::line_maps(c.factored ? c.step_f : direct, lp::piece_len(P.width));
-        c.col_maps = lp::line_maps(c.factored ? c.step_f : direct, lp::piece_len(P.height));
-        P.direct |= !c.factored;
+        c.row_maps = lp::line_maps(c.factored ? c.step_f : direct, piece_of(P, P.width, P.row_pairs));
+        c.col_maps = lp::line_maps(c.factored ? c.step_f : direct, piece_of(P, P.height, P.col_pairs));
     }
     for (int ch = 0; ch < 3; ++ch) {
         P.base[ch] = base ? next : nullptr;
@@ -399,28 +457,28 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         fjb::count_launch();
         dir_starts_kernel<false><<<dim3((P.height + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        const size_t smem = P.row_warps * lp::line_bytes(P.width);
+        const size_t smem = lp::cta_bytes(P.row_pairs, P.width);
         auto* k = P.direct ? rows_variant<true>(P) : rows_variant<false>(P);
         e = fjb::allow_dynamic_smem(k, smem);
         if (e != cudaSuccess) return e;
-        const int rows = 2 * P.row_warps;
+        const int rows = 2 * P.row_pairs;
         P.rows_ahead = rows * lp::resident_ctas(smem);
         fjb::count_launch();
-        k<<<dim3((P.height + rows - 1) / rows, 3), 32 * P.row_warps, smem, s>>>(P);
+        k<<<dim3((P.height + rows - 1) / rows, 3), 32 * warps_of(P, P.row_pairs, P.row_pairs), smem, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         fjb::count_launch();
         dir_starts_kernel<true>
             <<<dim3((2 * lp::plane_pairs(P.width) + kLinesPerCta - 1) / kLinesPerCta, 3, P.count), 32 * kStartWarps, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    const int warps = P.recursions * P.col_pairs;
-    const size_t smem = warps * lp::line_bytes(P.height);
+    const int columns = P.recursions * P.col_pairs;
+    const size_t smem = lp::cta_bytes(columns, P.height);
     auto* k = P.direct ? cols_variant<true>(P) : cols_variant<false>(P);
     e = fjb::allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     P.cols_ahead = lp::resident_ctas(smem);
     fjb::count_launch();
-    k<<<dim3(lp::plane_pairs(P.width) / P.col_pairs, 3), 32 * warps, smem, s>>>(P);
+    k<<<dim3(lp::plane_pairs(P.width) / P.col_pairs, 3), 32 * warps_of(P, P.col_pairs, columns), smem, s>>>(P);
     return cudaGetLastError();
 }
 

@@ -11,7 +11,7 @@
 // column passes).
 //
 // B200 schedule: fjb_halation_lines.cu. The kernels of this file are the form for what that
-// one does not cover: frames above 29056 samples in a line. Here the recursions run block-parallel
+// one does not cover: frames above 29020 samples in a line. Here the recursions run block-parallel
 // over global memory; the row kernels write one row-filtered plane per Gaussian, and the
 // last column kernel runs all column filters of a channel together and applies the
 // scatter/bounce combination in its epilogue. All three channels run in each launch

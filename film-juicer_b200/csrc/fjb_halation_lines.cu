@@ -56,6 +56,31 @@ __device__ __forceinline__ void filter_chunks(const lp::DirectStep& op, const lp
     __syncwarp();
 }
 
+// A pair of lines by the CTA's team.
+template <bool kDown, bool kFactored, typename Op>
+__device__ __forceinline__ void filter_team(const Op& op, const lp::LineMaps& maps, Pair* line, int n, int chunks,
+                                            lp::TeamExchange& ex) {
+    const int k = lp::team_piece_len(n, chunks);
+    const Pair zero{0ull};
+    const Pair v0 = line[kDown ? n - 1 : 0];
+    Pair start[3] = {v0, v0, kFactored ? zero : v0}, s[3];
+    __syncthreads(); // every thread has read the first sample
+    lp::direction_team<!kDown>(op, maps, line, 0, n, k, chunks, start, s, ex);
+    const Pair v1 = kFactored ? s[1] : s[0];
+    start[0] = start[1] = v1;
+    start[2] = kFactored ? zero : v1;
+    lp::direction_team<kDown>(op, maps, line, 0, n, k, chunks, start, s, ex);
+}
+template <bool kDown, bool kLong>
+__device__ __forceinline__ void filter_team(const OpticGauss& g, Pair* line, int n, lp::TeamExchange& ex) {
+    const lp::LineMaps& maps = kDown ? g.col_maps : g.row_maps;
+    if (!kLong || g.kind == kGaussYvvFactored)
+        filter_team<kDown, true>(lp::FactoredStep(g.yvv[0], g.yvv[1], g.yvv[2]), maps, line, n, 1, ex);
+    else
+        filter_team<kDown, false>(lp::DirectStep(g.yvv[0], g.yvv[1], g.yvv[2], g.yvv[3]), maps, line, n,
+                                  lp::team_chunks(n), ex);
+}
+
 // kLong: a Gaussian in the direct form has its lines cut into chunks. A variant of its own: the
 // states between chunks take 24 registers more, with which 1283x719 took 161 us instead of 144.
 template <bool kDown, bool kLong>
@@ -72,27 +97,33 @@ __device__ __forceinline__ void filter(const OpticGauss& g, Pair* line, int n, i
     }
 }
 
-// Four rows of one channel per CTA (kWarps pairs) through every recursive Gaussian of the job.
-template <bool kLong, int kWarps>
-__global__ void __launch_bounds__(32 * kWarps) optic_rows_kernel(const __grid_constant__ OpticPass P) {
+// Four rows of one channel per CTA (kPairs pairs) through every recursive Gaussian of the job.
+template <bool kLong, int kPairs>
+__global__ void __launch_bounds__(32 * (kPairs == 1 ? lp::kTeam : kPairs)) optic_rows_kernel(const __grid_constant__ OpticPass P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const OpticJob& J = P.job[blockIdx.y];
-    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = kPairs == 1 ? 0 : threadIdx.x >> 5;
     const int words = lp::line_words(W);
     Pair* rows = reinterpret_cast<Pair*>(sm);
     Pair* buf = rows + warp * words;
     // rows past the frame's end repeat the last one; their results land in the planes' padding
-    const int y0 = 2 * kWarps * blockIdx.x, y = y0 + 2 * warp;
+    const int y0 = 2 * kPairs * blockIdx.x, y = y0 + 2 * warp;
     const float* a = J.src + (long long)min(y, H - 1) * J.stride;
     const float* b = J.src + (long long)min(y + 1, H - 1) * J.stride;
-    if (lane < 2 && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (long long)(lane + P.rows_ahead) * J.stride, W);
+    if (lane < 2 && (kPairs > 1 || threadIdx.x < 2) && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (long long)(lane + P.rows_ahead) * J.stride, W);
 #pragma unroll 1
     for (int gi = 0; gi < J.count; ++gi) {
         const OpticGauss& g = J.g[gi];
         if (!is_yvv(g.kind)) continue;
-        lp::load_rows(buf, a, b, W, lane);
-        filter<false, kLong>(g, buf, W, lane);
-        lp::store_pairs<kWarps>(rows, words, J.temp[gi], W, H, y0);
+        if constexpr (kPairs == 1) {
+            lp::TeamExchange& ex = lp::exchange(buf, words);
+            lp::load_rows<lp::kTeam>(buf, a, b, W, threadIdx.x);
+            filter_team<false, kLong>(g, buf, W, ex);
+        } else {
+            lp::load_rows(buf, a, b, W, lane);
+            filter<false, kLong>(g, buf, W, lane);
+        }
+        lp::store_pairs<kPairs>(rows, words, J.temp[gi], W, H, y0);
     }
 }
 
@@ -100,15 +131,15 @@ __global__ void __launch_bounds__(32 * kWarps) optic_rows_kernel(const __grid_co
 // waits in the first launch's plane or, where channels have none (kRow), in the carrier between
 // the rounds (more than one only for columns too long for all recursions of the channel to fit).
 template <bool kLong, bool kRow, int kPairs>
-__global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1) __launch_bounds__(32 * lp::kMaxRecursions * kPairs)
+__global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1) __launch_bounds__(32 * (kPairs == 1 ? lp::kTeam : lp::kMaxRecursions * kPairs))
     optic_cols_kernel(const __grid_constant__ OpticPass P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();
     const OpticJob& J = P.job[blockIdx.y];
-    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = kPairs == 1 ? 0 : threadIdx.x >> 5;
     Pair* lines = reinterpret_cast<Pair*>(sm);
     Pair* line = lines + warp * lp::line_words(H);
-    if (lane == 0) {
+    if (lane == 0 && (kPairs > 1 || threadIdx.x == 0)) {
         const unsigned next = blockIdx.y * gridDim.x + blockIdx.x + P.cols_ahead;
         if (next < gridDim.x * gridDim.y) {
             const OpticJob& N = P.job[next / gridDim.x];
@@ -129,8 +160,15 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1) __launch_bounds
             const OpticGauss& g = J.g[gi];
             if (!is_yvv(g.kind)) continue;
             if (warp / kPairs == count) {
-                lp::load_line(line, J.temp[gi], blockIdx.x * kPairs + warp % kPairs, H, lane);
-                filter<true, kLong>(g, line, H, lane);
+                const int pair = blockIdx.x * kPairs + warp % kPairs;
+                if constexpr (kPairs == 1) {
+                    lp::TeamExchange& ex = lp::exchange(line, lp::line_words(H));
+                    lp::load_line<lp::kTeam>(line, J.temp[gi], pair, H, threadIdx.x);
+                    filter_team<true, kLong>(g, line, H, ex);
+                } else {
+                    lp::load_line(line, J.temp[gi], pair, H, lane);
+                    filter<true, kLong>(g, line, H, lane);
+                }
             }
             weight[count++] = J.weight[gi];
         }
@@ -169,8 +207,14 @@ static void balance_weights(OpticJob& J, double carrier, const double* exact) {
     if (least >= 0) J.weight[least] = (float)((double)J.weight[least] + left);
 }
 
+// Samples per piece of a line of n samples in a CTA of `pairs` pairs.
+static int piece_of(int n, int pairs, bool direct) {
+    if (pairs == 1) return lp::team_piece_len(n, direct ? lp::team_chunks(n) : 1);
+    return lp::chunk_piece_len(n, direct ? lp::direct_chunks(n) : 1);
+}
+
 // Whether this form covers the pass: a pair of rows and a pair of columns fit in shared memory
-// (lines up to 29056 samples). The planes between the launches, whole sectors of rows and
+// (lines up to 29020 samples). The planes between the launches, whole sectors of rows and
 // columns each, fit the pass's scratch.
 bool optic_lines_plan(OpticPass& P) {
     int most = 1;
@@ -187,9 +231,9 @@ bool optic_lines_plan(OpticPass& P) {
         taps += fir[j];
         most = n > most ? n : most;
     }
-    P.row_warps = lp::rows_per_cta(P.width);
+    P.row_pairs = lp::pairs_per_cta(P.width);
     P.col_pairs = lp::pairs_per_cta(P.height);
-    if (P.row_warps < 1 || P.col_pairs < 1) return false;
+    if (P.row_pairs < 1 || P.col_pairs < 1) return false;
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.scratch) + 31) / 32 * 32);
     const size_t room = P.scratch_floats - (size_t)(next - P.scratch);
@@ -218,8 +262,8 @@ bool optic_lines_plan(OpticPass& P) {
             double m[9];
             optic_step_map(q, m);
             const bool direct = q.kind == kGaussYvv;
-            q.row_maps = lp::line_maps(m, lp::chunk_piece_len(P.width, direct ? lp::direct_chunks(P.width) : 1));
-            q.col_maps = lp::line_maps(m, lp::chunk_piece_len(P.height, direct ? lp::direct_chunks(P.height) : 1));
+            q.row_maps = lp::line_maps(m, piece_of(P.width, P.row_pairs, direct));
+            q.col_maps = lp::line_maps(m, piece_of(P.height, P.col_pairs, direct));
         }
         J.carrier_weight = (float)carrier;
         balance_weights(J, carrier, exact);
@@ -263,21 +307,21 @@ cudaError_t launch_optic_lines(OpticPass& P, cudaStream_t s) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (rows) {
-        const size_t smem = P.row_warps * lp::line_bytes(P.width);
+        const size_t smem = lp::cta_bytes(P.row_pairs, P.width);
         const bool chunks = direct && lp::direct_chunks(P.width) > 1;
-        auto* k = P.row_warps == lp::kRowWarps
+        auto* k = P.row_pairs == lp::kRowWarps
                       ? (chunks ? optic_rows_kernel<true, lp::kRowWarps> : optic_rows_kernel<false, lp::kRowWarps>)
                       : (chunks ? optic_rows_kernel<true, 1> : optic_rows_kernel<false, 1>);
         e = fjb::allow_dynamic_smem(k, smem);
         if (e != cudaSuccess) return e;
-        const int lines = 2 * P.row_warps;
+        const int lines = 2 * P.row_pairs;
         P.rows_ahead = lines * lp::resident_ctas(smem);
         fjb::count_launch();
-        k<<<dim3((P.height + lines - 1) / lines, P.jobs), 32 * P.row_warps, smem, s>>>(P);
+        k<<<dim3((P.height + lines - 1) / lines, P.jobs), 32 * (P.row_pairs == 1 ? lp::kTeam : P.row_pairs), smem, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    const int warps = P.recursions * P.col_pairs;
-    const size_t smem = warps * lp::line_bytes(P.height);
+    const int lines = P.recursions * P.col_pairs, warps = P.col_pairs == 1 ? lp::kTeam : lines;
+    const size_t smem = lp::cta_bytes(lines, P.height);
     auto* k = P.col_pairs == lp::kColPairs
                   ? cols_variant<lp::kColPairs>(direct && lp::direct_chunks(P.height) > 1, !P.taps_for_all)
                   : cols_variant<1>(direct && lp::direct_chunks(P.height) > 1, !P.taps_for_all);

@@ -20,9 +20,10 @@
 // block. Columns: a CTA holds two pairs of columns for each of a channel's recursions, one
 // warp per pair and recursion; two CTAs (a cluster) sum eight columns in their epilogue
 // through each other's shared memory and write whole sectors of the frame's rows.
-// Lines above 14528 samples: a CTA holds one pair of rows, or of columns (clusters of four);
-// above 29056 not even one pair fits. 16000x2000: DIR 5.3 ms, scatter/halation 7.0; 2000x16000:
-// 5.8 and 7.7; as launches over segments in global memory 10.0, 13.9, 8.6 and 11.9 ms.
+// Lines above 14528 samples: a CTA holds one pair of rows, or of columns (clusters of four), which
+// a team of four warps shares (direction_team); above 29020 not even one pair fits. 16000x2000:
+// DIR 3.8 ms, scatter/halation 4.9; 2000x16000: 2.9 and 3.4; with one warp per pair 5.3, 7.0,
+// 5.8 and 7.7; as launches over segments in global memory 10.0, 13.9, 8.6 and 11.9.
 //
 // What bounds it: shared-memory bandwidth, seven 8-byte accesses per pair and position and
 // recursion (28 bytes per sample; 128 bytes per clock and SM), next to one read and one
@@ -52,6 +53,7 @@ constexpr int kRowWarps = 2;      // warps (pairs of rows) of a row CTA
 constexpr int kMaxRecursions = 5; // of one channel
 constexpr int kColPairs = 2;      // pairs of columns of a column CTA
 constexpr int kStripPairs = 4;    // pairs of columns whose CTAs (a cluster) write rows together
+constexpr int kTeam = 4;          // warps of the one pair of lines that a CTA holds above 14528 samples
 constexpr size_t kSmemLimit = 227 * 1024;
 
 // M^(K 2^i): the powers of the one-step zero-input map over one piece.
@@ -75,6 +77,11 @@ __host__ __device__ inline int direct_chunks(int n) {
 }
 // Samples per piece of a line in so many chunks.
 __host__ __device__ inline int chunk_piece_len(int n, int chunks) { return piece_len((n + chunks - 1) / chunks); }
+// The same for a team's line: so many chunks of 32 kTeam pieces.
+__host__ __device__ inline int team_chunks(int n) { return (n + kTeam * kPieces * 63 - 1) / (kTeam * kPieces * 63); }
+__host__ __device__ inline int team_piece_len(int n, int chunks) {
+    return ((n + chunks * kTeam * kPieces - 1) / (chunks * kTeam * kPieces)) | 1;
+}
 // Words (pairs of samples) of a line as stored, a whole number of 32-byte sectors.
 __host__ __device__ inline int line_words(int n) { return (n + 3) / 4 * 4; }
 __host__ __device__ inline size_t line_bytes(int n) { return (size_t)line_words(n) * sizeof(float2); }
@@ -323,6 +330,100 @@ __device__ __forceinline__ void direction_chunks(const DirectStep& op, const Lin
     }
 }
 
+// ---------------------------------------------------------------------------
+// One pair of lines by a team of warps, the whole CTA: 32 kTeam pieces, more of them in flight
+// and shorter than one warp's. The warps scan their own pieces, pass their exit states on through
+// shared memory, and scan again from their entry states.
+// ---------------------------------------------------------------------------
+struct TeamExchange {
+    double exit[kTeam + 1][6];
+    unsigned long long start[3];
+    __device__ __forceinline__ void put(int i, const State2& s) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) exit[i][k] = s.a[k], exit[i][3 + k] = s.b[k];
+    }
+    __device__ __forceinline__ State2 get(int i) const {
+        State2 s;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s.a[k] = exit[i][k], s.b[k] = exit[i][3 + k];
+        return s;
+    }
+};
+
+// Behind the CTA's line in shared memory.
+__device__ __forceinline__ TeamExchange& exchange(Pair* line, int words) {
+    return *reinterpret_cast<TeamExchange*>(line + words);
+}
+// Shared memory of a CTA of `lines` lines (pairs) of n samples.
+inline size_t cta_bytes(int lines, int n) { return lines * line_bytes(n) + (lines == 1 ? sizeof(TeamExchange) : 0); }
+
+template <bool kFwd>
+__device__ __forceinline__ void scan(State2& s, const LineMaps& m, int order) {
+#pragma unroll 1
+    for (int l = 0; l < kLevels; ++l) {
+        const State2 t = s.from<kFwd>(1 << l);
+        if (order >= (1 << l)) s.add(m.m[l], t);
+    }
+}
+
+// One direction over samples [lo, hi) of the line, its pieces of `k` samples counted from 0, in
+// `chunks` chunks one after the other. `s` receives the exit state of the thread's piece in the
+// last chunk processed. Begins with the line complete and ends with a barrier.
+template <bool kFwd, typename Op>
+__device__ __forceinline__ void direction_team(const Op& op, const LineMaps& m, Pair* line, int lo, int hi, int k,
+                                               int chunks, const Pair (&start)[3], Pair (&s)[3], TeamExchange& ex) {
+    const Pair zero{0ull};
+    const int lane = threadIdx.x & 31, member = threadIdx.x >> 5;
+    const int order = kFwd ? lane : kPieces - 1 - lane, rank = kFwd ? member : kTeam - 1 - member;
+    State2 carry{};
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+        const int from = (kFwd ? c : chunks - 1 - c) * kTeam * kPieces * k, base = from + (int)threadIdx.x * k;
+        const int plo = min(max(base, lo), hi), phi = min(max(base + k, lo), hi), nv = phi - plo;
+        const bool first = nv > 0 && (kFwd ? plo == max(from, lo) : phi == min(from + kTeam * kPieces * k, hi));
+        Pair* w = line + (kFwd ? plo : phi - 1);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s[i] = first && c == 0 ? start[i] : zero;
+        run<kFwd, false>(op, w, nv, s);
+        State2 own;
+        own.set(s);
+        if (first && c > 0) own.add(m.m[0], carry);
+        State2 S = own;
+        scan<kFwd>(S, m, order);
+        if (order == kPieces - 1) ex.put(member, S);
+        __syncthreads();
+        // the state that this warp's pieces start from: earlier warps' exits, 32 pieces apart
+        State2 entry{};
+#pragma unroll 1
+        for (int r = 0; r < rank; ++r) {
+            State2 half{}, next = ex.get(kFwd ? r : kTeam - 1 - r);
+            half.add(m.m[kLevels - 1], entry); // 16 pieces
+            next.add(m.m[kLevels - 1], half);
+            entry = next;
+        }
+        if (order == 0) own.add(m.m[0], entry);
+        scan<kFwd>(own, m, order);
+        const State2 before = own.from<kFwd>(1);
+        (order == 0 ? entry : before).get(s);
+        if (first) {
+            if (c == 0) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) s[i] = start[i];
+            } else {
+                carry.get(s);
+            }
+        }
+        if (chunks > 1) {
+            // the chunks followed by another are whole: the piece processed last has their exit state
+            if (rank == kTeam - 1 && order == kPieces - 1) ex.put(kTeam, own);
+            __syncthreads();
+            carry = ex.get(kTeam);
+        }
+        run<kFwd, true>(op, w, nv, s);
+        __syncthreads();
+    }
+}
+
 // Brings a block of global memory into L2. The CTAs of a launch start together and would all
 // load, then all compute: each one asks for what the CTA that takes its place will load.
 __device__ __forceinline__ void prefetch_block(const float* p, size_t floats) {
@@ -342,33 +443,44 @@ inline int resident_ctas(size_t smem) {
 // ---------------------------------------------------------------------------
 // Rows: from a plane, to a plane by pairs of columns
 // ---------------------------------------------------------------------------
-// Two rows of n floats, interleaved, by one warp (4-byte asynchronous copies: no alignment
-// asked for, everything in flight at once). The copies are in place when this returns.
+// Waits for the caller's copies and those of the other threads that hold its lines.
+template <int kWarps>
+__device__ __forceinline__ void loaded() {
+    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if constexpr (kWarps == 1)
+        __syncwarp();
+    else
+        __syncthreads();
+}
+
+// Two rows of n floats, interleaved, by the kWarps warps that hold them (4-byte asynchronous
+// copies: no alignment asked for, everything in flight at once). The copies are in place when
+// this returns.
+template <int kWarps = 1>
 __device__ __forceinline__ void load_rows(Pair* buf, const float* a, const float* b, int n, int lane) {
     unsigned d = (unsigned)__cvta_generic_to_shared(buf) + 8u * (unsigned)lane;
 #pragma unroll 4
-    for (int p = lane; p < n; p += 32, d += 256) {
+    for (int p = lane; p < n; p += 32 * kWarps, d += 256 * kWarps) {
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(a + p));
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4), "l"(b + p));
     }
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncwarp();
+    loaded<kWarps>();
 }
 
 // The CTA's rows y .. y + 3 (two pairs, `words` apart) of `width` samples to the plane by
 // pairs of columns: one sector per pair of columns and thread; or its one pair of rows, half a
 // sector. A barrier before (the rows are complete) and after (the buffers are free).
-template <int kWarps>
+template <int kPairs>
 __device__ __forceinline__ void store_pairs(const Pair* buf, int words, float* plane, int width, int height, int y) {
-    static_assert(kWarps == 1 || kWarps == 2, "rows of a CTA");
+    static_assert(kPairs == 1 || kPairs == 2, "pairs of rows of a CTA");
     __syncthreads();
     const int pitch = 2 * line_words(height);
     float* out = plane + 2 * y;
 #pragma unroll 2
-    for (int j = threadIdx.x; 2 * j < width; j += 32 * kWarps) {
+    for (int j = threadIdx.x; 2 * j < width; j += blockDim.x) {
         const float4 a = *reinterpret_cast<const float4*>(buf + 2 * j); // rows y, y + 1 of two columns
-        if constexpr (kWarps == 1) {
+        if constexpr (kPairs == 1) {
             *reinterpret_cast<float4*>(out + (size_t)j * pitch) = make_float4(a.x, a.z, a.y, a.w);
             continue;
         }
@@ -383,17 +495,16 @@ __device__ __forceinline__ void store_pairs(const Pair* buf, int words, float* p
 // ---------------------------------------------------------------------------
 // Columns
 // ---------------------------------------------------------------------------
-// One pair of columns of n rows by one warp, a contiguous block.
+// One pair of columns of n rows by the kWarps warps that hold it, a contiguous block.
+template <int kWarps = 1>
 __device__ __forceinline__ void load_line(Pair* buf, const float* plane, int pair, int n, int lane) {
     const int words = line_words(n);
     const float* src = plane + (size_t)pair * 2 * words;
     const unsigned d = (unsigned)__cvta_generic_to_shared(buf);
 #pragma unroll 4
-    for (int i = 2 * lane; i < words; i += 64)
+    for (int i = 2 * lane; i < words; i += 64 * kWarps)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + 8u * (unsigned)i), "l"(src + 2 * i));
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncwarp();
+    loaded<kWarps>();
 }
 
 // The line of load_line into L2, by one lane.
@@ -510,10 +621,11 @@ __device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const 
     }
 }
 
-// Pairs of rows of a row CTA; 0: not one fits.
-inline int rows_per_cta(int n) { return std::min(kRowWarps, (int)(kSmemLimit / line_bytes(n))); }
-// Pairs of columns of a column CTA; 0: not one fits.
-inline int pairs_per_cta(int n) { return std::min(kColPairs, (int)(kSmemLimit / line_bytes(n))); }
+// Pairs of rows of a row CTA, and of columns of a column CTA; 0: not one fits.
+inline int pairs_per_cta(int n) {
+    static_assert(kRowWarps == 2 && kColPairs == 2, "two pairs, or one");
+    return cta_bytes(2, n) <= kSmemLimit ? 2 : cta_bytes(1, n) <= kSmemLimit ? 1 : 0;
+}
 // Recursions a column CTA of `pairs` pairs holds at once, as many as fit.
 inline int recursions_per_cta(int count, int pairs, int n) {
     count = std::max(1, std::min(count, kMaxRecursions));

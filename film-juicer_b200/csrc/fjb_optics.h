@@ -67,7 +67,7 @@ struct OpticPass {
     // CTA and the one after it, and whether every job has a plane `base`
     float* scratch;
     size_t scratch_floats;
-    int row_warps, col_pairs, recursions, rows_ahead, cols_ahead;
+    int row_pairs, col_pairs, recursions, rows_ahead, cols_ahead;
     bool taps_for_all;
 };
 

@@ -1,6 +1,6 @@
 """Spatial DIR and scatter/halation on lines at the ends of each form's range: frames of a few
 samples (the line form's planes are padded), one pair of rows or columns per CTA from 14529
-samples on, the many-launch form in global memory above 29056. The launch count tells the
+samples on, the many-launch form in global memory above 29020. The launch count tells the
 forms apart. Oracle and bounds are those of test_line_pairs_gpu.py."""
 import numpy as np
 import pytest
@@ -8,8 +8,8 @@ import pytest
 from test_line_rounds_gpu import dir_oracle, launches, planes
 
 pytestmark = pytest.mark.gpu
-LINES = [(1, 1), (3, 2), (9, 9), (17, 17), (25, 25), (14528, 5), (14529, 6), (14531, 5), (5, 14532), (9, 14529), (18, 14528), (29056, 3), (8, 29056)]
-GLOBAL = [(29060, 4), (3, 29061)]
+LINES = [(1, 1), (3, 2), (9, 9), (17, 17), (25, 25), (14528, 5), (14529, 6), (14531, 5), (5, 14532), (9, 14529), (18, 14528), (29020, 3), (8, 29020)]
+GLOBAL = [(29024, 4), (3, 29021)]
 
 
 def check_dir(torch, w, h):
