@@ -38,7 +38,6 @@ struct DirComponentDev {
     float weight;
     int radius;
     const float* taps; // device, 2r+1
-    int symmetric_taps; // taps[i] == taps[2r - i] bit for bit
     double ff;
     double fb[3];
     const double* h_init;
@@ -116,8 +115,6 @@ struct DirPlan {
 
 bool dir_plan_create(const FjSpatialDir& sd, int width, int height, cudaStream_t stream, DirPlan& plan,
                      std::string& why, cudaError_t& err);
-
-size_t dir_scratch_floats(int width, int height);
 
 } // namespace fjb
 

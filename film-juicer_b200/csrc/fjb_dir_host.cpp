@@ -268,11 +268,6 @@ size_t dir_recursion_bytes(int width, int height) {
            sizeof(double);
 }
 
-size_t dir_scratch_floats(int width, int height) {
-    // raw corrections (3) + log raw (3) + filtered (3) + one temp per channel/component
-    return (size_t)(9 + 3 * kDirMaxComponents) * (size_t)width * (size_t)height;
-}
-
 namespace {
 
 // The recursion 1 / (1 - fb0 z^-1 - fb1 z^-2 - fb2 z^-3) as (1 - p z^-1)(1 - a1 z^-1 -
@@ -367,9 +362,6 @@ bool dir_plan_create(const FjSpatialDir& sd, int width, int height, cudaStream_t
                 if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return false;
                 c.taps = static_cast<const float*>(d);
                 for (int i = 0; i < 19 && i < (int)taps.size(); ++i) c.host_taps[i] = taps[i];
-                c.symmetric_taps = 1;
-                for (int i = 0; i <= 2 * g.radius; ++i)
-                    if (std::memcmp(&taps[i], &taps[2 * g.radius - i], sizeof(float)) != 0) c.symmetric_taps = 0;
                 break;
             }
             case FJ_DIR_OPERATOR_YVV_REFLECT: {

@@ -250,7 +250,8 @@ constexpr int team_warps() {
 
 // Four rows of one channel per CTA (kPairs pairs) through every recursive component.
 template <int kPairs, bool kDirect>
-__global__ void __launch_bounds__(32 * (kPairs == 1 ? team_warps<kDirect>() : kPairs)) dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
+__global__ void __launch_bounds__(32 * (kPairs == 1 ? team_warps<kDirect>() : kPairs))
+    dir_rows_kernel(const __grid_constant__ DirBlurParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int ch = blockIdx.y;
     const int W = P.width, H = P.height, lane = threadIdx.x & 31, warp = kPairs == 1 ? 0 : threadIdx.x >> 5;
@@ -261,7 +262,8 @@ __global__ void __launch_bounds__(32 * (kPairs == 1 ? team_warps<kDirect>() : kP
     const int y0 = 2 * kPairs * blockIdx.x, y = y0 + 2 * warp;
     const float* a = P.raw[ch] + (size_t)min(y, H - 1) * W;
     const float* b = P.raw[ch] + (size_t)min(y + 1, H - 1) * W;
-    if (lane < 2 && (kPairs > 1 || threadIdx.x < 2) && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (size_t)(lane + P.rows_ahead) * W, W);
+    if (lane < 2 && (kPairs > 1 || threadIdx.x < 2) && y + lane + P.rows_ahead < H)
+        lp::prefetch_block(a + (size_t)(lane + P.rows_ahead) * W, W);
 #pragma unroll 1
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];

@@ -11,9 +11,9 @@
 // each of them cost a plane written and read twice.
 //
 // What bounds it: FP32 sums, instruction issue and the barriers between the phases
-// (3840x2160, three planes: 95 us for the scatter's Gaussians, 29 for the
-// back-reflection's; two sums per packed instruction, in 76 registers, took 20 to 45 % longer); FP64 sums, the conversions between FP32 and FP64 (56 % of that unit) and
-// the FP64 pipe (38 %): 144 us.
+// (3840x2160, three planes: 95 us for the scatter's Gaussians, 29 for the back-reflection's; two
+// sums per packed instruction, in 76 registers, took 20 to 45 % longer); FP64 sums, the
+// conversions between FP32 and FP64 (56 % of that unit) and the FP64 pipe (38 %): 147 us.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(32 * (kPairs == 1 ? lp::kTeam : kPairs)) optic
     const int y0 = 2 * kPairs * blockIdx.x, y = y0 + 2 * warp;
     const float* a = J.src + (long long)min(y, H - 1) * J.stride;
     const float* b = J.src + (long long)min(y + 1, H - 1) * J.stride;
-    if (lane < 2 && (kPairs > 1 || threadIdx.x < 2) && y + lane + P.rows_ahead < H) lp::prefetch_block(a + (long long)(lane + P.rows_ahead) * J.stride, W);
+    if (lane < 2 && (kPairs > 1 || threadIdx.x < 2) && y + lane + P.rows_ahead < H)
+        lp::prefetch_block(a + (long long)(lane + P.rows_ahead) * J.stride, W);
 #pragma unroll 1
     for (int gi = 0; gi < J.count; ++gi) {
         const OpticGauss& g = J.g[gi];
@@ -131,7 +132,8 @@ __global__ void __launch_bounds__(32 * (kPairs == 1 ? lp::kTeam : kPairs)) optic
 // waits in the first launch's plane or, where channels have none (kRow), in the carrier between
 // the rounds (more than one only for columns too long for all recursions of the channel to fit).
 template <bool kLong, bool kRow, int kPairs>
-__global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1) __launch_bounds__(32 * (kPairs == 1 ? lp::kTeam : lp::kMaxRecursions * kPairs))
+__global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
+    __launch_bounds__(32 * (kPairs == 1 ? lp::kTeam : lp::kMaxRecursions * kPairs))
     optic_cols_kernel(const __grid_constant__ OpticPass P) {
     extern __shared__ __align__(16) unsigned char sm[];
     const auto cluster = cooperative_groups::this_cluster();

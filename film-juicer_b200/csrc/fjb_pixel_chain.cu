@@ -8,8 +8,8 @@
 // What bounds it: scanning density planes with the print, instruction issue (75 % active, 1490
 // instructions per pixel) beside the conversion and transcendental unit (56 %: 82 exponentials
 // per pixel); camera exposure, the L1 passes of its 16 scattered float4 taps (86 %). 3840x2160:
-// print scan 741 -> 455 us, camera exposure 164 -> 140, spatial-DIR source 196 -> 138, capture
-// density 176 -> 98; 1920x1080 RGBA, everything in one kernel, 335 -> 213.
+// print scan 741 -> 474 us, camera exposure 164 -> 134, spatial-DIR source 196 -> 146, capture
+// density 176 -> 103; 1920x1080 RGBA, everything in one kernel, 335 -> 221.
 //
 // Variants (template flags) cover the reference's fused kernels
 // (src/Cuda/Scan/JuicerCudaScanPipeline.cu:1700-1868 pipeline_direct/carrier_kernel,
