@@ -52,7 +52,8 @@ class CallMemory {
     static constexpr uint64_t kKeep = 64ull << 20;
     static constexpr size_t kLargest = (size_t)256 << 20;
     // Number of the current context, never given twice: cudaDeviceReset destroys the pools of a
-    // device, and the context made after it has another number. 0 where the driver cannot tell.
+    // device, and the context made after it has another number. 0 where the thread has no context
+    // or the driver cannot tell.
     static unsigned long long context_number() {
         using GetId = int (*)(void*, unsigned long long*);
         static const GetId get = [] {
@@ -75,9 +76,12 @@ class CallMemory {
         static std::vector<DevicePool> pools;
         int device = 0;
         cudaError_t e = cudaGetDevice(&device);
-        if (e == cudaSuccess) e = cudaFree(nullptr); // makes the device's context current
         if (e != cudaSuccess) return e;
-        const unsigned long long context = context_number();
+        unsigned long long context = context_number();
+        if (!context) { // the thread's first call: makes the device's context current
+            if ((e = cudaSetDevice(device)) != cudaSuccess) return e;
+            context = context_number();
+        }
         std::lock_guard<std::mutex> lock(gate);
         for (const DevicePool& p : pools)
             if (p.device == device && p.context == context) {
