@@ -1,6 +1,6 @@
 // fjb_fir2d.cuh -- short separable taps (radius 1..9), both axes in one pass.
 //
-// dst = src_weight src + sum_i weight_i columns_i(rows_i(src)), each sum over taps in Acc
+// dst = sum_i weight_i columns_i(rows_i(src)) + src_weight src, each sum over taps in Acc
 // precision and rounded to FP32 between the axes, half-sample reflection at the frame's
 // edges. A CTA makes a 64 x 32 tile: the input with the widest halo goes to shared memory
 // once, then for each set of taps every thread makes eight neighbouring row outputs from
@@ -159,10 +159,7 @@ __global__ void __launch_bounds__(kThreads, 3) kernel(const __grid_constant__ Jo
     stage(P, J, rad, in);
     __syncthreads();
     const int c = threadIdx.x % kTileW, r = threadIdx.x / kTileW * 8;
-    float sum[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        sum[j] = J.src_weight != 0.0f ? J.src_weight * in[(rad + r + j) * kInPitch + kHalo + c] : 0.0f;
+    float sum[8] = {};
 #pragma unroll 1
     for (int i = 0; i < J.count; ++i) {
         const Taps& T = J.set[i];
@@ -178,6 +175,10 @@ __global__ void __launch_bounds__(kThreads, 3) kernel(const __grid_constant__ Jo
             default: taps<Acc, 9>(T, rad, in, mid, sum); break;
         }
     }
+    // the source's own share last: it is the largest term as a rule
+    if (J.src_weight != 0.0f)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = fmaf(J.src_weight, in[(rad + r + j) * kInPitch + kHalo + c], sum[j]);
     // transposed through shared memory: a warp stores 32 rows of a pair of columns
     constexpr int kPitch = kTileH + 1;
     __syncthreads();

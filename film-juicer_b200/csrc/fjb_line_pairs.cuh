@@ -546,6 +546,10 @@ __device__ __forceinline__ void row_samples(const float* p, bool wide, int left,
 // The epilogue of a column cluster: `count` recursions' lines in its CTAs' shared memory
 // (line i * kPairs + pair), eight columns of an n x width plane, each CTA its share of the
 // rows. The caller has synchronised the cluster and does so again before the lines go.
+// The recursions are added up first, then the rest: they are the small terms, and the error of
+// the sum is that of its last addition or two (scatter/halation, 1283x719 to 4060x800, factored
+// form: rms 4.7e-8 of the result, the other way round 6.2e-8 to 6.5e-8). The rest is loaded
+// after the recursions: held across them it took registers, and 1.5 % of the columns' passes.
 // Without kRow there is a plane by pairs of columns (a variant of its own: with the rest,
 // scatter/halation took 784 us at 3840x2160 instead of 771).
 template <bool kRow, int kPairs>
@@ -564,23 +568,7 @@ __device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const 
     const bool wide = kRow && S.row && S.row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(S.row) & 15u) == 0;
     const unsigned align = S.dst_stride % 8 == 0 ? (unsigned)(reinterpret_cast<uintptr_t>(S.dst) & 31u) : 4u;
     for (int y0 = ylo + threadIdx.x; y0 < yhi; y0 += kBatch * blockDim.x) {
-        float2 sum[kBatch][kAll];
-#pragma unroll
-        for (int r = 0; r < kBatch; ++r) {
-            const int y = min(y0 + r * (int)blockDim.x, yhi - 1);
-            if (!kRow || base) {
-#pragma unroll
-                for (int q = 0; q < kAll; ++q) sum[r][q] = base[(size_t)q * words + y];
-            } else if (S.row) {
-                row_samples(S.row + (long long)y * S.row_stride + x0, wide, width - x0, sum[r]);
-#pragma unroll
-                for (int q = 0; q < kAll; ++q)
-                    sum[r][q] = make_float2(S.row_weight * sum[r][q].x, S.row_weight * sum[r][q].y);
-            } else {
-#pragma unroll
-                for (int q = 0; q < kAll; ++q) sum[r][q] = make_float2(0.0f, 0.0f);
-            }
-        }
+        float2 sum[kBatch][kAll] = {};
 #pragma unroll 1
         for (int i = 0; i < count; ++i) {
             const float w = weight[i];
@@ -595,6 +583,28 @@ __device__ __forceinline__ void strip_sum(const StripSum& S, Pair* lines, const 
                 }
             }
         }
+        float2 rest[kBatch][kAll];
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const int y = min(y0 + r * (int)blockDim.x, yhi - 1);
+            if (!kRow || base) {
+#pragma unroll
+                for (int q = 0; q < kAll; ++q) rest[r][q] = base[(size_t)q * words + y];
+            } else if (S.row) {
+                row_samples(S.row + (long long)y * S.row_stride + x0, wide, width - x0, rest[r]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < kAll; ++q) rest[r][q] = make_float2(0.0f, 0.0f);
+            }
+        }
+        const float rest_weight = kRow && !base ? S.row_weight : 1.0f;
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r)
+#pragma unroll
+            for (int q = 0; q < kAll; ++q) {
+                sum[r][q].x = fmaf(rest_weight, rest[r][q].x, sum[r][q].x);
+                sum[r][q].y = fmaf(rest_weight, rest[r][q].y, sum[r][q].y);
+            }
 #pragma unroll
         for (int r = 0; r < kBatch; ++r) {
             const int y = y0 + r * blockDim.x;
