@@ -83,6 +83,7 @@ struct DirBlurParams {
     size_t region_floats;
     int row_pairs, col_pairs, recursions, rows_ahead, cols_ahead;
     float* base[3];
+    float* wide[3]; // rows of a component with wide taps, before the recursions' planes are written
     float raw_weight;
     bool direct; // some component has no factored form
     double* row_start;

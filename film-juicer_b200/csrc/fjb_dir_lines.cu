@@ -11,7 +11,8 @@
 // the columns' reflected starts; the columns, one warp per pair of columns and recursive
 // component, then the weighted sum of all of them and the plane of the first launch.
 // Only short components take a plane of their own, so the planes are never more than the
-// components, which is what the scratch holds.
+// components, which is what the scratch holds. The filtered planes are written by the last launch
+// alone, which does not read the corrections: one channel's may be another's corrections.
 //
 // The starts are launches of their own because their weights (three doubles for each of the
 // first 21 sigma samples, 55 KB at 3840x2160) do not fit what the line kernels leave of L1:
@@ -308,7 +309,7 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
             if (P.base[nch] && warp < kPairs) lp::prefetch_line(P.base[nch], first + warp, H);
         }
     }
-    lp::StripSum out{P.base[ch], P.filtered[ch], W, false, P.raw_weight != 0.0f ? P.raw[ch] : nullptr, W, P.raw_weight};
+    lp::StripSum out{P.base[ch], P.filtered[ch], W, false, nullptr, W, 1.0f};
     int k = 0;
     do {
         float weight[lp::kMaxRecursions];
@@ -338,10 +339,7 @@ __global__ void __cluster_dims__(lp::kStripPairs / kPairs, 1, 1)
         cluster.sync();
         out.last = k >= P.count;
         lp::strip_sum<kRow, kPairs>(out, lines, weight, count, W, H);
-        if constexpr (kRow) {
-            out.row = P.filtered[ch];
-            out.row_weight = 1.0f;
-        }
+        if constexpr (kRow) out.row = P.filtered[ch];
         cluster.sync(); // the other CTAs have read these lines
     } while (k < P.count);
 }
@@ -381,21 +379,22 @@ size_t dir_lines_floats(int width, int height) {
 
 bool dir_lines_plan(DirBlurParams& P) {
     int lines = 0;
-    bool base = false;
+    bool base = false, wide = false;
     P.direct = false;
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];
         lines += c.op == kDirOpYvv;
         P.direct |= c.op == kDirOpYvv && !c.factored;
-        base |= c.op == kDirOpFir;
+        base |= c.op != kDirOpYvv;
+        wide |= c.op == kDirOpFir && c.radius > fir::kMaxRadius;
     }
     P.row_pairs = lp::pairs_per_cta(P.width);
     P.col_pairs = lp::pairs_per_cta(P.height);
     if (P.row_pairs < 1 || P.col_pairs < 1) return false;
     const size_t plane = lp::plane_floats(P.width, P.height);
     float* next = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(P.region) + 31) / 32 * 32);
-    if ((size_t)(next - P.region) + 3 * (size_t)(lines + base) * plane + starts_floats(P.width, P.height) > P.region_floats)
-        return false;
+    const size_t planes = 3 * (size_t)(lines + base + (wide && lines == 0));
+    if ((size_t)(next - P.region) + planes * plane + starts_floats(P.width, P.height) > P.region_floats) return false;
     P.recursions = lp::recursions_per_cta(lines, P.col_pairs, P.height);
     P.raw_weight = 0.0f;
     for (int k = 0; k < P.count; ++k) {
@@ -411,6 +410,13 @@ bool dir_lines_plan(DirBlurParams& P) {
     for (int ch = 0; ch < 3; ++ch) {
         P.base[ch] = base ? next : nullptr;
         if (base) next += plane;
+        P.wide[ch] = P.temp[ch][0];
+        for (int k = P.count - 1; k >= 0; --k)
+            if (P.comp[k].op == kDirOpYvv) P.wide[ch] = P.temp[ch][k];
+        if (wide && lines == 0) {
+            P.wide[ch] = next;
+            next += plane;
+        }
     }
     P.row_start = reinterpret_cast<double*>(next);
     P.col_start = P.row_start + 3 * (size_t)kDirMaxComponents * 3 * P.height;
@@ -447,11 +453,11 @@ cudaError_t launch_dir_lines(DirBlurParams& P, cudaStream_t s) {
         fir::kernel<double><<<fir::grid(F), fir::kThreads, 0, s>>>(F);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    // wider taps, a component after the other; the filtered planes hold its rows
+    // wider taps, a component after the other
     for (int k = 0; k < P.count; ++k) {
         const DirComponentDev& c = P.comp[k];
         if (c.op != kDirOpFir || c.radius <= fir::kMaxRadius) continue;
-        e = launch_blur_into_pairs(P.raw, P.filtered, P.base, 3, P.width, P.height, c.taps, c.radius, c.weight, s);
+        e = launch_blur_into_pairs(P.raw, P.wide, P.base, 3, P.width, P.height, c.taps, c.radius, c.weight, s);
         if (e != cudaSuccess) return e;
     }
     constexpr int kLinesPerCta = 4 * kStartWarps;

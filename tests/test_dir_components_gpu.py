@@ -56,3 +56,31 @@ def test_wide_taps(torch_cuda, w, h, radii):
     wide = sum(r > 9 for r in radii)
     recursive = 3 if len(radii) < 4 else 0  # starts, rows, starts
     check_dir(torch_cuda, sd, planes(w, h, 12), 1 + 2 * wide + recursive + 1)
+
+
+@pytest.mark.parametrize("w,h,kind", [(643, 361, "taps"), (643, 361, "recursive"), (160, 90, "default"),
+                                      (643, 361, "default"), (64, 3700, "recursive"), (643, 361, "only taps")])
+def test_outputs_in_other_channels_inputs(torch_cuda, w, h, kind):
+    """The corrections of all channels are read before a filtered plane is written."""
+    from film_juicer_b200 import descriptors, runtime
+
+    torch = torch_cuda
+    if kind == "default":
+        sd = descriptors.spatial_dir_record(35000.0 / w, w, h)
+    else:
+        sd = descriptors.spatial_dir_record(5.0, w, h, diffusion_size_um=20.0, tail_um=60.0, tail_weight=0.3)
+    if kind == "taps":
+        taps(sd.components[0], 2.9, 12)
+    if kind == "only taps":
+        for k, r in enumerate((11, 40, 2, 64)):
+            taps(sd.components[k], 2.9 if r > 2 else 0.7, r)
+    f = runtime.DirFilter(sd, w, h)
+    src = [torch.from_numpy(p).cuda() for p in planes(w, h, 13)]
+    want = [torch.empty_like(p) for p in src]
+    f.apply(src, want)
+    work = [p.clone() for p in src]
+    f.apply(work, [work[1], work[2], work[0]])
+    got = [work[1], work[2], work[0]]
+    f.close()
+    for g, t in zip(got, want):
+        assert torch.equal(g, t)
